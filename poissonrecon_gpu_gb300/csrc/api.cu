@@ -101,7 +101,7 @@ void Ctx::kflush() {
     kev_next = 0;
 }
 
-int cg_csr_impl(int n, const int* rowptr, const int* col, const float* val, const float* rhs, float* x, float tol,
+int cg_csr_impl(int n, int nz, const int* rowptr, const int* col, const float* val, const float* rhs, float* x, float tol,
                 int max_iter, int* iters, float* ms);
 
 // timed stage runner: CUDA events on the context stream
@@ -1033,10 +1033,9 @@ int prgpu_mlp_gradients(void* t, const uint16_t* features, const float* targets,
 
 int prgpu_cg_csr(int32_t n, int32_t nz, const int32_t* rowptr, const int32_t* col, const float* val, const float* rhs,
                  float* x, float tol, int32_t max_iter, int32_t* iters, float* kernel_ms) {
-    (void)nz;
     if (n <= 0 || !rowptr || !col || !val || !rhs || !x || max_iter < 0) return PRGPU_ERR_ARG;
     API_BEGIN
-    return cg_csr_impl(n, rowptr, col, val, rhs, x, tol, max_iter, iters, kernel_ms);
+    return cg_csr_impl(n, nz, rowptr, col, val, rhs, x, tol, max_iter, iters, kernel_ms);
     API_END
 }
 

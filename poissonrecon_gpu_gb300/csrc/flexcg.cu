@@ -53,15 +53,6 @@ struct FcgState {           // one per depth
 
 constexpr int FCG_NV = 3;
 
-struct alignas(128) FcgSync {
-    unsigned count;
-    unsigned pad0[31];
-    unsigned gen;
-    unsigned pad1[31];
-    double res[2][4];
-    double pad2[8];
-};
-
 struct FcgArgs {
     int mode;
     float tol2;
@@ -80,8 +71,8 @@ struct FcgArgs {
     float* p;               // search direction, two buffers used alternately
     float* q;
     FcgState* state;
-    FcgSync* sync;          // one per depth
-    double* partial;        // 4 per block
+    u64* slots;             // grid_sum's slots: one per block, one per depth (results), one never written
+    int nslots;
     int* err;
     long long spin_limit;
     int extra;
@@ -103,76 +94,6 @@ constexpr int FCG_WARP_TILES = 2;
 constexpr i64 FCG_MIN_ROWS = 256;
 constexpr int FCG_DSMEM = 8192 + 8192 + FCG_GROUPS * 16384 + 1024;   // W1, W2, feature tiles (+ alignment)
 
-// sum of FCG_NV doubles over the blocks of a partition, in a fixed order, returned
-// to every thread; false when a wait gave up (error flag set)
-__device__ bool fcg_reduce(FcgSync* ps, double* partial, int first_block, int nblocks, int slot,
-                           double (&v)[FCG_NV], const FcgArgs& a, double* sh, int* sh_flag, double* sh_val) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int j = 0; j < FCG_NV; ++j) {
-        double t = v[j];
-        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) sh[w * FCG_NV + j] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 0; j < FCG_NV; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < nw; ++k) s += sh[k * FCG_NV + j];
-            partial[(i64)blockIdx.x * 4 + j] = s;
-        }
-        __threadfence();
-        const unsigned g = *(volatile unsigned*)&ps->gen;
-        const unsigned arrived = atomicAdd(&ps->count, 1u);
-        sh_flag[0] = (arrived == (unsigned)(nblocks + a.extra) - 1) ? 1 : 0;
-        sh_flag[1] = (int)g;
-    }
-    __syncthreads();
-    if (sh_flag[0]) {
-        __threadfence();
-        double t[FCG_NV] = {0.0, 0.0, 0.0};
-        for (int k = threadIdx.x; k < nblocks; k += blockDim.x)
-#pragma unroll
-            for (int j = 0; j < FCG_NV; ++j) t[j] += *(volatile double*)&partial[(i64)(first_block + k) * 4 + j];
-#pragma unroll
-        for (int j = 0; j < FCG_NV; ++j) {
-            for (int o = 16; o; o >>= 1) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
-            if (lane == 0) sh[w * FCG_NV + j] = t[j];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int j = 0; j < FCG_NV; ++j) {
-                double s = 0.0;
-                for (int k = 0; k < nw; ++k) s += sh[k * FCG_NV + j];
-                ps->res[slot][j] = s;
-                sh_val[j] = s;
-            }
-            atomicExch(&ps->count, 0u);
-            __threadfence();
-            atomicAdd(&ps->gen, 1u);
-            sh_flag[2] = 1;
-        }
-    } else if (threadIdx.x == 0) {
-        const unsigned g = (unsigned)sh_flag[1];
-        volatile unsigned* vgen = &ps->gen;
-        long long spins = 0;
-        int good = 1;
-        while (*vgen == g) {
-            if (++spins > a.spin_limit || *(volatile int*)a.err) { good = 0; break; }
-            __nanosleep(64);
-        }
-        __threadfence();
-        if (!good) atomicExch(a.err, PRGPU_ERR_TIMEOUT);
-        for (int j = 0; j < FCG_NV; ++j) sh_val[j] = *(volatile double*)&ps->res[slot][j];
-        sh_flag[2] = good && !*(volatile int*)a.err;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < FCG_NV; ++j) v[j] = sh_val[j];
-    return sh_flag[2] != 0;
-}
-
 __global__ void __launch_bounds__(FCG_THREADS, 1) k_fcg_all(FcgArgs a, const CgDepth* __restrict__ deps,
                                                           const int* __restrict__ block_depth) {
     extern __shared__ __align__(1024) uint8_t dsm[];
@@ -184,9 +105,7 @@ __global__ void __launch_bounds__(FCG_THREADS, 1) k_fcg_all(FcgArgs a, const CgD
     __shared__ float sb[192];
     __shared__ float red[FCG_GROUPS][256];
     __shared__ float ss[FCG_GROUPS][128];
-    __shared__ double sh[FCG_WARPS * FCG_NV];
-    __shared__ double sh_val[FCG_NV];
-    __shared__ int sh_flag[3];
+    __shared__ GridSumShared<FCG_NV> gsm;
     __shared__ int gflag[FCG_GROUPS];
     __shared__ uint64_t bars[FCG_GROUPS];
     __shared__ uint32_t tslot;
@@ -224,16 +143,18 @@ __global__ void __launch_bounds__(FCG_THREADS, 1) k_fcg_all(FcgArgs a, const CgD
     tc_fence_after();
     const uint32_t tbase = tslot + (uint32_t)(grp * 128);
     uint32_t phase = 0;
-    FcgSync* psync = &a.sync[d];
     const int rank = blockIdx.x - dp.first_block;
     const i64 stride = (i64)dp.nblocks * blockDim.x;
     const i64 start = (i64)rank * blockDim.x + threadIdx.x;
     const i64 lo = dp.lo, n = dp.n;
-    int red_n = 0;
+    unsigned epoch = 0;
     bool ok = true, mma_ok = true;
+    const GridSum gs{a.slots, a.nslots, dp.first_block, dp.nblocks, rank, (int)gridDim.x + d, a.err, a.spin_limit, a.extra};
     auto reduce = [&](double (&v)[FCG_NV]) -> bool {
-        const bool r = fcg_reduce(psync, a.partial, dp.first_block, dp.nblocks, red_n & 1, v, a, sh, sh_flag, sh_val);
-        ++red_n;
+        double t[FCG_NV];
+        const bool r = grid_sum(gs, ++epoch, true, v, gsm, t);
+#pragma unroll
+        for (int j = 0; j < FCG_NV; ++j) v[j] = r ? t[j] : 0.0;
         return r;
     };
 
@@ -630,13 +551,14 @@ void stage_solve_learned(Ctx& c) {
     CgDepth* ddeps = dalloc<CgDepth>(D + 1, s);
     int* dbd = dalloc<int>(nblk, s);
     FcgState* st = dalloc<FcgState>(D + 1, s);
-    FcgSync* psync = dalloc<FcgSync>(D + 1, s);
-    double* partial = dalloc<double>((i64)nblk * 4, s);
+    const int nslots = nblk + D + 2;
+    const i64 words = grid_sum_words(nslots, FCG_NV);
+    u64* slots = dalloc<u64>(words, s);
     int* err = dalloc<int>(1, s);
     CK(cudaMemcpyAsync(ddeps, deps.data(), (D + 1) * sizeof(CgDepth), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dbd, block_depth.data(), nblk * sizeof(int), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(st, 0, (D + 1) * sizeof(FcgState), s));
-    CK(cudaMemsetAsync(psync, 0, (D + 1) * sizeof(FcgSync), s));
+    CK(cudaMemsetAsync(slots, 0, words * sizeof(u64), s));
     CK(cudaMemsetAsync(err, 0, sizeof(int), s));
     FcgArgs a;
     a.mode = c.params.solve_mode;
@@ -657,8 +579,8 @@ void stage_solve_learned(Ctx& c) {
     a.p = p;
     a.q = q;
     a.state = st;
-    a.sync = psync;
-    a.partial = partial;
+    a.slots = slots;
+    a.nslots = nslots;
     a.err = err;
     const WaitLimits wl = wait_limits();
     a.spin_limit = wl.spin_limit;
@@ -700,8 +622,8 @@ void stage_solve_learned(Ctx& c) {
     }
     if (kt >= 0) c.kpending[kt].bytes = bytes;
     dfree(ra, s); dfree(rb, s); dfree(z, s); dfree(p, s); dfree(q, s);
-    dfree(dcn, s); dfree(dcentre, s); dfree(ddeps, s); dfree(dbd, s); dfree(st, s); dfree(psync, s);
-    dfree(partial, s); dfree(err, s);
+    dfree(dcn, s); dfree(dcentre, s); dfree(ddeps, s); dfree(dbd, s); dfree(st, s); dfree(slots, s);
+    dfree(err, s);
     if (herr) {
         set_last_error("flexible CG: a device wait timed out");
         throw Error{PRGPU_ERR_TIMEOUT, {0}};

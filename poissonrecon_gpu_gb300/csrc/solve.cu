@@ -52,95 +52,13 @@ struct CgArgs {
     float* p;               // search direction
     float* q;               // A p
     PartState* state;
-    PartSync* sync;         // one per depth
-    double* partial;        // one per block
+    u64* slots;             // grid_sum's slots: one per block, one per depth (results), one never written
+    int nslots;
     int* err;
     long long spin_limit;   // bounded waits (WaitLimits)
     int extra;
     int refine;             // relative mode: FP64 true-residual check and refinement
 };
-
-// barrier over the blocks of one partition; returns false after a timeout
-__device__ bool part_barrier(PartState* ps, int nblocks, int* err, int* sh_ok, long long spin_limit, int extra) {
-    __syncthreads();
-    if (nblocks + extra > 1) {
-        if (threadIdx.x == 0) {
-            volatile unsigned* vgen = &ps->gen;
-            unsigned g = *vgen;
-            __threadfence();
-            unsigned arrived = atomicAdd(&ps->count, 1u);
-            int ok = 1;
-            if (arrived == (unsigned)(nblocks + extra) - 1) {
-                atomicExch(&ps->count, 0u);
-                __threadfence();
-                atomicAdd(&ps->gen, 1u);
-            } else {
-                long long spins = 0;
-                while (*vgen == g) {
-                    if (++spins > spin_limit || *(volatile int*)err) { ok = 0; break; }
-                    __nanosleep(32);
-                }
-            }
-            __threadfence();
-            if (!ok) atomicExch(err, PRGPU_ERR_TIMEOUT);
-            *sh_ok = ok && !*(volatile int*)err;
-        }
-    } else if (threadIdx.x == 0) {
-        __threadfence_block();
-        *sh_ok = 1;
-    }
-    __syncthreads();
-    return *sh_ok != 0;
-}
-
-// sum of v over the blocks of a partition, returned to every thread: each block
-// stores its partial, the last to arrive sums them all in a fixed order (so the
-// result does not depend on arrival order) and releases the others.  Waits spin
-// with a limit; on expiry the error flag is set and false returned.
-__device__ double part_reduce(PartSync* ps, double* partial, int first_block, int nblocks, int slot, double v,
-                              int* err, double* sh, int* sh_flag, double* sh_val, bool& ok, long long spin_limit,
-                              int extra) {
-    const double s = block_sum(v, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = s;
-        __threadfence();
-        const unsigned g = *(volatile unsigned*)&ps->gen;
-        const unsigned arrived = atomicAdd(&ps->count, 1u);
-        sh_flag[0] = (arrived == (unsigned)(nblocks + extra) - 1) ? 1 : 0;
-        sh_flag[1] = (int)g;
-    }
-    __syncthreads();
-    if (sh_flag[0]) {
-        __threadfence();
-        double t = 0.0;
-        for (int k = threadIdx.x; k < nblocks; k += blockDim.x) t += *(volatile double*)&partial[first_block + k];
-        t = block_sum(t, sh);
-        if (threadIdx.x == 0) {
-            ps->res[slot] = t;
-            atomicExch(&ps->count, 0u);
-            __threadfence();
-            atomicAdd(&ps->gen, 1u);
-            *sh_val = t;
-            sh_flag[2] = 1;
-        }
-    } else if (threadIdx.x == 0) {
-        const unsigned g = (unsigned)sh_flag[1];
-        volatile unsigned* vgen = &ps->gen;
-        long long spins = 0;
-        int good = 1;
-        while (*vgen == g) {
-            if (++spins > spin_limit || *(volatile int*)err) { good = 0; break; }
-            __nanosleep(64);
-        }
-        __threadfence();
-        if (!good) atomicExch(err, PRGPU_ERR_TIMEOUT);
-        *sh_val = *(volatile double*)&ps->res[slot];
-        sh_flag[2] = good && !*(volatile int*)err;
-    }
-    __syncthreads();
-    ok = sh_flag[2] != 0;
-    return *sh_val;
-}
 
 // per sibling group: first child of each of the parent's 27 neighbours (-1: none or a leaf)
 __global__ void k_group_table(NodeArrays nd, i64 ngroups, int* __restrict__ gn) {
@@ -165,6 +83,7 @@ __global__ void k_group_rows(const int* __restrict__ gn, i64 ngroups, int* __res
 
 constexpr int CG_TILE_GROUPS = CG_BLOCK / 8;   // sibling groups per tile, one thread per row
 constexpr int CG_WARP_TILES = 2;               // tiles of 4 groups a warp stages at once
+constexpr int CG_BLOCK_ROWS = CG_BLOCK * CG_WARP_TILES;   // rows of a block's warps at once, consecutive
 
 // 5 blocks per SM (48 registers): the partitions' warps wait on gathers and grid reductions, and
 // 40 warps per SM hide more of that latency than 32 (measured: 2.41 -> 1.90 ms on the 1M-point
@@ -174,8 +93,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
     __shared__ float sp[(CG_BLOCK / 32) * CG_WARP_TILES * CG_TILE_WORDS];
     __shared__ int sgn[(CG_BLOCK / 32) * CG_WARP_TILES * 4 * GN_ROW];
     __shared__ float sst[27];
-    __shared__ double sh[CG_BLOCK / 32];
-    __shared__ double sh_val;
+    __shared__ GridSumShared<1> gsm;
     const int d = block_depth[blockIdx.x];
     const CgDepth& dp = deps[d];
     if (threadIdx.x < 27) sst[threadIdx.x] = dp.st[threadIdx.x];
@@ -185,15 +103,15 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
     const int rank = blockIdx.x - dp.first_block;
     const i64 stride = (i64)dp.nblocks * blockDim.x;
     const i64 start = (i64)rank * blockDim.x + threadIdx.x;
-    int red = 0;   // reduction counter selects the accumulator slot
+    unsigned epoch = 0;
+    const GridSum gs{a.slots, a.nslots, dp.first_block, dp.nblocks, rank, (int)gridDim.x + d, a.err, a.spin_limit, a.extra};
 
-    // reduce a per-thread double over the partition; every thread gets the sum
-    __shared__ int sh_flag[3];
-    auto preduce = [&](double v, bool& ok) -> double {
-        const double res = part_reduce(&a.sync[d], a.partial, dp.first_block, dp.nblocks, red & 1, v, a.err, sh,
-                                       sh_flag, &sh_val, ok, a.spin_limit, a.extra);
-        ++red;
-        return res;
+    // reduce a per-thread value over the partition; every thread gets the sum
+    auto preduce = [&](auto v, bool data, bool& ok) -> double {
+        const decltype(v) s[1] = {v};
+        double t[1] = {0.0};
+        ok = grid_sum(gs, ++epoch, data, s, gsm, t);
+        return t[0];
     };
 
     // x = 0, r = b  (the host-side initialisation of CG_CUDA.cuh:435-439)
@@ -206,7 +124,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
         loc.add(bi * bi);
     }
     bool ok = true;
-    const double bb = preduce(loc.value(), ok);   // ||b||^2 in double (relative mode)
+    const double bb = preduce(loc, true, ok);   // ||b||^2 in double (relative mode)
     float r1 = (float)bb;
     float r0 = 0.f;
     int k = 1;
@@ -220,7 +138,10 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
         const bool go = (a.mode == PRGPU_SOLVE_REFERENCE) ? (r1 > a.tol2) : ((double)r1 > a.rel2 * bb);
         if (!go || k > a.max_iter) {
             if (!a.refine || a.mode != PRGPU_SOLVE_RELATIVE || k > a.max_iter) break;
-            // the recurrence says converged: recompute r = b - A x with FP64 accumulation
+            // the recurrence says converged: recompute r = b - A x with FP64 accumulation (x was
+            // written after its r.r was published, so its rows are made visible first)
+            preduce(0.0, true, ok);
+            if (!ok) break;
             double tsum = 0.0;
             for (i64 t = start; t < dp.n; t += stride) {
                 const i64 i = dp.lo + t;
@@ -233,7 +154,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
                 a.r[i] = (float)acc;
                 tsum = fma(acc, acc, tsum);
             }
-            rr_true = preduce(tsum, ok);
+            rr_true = preduce(tsum, true, ok);
             if (!ok || rr_true <= a.rel2 * bb || refines >= 2) break;
             // restart CG from the current x on the true residual
             ++refines;
@@ -256,7 +177,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
             loc.add(pi * qi);
         };
         loc = FSum();
-        if (d == 0) {
+        if (d == 0) {   // one row, one block
             for (i64 t = start; t < dp.n; t += stride) {
                 const i64 i = dp.lo + t;
                 float o = 0.f;
@@ -330,40 +251,55 @@ __global__ void __launch_bounds__(CG_BLOCK, 5) k_cg_all(CgArgs a, const CgDepth*
                 }
             }
         }
-        const double pq = preduce(loc.value(), ok);
+        // p.q carries no data: the update takes the rows whose p and q this block's product wrote
+        // (CG_BLOCK_ROWS at a time), and r only after every block has read it
+        const double pq = preduce(loc, false, ok);
         if (!ok) break;
         const float al = (float)((double)r1 / pq);
         const float nal = -al;
         loc = FSum();
-        {
-            // four rows per thread per step, loads first (independent requests in flight)
-            i64 t = start;
-            for (; t + 3 * stride < dp.n; t += 4 * stride) {
-                float pv[4], qv[4], xv[4], rv[4];
+        const i64 ustride = (i64)dp.nblocks * CG_BLOCK_ROWS;
+        // four rows per thread per step, loads first (independent requests in flight)
+        auto row4 = [&](i64 t, int u) { return t + (u & 1) * CG_BLOCK + (u >> 1) * ustride; };
+        for (i64 t = (i64)rank * CG_BLOCK_ROWS + threadIdx.x; t < dp.n; t += 2 * ustride) {
+            float qv[4], rv[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const i64 i = dp.lo + t + u * stride;
-                    pv[u] = a.p[i]; qv[u] = a.q[i]; xv[u] = a.x[i]; rv[u] = a.r[i];
-                }
+            for (int u = 0; u < 4; ++u) {
+                const bool in = row4(t, u) < dp.n;
+                const i64 i = dp.lo + row4(t, u);
+                qv[u] = in ? a.q[i] : 0.f;
+                rv[u] = in ? a.r[i] : 0.f;
+            }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const i64 i = dp.lo + t + u * stride;
-                    a.x[i] = fmaf(al, pv[u], xv[u]);
+            for (int u = 0; u < 4; ++u)
+                if (row4(t, u) < dp.n) {
                     const float ri = fmaf(nal, qv[u], rv[u]);
-                    a.r[i] = ri;
+                    a.r[dp.lo + row4(t, u)] = ri;
                     loc.add(ri * ri);
                 }
-            }
-            for (; t < dp.n; t += stride) {
-                const i64 i = dp.lo + t;
-                a.x[i] = fmaf(al, a.p[i], a.x[i]);
-                const float ri = fmaf(nal, a.q[i], a.r[i]);
-                a.r[i] = ri;
-                loc.add(ri * ri);
-            }
         }
-        r0 = r1;
-        r1 = (float)preduce(loc.value(), ok);
+        {
+            // x (read by nobody else) while r.r travels
+            const FSum s[1] = {loc};
+            grid_publish(gs, ++epoch, true, s, gsm);
+            for (i64 t = (i64)rank * CG_BLOCK_ROWS + threadIdx.x; t < dp.n; t += 2 * ustride) {
+                float pv[4], xv[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool in = row4(t, u) < dp.n;
+                    const i64 i = dp.lo + row4(t, u);
+                    pv[u] = in ? a.p[i] : 0.f;
+                    xv[u] = in ? a.x[i] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (row4(t, u) < dp.n) a.x[dp.lo + row4(t, u)] = fmaf(al, pv[u], xv[u]);
+            }
+            double rr[1] = {0.0};
+            ok = grid_collect(gs, epoch, true, gsm, rr);
+            r0 = r1;
+            r1 = (float)rr[0];
+        }
         ++k;
     }
     if (rank == 0 && threadIdx.x == 0) {
@@ -655,9 +591,9 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
     CgDepth* ddeps = dalloc<CgDepth>(D + 1, s);
     int* dbd = dalloc<int>((i64)block_depth.size(), s);
     PartState* st = dalloc<PartState>(D + 1, s);
-    PartSync* psync = dalloc<PartSync>(D + 1, s);
-    double* partial = dalloc<double>((i64)block_depth.size(), s);
-    CK(cudaMemsetAsync(psync, 0, (D + 1) * sizeof(PartSync), s));
+    const int nslots = (int)block_depth.size() + D + 2;
+    u64* slots = dalloc<u64>(grid_sum_words(nslots, 1), s);
+    CK(cudaMemsetAsync(slots, 0, grid_sum_words(nslots, 1) * sizeof(u64), s));
     int* err = dalloc<int>(1, s);
     CK(cudaMemcpyAsync(ddeps, deps.data(), (D + 1) * sizeof(CgDepth), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dbd, block_depth.data(), block_depth.size() * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -681,8 +617,8 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
     a.p = p;
     a.q = q;
     a.state = st;
-    a.sync = psync;
-    a.partial = partial;
+    a.slots = slots;
+    a.nslots = nslots;
     a.err = err;
     const WaitLimits wl = wait_limits();
     a.spin_limit = wl.spin_limit;
@@ -722,7 +658,7 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
         c.kpending[kt].bytes = bytes;
     }
     dfree(r, s); dfree(p, s); dfree(q, s);
-    dfree(ddeps, s); dfree(dbd, s); dfree(st, s); dfree(psync, s); dfree(partial, s); dfree(err, s);
+    dfree(ddeps, s); dfree(dbd, s); dfree(st, s); dfree(slots, s); dfree(err, s);
     if (herr) {
         set_last_error("solver barrier timed out");
         throw Error{PRGPU_ERR_TIMEOUT, {0}};
@@ -745,31 +681,177 @@ struct CsrArgs {
     float tol2;
     int max_iter;
     PartState* state;
+    u64* slots;             // grid_sum's slots
     int* err;
     long long spin_limit;
     int extra;
 };
 
-__global__ void __launch_bounds__(CG_BLOCK) k_cg_csr(CsrArgs a) {
-    __shared__ double sh[CG_BLOCK / 32];
-    __shared__ int sh_ok;
-    __shared__ double sh_val;
-    PartState* ps = a.state;
-    const int nblocks = gridDim.x;
+// Two products, the same q bit for bit (a row's entries in order, one FMA each).
+//
+// Rows of few entries, or few rows: a thread per row walks its own entries.
+//
+// Rows of many entries (csr_stream): the product is bound by the matrix, 8 bytes an entry, once per
+// iteration.  A thread per row reads a warp's lines a row apart, an eighth of each request used; on the
+// 27-point stencil of 915 K rows (195 MB) an iteration took 84 us against 29 us of matrix bytes.  So a
+// warp takes 32 consecutive rows, whose entries are one run of the arrays, in pieces of at most
+// CSR_CHUNK entries: columns and values come into shared memory by asynchronous copies, the next piece
+// while this one is summed, and each lane walks its own row there.  p is gathered in that walk, where
+// the 32 lanes are at the same place of 32 rows (near columns, one or two lines a request), and not in
+// the order of the entries (ten).  Pieces end where the 32 rows end: with a fixed size a piece holds
+// parts of few rows and most lanes idle.  Two pieces of 7 KB for each of 15 warps fill an SM's shared
+// memory, one block per SM.  Measured: 47 us a product (DRAM 3.2 TB/s and as much again from L2, which
+// serves the gathers), 67 us an iteration.
+constexpr int CSR_CHUNK = 896;
+constexpr int CSR_BLOCK = 480;
+constexpr int CSR_U = 9;                               // gathers in flight per lane
+constexpr int CSR_WARPS = CSR_BLOCK / 32;
+struct CsrWarpShared {
+    int col[2][CSR_CHUNK];
+    float val[2][CSR_CHUNK];
+};
+constexpr int CSR_DSMEM = CSR_WARPS * (int)sizeof(CsrWarpShared);
+
+// entries [s, e) into a stage, at s & 3 when 'wide' (both arrays 16-byte aligned), else at 0
+__device__ __forceinline__ void csr_fetch(const CsrArgs& a, int s, int e, bool wide, int* col, float* val) {
+    const int lane = threadIdx.x & 31;
+    const unsigned sc = (unsigned)__cvta_generic_to_shared(col), sv = (unsigned)__cvta_generic_to_shared(val);
+    if (wide) {
+        const int s0 = s & ~3;
+        for (int k = 4 * lane; k < e - s0; k += 128) {
+            const int bytes = 4 * min(e - s0 - k, 4);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sc + 4 * k), "l"(a.col + s0 + k), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sv + 4 * k), "l"(a.val + s0 + k), "r"(bytes) : "memory");
+        }
+    } else {
+        for (int k = lane; k < e - s; k += 32) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sc + 4 * k), "l"(a.col + s + k) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sv + 4 * k), "l"(a.val + s + k) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+struct CsrRows {                                       // 32 rows: this lane's row and its entries
+    int row, e0, e1;
+    int end;                                           // the last entry + 1
+    bool run;                                          // the offsets do not decrease
+};
+// the loads only; csr_rows_close makes them a group
+__device__ __forceinline__ CsrRows csr_rows_load(const CsrArgs& a, i64 g) {
+    CsrRows r;
+    r.row = (int)min(32 * g + (threadIdx.x & 31), (i64)a.n);
+    r.e0 = r.e1 = 0;
+    if (r.row < a.n) {
+        r.e0 = a.rowptr[r.row];
+        r.e1 = a.rowptr[r.row + 1];
+    }
+    return r;
+}
+__device__ __forceinline__ void csr_rows_close(const CsrArgs& a, CsrRows& r) {
+    r.run = __all_sync(0xffffffffu, r.e0 <= r.e1);
+    const unsigned m = __ballot_sync(0xffffffffu, r.row < a.n);
+    r.end = m ? __shfl_sync(0xffffffffu, r.e1, 31 - __clz(m)) : 0;
+}
+
+// the 32-row groups first, first + step, ... of q = A p, one warp.  Returns the lane's part of p.q
+__device__ __forceinline__ double csr_stream(const CsrArgs& a, int first, int step, bool wide, CsrWarpShared& sm) {
+    const int lane = threadIdx.x & 31;
+    double loc = 0.0;
+    const i64 ngroup = ((i64)a.n + 31) / 32;
+    i64 g = first;
+    if (g >= ngroup) return loc;
+    CsrRows cur = csr_rows_load(a, g), nxt = csr_rows_load(a, g + step), far = csr_rows_load(a, g + 2 * (i64)step);
+    csr_rows_close(a, cur);
+    csr_rows_close(a, nxt);
+    auto piece_end = [&](int from, const CsrRows& r) {
+        return (int)min((i64)r.end, (i64)from - (wide ? from & 3 : 0) + CSR_CHUNK);
+    };
+    int s = __shfl_sync(0xffffffffu, cur.e0, 0);       // the current piece [s, e)
+    int e = cur.run ? piece_end(s, cur) : s;
+    __syncwarp();                                      // the previous product's readers are done
+    csr_fetch(a, s, e, wide, sm.col[0], sm.val[0]);
+    float o = 0.f, po = cur.row < a.n ? a.p[cur.row] : 0.f;
+    for (int st = 0;; st ^= 1) {
+        // the next piece: of this group, or the next group's first
+        const bool last = e >= cur.end || !cur.run;
+        const bool more = !last || g + step < ngroup;
+        int s2 = e, e2 = e;
+        if (last && more) s2 = e2 = __shfl_sync(0xffffffffu, nxt.e0, 0);
+        if (more && (last ? nxt.run : true)) e2 = piece_end(s2, last ? nxt : cur);
+        csr_fetch(a, s2, e2, wide, sm.col[st ^ 1], sm.val[st ^ 1]);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const int base = wide ? s & ~3 : s;            // entry k lies at k - base
+        const int* col = sm.col[st];
+        const float* sv = sm.val[st];
+        const int t1 = min(cur.e1, e) - base;
+        for (int t = max(cur.e0, s) - base; t < t1; t += CSR_U) {
+            float pv[CSR_U], vv[CSR_U];
+#pragma unroll
+            for (int u = 0; u < CSR_U; ++u) pv[u] = t + u < t1 ? a.p[col[t + u]] : 0.f;
+#pragma unroll
+            for (int u = 0; u < CSR_U; ++u) vv[u] = t + u < t1 ? sv[t + u] : 0.f;
+#pragma unroll
+            for (int u = 0; u < CSR_U; ++u)
+                if (t + u < t1) o = fmaf(vv[u], pv[u], o);
+        }
+        if (last) {
+            if (cur.row < a.n) {
+                // offsets that decrease: each row by itself, without entries when its end lies before its start
+                if (!cur.run) {
+                    o = 0.f;
+                    for (int k = cur.e0; k < cur.e1; ++k) o = fmaf(a.val[k], a.p[a.col[k]], o);
+                }
+                a.q[cur.row] = o;
+                loc += (double)(po * o);
+            }
+            if (!more) break;
+            o = 0.f;
+            g += step;
+            cur = nxt;
+            po = cur.row < a.n ? a.p[cur.row] : 0.f;
+            nxt = far;
+            csr_rows_close(a, nxt);
+            far = csr_rows_load(a, g + 2 * (i64)step);
+        }
+        s = s2;
+        e = e2;
+        __syncwarp();                                  // this piece's readers are done
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return loc;
+}
+
+// f over this thread's rows, four at a time: load (row, slot) for all four first
+template <class L, class F>
+__device__ __forceinline__ void csr_each(i64 start, i64 stride, i64 n, L load, F use) {
+    for (i64 i = start; i < n; i += 4 * stride) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * stride < n) load(i + u * stride, u);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * stride < n) use(i + u * stride, u);
+    }
+}
+
+template <bool STREAM>
+__global__ void __launch_bounds__(STREAM ? CSR_BLOCK : CG_BLOCK, STREAM ? 1 : 4) k_cg_csr(CsrArgs a) {
+    extern __shared__ __align__(16) unsigned char csr_dsm[];
+    __shared__ GridSumShared<1> gsm;
     const i64 stride = (i64)gridDim.x * blockDim.x;
     const i64 start = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    int red = 0;
-    auto preduce = [&](double v, bool& ok) -> double {
-        double s = block_sum(v, sh);
-        if (threadIdx.x == 0) atomicAdd(&ps->acc[red % 3], s);
-        ok = part_barrier(ps, nblocks, a.err, &sh_ok, a.spin_limit, a.extra);
-        if (threadIdx.x == 0) sh_val = *(volatile double*)&ps->acc[red % 3];
-        __syncthreads();
-        double res = sh_val;
-        if (blockIdx.x == 0 && threadIdx.x == 0) ps->acc[(red + 2) % 3] = 0.0;
-        ++red;
-        return res;
+    const int w = threadIdx.x >> 5;
+    unsigned epoch = 0;
+    const GridSum gs{a.slots, (int)gridDim.x + 2, 0, (int)gridDim.x, (int)blockIdx.x, (int)gridDim.x, a.err, a.spin_limit, a.extra};
+    auto preduce = [&](double v, bool data, bool& ok) -> double {
+        const double s[1] = {v};
+        double t[1] = {0.0};
+        ok = grid_sum(gs, ++epoch, data, s, gsm, t);
+        return t[0];
     };
+    float l0[4], l1[4];
     double loc = 0;
     for (i64 i = start; i < a.n; i += stride) {
         a.x[i] = 0.f;
@@ -777,67 +859,97 @@ __global__ void __launch_bounds__(CG_BLOCK) k_cg_csr(CsrArgs a) {
         loc += (double)(a.b[i] * a.b[i]);
     }
     bool ok = true;
-    float r1 = (float)preduce(loc, ok), r0 = 0.f;
+    float r1 = (float)preduce(loc, true, ok), r0 = 0.f;
     int k = 1;
     while (ok && r1 > a.tol2 && k <= a.max_iter) {
-        if (k > 1) {
-            const float beta = r1 / r0;
-            for (i64 i = start; i < a.n; i += stride) a.p[i] = fmaf(beta, a.p[i], a.r[i]);
-        } else {
-            for (i64 i = start; i < a.n; i += stride) a.p[i] = a.r[i];
-        }
-        if (!part_barrier(ps, nblocks, a.err, &sh_ok, a.spin_limit, a.extra)) break;
+        const float beta = k > 1 ? r1 / r0 : 0.f;
+        csr_each(start, stride, a.n,
+                 [&](i64 i, int u) { l0[u] = a.r[i]; l1[u] = k > 1 ? a.p[i] : 0.f; },
+                 [&](i64 i, int u) { a.p[i] = k > 1 ? fmaf(beta, l1[u], l0[u]) : l0[u]; });
+        preduce(0.0, true, ok);   // p is complete
+        if (!ok) break;
         loc = 0;
-        for (i64 i = start; i < a.n; i += stride) {
-            float o = 0.f;
-            for (int e = a.rowptr[i]; e < a.rowptr[i + 1]; ++e) o = fmaf(a.val[e], a.p[a.col[e]], o);
-            a.q[i] = o;
-            loc += (double)(a.p[i] * o);
+        if constexpr (STREAM) {
+            const bool wide = ((reinterpret_cast<u64>(a.col) | reinterpret_cast<u64>(a.val)) & 15) == 0;
+            loc = csr_stream(a, blockIdx.x * CSR_WARPS + w, gridDim.x * CSR_WARPS, wide,
+                             reinterpret_cast<CsrWarpShared*>(csr_dsm)[w]);
+        } else {
+            for (i64 i = start; i < a.n; i += stride) {
+                float o = 0.f;
+                for (int e = a.rowptr[i]; e < a.rowptr[i + 1]; ++e) o = fmaf(a.val[e], a.p[a.col[e]], o);
+                a.q[i] = o;
+                loc += (double)(a.p[i] * o);
+            }
         }
-        const double pq = preduce(loc, ok);
+        const double pq = preduce(loc, STREAM, ok);   // (a thread per row updates the rows of its q)
         if (!ok) break;
         const float al = (float)((double)r1 / pq), nal = -al;
         loc = 0;
-        for (i64 i = start; i < a.n; i += stride) {
-            a.x[i] = fmaf(al, a.p[i], a.x[i]);
-            const float ri = fmaf(nal, a.q[i], a.r[i]);
-            a.r[i] = ri;
-            loc += (double)(ri * ri);
-        }
+        csr_each(start, stride, a.n,
+                 [&](i64 i, int u) { l0[u] = a.q[i]; l1[u] = a.r[i]; },
+                 [&](i64 i, int u) {
+                     const float ri = fmaf(nal, l0[u], l1[u]);
+                     a.r[i] = ri;
+                     loc += (double)(ri * ri);
+                 });
+        // r is read and written by its own thread only, and so is p until it is complete again: r.r
+        // carries no data, and x is updated while it travels
+        const double s[1] = {loc};
+        double rr[1] = {0.0};
+        grid_publish(gs, ++epoch, false, s, gsm);
+        csr_each(start, stride, a.n,
+                 [&](i64 i, int u) { l0[u] = a.p[i]; l1[u] = a.x[i]; },
+                 [&](i64 i, int u) { a.x[i] = fmaf(al, l0[u], l1[u]); });
+        ok = grid_collect(gs, epoch, false, gsm, rr);
         r0 = r1;
-        r1 = (float)preduce(loc, ok);
+        r1 = (float)rr[0];
         ++k;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ps->iters = k - 1;
-        ps->rr = r1;
+        a.state->iters = k - 1;
+        a.state->rr = r1;
     }
 }
 
-int cg_csr_impl(int n, const int* rowptr, const int* col, const float* val, const float* rhs, float* x, float tol,
+// Where the streamed product is the faster one (us an iteration, a thread per row against streamed): 27
+// entries a row, 1 M rows 98 against 67, 100 K rows 20 against 23; 7 entries, 1 M rows 33 against 54; 64
+// entries, 1 M rows (rows 16 quads apart, so lanes meet in a bank) 486 against 478.  A wrong nz only picks
+// the slower of two products.
+constexpr int CSR_STREAM_NNZ = 16, CSR_STREAM_ROWS = 1 << 17;
+
+int cg_csr_impl(int n, int nz, const int* rowptr, const int* col, const float* val, const float* rhs, float* x, float tol,
                 int max_iter, int* iters, float* ms) {
     cudaStream_t s = 0;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_csr, CG_BLOCK, 0));
-    i64 want = ((i64)n + CG_BLOCK - 1) / CG_BLOCK;
-    int G = (int)std::max<i64>(1, std::min<i64>((i64)sms * std::max(per_sm, 1), want));
+    const bool stream = nz / std::max(n, 1) >= CSR_STREAM_NNZ && n >= CSR_STREAM_ROWS;
+    const int block = stream ? CSR_BLOCK : CG_BLOCK, dsmem = stream ? CSR_DSMEM : 0;
+    void (*kernel)(CsrArgs) = stream ? k_cg_csr<true> : k_cg_csr<false>;
+    if (stream) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CSR_DSMEM));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, dsmem));
+    const i64 want = ((i64)n + block - 1) / block;
+    const int G = (int)std::max<i64>(1, std::min<i64>((i64)sms * std::max(per_sm, 1), want));
+    const i64 words = grid_sum_words(G + 2, 1);
     float *r = nullptr, *p = nullptr, *q = nullptr;
     PartState* st = nullptr;
+    u64* slots = nullptr;
     int* err = nullptr;
     CK(cudaMalloc(&r, sizeof(float) * std::max(n, 1)));
     CK(cudaMalloc(&p, sizeof(float) * std::max(n, 1)));
     CK(cudaMalloc(&q, sizeof(float) * std::max(n, 1)));
     CK(cudaMalloc(&st, sizeof(PartState)));
+    CK(cudaMalloc(&slots, sizeof(u64) * words));
     CK(cudaMalloc(&err, sizeof(int)));
     CK(cudaMemset(st, 0, sizeof(PartState)));
+    CK(cudaMemset(slots, 0, sizeof(u64) * words));
     CK(cudaMemset(err, 0, sizeof(int)));
     CsrArgs a;
     a.n = n; a.rowptr = rowptr; a.col = col; a.val = val; a.b = rhs; a.x = x; a.r = r; a.p = p; a.q = q;
     a.tol2 = tol * tol;
     a.max_iter = max_iter;
     a.state = st;
+    a.slots = slots;
     a.err = err;
     const WaitLimits wl = wait_limits();
     a.spin_limit = wl.spin_limit;
@@ -847,7 +959,7 @@ int cg_csr_impl(int n, const int* rowptr, const int* col, const float* val, cons
     CK(cudaEventCreate(&e1));
     void* kargs[] = {(void*)&a};
     CK(cudaEventRecord(e0, s));
-    CK(cudaLaunchCooperativeKernel((void*)k_cg_csr, dim3(G), dim3(CG_BLOCK), kargs, 0, s));
+    CK(cudaLaunchCooperativeKernel((void*)kernel, dim3(G), dim3(block), kargs, dsmem, s));
     ++g_kernel_launches;
     CK(cudaEventRecord(e1, s));
     CK(cudaEventSynchronize(e1));
@@ -857,7 +969,7 @@ int cg_csr_impl(int n, const int* rowptr, const int* col, const float* val, cons
     int herr = 0;
     CK(cudaMemcpy(&hs, st, sizeof hs, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&herr, err, sizeof herr, cudaMemcpyDeviceToHost));
-    cudaFree(r); cudaFree(p); cudaFree(q); cudaFree(st); cudaFree(err);
+    cudaFree(r); cudaFree(p); cudaFree(q); cudaFree(st); cudaFree(slots); cudaFree(err);
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     if (iters) *iters = hs.iters;
     if (ms) *ms = t;
