@@ -84,43 +84,72 @@ struct EvalArgs {
     const float* x;
     const float* x27;      // nodes [0, nx27): x of the 27 neighbours (0: none), 28 floats per node; or null
     i64 nx27;
-    const float* lb;       // basis values at finest-lattice points (see lattice_basis), or null
+    const float4* lb;      // basis values at finest-lattice points by cell (see lattice_at), or null
     int stable;            // params.stable_basis: closed-form basis values (basis_stable)
 };
 
-// start of depth d in the lattice basis table: sum_{l<d} 2^l (3 2^(D-l) + 1) = 3 d 2^D + 2^d - 1
-__device__ __host__ __forceinline__ i64 lattice_basis_offset(int D, int d) {
-    return 3ll * d * (1ll << D) + (1ll << d) - 1;
+// Basis values at the finest-lattice points, by depth-d cell c and point u = c w + k of its closure
+// (0 <= k <= w = 2^(D-d)): the values at u of the functions c - 1, c, c + 1 and c + 2, those a walk at u
+// through cell c multiplies with (c + 2 reaches u only at k = w; it serves corners whose owner is the
+// next cell), 0 for functions that do not exist or do not reach u.  One 16-byte load per axis and level
+// in place of three looked-up scalars.  Depth d starts at sum_{l<d} (2^D + 2^l) = d 2^D + 2^d - 1.
+__device__ __host__ __forceinline__ i64 lattice_offset(int D, int d) { return (i64)d * (1ll << D) + (1ll << d) - 1; }
+__device__ __forceinline__ float4 lattice_at(const EvalArgs& a, int d, int c, int k) {
+    return a.lb[lattice_offset(a.D, d) + (i64)c * ((1 << (a.D - d)) + 1) + k];
+}
+// entry t of lattice_at
+__device__ __forceinline__ float lattice_entry(const EvalArgs& a, int d, int c, int k, int t) {
+    return reinterpret_cast<const float*>(a.lb)[4 * (lattice_offset(a.D, d) + (i64)c * ((1 << (a.D - d)) + 1) + k) + t];
 }
 
-// B_{d,n}(u / 2^D) for a finest-lattice coordinate u: the value cpoly_value
-// computes, read from the table when u lies in the support [(n-1)w, (n+2)w]
-// (w = 2^(D-d), 3w+1 points per function), evaluated otherwise
+// B_{d,n}(u / 2^D), 0 <= n < 2^d, for any finest-lattice coordinate u: from the table where u lies in the
+// support [(n-1)w, (n+2)w], evaluated elsewhere (the table's values are the evaluated ones)
 __device__ __forceinline__ float lattice_basis(const EvalArgs& a, int d, int n, int u) {
     const int w = 1 << (a.D - d);
     const int k = u - (n - 1) * w;
-    if (a.lb && k >= 0 && k <= 3 * w) return a.lb[lattice_basis_offset(a.D, d) + (i64)n * (3 * w + 1) + k];
+    if (k >= 0 && k <= 3 * w) {
+        int c = min(u >> (a.D - d), (1 << d) - 1);   // a cell that holds u
+        if (c > n + 1) --c;                          // u is the support's right end: the cell left of it
+        return lattice_entry(a, d, c, u - c * w, n - c + 1);
+    }
     if (a.stable) return basis_stable(d, n, (float)u * (1.0f / (float)(1 << a.D)));
     return cpoly_value<3>(a.basis[(1 << d) - 1 + n], (float)u * (1.0f / (float)(1 << a.D)));
 }
 
 __global__ void k_lattice_basis(const CPoly* __restrict__ basis, int D, i64 total, float* __restrict__ lb, int stable) {
     const float inv = 1.0f / (float)(1 << D);
-    for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
-        // depth d holds 2^d functions of 3w+1 points: offset sum_{l<d} 2^l (3 2^(D-l) + 1)
+    for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < 4 * total; e += (i64)gridDim.x * blockDim.x) {
+        const i64 q = e >> 2;
         int d = 0;
-        i64 off = 0;
-        for (;;) {
-            const i64 len = (1ll << d) * (3ll * (1ll << (D - d)) + 1);
-            if (e < off + len) break;
-            off += len;
-            ++d;
-        }
+        while (q >= lattice_offset(D, d + 1)) ++d;
         const int w = 1 << (D - d);
-        const i64 r = e - off;
-        const int n = (int)(r / (3 * w + 1)), k = (int)(r % (3 * w + 1));
-        const float q = (float)((n - 1) * w + k) * inv;
-        lb[e] = stable ? basis_stable(d, n, q) : cpoly_value<3>(basis[(1 << d) - 1 + n], q);
+        const i64 r = q - lattice_offset(D, d);
+        const int c = (int)(r / (w + 1)), k = (int)(r % (w + 1)), n = c + (int)(e & 3) - 1;
+        const int u = c * w + k, ks = u - (n - 1) * w;
+        float v = 0.f;
+        if (n >= 0 && n < (1 << d) && ks >= 0 && ks <= 3 * w) {
+            const float x = (float)u * inv;
+            v = stable ? basis_stable(d, n, x) : cpoly_value<3>(basis[(1 << d) - 1 + n], x);
+        }
+        lb[e] = v;
+    }
+}
+
+// values at finest-lattice coordinate u of the functions c - 1, c, c + 1 of depth d (0 outside 0..2^d - 1)
+__device__ __forceinline__ void lattice_row(const EvalArgs& a, int d, int c, int u, float bv[3]) {
+    const int k = u - (c << (a.D - d));
+    if ((unsigned)k <= (1u << (a.D - d))) {
+        const float4 f = lattice_at(a, d, c, k);
+        bv[0] = f.x; bv[1] = f.y; bv[2] = f.z;
+        return;
+    }
+#pragma unroll 1
+    for (int t = 0; t < 3; ++t) {
+        const int n = c + t - 1;
+        const float v = (n >= 0 && n < (1 << d)) ? lattice_basis(a, d, n, u) : 0.f;
+        if (t == 0) bv[0] = v;
+        else if (t == 1) bv[1] = v;
+        else bv[2] = v;
     }
 }
 
@@ -192,15 +221,9 @@ inline float* build_x27(const Ctx& c, i64 n) {
 // level_sum at a finest-lattice point u (q = u / 2^D), basis values from the table
 __device__ __forceinline__ float level_sum_u(const EvalArgs& a, i64 node, int d, const int xyz[3], const int u[3],
                                              float val) {
-    const int lim = 1 << d;
     float bv[3][3];
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax)
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int c = xyz[ax] + t - 1;
-            bv[ax][t] = (c >= 0 && c < lim) ? lattice_basis(a, d, c, u[ax]) : 0.f;
-        }
+    for (int ax = 0; ax < 3; ++ax) lattice_row(a, d, xyz[ax], u[ax], bv[ax]);
     if (node < a.nx27) {
         const float4* row = reinterpret_cast<const float4*>(a.x27 + node * X27_STRIDE);
         float xs[28];
@@ -344,60 +367,6 @@ __device__ float owner_corner_value(const EvalArgs& a, i64 o, int kind, float is
     return val - iso;
 }
 
-// for each corner k in 'mask' of node 'node' (depth d, coordinates xyz): the
-// walk_up_u sum from the node to the root at the corner's lattice point
-// (xyz + bit) << sh, all corners sharing the walk (the same levels and
-// neighbour x, each corner with its own basis values and FMA chain)
-__device__ __forceinline__ void walk_up_corners(const EvalArgs& a, i64 node, int d, const int xyz[3], int sh,
-                                                unsigned mask, float val[8]) {
-    const NodeArrays& nd = a.nd;
-    const i64 M = nd.M;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) val[k] = 0.f;
-    int c[3] = {xyz[0], xyz[1], xyz[2]};
-    while (node != -1) {
-        float xs[27];
-        if (node < a.nx27) {
-            const float4* row = reinterpret_cast<const float4*>(a.x27 + node * X27_STRIDE);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                const float4 t = row[k];
-                xs[4 * k] = t.x; xs[4 * k + 1] = t.y; xs[4 * k + 2] = t.z; xs[4 * k + 3] = t.w;
-            }
-            const float4 t = row[6];
-            xs[24] = t.x; xs[25] = t.y; xs[26] = t.z;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 27; ++j) {
-                const int nb = nd.neigh[(i64)j * M + node];
-                xs[j] = nb == -1 ? 0.f : a.x[nb];   // absent: a zero product leaves the sum unchanged
-            }
-        }
-        const int lim = 1 << d;
-#pragma unroll 1
-        for (int kind = 0; kind < 8; ++kind) {
-            if (!((mask >> kind) & 1)) continue;
-            const int u[3] = {(xyz[0] + (kind & 1)) << sh, (xyz[1] + ((kind >> 1) & 1)) << sh,
-                              (xyz[2] + ((kind >> 2) & 1)) << sh};
-            float bv[3][3];
-#pragma unroll
-            for (int ax = 0; ax < 3; ++ax)
-#pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    const int n = c[ax] + t - 1;
-                    bv[ax][t] = (n >= 0 && n < lim) ? lattice_basis(a, d, n, u[ax]) : 0.f;
-                }
-            float v = val[kind];
-#pragma unroll
-            for (int j = 0; j < 27; ++j) v = fmaf(xs[j] * bv[0][j / 9] * bv[1][(j / 3) % 3], bv[2][j % 3], v);
-            val[kind] = v;
-        }
-        node = nd.parent[node];
-        --d;
-        c[0] >>= 1; c[1] >>= 1; c[2] >>= 1;
-    }
-}
-
 // finest-depth corners: each corner evaluated by its owner.  A node owns a
 // corner when no other existing node of the 8 around it has a smaller key.
 // Pass 1 (one thread per node): the mask of owned corners and their count.
@@ -533,57 +502,6 @@ __global__ void k_coarse_need(NodeArrays nd, i64 lo, i64 hi, unsigned char* __re
         }
     }
 }
-// the needed corners of one node share the walk up (owner_corner_value: walk
-// up, then for each corner its own descent through children[childrenVertexKind])
-__global__ void __launch_bounds__(128, 6) k_coarse_corner_values(EvalArgs a, i64 n, float iso,
-                                                                 const unsigned char* __restrict__ need,
-                                                                 float* __restrict__ cval) {
-    const NodeArrays& nd = a.nd;
-    const int D = a.D;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        unsigned mask = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) mask |= need[8 * i + k] ? (1u << k) : 0u;
-        if (!mask) continue;
-        float val[8];
-        if (i == 0) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) val[k] = 0.f;   // the root has no corner value of its own
-        } else {
-            const int d = nd.depth[i];
-            int xyz[3];
-            key_coords(nd.key[i], d, D, xyz);
-            const int sh = D - d;
-            walk_up_corners(a, i, d, xyz, sh, mask, val);
-            if (nd.child0[i] != -1) {
-#pragma unroll 1
-                for (int kind = 0; kind < 8; ++kind) {
-                    if (!((mask >> kind) & 1)) continue;
-                    const int u[3] = {(xyz[0] + (kind & 1)) << sh, (xyz[1] + ((kind >> 1) & 1)) << sh,
-                                      (xyz[2] + ((kind >> 2) & 1)) << sh};
-                    const int exceed = c_vid[kind];
-                    i64 node = i;
-                    float v = val[kind];
-                    int cx[3] = {xyz[0], xyz[1], xyz[2]};
-                    for (int dd = d + 1; dd <= D; ++dd) {
-                        const int c0 = nd.child0[node];
-                        if (c0 == -1) break;
-                        node = c0 + exceed;
-                        cx[0] = (cx[0] << 1) | ((exceed >> 2) & 1);
-                        cx[1] = (cx[1] << 1) | ((exceed >> 1) & 1);
-                        cx[2] = (cx[2] << 1) | (exceed & 1);
-                        v = level_sum_u(a, node, dd, cx, u, v);
-                    }
-                    val[kind] = v;
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if ((mask >> k) & 1) cval[8 * i + k] = val[k] - iso;
-    }
-}
-
 // needed corners of each coarse node as a mask and a count
 __global__ void k_need_mask(const unsigned char* __restrict__ need, i64 n, unsigned char* __restrict__ mask,
                             int* __restrict__ count) {
@@ -704,11 +622,7 @@ __device__ float virtual_corner_value(const VArgs& v, int L, int r, const int oc
         }
         if (inner) continue;
         float bv[3][3];
-        for (int ax = 0; ax < 3; ++ax)
-            for (int t = 0; t < 3; ++t) {
-                int cc = V[ax] + t - 1;
-                bv[ax][t] = (cc >= 0 && cc < lim) ? lattice_basis(a, d, cc, qc[ax]) : 0.f;
-            }
+        for (int ax = 0; ax < 3; ++ax) lattice_row(a, d, V[ax], qc[ax], bv[ax]);
         for (int j = 0; j < 27; ++j) {
             const int N[3] = {V[0] + j / 9 - 1, V[1] + (j / 3) % 3 - 1, V[2] + j % 3 - 1};
             if (N[0] < 0 || N[1] < 0 || N[2] < 0 || N[0] >= lim || N[1] >= lim || N[2] >= lim) continue;
@@ -803,7 +717,7 @@ struct BrickIndex {                // bricks of all subdivided leaves, numbered 
     const i64* row_prefix;         // first brick row of each root (3 * bricks per edge rows each)
     int nroots;
     const float* rows;             // brick-row tables, PROW (D+1) floats each
-    const float* xl;               // per root: x of the 27 neighbours of each ancestor, 16 x 27
+    const int* up;                 // per root: its node and its ancestors by depth, BR_LEVELS each
     const float* anc;              // per root: the ancestor polynomial, ANC_STRIDE floats
     DepthLayout dl;
 };
@@ -866,8 +780,6 @@ __device__ __forceinline__ float bern_m(const float4& f) {
     return (fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fabsf(f.z)) + f.w) * (1.0f + 9.5367431640625e-07f);
 }
 
-__device__ __forceinline__ float x_or_zero(const EvalArgs& a, int node) { return node < 0 ? 0.f : a.x[node]; }
-
 // real node at depth d with coordinates N near leaf L (depth r, coords Lc), or -1 (none, or inside L)
 __device__ i64 shell_node(const VArgs& v, int L, int r, const int Lc[3], int d, const int N[3]) {
     const NodeArrays& nd = v.e.nd;
@@ -890,12 +802,12 @@ __device__ i64 shell_node(const VArgs& v, int L, int r, const int Lc[3], int d, 
 // within 5u of the exact factored end per row (3 terms, 2 products), against
 // 3u per term in the term-by-term form; the margins allow 2 BR_WEXT u A more.
 // amax gains sum |x| |Z| |Y| |X| >= sum |term| over the corners.
-__device__ __forceinline__ void ancestor_bound(const float* xl, const float* const row[3], int r, int D, int lane,
-                                               float& lo, float& hi, float& amax, int& cnt) {
+__device__ __forceinline__ void ancestor_bound(const EvalArgs& a, const int* up, const float* const row[3], int r,
+                                               int D, int lane, float& lo, float& hi, float& amax, int& cnt) {
     const int ra = ROW_RA * (D + 1);
     for (int t = lane; t < 9 * (r + 1); t += 32) {
         const int l = r - t / 9, jx = (t % 9) / 3, jy = t % 3;
-        const float* xs = xl + 27 * l + 9 * jx + 3 * jy;
+        const float* xs = a.x27 + (i64)up[l] * X27_STRIDE + 9 * jx + 3 * jy;
         float slo = 0.f, shi = 0.f, sabs = 0.f;
         for (int jz = 0; jz < 3; ++jz) {
             const float x = xs[jz];
@@ -958,17 +870,17 @@ __device__ __forceinline__ void window_axis(int g0, int B, int Lc_ax, int r, int
     ext = Vhi - Vlo + 3 + extra;
 }
 
-// BT[d][t][k] of the brick row starting at corner g0 (see above).  Every entry a
-// corner reads lies in its function's support [(n-1)w, (n+2)w] (the corner is
-// in the closure of the owner cell n - t + 1; for t = 3 at the support's left
-// end), so entries outside it -- never read -- are left 0.
-__device__ __forceinline__ float brick_bt(const EvalArgs& a, int r, int Lc_ax, int g0, int d, int t, int k) {
-    const int n = (d <= r) ? (Lc_ax >> (r - d)) + t - 1 : ((g0 + k - 1) >> (a.D - d)) + t - 1;
-    if (n < 0 || n >= (1 << d)) return 0.f;
-    const int w = 1 << (a.D - d);
-    const int kk = g0 + k - (n - 1) * w;
-    if (kk < 0 || kk > 3 * w) return 0.f;
-    return a.lb[lattice_basis_offset(a.D, d) + (i64)n * (3 * w + 1) + kk];
+// BT[d][0..3][k] of the brick row starting at corner g0 (see above): the corner is in the closure of its
+// ancestor cell (d <= r) or of the cell below it.  The corner 0 has no cell below it: the functions
+// -2..1 there are those of cell 0 moved by one.
+__device__ __forceinline__ float4 brick_bt(const EvalArgs& a, int r, int Lc_ax, int g0, int d, int k) {
+    const int u = g0 + k, sh = a.D - d;
+    const int c = (d <= r) ? (Lc_ax >> (r - d)) : ((u - 1) >> sh);
+    if (c < 0) {
+        const float4 f = lattice_at(a, d, 0, 0);
+        return make_float4(0.f, f.x, f.y, f.z);
+    }
+    return lattice_at(a, d, c, u - (c << sh));
 }
 
 // a / n for 0 <= a < 2^14 and 1 <= n <= 2^10 through the reciprocal inv = 1/n:
@@ -1055,16 +967,14 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
         float* out = rows + row * (i64)((super ? ROW_PER_DEPTH : PROW) * (D + 1));
         if (d <= r) {
             if (!super) continue;   // bricks: the leaf's ancestor polynomial (k_brick_xl)
-            for (int t = 0; t < 3; ++t) {
-                float mn = brick_bt(a, r, Lc[ax], g0, d, t, 0), mx = mn;
-                for (int k = 1; k <= B; ++k) {
-                    const float b = brick_bt(a, r, Lc[ax], g0, d, t, k);
-                    mn = fminf(mn, b);
-                    mx = fmaxf(mx, b);
-                }
-                out[ROW_RA * (D + 1) + (d * 3 + t) * 2] = mn;
-                out[ROW_RA * (D + 1) + (d * 3 + t) * 2 + 1] = mx;
+            float4 mn = brick_bt(a, r, Lc[ax], g0, d, 0), mx = mn;
+            for (int k = 1; k <= B; ++k) {
+                const float4 b = brick_bt(a, r, Lc[ax], g0, d, k);
+                mn.x = fminf(mn.x, b.x); mn.y = fminf(mn.y, b.y); mn.z = fminf(mn.z, b.z);
+                mx.x = fmaxf(mx.x, b.x); mx.y = fmaxf(mx.y, b.y); mx.z = fmaxf(mx.z, b.z);
             }
+            float* ra = out + ROW_RA * (D + 1) + d * 6;
+            ra[0] = mn.x; ra[1] = mx.x; ra[2] = mn.y; ra[3] = mx.y; ra[4] = mn.z; ra[5] = mx.z;
         } else {
             int wlo, ext;
             bool cross;
@@ -1074,7 +984,7 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
             // (the lower-face corner owns its own cell) is within one cell of N, else 0
             auto term = [&](int N, int k) {
                 const int Va = (k == 0 && c0 == 0) ? (g0 >> sh) : ((g0 + k - 1) >> sh);
-                return (N < Va - 1 || N > Va + 1) ? 0.f : lattice_basis(a, d, N, g0 + k);
+                return (N < Va - 1 || N > Va + 1) ? 0.f : lattice_entry(a, d, Va, g0 + k - (Va << sh), N - Va + 1);
             };
             if (!super && (1 << sh) >= B) {
                 float4* pw = reinterpret_cast<float4*>(out + d * PROW);
@@ -1104,8 +1014,18 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
     }
 }
 
-// Per root: x of the 27 neighbours of each ancestor (0: no neighbour; xl, for the evaluation),
-// and the leaf's ancestor polynomial (anc, for the bounds).  Every ancestor function is one
+// per root: its node and its ancestors, by depth (their x27 rows hold the neighbours' x of each level)
+__global__ void k_root_up(NodeArrays nd, const VRoot* __restrict__ roots, int nroots, int* __restrict__ up) {
+    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < nroots; k += (i64)gridDim.x * blockDim.x) {
+        int node = roots[k].node;
+        for (int l = roots[k].depth; l >= 0; --l) {
+            up[k * BR_LEVELS + l] = node;
+            node = nd.parent[node];
+        }
+    }
+}
+
+// Per root: the leaf's ancestor polynomial (anc, for the bounds).  Every ancestor function is one
 // quadratic piece per axis over the leaf (its knots are multiples of its cell width, and the leaf
 // lies in one such cell), so the ancestors' sum is one tri-quadratic over the leaf, kept in
 // Bernstein form over t = (corner - leaf origin) / S per axis:
@@ -1113,15 +1033,16 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
 // (lane k computes coefficient k, per level as sum_jx bx_i (sum_jy by_j (sum_jz x bz_l))), then
 // S3 = sum |x| Mx My Mz, the number of terms and FIT = sum |x| (dx My Mz + Mx dy Mz + Mx My dz)
 // (d the fits' residuals, M = bern_m), which bounds |sum x (vx vy vz - Qx Qy Qz)| at every corner.
-// Single-brick leaves whose corners change sign are never bounded: their polynomial is left 0.
+// Single-brick leaves whose corners change sign are never bounded: their entry is not written.
+// The x of the levels are rows of x27, which siblings and cousins share in L2; the copy of them per
+// root that the evaluation read before (1,728 bytes, 3.6 GB written and read at 4 M points, maxDepth
+// 11) was most of this kernel: 11.3 ms.
 constexpr int XL_WARPS = 4;
 __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots, const int* __restrict__ has_tri,
-                                                            float* __restrict__ xl, float* __restrict__ anc) {
-    // one warp per root: lane 0 walks up the leaf's ancestors once; the warp writes the 27
-    // neighbours' x of every level, fits the ancestor functions of all levels (lanes over
-    // level, axis, offset), then forms the polynomial
-    __shared__ int sanc[XL_WARPS][BR_LEVELS];
-    __shared__ float sx[XL_WARPS][BR_LEVELS * 27];
+                                                             const int* __restrict__ up, float* __restrict__ anc) {
+    // one warp per root: it stages the levels' x, fits the ancestor functions of all levels (lanes
+    // over level and axis), then forms the polynomial
+    __shared__ float4 sx[XL_WARPS][BR_LEVELS * 7];
     __shared__ float4 sfit[XL_WARPS][BR_LEVELS * 9];   // [level][axis][t]
     const NodeArrays& nd = v.e.nd;
     const int D = v.e.D;
@@ -1131,37 +1052,24 @@ __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots,
     for (i64 ri = warp; ri < nroots; ri += nwarps) {
         const VRoot R = v.roots[ri];
         const int r = R.depth, S = 1 << (D - r);
+        if (S <= BR && has_tri[R.node]) continue;
         __syncwarp();   // the previous root's readers are done
-        if (lane == 0) {
-            int node = R.node;
-            for (int q = r; q >= 0; --q) {
-                sanc[w][q] = node;
-                if (q > 0) node = nd.parent[node];
-            }
-        }
-        __syncwarp();
-        for (int t = lane; t < BR_LEVELS * 27; t += 32) {
-            const int l = t / 27, j = t % 27;
-            const float x = (l <= r) ? x_or_zero(v.e, nd.neigh[(i64)j * nd.M + sanc[w][l]]) : 0.f;
-            xl[ri * BR_LEVELS * 27 + t] = x;
-            sx[w][t] = x;
-        }
-        const bool poly = !(S <= BR && has_tri[R.node]);
+        for (int t = lane; t < 7 * (r + 1); t += 32)
+            sx[w][t] = reinterpret_cast<const float4*>(v.e.x27 + (i64)up[ri * BR_LEVELS + t / 7] * X27_STRIDE)[t % 7];
         int Lc[3];
         key_coords(nd.key[R.node], r, D, Lc);
-        if (poly) {
-            for (int f = lane; f < 9 * (r + 1); f += 32) {
-                const int l = f / 9, ax = (f % 9) / 3, t = f % 3, g0 = Lc[ax] * S;
-                sfit[w][f] = bern_fit([&](int k) { return brick_bt(v.e, r, Lc[ax], g0, l, t, k); }, S);
-            }
+        for (int f = lane; f < 9 * (r + 1); f += 32) {
+            const int l = f / 9, ax = (f % 9) / 3, t = f % 3, g0 = Lc[ax] * S, c = Lc[ax] >> (r - l);
+            const int k0 = g0 - (c << (D - l));
+            sfit[w][f] = bern_fit([&](int k) { return lattice_entry(v.e, l, c, k0 + k, t); }, S);
         }
         __syncwarp();
         float c = 0.f, s3 = 0.f, fit = 0.f;
         int cnt = 0;
-        if (poly && lane < 27) {
+        if (lane < 27) {
             const int i = lane / 9, j = (lane / 3) % 3, lz = lane % 3;
             for (int l = 0; l <= r; ++l) {
-                const float* xs = sx[w] + 27 * l;
+                const float* xs = reinterpret_cast<const float*>(sx[w] + 7 * l);
                 const float4* F = sfit[w] + 9 * l;
                 float acc = 0.f;
                 for (int jx = 0; jx < 3; ++jx) {
@@ -1359,7 +1267,7 @@ __device__ __forceinline__ void shell_terms(const VArgs& v, int L, int r, const 
 // the row tables (away from the leaf's boundary).  ssign = 1, -1 or 0.
 __global__ void __launch_bounds__(256) k_super_bound(VArgs v, DepthLayout dl,
                                                      const i64* __restrict__ srow_prefix,
-                                                     const float* __restrict__ srows, const float* __restrict__ xl_all,
+                                                     const float* __restrict__ srows, const int* __restrict__ up_all,
                                                      i64 nsuper, signed char* __restrict__ ssign) {
     __shared__ int s_anchor[256 / 32][SHELL_ANCHORS];
     const EvalArgs& a = v.e;
@@ -1383,11 +1291,10 @@ __global__ void __launch_bounds__(256) k_super_bound(VArgs v, DepthLayout dl,
         const float* row[3];
         for (int ax = 0; ax < 3; ++ax)
             row[ax] = srows + (srow_prefix[lo] + (i64)ax * ns + sb[ax]) * (i64)(ROW_PER_DEPTH * (D + 1));
-        const float* xl = xl_all + (i64)lo * BR_LEVELS * 27;
         float flo = 0.f, fhi = 0.f, amax = 0.f;
         int cnt = 0;
         bool decided = true;
-        ancestor_bound(xl, row, r, D, lane, flo, fhi, amax, cnt);
+        ancestor_bound(a, up_all + (i64)lo * BR_LEVELS, row, r, D, lane, flo, fhi, amax, cnt);
         for (int d = r + 1; d <= D && decided; ++d) {
             int wlo[3], ext[3];
             bool cross = false;
@@ -1831,16 +1738,12 @@ __global__ void __launch_bounds__(NT) k_brick_eval(VArgs v, BrickIndex bix, cons
             if (threadIdx.x == 0) atomicAdd(nforeign + 1, 1ull);
             continue;
         }
-        float* xl_s = reinterpret_cast<float*>(sm.xL);
-        for (int e = threadIdx.x; e < 28 * (r + 1); e += blockDim.x) {
-            const int l = e / 28, j = e % 28;
-            xl_s[e] = (j < 27) ? bix.xl[(i64)lb.root * BR_LEVELS * 27 + 27 * l + j] : 0.f;
-        }
-        float* bt_s = reinterpret_cast<float*>(sm.Bt);
-        for (int e = threadIdx.x; e < 3 * 4 * K1 * (D + 1); e += blockDim.x) {
-            const int ax = e / (4 * K1 * (D + 1)), q = e % (4 * K1 * (D + 1));
-            const int d = q / (4 * K1), k = (q % (4 * K1)) / 4, t = q % 4;
-            bt_s[ax * BR_LEVELS * 4 * K1 + q] = (k <= E) ? brick_bt(a, r, Lc[ax], g0[ax], d, t, k) : 0.f;
+        for (int e = threadIdx.x; e < 7 * (r + 1); e += blockDim.x)
+            sm.xL[e] = reinterpret_cast<const float4*>(a.x27 + (i64)bix.up[(i64)lb.root * BR_LEVELS + e / 7] * X27_STRIDE)[e % 7];
+        for (int e = threadIdx.x; e < 3 * K1 * (D + 1); e += blockDim.x) {
+            const int d = e / (3 * K1), ax = (e % (3 * K1)) / K1, k = e % K1;
+            sm.Bt[(ax * BR_LEVELS + d) * K1 + k] =
+                (k <= E) ? brick_bt(a, r, Lc[ax], g0[ax], d, k) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         for (int t = threadIdx.x; t < total; t += blockDim.x) sm.Xw[t] = 0.f;
         if (fposs && threadIdx.x < 27) {
@@ -2263,11 +2166,12 @@ void stage_mesh(Ctx& c) {
     const int kx = c.kbegin("mesh_tables", 0.0);
     float* x27 = build_x27(c, lo);
     EvalArgs ea{c.nodes, D, c.basis, c.x, x27, x27 ? lo : 0, nullptr, c.params.stable_basis};
-    float* lb = nullptr;
+    float4* lb = nullptr;
     {
-        const i64 total = lattice_basis_offset(D, D + 1);
-        lb = dalloc<float>(total, s);
-        k_lattice_basis<<<grid_for(total, 256), 256, 0, s>>>(c.basis, D, total, lb, c.params.stable_basis);
+        const i64 total = lattice_offset(D, D + 1);
+        lb = dalloc<float4>(total, s);
+        k_lattice_basis<<<grid_for(4 * total, 256), 256, 0, s>>>(c.basis, D, total, reinterpret_cast<float*>(lb),
+                                                                 c.params.stable_basis);
         CK_LAUNCH();
         ea.lb = lb;
     }
@@ -2470,9 +2374,9 @@ void stage_mesh(Ctx& c) {
         i64* dspre = dpre + 2 * (nr + 1);
         i64* dsrpre = dpre + 3 * (nr + 1);
         float* rows = dalloc<float>(nrows * PROW * (D + 1), s);
-        float* xl = dalloc<float>((i64)nr * BR_LEVELS * 27, s);
+        int* up = dalloc<int>((i64)nr * BR_LEVELS, s);
         float* anc = dalloc<float>((i64)nr * ANC_STRIDE, s);
-        BrickIndex bix{dbpre, drpre, nr, rows, xl, anc, {}};
+        BrickIndex bix{dbpre, drpre, nr, rows, up, anc, {}};
         for (int d = 0; d <= D; ++d) {
             bix.dl.first[d] = layout.first[d];
             bix.dl.lg[d] = std::max(D - d - 3, 0);          // bricks per edge 2^(D-d) / min(2^(D-d), 8)
@@ -2492,7 +2396,9 @@ void stage_mesh(Ctx& c) {
             k_brick_rows<<<grid_for(nsrows * (D + 1), 128), 128, 0, s>>>(va, bix.dl, nsrows, 1, c.d_has_tri, srows);
             CK_LAUNCH();
         }
-        k_brick_xl<<<grid_for((i64)nr * 32, 32 * XL_WARPS), 32 * XL_WARPS, 0, s>>>(va, nr, c.d_has_tri, xl, anc);
+        k_root_up<<<grid_for(nr, 256), 256, 0, s>>>(nd, droots, nr, up);
+        CK_LAUNCH();
+        k_brick_xl<<<grid_for((i64)nr * 32, 32 * XL_WARPS), 32 * XL_WARPS, 0, s>>>(va, nr, c.d_has_tri, up, anc);
         CK_LAUNCH();
         c.kend(kr);
         unsigned char* culled = dalloc<unsigned char>(nbricks, s);
@@ -2508,7 +2414,7 @@ void stage_mesh(Ctx& c) {
             ssign = dalloc<signed char>(nsuper, s);
             const int ksb = c.kbegin("super_bound", (double)nsrows * (6 + 2 * BR_WEXT) * (D + 1) * 4 +
                                                         (double)nr * BR_LEVELS * 27 * 4 + (double)nsuper);
-            k_super_bound<<<grid_for(nsuper * 32, 256, (i64)c.sms * 8), 256, 0, s>>>(va, bix.dl, dsrpre, srows, xl,
+            k_super_bound<<<grid_for(nsuper * 32, 256, (i64)c.sms * 8), 256, 0, s>>>(va, bix.dl, dsrpre, srows, up,
                                                                                     nsuper, ssign);
             CK_LAUNCH();
             c.kend(ksb);
@@ -2637,7 +2543,7 @@ void stage_mesh(Ctx& c) {
         dfree(root_of, s);
         dfree(dpre, s);
         dfree(rows, s);
-        dfree(xl, s);
+        dfree(up, s);
         vc.live = live;
         vc.nlive = nlive;
         vc.lat = lat_brick;
