@@ -683,13 +683,12 @@ __device__ __forceinline__ u64 cell_key_D(const int c[3], int D) { return coords
 constexpr int BR = 8;              // largest brick edge (cells); corners per axis up to BR+1
 constexpr int BR1 = BR + 1;
 constexpr int BR_CORNERS = BR1 * BR1 * BR1;
-constexpr int BR_BLOCK = 128;
 constexpr int BR_LEVELS = 16;      // depths 0..15
-constexpr int BR_WEXT = BR + 4;    // window edge at the finest depth, with the extra upper cell
-// window cells over all virtual depths of a brick whose first corner is a
-// multiple of its edge B <= 8, with the extra upper cell per axis (bricks
-// with foreign corners): at most 12^3 + 8^3 + 6^3 + 12 * 5^3 = 3956
-constexpr int BR_XW = 3968;
+constexpr int BR_WEXT = BR + 4;    // window cells per axis in the row tables (at most 11 are used)
+// window cells over all virtual depths of a brick of edge 8 whose first corner is a multiple of 8: per
+// axis the owner cells of its corners (8 cells and the one below) and one more to each side, 11, 7 and 5
+// cells at the finest depths and 4 at the others: 11^3 + 7^3 + 5^3 + 12 * 4^3 = 2567
+constexpr int BR_XW = 2568;
 // super-brick row table: RA (6 per depth), RW (24 per depth)
 constexpr int ROW_RA = 0, ROW_RW = 6, ROW_PER_DEPTH = 30;
 // brick row table: 24 floats per depth d > r (the ancestors, d <= r, are one polynomial per leaf)
@@ -838,21 +837,16 @@ __device__ __forceinline__ void ancestor_bound(const EvalArgs& a, const int* up,
 // leaf can have the least key only if one offset is -1 (Morton order is
 // monotone per axis).  So: only if such a neighbour is a root of the same batch
 // (batch_member's rule)
-__device__ __forceinline__ bool brick_foreign_possible(const VArgs& v, const VRoot& R, const int b[3], int nb) {
-    if (R.depth < 3 || (b[0] && b[1] && b[2])) return false;
-    const NodeArrays& nd = v.e.nd;
-    for (int j = 0; j < 27; ++j) {
-        const int off[3] = {j / 9 - 1, (j / 3) % 3 - 1, j % 3 - 1};
-        bool ok = false, allowed = true;
-        for (int ax = 0; ax < 3; ++ax) {
-            if (off[ax] == -1) { ok = true; if (b[ax] != 0) allowed = false; }
-            if (off[ax] == 1 && b[ax] != nb - 1) allowed = false;
-        }
-        if (!ok || !allowed) continue;
-        const int n = nd.neigh[(i64)j * nd.M + R.node];
-        if (n != -1 && v.batch_root_flag[n] == R.batch) return true;
+// (the test for the neighbour at offset j, given that it is such a root)
+__device__ __forceinline__ bool foreign_neighbour(int j, const int b[3], int nb) {
+    const int off[3] = {j / 9 - 1, (j / 3) % 3 - 1, j % 3 - 1};
+    bool lower = false, allowed = true;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        if (off[ax] == -1) { lower = true; if (b[ax] != 0) allowed = false; }
+        if (off[ax] == 1 && b[ax] != nb - 1) allowed = false;
     }
-    return false;
+    return lower && allowed;
 }
 
 // window of depth d around a brick (edge B) along one axis: origin and extent
@@ -1036,7 +1030,8 @@ __global__ void k_root_up(NodeArrays nd, const VRoot* __restrict__ roots, int nr
 // Single-brick leaves whose corners change sign are never bounded: their entry is not written.
 // The x of the levels are rows of x27, which siblings and cousins share in L2; the copy of them per
 // root that the evaluation read before (1,728 bytes, 3.6 GB written and read at 4 M points, maxDepth
-// 11) was most of this kernel: 11.3 ms.
+// 11) was half of this kernel (11.3 -> 6.1 ms without it); the nine coefficients a lane needs of a level
+// read as scalars and not picked from vectors in the inner loop take it to 2.1 ms.
 constexpr int XL_WARPS = 4;
 __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots, const int* __restrict__ has_tri,
                                                              const int* __restrict__ up, float* __restrict__ anc) {
@@ -1044,11 +1039,13 @@ __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots,
     // over level and axis), then forms the polynomial
     __shared__ float4 sx[XL_WARPS][BR_LEVELS * 7];
     __shared__ float4 sfit[XL_WARPS][BR_LEVELS * 9];   // [level][axis][t]
+    __shared__ float sm_[XL_WARPS][BR_LEVELS * 9];     // their bern_m
     const NodeArrays& nd = v.e.nd;
     const int D = v.e.D;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const i64 warp = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
+    const int i = min(lane / 9, 2), j = (lane / 3) % 3, lz = lane % 3;
     for (i64 ri = warp; ri < nroots; ri += nwarps) {
         const VRoot R = v.roots[ri];
         const int r = R.depth, S = 1 << (D - r);
@@ -1060,33 +1057,53 @@ __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots,
         key_coords(nd.key[R.node], r, D, Lc);
         for (int f = lane; f < 9 * (r + 1); f += 32) {
             const int l = f / 9, ax = (f % 9) / 3, t = f % 3, g0 = Lc[ax] * S, c = Lc[ax] >> (r - l);
-            const int k0 = g0 - (c << (D - l));
-            sfit[w][f] = bern_fit([&](int k) { return lattice_entry(v.e, l, c, k0 + k, t); }, S);
+            const float* tab = reinterpret_cast<const float*>(v.e.lb + lattice_offset(D, l) +
+                                                              (i64)c * ((1 << (D - l)) + 1) + (g0 - (c << (D - l)))) + t;
+            const float4 b = bern_fit([&](int k) { return tab[4 * k]; }, S);
+            sfit[w][f] = b;
+            sm_[w][f] = bern_m(b);
         }
         __syncwarp();
         float c = 0.f, s3 = 0.f, fit = 0.f;
         int cnt = 0;
         if (lane < 27) {
-            const int i = lane / 9, j = (lane / 3) % 3, lz = lane % 3;
-            for (int l = 0; l <= r; ++l) {
-                const float* xs = reinterpret_cast<const float*>(sx[w] + 7 * l);
-                const float4* F = sfit[w] + 9 * l;
+            // the lane's coefficient of each function is one scalar: nine loads a level
+            const float* F = reinterpret_cast<const float*>(sfit[w]);
+            const float* Mf = sm_[w];
+            for (int l = 0; l <= r; ++l, F += 36, Mf += 9) {
+                float xs[28];
+#pragma unroll
+                for (int q = 0; q < 7; ++q) {
+                    const float4 f = sx[w][7 * l + q];
+                    xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
+                }
+                float bx[3], by[3], bz[3];
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    bx[t] = F[4 * t + i];
+                    by[t] = F[4 * (3 + t) + j];
+                    bz[t] = F[4 * (6 + t) + lz];
+                }
                 float acc = 0.f;
+#pragma unroll
                 for (int jx = 0; jx < 3; ++jx) {
                     float ys = 0.f;
+#pragma unroll
                     for (int jy = 0; jy < 3; ++jy) {
                         float zs = 0.f;
-                        for (int jz = 0; jz < 3; ++jz) zs = fmaf(xs[9 * jx + 3 * jy + jz], f4_at(F[6 + jz], lz), zs);
-                        ys = fmaf(f4_at(F[3 + jy], j), zs, ys);
+#pragma unroll
+                        for (int jz = 0; jz < 3; ++jz) zs = fmaf(xs[9 * jx + 3 * jy + jz], bz[jz], zs);
+                        ys = fmaf(by[jy], zs, ys);
                     }
-                    acc = fmaf(f4_at(F[jx], i), ys, acc);
+                    acc = fmaf(bx[jx], ys, acc);
                 }
                 c += acc;
-                const float ax = fabsf(xs[lane]);   // the neighbour at offset (i, j, lz)
+                const float ax = fabsf(reinterpret_cast<const float*>(sx[w] + 7 * l)[lane]);   // the neighbour at offset (i, j, lz)
                 if (ax != 0.f) {
-                    const float Mx = bern_m(F[i]), My = bern_m(F[3 + j]), Mz = bern_m(F[6 + lz]);
+                    const float Mx = Mf[i], My = Mf[3 + j], Mz = Mf[6 + lz];
+                    const float dx = F[4 * i + 3], dy = F[4 * (3 + j) + 3], dz = F[4 * (6 + lz) + 3];
                     s3 += ax * Mx * My * Mz;
-                    fit += ax * (F[i].w * My * Mz + Mx * F[3 + j].w * Mz + Mx * My * F[6 + lz].w);
+                    fit += ax * (dx * My * Mz + Mx * dy * Mz + Mx * My * dz);
                     ++cnt;
                 }
             }
@@ -1101,36 +1118,36 @@ __global__ void __launch_bounds__(32 * XL_WARPS) k_brick_xl(VArgs v, int nroots,
     }
 }
 
-// lower_face_owner with the batch membership of the leaf's 27 neighbours looked up once
-// (member[j]: batch_member's answer for the leaf at offset j, 13 = the leaf itself)
-__device__ __forceinline__ int lower_face_owner_cached(const VArgs& v, const VRoot& R, const int Lc[3], const int qc[3],
-                                                       const int* member, int oc[3]) {
-    const int D = v.e.D, sh = D - R.depth, lim = 1 << D;
+// Owner of corner qc of leaf R: the cell with the least key among the 8 around the corner that belong to
+// the leaf or to another root of its batch (member[j]: batch_member's answer for the neighbour at offset
+// j, 13 = the leaf itself).  The keys are the OR of one spread coordinate per axis, two of each.
+__device__ __forceinline__ int corner_owner_cell(int D, int r, const int Lc[3], const int qc[3], const int* member,
+                                                 int oc[3]) {
+    const int sh = D - r, lim = 1 << D;
+    u64 key[3][2];
+    int off[3][2];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = qc[ax] - e;
+            key[ax][e] = morton_spread3((uint32_t)max(c, 0)) << (2 - ax);
+            off[ax][e] = (c < 0 || c >= lim) ? -1 : (c >> sh) - Lc[ax] + 1;   // 0..2, or outside the cube
+        }
     u64 best = ~0ull;
-    int own = -1;
+    int own = -1, eb = 0;
+#pragma unroll
     for (int eo = 0; eo < 8; ++eo) {
-        const int cell[3] = {qc[0] - (eo & 1), qc[1] - ((eo >> 1) & 1), qc[2] - ((eo >> 2) & 1)};
-        if (cell[0] < 0 || cell[1] < 0 || cell[2] < 0 || cell[0] >= lim || cell[1] >= lim || cell[2] >= lim) continue;
-        const int j = 9 * ((cell[0] >> sh) - Lc[0] + 1) + 3 * ((cell[1] >> sh) - Lc[1] + 1) + ((cell[2] >> sh) - Lc[2] + 1);
-        const int m = member[j];
-        if (m < 0) continue;
-        const u64 kk = cell_key_D(cell, D);
-        if (kk < best) { best = kk; own = m; oc[0] = cell[0]; oc[1] = cell[1]; oc[2] = cell[2]; }
+        const int ex = eo & 1, ey = (eo >> 1) & 1, ez = eo >> 2;
+        if ((off[0][ex] | off[1][ey] | off[2][ez]) < 0) continue;
+        const int m = member[9 * off[0][ex] + 3 * off[1][ey] + off[2][ez]];
+        const u64 kk = key[0][ex] | key[1][ey] | key[2][ez];
+        if (m >= 0 && kk < best) { best = kk; own = m; eb = eo; }
     }
-    return own;
-}
-
-// owner of a lower-face corner (min key among batch cells sharing it)
-__device__ __forceinline__ int lower_face_owner(const VArgs& v, const VRoot& R, const int Lc[3], const int qc[3],
-                                                int oc[3]) {
-    u64 best = ~0ull;
-    int own = -1;
-    for (int eo = 0; eo < 8; ++eo) {
-        const int cell[3] = {qc[0] - (eo & 1), qc[1] - ((eo >> 1) & 1), qc[2] - ((eo >> 2) & 1)};
-        const int m = batch_member(v, R, Lc, cell);
-        if (m < 0) continue;
-        const u64 kk = cell_key_D(cell, v.e.D);
-        if (kk < best) { best = kk; own = m; oc[0] = cell[0]; oc[1] = cell[1]; oc[2] = cell[2]; }
+    if (own >= 0) {
+        oc[0] = qc[0] - (eb & 1);
+        oc[1] = qc[1] - ((eb >> 1) & 1);
+        oc[2] = qc[2] - (eb >> 2);
     }
     return own;
 }
@@ -1434,6 +1451,9 @@ constexpr int BB_BLOCK = 256;
 // its brick's corners include the leaf's corners, so its bound straddles iso (and a brick left
 // unproven is only evaluated exactly, which changes no value).
 // (4 blocks per SM: 64 registers, no spills; unbounded it takes 104 and halves the resident warps)
+// The launch has up to 256 blocks per SM: bricks differ in cost (skipped, decided, deep windows), and
+// with 8 blocks per SM striding over all of them the last blocks ran alone (22.0 -> 15.9 ms at 4 M points,
+// 2.41 -> 1.90 on the 1M torus).
 __global__ void __launch_bounds__(BB_BLOCK, 4) k_brick_bound(VArgs v, BrickIndex bix, i64 first, i64 nbricks,
                                                           const i64* __restrict__ sprefix,
                                                           const signed char* __restrict__ ssign,
@@ -1598,97 +1618,6 @@ __global__ void k_root_of(const VRoot* __restrict__ roots, int nroots, int* __re
         root_of[roots[k].node] = k;
 }
 
-// shared memory of one brick of edge at most EB: bricks of edge 8 (leaves with
-// lattice edge >= 8) and of edge 2 or 4 (the smallest leaves) are evaluated by
-// two instances.  Window bound for EB = 4 with the extra upper cell: 8^3 + 6^3.
-template <int EB>
-struct BrickShared {
-    static constexpr int K1 = EB + 1;         // corners per axis
-    // edge 2 (leaves one depth above the finest): one virtual depth, at most 5^3 window cells
-    static constexpr int XW = (EB == BR) ? BR_XW : (EB == 4 ? 728 : 128);
-    float4 Bt[3 * BR_LEVELS * K1];            // [axis][depth][k], the four t of a corner in one vector
-    float4 xL[BR_LEVELS * 7];                 // neighbours of the leaf and its ancestors (0: none), 27 + 1 per level
-    float Xw[XW];                             // window coefficients, virtual depths (0: none or inside the leaf)
-    int wlo[BR_LEVELS][3];                    // window origin (cell coordinates at that depth)
-    int wext[BR_LEVELS][3];
-    int woff[BR_LEVELS];                      // offset into Xw, -1 when no corner reaches outside the leaf
-    int member[27];                           // batch_member of the leaf at each neighbour offset
-};
-template <int EB>
-__device__ __forceinline__ float4 bt_at(const BrickShared<EB>& sm, int ax, int d, int k) {
-    return sm.Bt[(ax * BR_LEVELS + d) * BrickShared<EB>::K1 + k];
-}
-
-// virtual-depth part of the value of corner qc (brick-local kk) whose owner
-// cell is oc -- in the brick's leaf or, for a foreign corner, in the leaf of
-// the batch that owns it -- from the shared window, in the order of
-// virtual_corner_value.  At depth d the owner cell is oc >> sh, the tabulated
-// one (qc - 1) >> sh, so the basis row is taken t + ((oc >> sh) - ((qc-1) >> sh))
-// (0 or 1).  Terms that virtual_corner_value skips (levels whose 3x3x3 block
-// lies inside the owner's leaf, cells inside either leaf, absent nodes) read 0
-// here, and adding a zero product leaves the sum unchanged, so the value is the
-// same.
-template <int EB>
-__device__ __forceinline__ float brick_virtual(const BrickShared<EB>& sm, int D, int r, const int Lc[3], const int oc[3],
-                                               const int qc[3], const int kk[3]) {
-    float val = 0.f;
-    for (int d = D; d > r; --d) {
-        const int off = sm.woff[d];
-        if (off < 0) continue;
-        const int sh = D - d;
-        const int V[3] = {oc[0] >> sh, oc[1] >> sh, oc[2] >> sh};
-        // a 3x3x3 block inside the leaf reads only zeros: its terms leave the sum unchanged
-        const int span = 1 << (d - r);
-        bool inside = true;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const int lo = Lc[ax] << (d - r);
-            inside &= (V[ax] - 1 >= lo) && (V[ax] + 1 < lo + span);
-        }
-        if (inside) continue;
-        float bv[3][3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const bool toff = V[ax] != ((qc[ax] - 1) >> sh);   // the owner cell is the tabulated one or the next
-            const float4 b = bt_at(sm, ax, d, kk[ax]);
-            bv[ax][0] = toff ? b.y : b.x;
-            bv[ax][1] = toff ? b.z : b.y;
-            bv[ax][2] = toff ? b.w : b.z;
-        }
-        const int e1 = sm.wext[d][1], e2 = sm.wext[d][2];
-        const float* xw = sm.Xw + off + ((V[0] - 1 - sm.wlo[d][0]) * e1 + (V[1] - 1 - sm.wlo[d][1])) * e2 +
-                          (V[2] - 1 - sm.wlo[d][2]);
-#pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            const int jx = j / 9, jy = (j / 3) % 3, jz = j % 3;
-            val = fmaf(xw[(jx * e1 + jy) * e2 + jz] * bv[0][jx] * bv[1][jy], bv[2][jz], val);
-        }
-    }
-    return val;
-}
-
-// the brick's leaf itself and its real ancestors (walk_up with absent neighbours as 0)
-template <int EB>
-__device__ __forceinline__ float brick_leaf_levels(const BrickShared<EB>& sm, int r, const int kk[3], float val) {
-    for (int l = r; l >= 0; --l) {
-        float xs[28];
-#pragma unroll
-        for (int q = 0; q < 7; ++q) {
-            const float4 v4 = sm.xL[7 * l + q];
-            xs[4 * q] = v4.x; xs[4 * q + 1] = v4.y; xs[4 * q + 2] = v4.z; xs[4 * q + 3] = v4.w;
-        }
-        float bv[3][3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const float4 b = bt_at(sm, ax, l, kk[ax]);
-            bv[ax][0] = b.x; bv[ax][1] = b.y; bv[ax][2] = b.z;
-        }
-#pragma unroll
-        for (int j = 0; j < 27; ++j) val = fmaf(xs[j] * bv[0][j / 9] * bv[1][(j / 3) % 3], bv[2][j % 3], val);
-    }
-    return val;
-}
-
 // live brick: root, brick coordinates; first corner value and first cell
 struct LiveBrick {
     int root;
@@ -1696,118 +1625,394 @@ struct LiveBrick {
     i64 lat;
     i64 cell;
 };
+// a corner of live brick li owned by another leaf of the batch, and the corner of that leaf's brick which
+// is the same point: brick << 10 | corner
+struct ForeignCorner {
+    int li;
+    int e;
+    u64 src;
+};
+__device__ __forceinline__ u64 foreign_src(int D, int r, int E, const DepthLayout& dl, int owner_root, const int oc[3],
+                                           const int qc[3]) {
+    const int sh = D - r, lg = dl.lg[r], E1 = E + 1;
+    int b[3], k[3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        const int l0 = (oc[ax] >> sh) << sh;         // the owner leaf's first cell
+        b[ax] = (oc[ax] - l0) / E;
+        k[ax] = qc[ax] - (l0 + b[ax] * E);
+    }
+    const i64 brick = dl.boff[r] + ((i64)(owner_root - dl.first[r]) << (3 * lg)) +
+                      (((((i64)b[0]) << lg) + b[1]) << lg) + b[2];
+    return ((u64)brick << 10) | (u64)((k[0] * E1 + k[1]) * E1 + k[2]);
+}
+// append the lanes' foreign corners (a whole warp calls): one atomic per warp
+__device__ __forceinline__ void push_foreign(bool isf, int li, int e, u64 src, unsigned long long* nforeign,
+                                             ForeignCorner* foreign, i64 cap) {
+    const unsigned fm = __ballot_sync(0xffffffffu, isf);
+    if (!fm) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(fm) - 1;
+    unsigned long long base = 0;
+    if (lane == leader) base = atomicAdd(nforeign, (unsigned long long)__popc(fm));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (isf) {
+        const unsigned long long f = base + (unsigned long long)__popc(fm & ((1u << lane) - 1u));
+        if ((i64)f < cap) foreign[f] = ForeignCorner{li, e, src};
+    }
+}
 
-// one block per live brick: exact corner values into the brick's (B+1)^3 slot
-template <int EB, int NT>
-__global__ void __launch_bounds__(NT) k_brick_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
+// Values of a live brick's corners, the same bit for bit as virtual_corner_value's: for every level, the
+// 27 terms in order, each fma((x bx) by, bz, value).
+//
+// A thread takes a column of corners along z.  A term's (x bx) by is the same for all corners of the
+// column that read the same x, so a level costs a column 54 products (the ancestors, whose 27 x are the
+// leaf's) or 18 per window cell along z (the virtual depths) and then 27 FMAs per corner, where a thread
+// per corner spends 54 products and 27 FMAs on each.  The values of the column are independent chains.
+// On the virtual depths the column slides along z: the products of the three z neighbours stay in
+// registers and move by one when the owner cell does.  Terms that virtual_corner_value skips (levels
+// whose 3x3x3 block lies inside the owner's leaf, cells inside the leaf, absent nodes) read 0 here,
+// and adding a zero product leaves the sum unchanged.
+template <int E>
+struct BrickShared {
+    static constexpr int K1 = E + 1;          // corners per axis
+    // window cells over the virtual depths and in the largest window above the finest depth; edge 4: the
+    // leaf itself, 6^3 + 4^3
+    static constexpr int XW = (E == BR) ? BR_XW : 280, PW3 = (E == BR) ? 343 : 64;
+    float4 Bt[3 * BR_LEVELS * K1];            // [axis][depth][k], the four t of a corner in one vector
+    float4 xL[BR_LEVELS * 7];                 // neighbours of the leaf and its ancestors (0: none), 27 + 1 per level
+    float Xw[XW];                             // window coefficients, virtual depths (0: none or inside the leaf)
+    int child[2][PW3];                        // first child of the window cells of the depth above (-1: none)
+    int wlo[BR_LEVELS][3];                    // window origin (cell coordinates at that depth)
+    int wext[BR_LEVELS][3];
+    int woff[BR_LEVELS];                      // offset into Xw, -1 when no corner reaches outside the leaf
+    int member[27];                           // batch_member of the leaf at each neighbour offset
+    int total, fposs;
+};
+
+// one level of a column whose corners all read the 27 x in xs: val[kz] += the 27 terms
+template <int K1>
+__device__ __forceinline__ void column_level(const float xs[28], const float4& bx, const float4& by, const float4* bz,
+                                             float val[K1]) {
+    const float x3[3] = {bx.x, bx.y, bx.z}, y3[3] = {by.x, by.y, by.z};
+    float p[27];
+#pragma unroll
+    for (int j = 0; j < 27; ++j) p[j] = xs[j] * x3[j / 9] * y3[(j / 3) % 3];
+#pragma unroll
+    for (int kz = 0; kz < K1; ++kz) {
+        const float4 b = bz[kz];
+        const float z3[3] = {b.x, b.y, b.z};
+        float v = val[kz];
+#pragma unroll
+        for (int j = 0; j < 27; ++j) v = fmaf(p[j], z3[j % 3], v);
+        val[kz] = v;
+    }
+}
+
+// Bricks of edge 8 (96 threads, 81 columns) and 4 (a warp, 25 columns).  4 M points, maxDepth 11: 109 K
+// bricks of edge 8 in 3.8 ms (7.9 with a thread per corner and a descent per window cell), 0.4 M of edge 4
+// in 3.2.  At most 85 registers, so that 7 blocks share an SM: with 128 (5 blocks) the edge-8 bricks take
+// 8.7 ms, set-up and window loads waiting.
+template <int E, int NT>
+__global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
                                                    const LiveBrick* __restrict__ live, const int* __restrict__ list,
                                                    i64 nlist, float* __restrict__ blat,
                                                    unsigned long long* __restrict__ nforeign,
-                                                   int2* __restrict__ foreign, i64 foreign_cap) {
-    __shared__ BrickShared<EB> sm;
-    constexpr int K1 = BrickShared<EB>::K1;
+                                                   ForeignCorner* __restrict__ foreign, i64 foreign_cap) {
+    __shared__ BrickShared<E> sm;
+    constexpr int K1 = E + 1;
+    static_assert(K1 * K1 <= NT, "a thread per column");
     const EvalArgs& a = v.e;
     const int D = a.D;
     for (i64 it = blockIdx.x; it < nlist; it += gridDim.x) {
-        const i64 li = list[it];
+        const int li = list[it];
         const LiveBrick lb = live[li];
         const VRoot R = v.roots[lb.root];
-        const int r = R.depth, S = 1 << (D - r), L = R.node, E = brick_edge(D, r), nb = S / E, E1 = E + 1;
+        const int r = R.depth, S = 1 << (D - r), L = R.node, nb = S / E;
         int Lc[3];
         key_coords(a.nd.key[L], r, D, Lc);
         const int g0[3] = {Lc[0] * S + lb.b[0] * E, Lc[1] * S + lb.b[1] * E, Lc[2] * S + lb.b[2] * E};
-        const bool fposs = brick_foreign_possible(v, R, lb.b, nb);
-        __syncthreads();
-        // window layout (every thread sizes it; thread 0 records it), leaf tables, zeroed window
-        int total = 0;
-        for (int d = r + 1; d <= D; ++d) {
-            int wl[3], we[3];
+        __syncthreads();   // the previous brick's readers are done
+        if (threadIdx.x < 32) {
+            // the leaf's neighbours: first children, batch membership (batch_member's rule)
+            const int lane = threadIdx.x;
+            bool fp = false;
+            if (lane < 27) {
+                const int n = a.nd.neigh[(i64)lane * a.nd.M + L];
+                int m = lane == 13 ? L : -1;
+                if (r >= 3 && n != -1 && lane != 13 && v.batch_root_flag[n] == R.batch) {
+                    m = n;
+                    fp = foreign_neighbour(lane, lb.b, nb);
+                }
+                sm.member[lane] = m;
+                sm.child[r & 1][lane] = n == -1 ? -1 : a.nd.child0[n];
+            }
+            fp = __any_sync(0xffffffffu, fp);
+            // window layout, a lane per depth
+            int wl[3] = {0, 0, 0}, we[3] = {0, 0, 0}, size = 0;
             bool cross = false;
-            for (int ax = 0; ax < 3; ++ax) {
-                bool c;
-                window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wl[ax], we[ax], c);
-                cross |= c;
+            if (lane > r && lane <= D) {
+                for (int ax = 0; ax < 3; ++ax) {
+                    bool c;
+                    window_axis(g0[ax], E, Lc[ax], r, lane, D, 0, wl[ax], we[ax], c);
+                    cross |= c;
+                }
+                if (cross) size = we[0] * we[1] * we[2];
             }
-            if (threadIdx.x == 0) {
-                for (int ax = 0; ax < 3; ++ax) { sm.wlo[d][ax] = wl[ax]; sm.wext[d][ax] = we[ax]; }
-                sm.woff[d] = cross ? total : -1;
+            int inc = size;
+            for (int o = 1; o < 16; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
             }
-            if (cross) total += we[0] * we[1] * we[2];
+            if (lane < BR_LEVELS) {
+                for (int ax = 0; ax < 3; ++ax) { sm.wlo[lane][ax] = wl[ax]; sm.wext[lane][ax] = we[ax]; }
+                sm.woff[lane] = cross ? inc - size : -1;
+            }
+            if (lane == BR_LEVELS - 1) sm.total = inc;
+            if (lane == 0) sm.fposs = fp;
         }
-        if (total > BrickShared<EB>::XW) {   // cannot happen for aligned bricks: reported, brick skipped
+        for (int e = threadIdx.x; e < 7 * (r + 1); e += NT)
+            sm.xL[e] = reinterpret_cast<const float4*>(a.x27 + (i64)bix.up[(i64)lb.root * BR_LEVELS + e / 7] * X27_STRIDE)[e % 7];
+        for (int e = threadIdx.x; e < 3 * K1 * (D + 1); e += NT) {
+            const int d = e / (3 * K1), ax = (e % (3 * K1)) / K1, k = e % K1;
+            sm.Bt[(ax * BR_LEVELS + d) * K1 + k] = brick_bt(a, r, Lc[ax], g0[ax], d, k);
+        }
+        __syncthreads();
+        const bool fposs = sm.fposs;
+        if (sm.total > BrickShared<E>::XW) {   // cannot happen for aligned bricks: reported, brick skipped
             if (threadIdx.x == 0) atomicAdd(nforeign + 1, 1ull);
             continue;
         }
-        for (int e = threadIdx.x; e < 7 * (r + 1); e += blockDim.x)
-            sm.xL[e] = reinterpret_cast<const float4*>(a.x27 + (i64)bix.up[(i64)lb.root * BR_LEVELS + e / 7] * X27_STRIDE)[e % 7];
-        for (int e = threadIdx.x; e < 3 * K1 * (D + 1); e += blockDim.x) {
-            const int d = e / (3 * K1), ax = (e % (3 * K1)) / K1, k = e % K1;
-            sm.Bt[(ax * BR_LEVELS + d) * K1 + k] =
-                (k <= E) ? brick_bt(a, r, Lc[ax], g0[ax], d, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        // the windows from the coarsest depth down: a cell's node is the child of its parent, a cell of the
+        // window above (the windows are nested; below depth r, the leaf's 27 neighbours), so a depth costs
+        // a cell one more load instead of a descent from the leaf's neighbour.  The leaf has no children:
+        // cells inside it come out absent.
+        {
+            int plo[3] = {Lc[0] - 1, Lc[1] - 1, Lc[2] - 1}, p1 = 3, p2 = 3;
+            for (int d = r + 1; d <= D; ++d) {
+                const int off = sm.woff[d];
+                if (off < 0) break;            // and so are the finer ones
+                const int wl[3] = {sm.wlo[d][0], sm.wlo[d][1], sm.wlo[d][2]};
+                const int e0 = sm.wext[d][0], e1 = sm.wext[d][1], e2 = sm.wext[d][2], n12 = e1 * e2, ncell = e0 * n12;
+                const float inv12 = 1.0f / (float)n12, inv2 = 1.0f / (float)e2;
+                const int* up = sm.child[(d - 1) & 1];
+                int* down = sm.child[d & 1];
+                for (int t = threadIdx.x; t < ncell; t += NT) {
+                    const int i0 = small_div(t, inv12), rem = t - i0 * n12, i1 = small_div(rem, inv2), i2 = rem - i1 * e2;
+                    const int N[3] = {wl[0] + i0, wl[1] + i1, wl[2] + i2};
+                    const int c0 = up[(((N[0] >> 1) - plo[0]) * p1 + ((N[1] >> 1) - plo[1])) * p2 + ((N[2] >> 1) - plo[2])];
+                    float x = 0.f;
+                    int c = -1;
+                    if (c0 != -1) {
+                        const int node = c0 + (((N[0] & 1) << 2) | ((N[1] & 1) << 1) | (N[2] & 1));
+                        x = a.x[node];
+                        if (d < D) c = a.nd.child0[node];
+                    }
+                    sm.Xw[off + t] = x;
+                    if (d < D) down[t] = c;
+                }
+                plo[0] = wl[0]; plo[1] = wl[1]; plo[2] = wl[2];
+                p1 = e1;
+                p2 = e2;
+                __syncthreads();
+            }
         }
-        for (int t = threadIdx.x; t < total; t += blockDim.x) sm.Xw[t] = 0.f;
-        if (fposs && threadIdx.x < 27) {
-            const int j = threadIdx.x;
-            const int cell[3] = {(Lc[0] + j / 9 - 1) << (D - r), (Lc[1] + (j / 3) % 3 - 1) << (D - r),
-                                 (Lc[2] + j % 3 - 1) << (D - r)};
-            sm.member[j] = batch_member(v, R, Lc, cell);
-        }
-        __syncthreads();
-        // only window cells outside the leaf can hold a real node
-        for (int d = r + 1; d <= D; ++d) {
+        // this thread's column (threads beyond the last column repeat it and store nothing)
+        const bool col = threadIdx.x < K1 * K1;
+        const int ci = col ? threadIdx.x : K1 * K1 - 1, kx = ci / K1, ky = ci % K1;
+        const int qx = g0[0] + kx, qy = g0[1] + ky;
+        // the leaf's lower faces: there a corner's own cell is the one above it
+        const bool lowx = lb.b[0] == 0 && kx == 0, lowy = lb.b[1] == 0 && ky == 0, lowz = lb.b[2] == 0;
+        float val[K1];
+#pragma unroll
+        for (int kz = 0; kz < K1; ++kz) val[kz] = 0.f;
+#pragma unroll 1
+        for (int d = D; d > r; --d) {
             const int off = sm.woff[d];
             if (off < 0) continue;
-            const int span = 1 << (d - r);
-            const int llo[3] = {Lc[0] * span, Lc[1] * span, Lc[2] * span};
-            const int wlo[3] = {sm.wlo[d][0], sm.wlo[d][1], sm.wlo[d][2]};
-            const int ext[3] = {sm.wext[d][0], sm.wext[d][1], sm.wext[d][2]};
-            Box3 bxs[6];
-            const int nbx = outside_boxes(wlo, ext, llo, span, bxs);
-            for (int q = 0; q < nbx; ++q) {
-                const Box3& bx = bxs[q];
-                const int n12 = bx.n[1] * bx.n[2], ncell = bx.n[0] * n12;
-                const float inv12 = 1.0f / (float)n12, inv2 = 1.0f / (float)bx.n[2];
-                for (int t = threadIdx.x; t < ncell; t += blockDim.x) {
-                    const int i0 = small_div(t, inv12), rem = t - i0 * n12, i1 = small_div(rem, inv2),
-                              i2 = rem - i1 * bx.n[2];
-                    const int N[3] = {bx.lo[0] + i0, bx.lo[1] + i1, bx.lo[2] + i2};
-                    const i64 node = shell_node(v, L, r, Lc, d, N);
-                    if (node >= 0)
-                        sm.Xw[off + ((N[0] - wlo[0]) * ext[1] + (N[1] - wlo[1])) * ext[2] + (N[2] - wlo[2])] = a.x[node];
+            const int sh = D - d;
+            const int V0 = (qx - 1 + lowx) >> sh, V1 = (qy - 1 + lowy) >> sh;
+            // the row holds the functions around the cell below the corner: one further on the lower face
+            const float4 fx = sm.Bt[d * K1 + kx], fy = sm.Bt[(BR_LEVELS + d) * K1 + ky];
+            const float x3[3] = {lowx ? fx.y : fx.x, lowx ? fx.z : fx.y, lowx ? fx.w : fx.z};
+            const float y3[3] = {lowy ? fy.y : fy.x, lowy ? fy.z : fy.y, lowy ? fy.w : fy.z};
+            const int e1 = sm.wext[d][1], e2 = sm.wext[d][2];
+            const float* xw = sm.Xw + off + ((V0 - 1 - sm.wlo[d][0]) * e1 + (V1 - 1 - sm.wlo[d][1])) * e2;
+            float p[3][9];                  // (x bx) by of the z neighbours below, at and above the owner cell
+            auto slice = [&](int z, float q[9]) {
+#pragma unroll
+                for (int j = 0; j < 9; ++j) q[j] = xw[((j / 3) * e1 + j % 3) * e2 + z] * x3[j / 3] * y3[j % 3];
+            };
+            int zc = ((g0[2] - 1 + lowz) >> sh) - 1 - sm.wlo[d][2];   // window cell of p[0]
+            slice(zc, p[0]);
+            slice(zc + 1, p[1]);
+            slice(zc + 2, p[2]);
+#pragma unroll
+            for (int kz = 0; kz < K1; ++kz) {
+                const int qz = g0[2] + kz;
+                const int zk = ((qz - 1 + (lowz && kz == 0)) >> sh) - 1 - sm.wlo[d][2];
+                if (kz > 0 && zk != zc) {   // the owner cell moved up by one
+                    zc = zk;
+#pragma unroll
+                    for (int j = 0; j < 9; ++j) { p[0][j] = p[1][j]; p[1][j] = p[2][j]; }
+                    slice(zc + 2, p[2]);
                 }
+                const float4 fz = sm.Bt[(2 * BR_LEVELS + d) * K1 + kz];
+                const bool lz = lowz && kz == 0;
+                const float z3[3] = {lz ? fz.y : fz.x, lz ? fz.z : fz.y, lz ? fz.w : fz.z};
+                float t = val[kz];
+#pragma unroll
+                for (int j = 0; j < 27; ++j) t = fmaf(p[j % 3][j / 3], z3[j % 3], t);
+                val[kz] = t;
             }
         }
-        __syncthreads();
-        float* out = blat + lb.lat;
-        const int ncorner = E1 * E1 * E1;
-        const int lane = threadIdx.x & 31;
-        // the warp's lanes take the same iterations (e = e0 + lane), so the foreign slots are
-        // claimed with one atomic per warp
-        for (int e0 = threadIdx.x - lane; e0 < ncorner; e0 += blockDim.x) {
-            const int e = e0 + lane;
-            const bool valid = e < ncorner;
-            const int kk[3] = {e / (E1 * E1), (e / E1) % E1, e % E1};
-            const int uu = lb.b[0] * E + kk[0], ww = lb.b[1] * E + kk[1], zz = lb.b[2] * E + kk[2];
-            const int qc[3] = {g0[0] + kk[0], g0[1] + kk[1], g0[2] + kk[2]};
-            // owner cell: the cell below the corner on every axis, except on the leaf's lower faces
-            int oc[3] = {qc[0] - 1 + (uu == 0), qc[1] - 1 + (ww == 0), qc[2] - 1 + (zz == 0)};
-            int own = L;
-            if (valid && fposs && (uu == 0 || ww == 0 || zz == 0))
-                own = lower_face_owner_cached(v, R, Lc, qc, sm.member, oc);
-            // owned by another leaf of the batch: filled by k_foreign_fill
-            const bool isf = valid && own != L;
-            const unsigned fm = __ballot_sync(0xffffffffu, isf);
-            if (fm) {
-                const int leader = __ffs(fm) - 1;
-                unsigned long long base = 0;
-                if (lane == leader) base = atomicAdd(nforeign, (unsigned long long)__popc(fm));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (isf) {
-                    const unsigned long long f = base + (unsigned long long)__popc(fm & ((1u << lane) - 1u));
-                    if ((i64)f < foreign_cap) foreign[f] = make_int2((int)li, e);
-                }
+        // the leaf itself and its real ancestors
+#pragma unroll 1
+        for (int l = r; l >= 0; --l) {
+            float xs[28];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const float4 f = sm.xL[7 * l + q];
+                xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
             }
-            if (valid && !isf) out[e] = brick_leaf_levels(sm, r, kk, brick_virtual(sm, D, r, Lc, oc, qc, kk)) - v.iso;
+            column_level<K1>(xs, sm.Bt[l * K1 + kx], sm.Bt[(BR_LEVELS + l) * K1 + ky], sm.Bt + (2 * BR_LEVELS + l) * K1, val);
+        }
+        float* out = blat + lb.lat + (i64)ci * K1;
+        unsigned fmask = 0;                 // corners of the column that another leaf owns
+        if (fposs) {
+#pragma unroll 1
+            for (int kz = 0; kz < K1; ++kz) {
+                const bool low = lowx || lowy || (lowz && kz == 0);
+                if (!__any_sync(0xffffffffu, col && low)) continue;
+                const int qc[3] = {qx, qy, g0[2] + kz};
+                int oc[3] = {0, 0, 0};
+                int own = L;
+                if (col && low) own = corner_owner_cell(D, r, Lc, qc, sm.member, oc);
+                // owned by another leaf of the batch: filled by k_foreign_fill
+                const bool isf = own != L;
+                const u64 src = isf ? foreign_src(D, r, E, bix.dl, root_of[own], oc, qc) : 0ull;
+                push_foreign(isf, li, ci * K1 + kz, src, nforeign, foreign, foreign_cap);
+                if (isf) fmask |= 1u << kz;
+            }
+        }
+        if (col) {
+#pragma unroll
+            for (int kz = 0; kz < K1; ++kz)
+                if (!((fmask >> kz) & 1)) out[kz] = val[kz] - v.iso;
+        }
+    }
+}
+
+// Bricks of edge 2 (leaves one depth above the finest), three to a warp, nine columns of three corners each.
+// The only virtual depth is the finest, and its window, the 4x4x4 cells around the leaf, are the children
+// of the leaf's 27 neighbours, so a cell's x is two loads away without a descent.  A level costs a warp 45
+// instructions of arithmetic per brick where a lane per corner takes 81 on 27 of 32 lanes, and its set-up
+// is shared by three.  4 M points, maxDepth 11, 1.6 M such bricks: 4.1 ms (with the edge-4 bricks 7.4 ms,
+// 19.7 before); half of the issue slots idle on the gathers of x27 rows.
+constexpr int E2_WARPS = 4;
+__global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
+                                                              const LiveBrick* __restrict__ live,
+                                                              const int* __restrict__ list, i64 nlist,
+                                                              float* __restrict__ blat,
+                                                              unsigned long long* __restrict__ nforeign,
+                                                              ForeignCorner* __restrict__ foreign, i64 foreign_cap) {
+    __shared__ float s_x[E2_WARPS][3][64];
+    __shared__ int s_child[E2_WARPS][3][27];
+    __shared__ int s_member[E2_WARPS][3][27];
+    __shared__ int s_up[E2_WARPS][3][BR_LEVELS];
+    const EvalArgs& a = v.e;
+    const int D = a.D, r = D - 1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int gi = min(lane / 9, 2), ci = lane - 9 * gi < 9 ? lane - 9 * gi : 8, kx = ci / 3, ky = ci % 3;
+    const i64 nwarps = (i64)gridDim.x * E2_WARPS;
+    for (i64 it = ((i64)blockIdx.x * E2_WARPS + w) * 3; it < nlist; it += nwarps * 3) {
+        const int nbr = (int)min(nlist - it, (i64)3);
+        __syncwarp();                       // the previous bricks' readers are done
+        for (int e = lane; e < nbr * 27; e += 32) {
+            const int b = e / 27, j = e % 27;
+            const VRoot R = v.roots[live[list[it + b]].root];
+            const int n = a.nd.neigh[(i64)j * a.nd.M + R.node];
+            s_child[w][b][j] = n == -1 ? -1 : a.nd.child0[n];
+            // batch_member's rule (R.depth >= 3: one batch per depth)
+            s_member[w][b][j] = j == 13 ? R.node : (r >= 3 && n != -1 && v.batch_root_flag[n] == R.batch) ? n : -1;
+        }
+        for (int e = lane; e < nbr * BR_LEVELS; e += 32) {
+            const int b = e / BR_LEVELS, l = e % BR_LEVELS;
+            if (l <= r) s_up[w][b][l] = bix.up[(i64)live[list[it + b]].root * BR_LEVELS + l];
+        }
+        __syncwarp();
+        for (int e = lane; e < nbr * 64; e += 32) {
+            const int b = e >> 6, cell = e & 63, bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
+            const int c0 = s_child[w][b][9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
+            s_x[w][b][cell] = c0 == -1 ? 0.f : a.x[c0 + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
+        }
+        __syncwarp();
+        const bool on = lane < 27 && gi < nbr;
+        const int g = min(gi, nbr - 1);
+        const int li = list[it + g];
+        const i64 lat = live[li].lat;
+        int Lc[3];
+        key_coords(a.nd.key[s_up[w][g][r]], r, D, Lc);
+        const int g0[3] = {2 * Lc[0], 2 * Lc[1], 2 * Lc[2]};
+        const int u[3] = {g0[0] + kx, g0[1] + ky, g0[2]};
+        float val[3] = {0.f, 0.f, 0.f};
+        {
+            // the finest depth: owner cell = the one below the corner, its own on the leaf's lower face
+            const int sx = kx == 2, sy = ky == 2;
+            const float4 fx = lattice_at(a, D, g0[0] + sx, kx - sx), fy = lattice_at(a, D, g0[1] + sy, ky - sy);
+            const float x3[3] = {fx.x, fx.y, fx.z}, y3[3] = {fy.x, fy.y, fy.z};
+            float p[4][9];
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+#pragma unroll
+                for (int j = 0; j < 9; ++j)
+                    p[z][j] = s_x[w][g][(sx + j / 3) * 16 + (sy + j % 3) * 4 + z] * x3[j / 3] * y3[j % 3];
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz) {
+                const int sz = kz == 2;
+                const float4 fz = lattice_at(a, D, g0[2] + sz, kz - sz);
+                const float z3[3] = {fz.x, fz.y, fz.z};
+#pragma unroll
+                for (int j = 0; j < 27; ++j) val[kz] = fmaf(p[sz + j % 3][j / 3], z3[j % 3], val[kz]);
+            }
+        }
+#pragma unroll 1
+        for (int l = r; l >= 0; --l) {
+            const float4* row = reinterpret_cast<const float4*>(a.x27 + (i64)s_up[w][g][l] * X27_STRIDE);
+            float xs[28];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const float4 f = row[q];
+                xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
+            }
+            const int sh = D - l;
+            int c[3], k[3];
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                c[ax] = Lc[ax] >> (r - l);
+                k[ax] = u[ax] - (c[ax] << sh);
+            }
+            const float4* bz = a.lb + lattice_offset(D, l) + (i64)c[2] * ((1 << sh) + 1) + k[2];
+            const float4 b3[3] = {bz[0], bz[1], bz[2]};
+            column_level<3>(xs, lattice_at(a, l, c[0], k[0]), lattice_at(a, l, c[1], k[1]), b3, val);
+        }
+        unsigned fmask = 0;
+#pragma unroll
+        for (int kz = 0; kz < 3; ++kz) {
+            const int qc[3] = {u[0], u[1], u[2] + kz};
+            int oc[3] = {0, 0, 0};
+            int own = -1;
+            const bool low = on && (kx == 0 || ky == 0 || kz == 0);
+            if (low) own = corner_owner_cell(D, r, Lc, qc, s_member[w][g], oc);
+            const bool isf = low && own != s_up[w][g][r];
+            const u64 src = isf ? foreign_src(D, r, 2, bix.dl, root_of[own], oc, qc) : 0ull;
+            push_foreign(isf, li, ci * 3 + kz, src, nforeign, foreign, foreign_cap);
+            if (isf) fmask |= 1u << kz;
+        }
+        if (on) {
+            float* out = blat + lat + ci * 3;
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz)
+                if (!((fmask >> kz) & 1)) out[kz] = val[kz] - v.iso;
         }
     }
 }
@@ -1815,40 +2020,36 @@ __global__ void __launch_bounds__(NT) k_brick_eval(VArgs v, BrickIndex bix, cons
 // corners on a leaf's lower faces owned by a cell of another leaf L' of the
 // batch: the same value is a corner of L''s brick holding the owner cell, where
 // L' owns it -- copied when that brick is live, evaluated otherwise
-__global__ void k_foreign_fill(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
-                               const LiveBrick* __restrict__ live, const unsigned char* __restrict__ culled,
-                               const int* __restrict__ live_pos, const int2* __restrict__ foreign, i64 n,
-                               float* __restrict__ blat, unsigned long long* __restrict__ nslow) {
+__global__ void k_foreign_fill(VArgs v, BrickIndex bix, const LiveBrick* __restrict__ live,
+                               const unsigned char* __restrict__ culled, const int* __restrict__ live_pos,
+                               const ForeignCorner* __restrict__ foreign, i64 n, float* __restrict__ blat,
+                               unsigned long long* __restrict__ nslow) {
     const int D = v.e.D;
     for (i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
-        const int2 fe = foreign[f];
-        const LiveBrick lb = live[fe.x];
-        const VRoot R = v.roots[lb.root];
-        const int r = R.depth, S = 1 << (D - r), E = brick_edge(D, r), E1 = E + 1, nb = S / E;
-        int Lc[3];
-        key_coords(v.e.nd.key[R.node], r, D, Lc);
-        const int e = fe.y;
-        const int qc[3] = {Lc[0] * S + lb.b[0] * E + e / (E1 * E1), Lc[1] * S + lb.b[1] * E + (e / E1) % E1,
-                           Lc[2] * S + lb.b[2] * E + e % E1};
-        int oc[3] = {0, 0, 0};
-        const int own = lower_face_owner(v, R, Lc, qc, oc);
-        const int k2 = root_of[own];
-        int Lc2[3];
-        key_coords(v.e.nd.key[own], r, D, Lc2);
-        int b2[3], kk2[3];
-        for (int ax = 0; ax < 3; ++ax) {
-            b2[ax] = (oc[ax] - Lc2[ax] * S) / E;
-            kk2[ax] = qc[ax] - (Lc2[ax] * S + b2[ax] * E);
-        }
-        const i64 bi2 = bix.prefix[k2] + ((i64)b2[0] * nb + b2[1]) * nb + b2[2];
+        const ForeignCorner fe = foreign[f];
+        const i64 brick = (i64)(fe.src >> 10);
+        const int e = (int)(fe.src & 1023);
         float val;
-        if (!culled[bi2]) {
-            val = blat[live[live_pos[bi2]].lat + (kk2[0] * E1 + kk2[1]) * E1 + kk2[2]];
+        if (!culled[brick]) {
+            val = blat[live[live_pos[brick]].lat + e];
         } else {
             atomicAdd(nslow, 1ull);
-            val = virtual_corner_value(v, own, r, oc, qc) - v.iso;
+            // the owner brick's corner e, evaluated by its own leaf
+            const VBrick B = brick_of(v, bix, brick);
+            const VRoot R = v.roots[B.root];
+            const int r = R.depth, S = 1 << (D - r), E = brick_edge(D, r), E1 = E + 1;
+            int Lc[3];
+            key_coords(v.e.nd.key[R.node], r, D, Lc);
+            const int kk[3] = {e / (E1 * E1), (e / E1) % E1, e % E1};
+            int oc[3], qc[3];
+            for (int ax = 0; ax < 3; ++ax) {
+                const int l0 = Lc[ax] * S;
+                qc[ax] = l0 + B.b[ax] * E + kk[ax];
+                oc[ax] = max(qc[ax] - 1, l0);
+            }
+            val = virtual_corner_value(v, R.node, r, oc, qc) - v.iso;
         }
-        blat[lb.lat + e] = val;
+        blat[live[fe.li].lat + fe.e] = val;
     }
 }
 
@@ -2430,13 +2631,13 @@ void stage_mesh(Ctx& c) {
         // bricks of leaves with lattice edge >= 16 come first (roots are in depth order)
         const int kb = c.kbegin("brick_bound", (double)nrows * PROW * (D + 1) * 4 +
                                                    (double)nr * ANC_STRIDE * 4 + (double)nbricks * 3);
-        k_brick_bound<<<grid_for(nbig * 32, BB_BLOCK, (i64)c.sms * 8), BB_BLOCK, 0, s>>>(va, bix, 0, nbig, dspre,
+        k_brick_bound<<<grid_for(nbig * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(va, bix, 0, nbig, dspre,
                                                                                          ssign, c.d_has_tri, bsign);
         CK_LAUNCH();
         c.kend(kb);
         const int kb2 = c.kbegin("brick_bound_small", (double)(nbricks - nbig) * 3);
         if (nbricks > nbig) {
-            k_brick_bound<<<grid_for((nbricks - nbig) * 32, BB_BLOCK, (i64)c.sms * 8), BB_BLOCK, 0, s>>>(
+            k_brick_bound<<<grid_for((nbricks - nbig) * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(
                 va, bix, nbig, nbricks, dspre, ssign, c.d_has_tri, bsign);
             CK_LAUNCH();
         }
@@ -2479,32 +2680,33 @@ void stage_mesh(Ctx& c) {
             unsigned long long* cnt3 = dalloc<unsigned long long>(6, s);
             int* lists = dalloc<int>(3 * nlive, s);
             CK(cudaMemsetAsync(cnt3, 0, 6 * sizeof(unsigned long long), s));
-            // corners owned by another leaf: at most the lower-face corners of the live bricks
-            const i64 fcap = std::min<i64>(lat_total, nlive * (BR_CORNERS - BR * BR * BR));
-            int2* foreign = dalloc<int2>(std::max<i64>(fcap, 1), s);
             k_live_split<<<grid_for(nlive, 256), 256, 0, s>>>(va, live, nlive, lists, lists + nlive,
                                                               lists + 2 * nlive, cnt3);
             CK_LAUNCH();
             unsigned long long hc[6];
             CK(cudaMemcpyAsync(hc, cnt3, sizeof hc, cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
+            // corners owned by another leaf: at most the lower-face corners of the live bricks
+            const i64 fcap = (i64)hc[0] * (9 * 9 * 9 - 8 * 8 * 8) + (i64)hc[1] * (5 * 5 * 5 - 4 * 4 * 4) +
+                             (i64)hc[5] * (3 * 3 * 3 - 2 * 2 * 2);
+            ForeignCorner* foreign = dalloc<ForeignCorner>(fcap, s);
             c.kend(kg);
             // compulsory: the corner values written (bricks of edge 8: 729 each)
             const int ke = c.kbegin("brick_eval", (double)hc[0] * BR_CORNERS * 4);
             if (hc[0] > 0) {
-                k_brick_eval<BR, BR_BLOCK><<<grid_for((i64)hc[0], 1, (i64)c.sms * 16), BR_BLOCK, 0, s>>>(
+                k_brick_eval<8, 96><<<grid_for((i64)hc[0], 1, (i64)c.sms * 16), 96, 0, s>>>(
                     va, bix, root_of, live, lists, (i64)hc[0], lat_brick, cnt3 + 2, foreign, fcap);
                 CK_LAUNCH();
             }
             c.kend(ke);
             const int ks = c.kbegin("brick_eval_small", (double)(lat_total - (i64)hc[0] * BR_CORNERS) * 4);
             if (hc[1] > 0) {
-                k_brick_eval<4, 64><<<grid_for((i64)hc[1], 1, (i64)c.sms * 24), 64, 0, s>>>(
+                k_brick_eval<4, 32><<<grid_for((i64)hc[1], 1, (i64)c.sms * 32), 32, 0, s>>>(
                     va, bix, root_of, live, lists + nlive, (i64)hc[1], lat_brick, cnt3 + 2, foreign, fcap);
                 CK_LAUNCH();
             }
-            if (hc[5] > 0) {   // 27 corners: one warp per brick
-                k_brick_eval<2, 32><<<grid_for((i64)hc[5], 1, (i64)c.sms * 32), 32, 0, s>>>(
+            if (hc[5] > 0) {
+                k_edge2_eval<<<grid_for((i64)hc[5], 3 * E2_WARPS, (i64)c.sms * 64), 32 * E2_WARPS, 0, s>>>(
                     va, bix, root_of, live, lists + 2 * nlive, (i64)hc[5], lat_brick, cnt3 + 2, foreign, fcap);
                 CK_LAUNCH();
             }
@@ -2524,7 +2726,7 @@ void stage_mesh(Ctx& c) {
             if (hf[0] > 0) {
                 const int kf = c.kbegin("foreign_fill", (double)hf[0] * 8);
                 k_foreign_fill<<<grid_for((i64)hf[0], 128, 1ll << 30), 128, 0, s>>>(
-                    va, bix, root_of, live, culled, bp, foreign, (i64)hf[0], lat_brick, cnt3 + 4);
+                    va, bix, live, culled, bp, foreign, (i64)hf[0], lat_brick, cnt3 + 4);
                 CK_LAUNCH();
                 c.kend(kf);
                 c.foreign_slow = (i64)read_scalar(cnt3 + 4, s);

@@ -688,7 +688,7 @@ void stage_divergence(Ctx& c) {
             CK_LAUNCH();
             if (ngitems > 0) {
                 const int kt3 = c.kbegin("divergence_groups", 0.0);
-                k_div_groups<<<grid_for(ngitems * 32, DIV_WARPS * 32, (i64)c.sms * 8), DIV_WARPS * 32, 0, s>>>(
+                k_div_groups<<<grid_for(ngitems * 32, DIV_WARPS * 32, (i64)c.sms * 256), DIV_WARPS * 32, 0, s>>>(
                     c.nodes, a, c.gn, ngroups_all, item_group, gfirst, ngitems, gpartial);
                 CK_LAUNCH();
                 c.kend(kt3);
