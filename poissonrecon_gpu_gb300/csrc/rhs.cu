@@ -140,40 +140,133 @@ __device__ __forceinline__ void node_rows(const DivArgs& a, u64 key, int d, cons
     for (int q = 0; q < 3; ++q) t0[q] = (xyz[q] - 1) * (1 << (a.D - d));
 }
 
-// nodes with few terms: one thread per node, terms in neighbour order
-__global__ void k_div_thread(NodeArrays nd, DivArgs a, i64 lo, i64 hi, float* __restrict__ out) {
-    for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
+// The value of a double sum of floats added one after the other, rounded to float at the end, without
+// the FP64 pipe (2 operations a cycle and SM: a conversion and an addition per term were most of the two
+// finest depths' divergence).  The terms go into three floats by error-free additions: h + l + m differs
+// from the exact sum S by at most n^3 u^3 T (u = 2^-24, T the sum of the terms' magnitudes), the double
+// sum by at most n 2^-53 T, both together below 2^-44 T for n <= 216.  Where every value within that of
+// h + l + m rounds to the same float, that is the double sum's rounding too.  Ties of that rounding (two
+// terms of one exponent make one in two cases) are settled by exactness: when T has less than 2^29 times
+// the smallest non-zero term's power of two, every partial sum is a multiple of that term's last place
+// below 2^53 of it, so the double sum is exact and so are h + l + m and its value in double.  Elsewhere
+// ('sure' false: about one node in a million, and sums that are not finite) the caller adds in double.
+struct FloatSum3 {
+    float h = 0.f, l = 0.f, m = 0.f, T = 0.f;
+    unsigned least = 0xffffffffu;   // bits of the smallest non-zero magnitude, less one
+    __device__ __forceinline__ void add(float t) {
+        const float s = h + t, a = s - h, e = (h - (s - a)) + (t - a);
+        const float q = l + e, b = q - l;
+        m += (l - (q - b)) + (e - b);
+        h = s;
+        l = q;
+        T += fabsf(t);
+        least = min(least, (__float_as_uint(t) & 0x7fffffffu) - 1u);
+    }
+    __device__ __forceinline__ float rounded(bool& sure) const {
+        const double v = (double)h + ((double)l + (double)m), d = (double)T * 5.684341886080802e-14;   // 2^-44
+        // exponents of T and the smallest term (a subnormal counts as exponent 1), T finite
+        const int eT = (int)(__float_as_uint(T) >> 23), en = max((int)((least + 1u) >> 23), 1);
+        const float f = (float)(v - d);
+        if (f == (float)(v + d)) {
+            sure = true;
+            return f;
+        }
+        sure = eT < 255 && eT - en <= 28;
+        return (float)v;
+    }
+};
+
+// Depth D - 1 by sibling groups: the 27 neighbours of a group's 8 nodes are the 4x4x4 block of the children
+// of the parent's 27 neighbours (the group table), and each block cell's finest descendants are its 8
+// children (or none), consecutive finest slots whose V is 96 aligned bytes.  A lane takes a node and adds
+// its at most 216 terms in neighbour order, each neighbour's children in order.  The row entry of a
+// child along an axis is 2 j + bit of the node's 6 (j the neighbour's offset 0..2), so no coordinates are
+// read.  1M torus: 0.98 ms with a thread per node, its 27 neighbour loops unrolled (half the issue slots
+// waiting for instructions, four loads a term) and a double addition per term.
+__device__ __forceinline__ float div_child_term(float vx, float vy, float vz, float u0, float u1, float u2) {
+    float t = vx * u0;
+    t = fmaf(vy, u1, t);
+    return fmaf(vz, u2, t);
+}
+constexpr int DIV_PARENT_WARPS = 4;
+__global__ void __launch_bounds__(32 * DIV_PARENT_WARPS) k_div_parents(NodeArrays nd, DivArgs a, const int* __restrict__ gn,
+                                                                       i64 ngroups_all, i64 gfirst, i64 ng, i64 lo,
+                                                                       i64 finest, float* __restrict__ out) {
+    __shared__ int s_slot[DIV_PARENT_WARPS][4][64];   // first finest slot of each block cell, -1: none
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int ch = lane & 7, sx = ch >> 2, sy = (ch >> 1) & 1, sz = ch & 1;
+    const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
+    for (i64 tile = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile * 4 < ng; tile += nwarps) {
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int e = lane + 32 * q;
+            const i64 g = tile * 4 + (e >> 6);
+            const int cell = e & 63, bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
+            int s0 = -1;
+            if (g < ng) {
+                const int c0 = gn[(i64)(9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)) * ngroups_all + gfirst + g];
+                if (c0 != -1) {
+                    const int f = nd.child0[c0 + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
+                    if (f != -1) s0 = (int)(f - finest);
+                }
+            }
+            s_slot[w][e >> 6][cell] = s0;
+        }
+        __syncwarp();
+        const i64 g = tile * 4 + (lane >> 3);
+        if (g >= ng) continue;
+        const i64 i = lo + 8 * g + ch;
         const float *r0, *r1, *r2;
         int t0[3];
-        node_rows(a, nd.key[i], nd.depth[i], r0, r1, r2, t0);
-        double val = 0.0;
-        // neighbours in three batches of nine: indices, then descendant ranges, then terms,
-        // so that each batch's loads are in flight together
+        node_rows(a, nd.key[i], a.D - 1, r0, r1, r2, t0);
+        float u2[6];
 #pragma unroll
-        for (int jb = 0; jb < 27; jb += 9) {
-            int nb[9], s0[9], sn[9];
+        for (int k = 0; k < 6; ++k) u2[k] = r2[k];
+        const int* blk = s_slot[w][lane >> 3];
+        // f for each term, in order
+        auto each = [&](auto f) {
+#pragma unroll 1
+            for (int jxy = 0; jxy < 9; ++jxy) {
+                const int jx = jxy / 3, jy = jxy % 3;
+                const float u0a = r0[2 * jx], u0b = r0[2 * jx + 1], u1a = r1[2 * jy], u1b = r1[2 * jy + 1];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) nb[q] = nd.neigh[(i64)(jb + q) * a.M + i];
+                for (int jz = 0; jz < 3; ++jz) {
+                    const int s0 = blk[(sx + jx) * 16 + (sy + jy) * 4 + sz + jz];
+                    if (s0 < 0) continue;
+                    const float4* V = reinterpret_cast<const float4*>(a.vfield + 3 * (i64)s0);
+                    float vv[24];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) {
-                s0[q] = nb[q] == -1 ? 0 : nd.didx[nb[q]];
-                sn[q] = nb[q] == -1 ? 0 : nd.dnum[nb[q]];
+                    for (int k = 0; k < 6; ++k) {
+                        const float4 q = V[k];
+                        vv[4 * k] = q.x; vv[4 * k + 1] = q.y; vv[4 * k + 2] = q.z; vv[4 * k + 3] = q.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        f(div_child_term(vv[3 * k], vv[3 * k + 1], vv[3 * k + 2], (k >> 2) ? u0b : u0a,
+                                         ((k >> 1) & 1) ? u1b : u1a, u2[2 * jz + (k & 1)]));
+                }
             }
-#pragma unroll
-            for (int q = 0; q < 9; ++q)
-                for (int k = 0; k < sn[q]; ++k) val += (double)div_term(a, r0, r1, r2, t0, (i64)s0[q] + k);
+        };
+        FloatSum3 s;
+        each([&](float t) { s.add(t); });
+        bool sure;
+        float val = s.rounded(sure);
+        if (!sure) {
+            double d = 0.0;
+            each([&](float t) { d += (double)t; });
+            val = (float)d;
         }
-        out[i] = (float)val;
+        out[i] = val;
     }
 }
 
 // finest depth by sibling groups: the 27 neighbours of the 8 children of a node
 // are the 4x4x4 block of the children of the parent's 27 neighbours (the solve's
 // group table).  One warp stages the V of the blocks of 4 groups in shared
-// memory; each row then sums its 27 terms in neighbour order in FP64, as
-// k_div_thread does.  Every finest node has exactly one finest descendant
-// (itself), and the neighbour at offset j = (jx,jy,jz) reads the row entries
-// jx, jy, jz of the node's 3-entry rows.
+// memory; each row then adds its 27 terms in neighbour order.  Every finest node
+// has exactly one finest descendant (itself), and the neighbour at offset
+// j = (jx,jy,jz) reads the row entries jx, jy, jz of the node's 3-entry rows.
 __global__ void __launch_bounds__(256) k_div_finest(NodeArrays nd, DivArgs a, const int* __restrict__ gn,
                                                     i64 ngroups_all, i64 gfirst, i64 ng, i64 lo,
                                                     float* __restrict__ out) {
@@ -214,18 +307,30 @@ __global__ void __launch_bounds__(256) k_div_finest(NodeArrays nd, DivArgs a, co
 #pragma unroll
                 for (int t = 0; t < 3; ++t) R[ax][t] = rr[xyz[ax] * 3 + t];
             const float4* b = blk + gl * 64;
-            double val = 0.0;
+            FloatSum3 s;
 #pragma unroll
             for (int j = 0; j < 27; ++j) {
                 const int jx = j / 9, jy = (j / 3) % 3, jz = j % 3;
                 const float4 c = b[(sx + jx) * 16 + (sy + jy) * 4 + (sz + jz)];
-                if (c.w == 0.f) continue;   // no neighbour
-                float t = c.x * R[0][jx];
-                t = fmaf(c.y, R[1][jy], t);
-                t = fmaf(c.z, R[2][jz], t);
-                val += (double)t;
+                if (c.w != 0.f) s.add(div_child_term(c.x, c.y, c.z, R[0][jx], R[1][jy], R[2][jz]));   // else no neighbour
             }
-            out[i] = (float)val;
+            bool sure;
+            float val = s.rounded(sure);
+            if (!sure) {
+                double d = 0.0;
+#pragma unroll 1
+                for (int jxy = 0; jxy < 9; ++jxy) {
+                    const int jx = jxy / 3, jy = jxy % 3;
+#pragma unroll
+                    for (int jz = 0; jz < 3; ++jz) {
+                        const float4 c = b[(sx + jx) * 16 + (sy + jy) * 4 + (sz + jz)];
+                        if (c.w != 0.f)
+                            d += (double)div_child_term(c.x, c.y, c.z, rr[xyz[0] * 3 + jx], rr[xyz[1] * 3 + jy], R[2][jz]);
+                    }
+                }
+                val = (float)d;
+            }
+            out[i] = val;
         }
     }
 }
@@ -634,15 +739,18 @@ void stage_divergence(Ctx& c) {
     const int split = D >= 1 ? D - 1 : 0;
     // compulsory: every node's key, depth, neighbours and b; V and coordinates of the finest slots
     const int kt = c.kbegin("divergence", (double)M * (8 + 1 + 108 + 4) + (double)nD * (12 + 8));
-    // depth D - 1 one thread per node; depth D by sibling groups
-    const int kt1 = c.kbegin("divergence_d1", 0.0);
-    k_div_thread<<<grid_for(c.base[D] - c.base[split], 128, 1ll << 30), 128, 0, s>>>(c.nodes, a, c.base[split],
-                                                                                      c.base[D], c.divergence);
-    CK_LAUNCH();
-    c.kend(kt1);
+    // depth D - 1 by sibling groups (a depth-1 group hangs off the root; depth 0 has no group), depth D too
     const int ktg = c.kbegin("group_table", 0.0);
     ensure_group_table(c);
     c.kend(ktg);
+    const int kt1 = c.kbegin("divergence_d1", 0.0);
+    if (split >= 1) {
+        const i64 ngroups_all = (M - 1) / 8, plo = c.base[split], png = (c.base[D] - plo) / 8;
+        k_div_parents<<<grid_for(png * 8, 32 * DIV_PARENT_WARPS, 1ll << 30), 32 * DIV_PARENT_WARPS, 0, s>>>(
+            c.nodes, a, c.gn, ngroups_all, (plo - 1) / 8, png, plo, lo, c.divergence);
+        CK_LAUNCH();
+    }
+    c.kend(kt1);
     const int kt2 = c.kbegin("divergence_d", 0.0);
     {
         const i64 ngroups_all = (M - 1) / 8, gfirst = (lo - 1) / 8, ng = nD / 8;
