@@ -689,16 +689,17 @@ constexpr int BR_WEXT = BR + 4;    // window cells per axis in the row tables (a
 // axis the owner cells of its corners (8 cells and the one below) and one more to each side, 11, 7 and 5
 // cells at the finest depths and 4 at the others: 11^3 + 7^3 + 5^3 + 12 * 4^3 = 2567
 constexpr int BR_XW = 2568;
-// super-brick row table: RA (6 per depth), RW (24 per depth)
-constexpr int ROW_RA = 0, ROW_RW = 6, ROW_PER_DEPTH = 30;
-// brick row table: 24 floats per depth d > r (the ancestors, d <= r, are one polynomial per leaf)
+// Row table of a brick or super-brick of edge E, 24 floats per depth d > r (the ancestors, d <= r, are one
+// polynomial per leaf):
 //   d <= D - lg E  PW[n]  window cell n < 4: Bernstein form over the brick's corners (b0, b1, b2, M,
 //                         see bern_fit) of its function, masked as RW is; the function's knots are
 //                         multiples of its cell width 2^(D-d) >= E, so it is one quadratic piece there
-//   d >  D - lg E  RW[n]  as above (12 cells, range with 0)
+//   d >  D - lg E  RW[n]  as above (12 cells, range with 0; bricks only)
 constexpr int PROW = 24;
 constexpr int PW = 4;              // window cells per axis at the depths of knot spacing >= E
 constexpr int ANC_STRIDE = 32;     // per root: Bernstein coefficients C[27] of the ancestors, S3, count, FIT
+constexpr int SUPER = 4 * BR;      // edge of a super-brick (leaves of lattice edge >= 64)
+constexpr int BELOW = 5;           // depths below a node whose range of x k_x_below keeps
 
 __device__ __forceinline__ int brick_edge(int D, int r) { return min(1 << (D - r), BR); }
 
@@ -718,6 +719,9 @@ struct BrickIndex {                // bricks of all subdivided leaves, numbered 
     const float* rows;             // brick-row tables, PROW (D+1) floats each
     const int* up;                 // per root: its node and its ancestors by depth, BR_LEVELS each
     const float* anc;              // per root: the ancestor polynomial, ANC_STRIDE floats
+    const float2* below;           // k_x_below
+    i64 below0;                    // its first node
+    const float2* bsum;            // k_basis_sums, per depth
     DepthLayout dl;
 };
 struct VBrick {
@@ -739,8 +743,9 @@ __device__ __forceinline__ VBrick brick_of(const VArgs& v, const BrickIndex& bx,
     b.b[2] = (int)l & m;
     return b;
 }
-__device__ __forceinline__ const float* brick_row(const BrickIndex& bx, int D, int root, int nb, int ax, int b) {
-    return bx.rows + (bx.row_prefix[root] + (i64)ax * nb + b) * (i64)(PROW * (D + 1));
+__device__ __forceinline__ const float* brick_row(const float* rows, const i64* row_prefix, int D, int root, int nb,
+                                                  int ax, int b) {
+    return rows + (row_prefix[root] + (i64)ax * nb + b) * (i64)(PROW * (D + 1));
 }
 
 __device__ __forceinline__ float f4_at(const float4& f, int i) { return i == 0 ? f.x : (i == 1 ? f.y : f.z); }
@@ -791,43 +796,6 @@ __device__ i64 shell_node(const VArgs& v, int L, int r, const int Lc[3], int d, 
     const int an = nd.neigh[(i64)(9 * (dx + 1) + 3 * (dy + 1) + (dz + 1)) * nd.M + L];
     if (an == -1) return -1;
     return descend(nd, an, r, d, N);
-}
-
-// the leaf's ancestor levels l <= r of a bound, factored by axis: for every
-// (l, jx, jy) the three z terms x[j] * Z[jz] (scalar times interval) are summed,
-// then multiplied by the intervals Y[jy] and X[jx].  Interval arithmetic is
-// subdistributive, so this encloses every corner's exact ancestor sum as the
-// term-by-term form does, with a third of its interval products.  Each end is
-// within 5u of the exact factored end per row (3 terms, 2 products), against
-// 3u per term in the term-by-term form; the margins allow 2 BR_WEXT u A more.
-// amax gains sum |x| |Z| |Y| |X| >= sum |term| over the corners.
-__device__ __forceinline__ void ancestor_bound(const EvalArgs& a, const int* up, const float* const row[3], int r,
-                                               int D, int lane, float& lo, float& hi, float& amax, int& cnt) {
-    const int ra = ROW_RA * (D + 1);
-    for (int t = lane; t < 9 * (r + 1); t += 32) {
-        const int l = r - t / 9, jx = (t % 9) / 3, jy = t % 3;
-        const float* xs = a.x27 + (i64)up[l] * X27_STRIDE + 9 * jx + 3 * jy;
-        float slo = 0.f, shi = 0.f, sabs = 0.f;
-        for (int jz = 0; jz < 3; ++jz) {
-            const float x = xs[jz];
-            if (x == 0.f) continue;
-            const float zl = row[2][ra + (l * 3 + jz) * 2], zh = row[2][ra + (l * 3 + jz) * 2 + 1];
-            const float p0 = x * zl, p1 = x * zh;
-            slo += fminf(p0, p1);
-            shi += fmaxf(p0, p1);
-            sabs += fabsf(x) * fmaxf(fabsf(zl), fabsf(zh));
-            ++cnt;
-        }
-        if (sabs == 0.f) continue;
-        const float yl = row[1][ra + (l * 3 + jy) * 2], yh = row[1][ra + (l * 3 + jy) * 2 + 1];
-        const float xl0 = row[0][ra + (l * 3 + jx) * 2], xh0 = row[0][ra + (l * 3 + jx) * 2 + 1];
-        float c0 = slo * yl, c1 = slo * yh, c2 = shi * yl, c3 = shi * yh;
-        const float alo = fminf(fminf(c0, c1), fminf(c2, c3)), ahi = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
-        c0 = alo * xl0; c1 = alo * xh0; c2 = ahi * xl0; c3 = ahi * xh0;
-        lo += fminf(fminf(c0, c1), fminf(c2, c3));
-        hi += fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
-        amax += sabs * fmaxf(fabsf(yl), fabsf(yh)) * fmaxf(fabsf(xl0), fabsf(xh0));
-    }
 }
 
 // can a corner of brick b[] (nb bricks per edge) be owned by a cell of another
@@ -929,7 +897,7 @@ __global__ void k_batch_flags(const VRoot* __restrict__ roots, int nroots, int* 
 // edge of the bricks (super == 0) or of the super-bricks (super == 1: 4^3 bricks of 8^3
 // cells, in leaves with lattice edge >= 64; 0 elsewhere)
 __device__ __forceinline__ int row_edge(int D, int r, int super) {
-    return super ? ((D - r >= 6) ? 4 * BR : 0) : brick_edge(D, r);
+    return super ? ((D - r >= 6) ? SUPER : 0) : brick_edge(D, r);
 }
 
 // one thread per (brick row, depth); rows numbered root by root (row_prefix), 3 x bricks-per-edge each
@@ -958,18 +926,9 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
         key_coords(a.nd.key[R.node], r, D, Lc);
         const int g0 = Lc[ax] * S + rd.z * B;
         const int c0 = rd.z * B;
-        float* out = rows + row * (i64)((super ? ROW_PER_DEPTH : PROW) * (D + 1));
-        if (d <= r) {
-            if (!super) continue;   // bricks: the leaf's ancestor polynomial (k_brick_xl)
-            float4 mn = brick_bt(a, r, Lc[ax], g0, d, 0), mx = mn;
-            for (int k = 1; k <= B; ++k) {
-                const float4 b = brick_bt(a, r, Lc[ax], g0, d, k);
-                mn.x = fminf(mn.x, b.x); mn.y = fminf(mn.y, b.y); mn.z = fminf(mn.z, b.z);
-                mx.x = fmaxf(mx.x, b.x); mx.y = fmaxf(mx.y, b.y); mx.z = fmaxf(mx.z, b.z);
-            }
-            float* ra = out + ROW_RA * (D + 1) + d * 6;
-            ra[0] = mn.x; ra[1] = mx.x; ra[2] = mn.y; ra[3] = mx.y; ra[4] = mn.z; ra[5] = mx.z;
-        } else {
+        float* out = rows + row * (i64)(PROW * (D + 1));
+        if (d <= r) continue;   // the leaf's ancestor polynomial (k_brick_xl)
+        {
             int wlo, ext;
             bool cross;
             window_axis(g0, B, Lc[ax], r, d, D, 0, wlo, ext, cross);
@@ -980,7 +939,7 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
                 const int Va = (k == 0 && c0 == 0) ? (g0 >> sh) : ((g0 + k - 1) >> sh);
                 return (N < Va - 1 || N > Va + 1) ? 0.f : lattice_entry(a, d, Va, g0 + k - (Va << sh), N - Va + 1);
             };
-            if (!super && (1 << sh) >= B) {
+            if ((1 << sh) >= B) {
                 float4* pw = reinterpret_cast<float4*>(out + d * PROW);
                 for (int n = 0; n < PW; ++n) {
                     const int N = wlo + n;
@@ -990,7 +949,8 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
                 }
                 continue;
             }
-            float* rw = super ? out + ROW_RW * (D + 1) + d * BR_WEXT * 2 : out + d * PROW;
+            if (super) continue;   // k_super_bound reads no ranges
+            float* rw = out + d * PROW;
             for (int n = 0; n < BR_WEXT; ++n) {
                 const int N = wlo + n;
                 float mn = 0.f, mx = 0.f;             // 0: corners without this term
@@ -1152,23 +1112,6 @@ __device__ __forceinline__ int corner_owner_cell(int D, int r, const int Lc[3], 
     return own;
 }
 
-// sign of a bound [lo, hi] of a brick's corner values against iso: 1 (all above), -1 (all
-// below), 0 (not proven).  The margin m = (2 cnt + 2 BR_WEXT + 8) u A + 4u (|lo| + |hi| + 2|iso|),
-// A = 1.01 amax, covers the evaluation's FMA chain and this bound's own float arithmetic.  It is
-// evaluated in float: every operation of it rounds by at most u relative and every term is
-// non-negative, so scaling by 1 + 2^-16 bounds the exact value from above; the tests are made as
-// lo - iso > m and iso - hi > m, whose float differences are within u of exact, which the extra
-// 2u (|lo| + |hi| + 2|iso|) covers.  (A non-finite bound compares false: not proven.)
-__device__ __forceinline__ signed char bound_sign(float lo, float hi, float amax, int cnt, float iso) {
-    const float u = 5.9604644775390625e-08f;   // 2^-24
-    const float A = amax * 1.01f;
-    const float m = ((2.0f * (float)cnt + (2.0f * BR_WEXT + 8.0f)) * u * A +
-                     6.0f * u * (fabsf(lo) + fabsf(hi) + 2.0f * fabsf(iso)) + 1e-30f) * (1.0f + 1.52587890625e-05f);
-    if (lo - iso > m) return 1;
-    if (iso - hi > m) return -1;
-    return 0;
-}
-
 // Shell terms of a bound at virtual depth d: the window cells outside the leaf that hold a
 // real node, each term x * X * Y * Z over the row tables' ranges RW.
 //  * Nodes: a cell's node is found by descending from the leaf's neighbour at depth r, through
@@ -1279,139 +1222,74 @@ __device__ __forceinline__ void shell_terms(const VArgs& v, int L, int r, const 
     }
 }
 
-// one warp per super-brick (4^3 bricks of leaves with lattice edge >= 64): the
-// same bound over all its corners; decided only when every window it needs fits
-// the row tables (away from the leaf's boundary).  ssign = 1, -1 or 0.
-__global__ void __launch_bounds__(256) k_super_bound(VArgs v, DepthLayout dl,
-                                                     const i64* __restrict__ srow_prefix,
-                                                     const float* __restrict__ srows, const int* __restrict__ up_all,
-                                                     i64 nsuper, signed char* __restrict__ ssign) {
-    __shared__ int s_anchor[256 / 32][SHELL_ANCHORS];
-    const EvalArgs& a = v.e;
-    const int D = a.D;
-    const int lane = threadIdx.x & 31;
-    const i64 warp = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
-    for (i64 si = warp; si < nsuper; si += nwarps) {
-        int dd = 0;
-        while (dd < D - 1 && dl.soff[dd + 1] <= si) ++dd;
-        const i64 loc = si - dl.soff[dd];
-        const int slg = dl.slg[dd];
-        const int lo = dl.first[dd] + (int)(loc >> (3 * slg));
-        const VRoot R = v.roots[lo];
-        const int r = R.depth, S = 1 << (D - r), E = 4 * BR, ns = S / E, L = R.node;
-        const i64 l = loc & ((1ll << (3 * slg)) - 1);
-        const int sb[3] = {(int)(l >> (2 * slg)), (int)(l >> slg) & (ns - 1), (int)l & (ns - 1)};
-        int Lc[3];
-        key_coords(a.nd.key[L], r, D, Lc);
-        const int g0[3] = {Lc[0] * S + sb[0] * E, Lc[1] * S + sb[1] * E, Lc[2] * S + sb[2] * E};
-        const float* row[3];
-        for (int ax = 0; ax < 3; ++ax)
-            row[ax] = srows + (srow_prefix[lo] + (i64)ax * ns + sb[ax]) * (i64)(ROW_PER_DEPTH * (D + 1));
-        float flo = 0.f, fhi = 0.f, amax = 0.f;
-        int cnt = 0;
-        bool decided = true;
-        ancestor_bound(a, up_all + (i64)lo * BR_LEVELS, row, r, D, lane, flo, fhi, amax, cnt);
-        for (int d = r + 1; d <= D && decided; ++d) {
-            int wlo[3], ext[3];
-            bool cross = false;
-            for (int ax = 0; ax < 3; ++ax) {
-                bool c;
-                window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], c);
-                cross |= c;
+// Per node of the depths [D - BELOW, D): the least and the largest x, with 0, among its descendants k = 1..
+// BELOW depths down (below[BELOW * node + k - 1]; one launch per depth, finest first).  A node whose
+// descendants hold a value that is not finite gets an infinite range, which proves nothing.
+__global__ void k_x_below(NodeArrays nd, const float* __restrict__ x, i64 lo, i64 hi, i64 node0, int kmax,
+                          float2* __restrict__ below) {
+    for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
+        const int c0 = nd.child0[i];
+        float2* out = below + BELOW * (i - node0);
+        float2 r = make_float2(0.f, 0.f);
+        if (c0 != -1)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float v = x[c0 + c];
+                if (!(fabsf(v) < INFINITY)) r = make_float2(-INFINITY, INFINITY);
+                r = make_float2(fminf(r.x, v), fmaxf(r.y, v));
             }
-            // the windows of successive depths are nested (in finest cells), so once a window
-            // lies inside the leaf so do all finer ones
-            if (!cross) break;
-            if (ext[0] > BR_WEXT || ext[1] > BR_WEXT || ext[2] > BR_WEXT) { decided = false; break; }
-            const float2* rw[3];
-            for (int ax = 0; ax < 3; ++ax) rw[ax] = reinterpret_cast<const float2*>(row[ax] + ROW_RW * (D + 1)) + d * BR_WEXT;
-            shell_terms(v, L, r, Lc, d, D, wlo, ext, rw, lane, s_anchor[threadIdx.x >> 5], flo, fhi, amax, cnt);
+        out[0] = r;
+        for (int k = 1; k < kmax; ++k) {
+            r = make_float2(0.f, 0.f);
+            if (c0 != -1)
+                for (int c = 0; c < 8; ++c) {
+                    const float2 q = below[BELOW * (c0 + c - node0) + k - 1];
+                    r = make_float2(fminf(r.x, q.x), fmaxf(r.y, q.y));
+                }
+            out[k] = r;
         }
-        for (int o = 16; o; o >>= 1) {
-            flo += __shfl_xor_sync(0xffffffffu, flo, o);
-            fhi += __shfl_xor_sync(0xffffffffu, fhi, o);
-            amax += __shfl_xor_sync(0xffffffffu, amax, o);
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        }
-        if (lane == 0) ssign[si] = decided ? bound_sign(flo, fhi, amax, cnt, v.iso) : 0;
     }
 }
 
-// Shell terms at a depth d of knot spacing >= the brick edge (d <= D - lg E): each window cell
-// outside the leaf with a real node contributes x Qx Qy Qz, Q the cell's PW entries (Bernstein
-// form over the brick), to the brick's coarse polynomial.  The window spans at most PW = 4 cells
-// per axis there (the brick lies in one cell of depth d, and its first corner's owner may lie in
-// the cell below), so the terms form a 4^3 grid X of x (0: no node, or inside the leaf; two cells
-// per lane), contracted one axis at a time through shared memory:
-//   T1[n0 n1 l] = sum_n2 X Qz_l(n2),  T2[n0 j l] = sum_n1 T1 Qy_j(n1),  C_ijl += sum_n0 T2 Qx_i(n0)
-// (lane k < 27 holds coefficient k = 9i + 3j + l).  s3 gains |x| Mx My Mz, fit
-// |x| (dx My Mz + Mx dy Mz + Mx My dz) (as k_brick_xl's), cnt the number of terms.
-constexpr int SHELL_POLY_BUF = 64 + 48 + 36;   // floats of shared memory per warp
-__device__ __forceinline__ void shell_poly(const VArgs& v, int L, int r, const int Lc[3], int d, const int wlo[3],
-                                           const int ext[3], const float4* const pw[3], int lane,
-                                           float* __restrict__ buf, float& coef, float& s3, float& fit, int& cnt) {
-    float* X = buf;
-    float* T1 = buf + 64;
-    float* T2 = buf + 112;
-    bool any = false;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int g = lane + 32 * h, n0 = g >> 4, n1 = (g >> 2) & 3, n2 = g & 3;
-        float x = 0.f;
-        if (n0 < ext[0] && n1 < ext[1] && n2 < ext[2]) {
-            const int N[3] = {wlo[0] + n0, wlo[1] + n1, wlo[2] + n2};
-            const i64 node = shell_node(v, L, r, Lc, d, N);
-            if (node >= 0) x = v.e.x[node];
+// Per depth, over all lattice points of all cells: the largest sum of the magnitudes of the three basis
+// values a walk multiplies with along an axis, and the largest sum of their negative parts (float noise of
+// the tabulated values; the B-spline itself is not negative), rounded up.  One block per depth.
+__global__ void k_basis_sums(const float4* __restrict__ lb, int D, float2* __restrict__ out) {
+    __shared__ float s_r[256], s_n[256];
+    const int d = blockIdx.x;
+    float r = 0.f, n = 0.f;
+    for (i64 e = lattice_offset(D, d) + threadIdx.x; e < lattice_offset(D, d + 1); e += blockDim.x) {
+        const float4 f = lb[e];
+        r = fmaxf(r, fabsf(f.x) + fabsf(f.y) + fabsf(f.z));
+        n = fmaxf(n, fmaxf(-f.x, 0.f) + fmaxf(-f.y, 0.f) + fmaxf(-f.z, 0.f));
+    }
+    s_r[threadIdx.x] = r;
+    s_n[threadIdx.x] = n;
+    __syncthreads();
+    for (int o = 128; o; o >>= 1) {
+        if ((int)threadIdx.x < o) {
+            s_r[threadIdx.x] = fmaxf(s_r[threadIdx.x], s_r[threadIdx.x + o]);
+            s_n[threadIdx.x] = fmaxf(s_n[threadIdx.x], s_n[threadIdx.x + o]);
         }
-        X[g] = x;
-        if (x != 0.f) {
-            const float4 QX = pw[0][n0], QY = pw[1][n1], QZ = pw[2][n2];
-            const float Mx = bern_m(QX), My = bern_m(QY), Mz = bern_m(QZ), ax = fabsf(x);
-            s3 += ax * Mx * My * Mz;
-            fit += ax * (QX.w * My * Mz + Mx * QY.w * Mz + Mx * My * QZ.w);
-            ++cnt;
-            any = true;
-        }
+        __syncthreads();
     }
-    if (!__any_sync(0xffffffffu, any)) return;   // no real node near the brick at this depth
-    __syncwarp();
-    for (int e = lane; e < 48; e += 32) {
-        const int nn = e / 3, l = e - 3 * nn;   // nn = 4 n0 + n1
-        float t = 0.f;
-#pragma unroll
-        for (int n2 = 0; n2 < 4; ++n2) t = fmaf(X[4 * nn + n2], f4_at(pw[2][n2], l), t);
-        T1[e] = t;
-    }
-    __syncwarp();
-    for (int e = lane; e < 36; e += 32) {
-        const int n0 = e / 9, j = (e / 3) % 3, l = e % 3;
-        float t = 0.f;
-#pragma unroll
-        for (int n1 = 0; n1 < 4; ++n1) t = fmaf(T1[(4 * n0 + n1) * 3 + l], f4_at(pw[1][n1], j), t);
-        T2[e] = t;
-    }
-    __syncwarp();
-    if (lane < 27) {
-        const int i = lane / 9, jl = lane % 9;
-        float t = 0.f;
-#pragma unroll
-        for (int n0 = 0; n0 < 4; ++n0) t = fmaf(T2[9 * n0 + jl], f4_at(pw[0][n0], i), t);
-        coef += t;
-    }
-    __syncwarp();   // the buffer is reused by the next depth
+    const float up = 1.0f + 9.5367431640625e-07f;
+    if (threadIdx.x == 0) out[d] = make_float2(s_r[0] * up, s_n[0] * up);
 }
 
 // sign of a bound lo = min C + flo, hi = max C + fhi against iso: C the Bernstein coefficients over
 // the brick of its coarse polynomial P (the leaf's ancestors and the shell terms of knot spacing
 // >= E; P lies within their range over the brick's box), [flo, fhi] the interval sum of the finer
-// shell terms.  The margin is bound_sign's over A = amax + s3 (the evaluation's FMA chain over all
-// the terms, and the interval part's own arithmetic), plus fit (the fits' residuals: the corner
-// values' coarse terms lie within fit of P), plus (cnt + 96) u s3 for P's coefficients,
-// s3 = sum |x| Mx My Mz over its terms: (cnt + 56)u for forming them (at most 9 roundings per
-// level and 16 levels for the ancestors, 12 per shell depth and one per further depth), 40u for the
-// restriction to the brick (3 rounded factors and 27 FMAs per coefficient; the blossom rows are
-// non-negative and sum to 1) and adding the two parts.
+// shell terms.  The margin is (2 cnt + 2 BR_WEXT + 8) u A over A = 1.01 (amax + s3) (the evaluation's
+// FMA chain over all the terms, and the interval part's own arithmetic), plus fit (the fits'
+// residuals: the corner values' coarse terms lie within fit of P), plus (cnt + 96) u s3 for P's
+// coefficients, s3 = sum |x| Mx My Mz over its terms: (cnt + 56)u for forming them (at most 9 roundings
+// per level and 16 levels for the ancestors, 12 per shell depth and one per further depth), 40u for the
+// restriction to the brick (three axes of 3 rounded factors and FMAs; the blossom rows are
+// non-negative and sum to 1) and adding the two parts.  Every operation of the margin rounds by at
+// most u relative and every term is non-negative, so scaling by 1 + 2^-16 bounds the exact value from
+// above; the tests are made as lo - iso > m and iso - hi > m, whose float differences are within u of
+// exact, which the last term's extra 2u covers.  (A non-finite bound compares false: not proven.)
 __device__ __forceinline__ signed char bound_sign_poly(float lo, float hi, float amax, float s3, float fit, int cnt,
                                                        float iso) {
     const float u = 5.9604644775390625e-08f;   // 2^-24
@@ -1427,145 +1305,323 @@ __device__ __forceinline__ signed char bound_sign_poly(float lo, float hi, float
 // row q of the blossom matrix that takes quadratic Bernstein coefficients over [0, S] to those over
 // [A, B] (0 <= A < B <= S, S a power of two <= 2^15): the blossom of the basis at (A, A), (A, B),
 // (B, B), divided by S^2 (exact in float for S <= 2^11, else rounded once); non-negative, sums to 1
-__device__ __forceinline__ void blossom_row(int A, int B, int S, int q, float out[3]) {
-    const i64 a = A, b = B, s = S;
-    i64 n0, n1, n2;
+__device__ __forceinline__ void blossom_row(unsigned a, unsigned b, unsigned s, int q, float out[3]) {
+    unsigned n0, n1, n2;   // below 2^31
     if (q == 0) { n0 = (s - a) * (s - a); n1 = 2 * a * (s - a); n2 = a * a; }
     else if (q == 1) { n0 = (s - a) * (s - b); n1 = a * (s - b) + b * (s - a); n2 = a * b; }
     else { n0 = (s - b) * (s - b); n1 = 2 * b * (s - b); n2 = b * b; }
-    const float inv = 1.0f / ((float)S * (float)S);
+    const float inv = 1.0f / ((float)s * (float)s);
     out[0] = (float)n0 * inv;
     out[1] = (float)n1 * inv;
     out[2] = (float)n2 * inv;
 }
 
-// one warp per brick: the bound over the corners the brick's leaf owns;
-// sign[bi] = 1 (all above iso), -1 (all below) or 0 (not proven).
+// shared memory of a warp that bounds bricks
+struct BoundShared {
+    float X[64], T1[48], T2[36];
+    int id[2][64];                 // nodes of the window cells at a depth, 4 x 4 x 4 (-1: none)
+    int anchor[SHELL_ANCHORS];
+};
+
+// The bound over the corners the leaf owns of the box of edge E at g0 (a brick or super-brick, one warp):
+// 1 (all above iso), -1 (all below) or 0 (not proven).
 //  * The coarse part, exact up to rounding and the tabulated values' noise: the leaf's ancestor
-//    polynomial (per root, k_brick_xl) and the shell terms of depths d <= D - lg E (shell_poly),
-//    bounded over the brick by the range of its Bernstein coefficients there.
-//  * The finer shell terms (depths d > D - lg E, one to three cells of the finest lattice wide
-//    around the leaf's faces) by intervals, as shell_terms sums them.
-constexpr int BB_BLOCK = 256;
-// A single-brick leaf whose own real corners change sign ('has_tri') is left unproven at once:
-// its brick's corners include the leaf's corners, so its bound straddles iso (and a brick left
-// unproven is only evaluated exactly, which changes no value).
-// (4 blocks per SM: 64 registers, no spills; unbounded it takes 104 and halves the resident warps)
-// The launch has up to 256 blocks per SM: bricks differ in cost (skipped, decided, deep windows), and
-// with 8 blocks per SM striding over all of them the last blocks ran alone (22.0 -> 15.9 ms at 4 M points,
-// 2.41 -> 1.90 on the 1M torus).
-__global__ void __launch_bounds__(BB_BLOCK, 4) k_brick_bound(VArgs v, BrickIndex bix, i64 first, i64 nbricks,
-                                                          const i64* __restrict__ sprefix,
-                                                          const signed char* __restrict__ ssign,
-                                                          const int* __restrict__ has_tri,
-                                                          signed char* __restrict__ sign) {
-    __shared__ int s_anchor[BB_BLOCK / 32][SHELL_ANCHORS];
-    __shared__ float s_stage[BB_BLOCK / 32][SHELL_POLY_BUF];
-    __shared__ float s_coef[BB_BLOCK / 32][27];   // the leaf's ancestor polynomial
+//    polynomial (per root, k_brick_xl), restricted to the box, and the shell terms of the depths of knot
+//    spacing >= E.  Each window cell outside the leaf with a real node contributes x Qx Qy Qz, Q the
+//    cell's PW entries (Bernstein form over the box).  The window spans at most PW = 4 cells per axis
+//    there (the box lies in one cell of depth d, and its first corner's owner may lie in the cell below),
+//    so the terms form a 4^3 grid X of x (0: no node, or inside the leaf; two cells per lane), contracted
+//    one axis at a time through shared memory:
+//      T1[n0 n1 l] = sum_n2 X Qz_l(n2),  T2[n0 j l] = sum_n1 T1 Qy_j(n1),  C_ijl += sum_n0 T2 Qx_i(n0)
+//    (lane k < 27 holds coefficient k = 9i + 3j + l).  s3 gains |x| Mx My Mz, fit
+//    |x| (dx My Mz + Mx dy Mz + Mx My dz) (as k_brick_xl's), cnt the number of terms.  The windows are
+//    nested, so a cell's node is the child of a cell of the window above, from the leaf's 27 neighbours.
+//    Bounded by the range of the Bernstein coefficients.
+//  * The finer shell terms only widen the bound (a term that some corners lack ranges over 0), so a box
+//    whose coarse part already straddles iso is left unproven without them.
+//  * First the finer terms together: at a corner the 27 terms of depth d are at most the largest |x| near
+//    the box times the product of the axes' sums of basis magnitudes (k_basis_sums), on the side of x's
+//    sign but for the basis values' negative noise.  The largest and least x come from the range of x
+//    below the nodes of the last coarse window (k_x_below) that the fine window touches: one load per
+//    depth and cell, where the terms themselves take a descent each.  In a dense shell this is also the
+//    tighter bound: a sum of intervals counts every cell of the window at its best corner.
+//  * Then, for a brick, the terms one by one (shell_terms).
+// Measured, bricks of leaves of edge >= 16 with their super-bricks: 4 M points, maxDepth 11, 8.3 M bricks
+// 15.9 -> 3.8 ms (92 % of the super-bricks decided, 36 % when they were bounded by interval products and
+// those at a leaf's face given up); 30 M points, maxDepth 12, 67 M bricks 147 -> 17; 1M torus 1.95 -> 0.42.
+__device__ __forceinline__ signed char bound_box(const VArgs& v, const BrickIndex& bix, int root, const VRoot& R,
+                                                 const int b[3], int E, const float* const row[3], int lane,
+                                                 BoundShared& sm) {
     const EvalArgs& a = v.e;
-    const int D = a.D;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const i64 warp = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
-    for (i64 bi = first + warp; bi < nbricks; bi += nwarps) {
-        const VBrick B = brick_of(v, bix, bi);
-        const VRoot R = v.roots[B.root];
-        if (ssign && v.e.D - R.depth >= 6) {   // decided by its super-brick?
-            const int ns = (1 << (v.e.D - R.depth)) / (4 * BR);
-            const signed char sg = ssign[sprefix[B.root] + ((i64)(B.b[0] >> 2) * ns + (B.b[1] >> 2)) * ns + (B.b[2] >> 2)];
-            if (sg != 0) {
-                if (lane == 0) sign[bi] = sg;
-                continue;
+    const NodeArrays& nd = a.nd;
+    const int D = a.D, r = R.depth, S = 1 << (D - r), L = R.node;
+    const int dpoly = D - (31 - __clz(E));   // depths of knot spacing >= E
+    int Lc[3];
+    key_coords(nd.key[L], r, D, Lc);
+    const int g0[3] = {Lc[0] * S + b[0] * E, Lc[1] * S + b[1] * E, Lc[2] * S + b[2] * E};
+    float s3 = 0.f, fit = 0.f, coef = 0.f;
+    int cnt = 0;
+    int plo[3] = {Lc[0] - 1, Lc[1] - 1, Lc[2] - 1}, cur = 0;
+    __syncwarp();   // the previous box's readers are done
+    {
+        const int n = lane < 27 ? nd.neigh[(i64)lane * nd.M + L] : -1;
+        sm.id[0][lane] = sm.id[0][lane + 32] = -1;
+        __syncwarp();
+        if (lane < 27) sm.id[0][(lane / 9) * 16 + ((lane / 3) % 3) * 4 + lane % 3] = n;
+    }
+    bool inside = false;
+    for (int d = r + 1; d <= dpoly; ++d) {
+        int wlo[3], ext[3];
+        bool cross = false;
+        for (int ax = 0; ax < 3; ++ax) {
+            bool c;
+            window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], c);
+            cross |= c;
+        }
+        if (!cross) { inside = true; break; }   // nested windows: the finer ones lie inside the leaf too
+        if (ext[0] > PW || ext[1] > PW || ext[2] > PW) return 0;   // (cannot happen)
+        const float4* pw[3];
+        for (int ax = 0; ax < 3; ++ax) pw[ax] = reinterpret_cast<const float4*>(row[ax] + d * PROW);
+        __syncwarp();
+        bool any = false;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int g = lane + 32 * h, n0 = g >> 4, n1 = (g >> 2) & 3, n2 = g & 3;
+            float x = 0.f;
+            int node = -1;
+            if (n0 < ext[0] && n1 < ext[1] && n2 < ext[2]) {
+                const int N[3] = {wlo[0] + n0, wlo[1] + n1, wlo[2] + n2};
+                const int p = sm.id[cur][((N[0] >> 1) - plo[0]) * 16 + ((N[1] >> 1) - plo[1]) * 4 + ((N[2] >> 1) - plo[2])];
+                const int c0 = p < 0 ? -1 : nd.child0[p];   // (the leaf itself has none: cells inside it come out absent)
+                if (c0 != -1) {
+                    node = c0 + (((N[0] & 1) << 2) | ((N[1] & 1) << 1) | (N[2] & 1));
+                    x = a.x[node];
+                }
+            }
+            sm.X[g] = x;
+            sm.id[cur ^ 1][g] = node;
+            if (x != 0.f) {
+                const float4 QX = pw[0][n0], QY = pw[1][n1], QZ = pw[2][n2];
+                const float Mx = bern_m(QX), My = bern_m(QY), Mz = bern_m(QZ), ax = fabsf(x);
+                s3 += ax * Mx * My * Mz;
+                fit += ax * (QX.w * My * Mz + Mx * QY.w * Mz + Mx * My * QZ.w);
+                ++cnt;
+                any = true;
             }
         }
-        const int r = R.depth, S = 1 << (D - r), L = R.node, E = brick_edge(D, r), nb = S / E;
-        if (nb == 1 && has_tri[L]) {
-            if (lane == 0) sign[bi] = 0;
-            continue;
+        cur ^= 1;
+        plo[0] = wlo[0]; plo[1] = wlo[1]; plo[2] = wlo[2];
+        if (!__any_sync(0xffffffffu, any)) continue;   // no real node near the box at this depth
+        __syncwarp();
+        for (int e = lane; e < 48; e += 32) {
+            const int nn = e / 3, l = e - 3 * nn;   // nn = 4 n0 + n1
+            float t = 0.f;
+#pragma unroll
+            for (int n2 = 0; n2 < 4; ++n2) t = fmaf(sm.X[4 * nn + n2], f4_at(pw[2][n2], l), t);
+            sm.T1[e] = t;
         }
-        int Lc[3];
-        key_coords(a.nd.key[L], r, D, Lc);
-        const int g0[3] = {Lc[0] * S + B.b[0] * E, Lc[1] * S + B.b[1] * E, Lc[2] * S + B.b[2] * E};
-        const float* row[3];
-        for (int ax = 0; ax < 3; ++ax) row[ax] = brick_row(bix, D, B.root, nb, ax, B.b[ax]);
-        const int dpoly = D - (31 - __clz(E));   // depths of knot spacing >= E
-        float lo = 0.f, hi = 0.f, amax = 0.f, s3 = 0.f, fit = 0.f, coef = 0.f;
-        int cnt = 0;
-        bool ok = true, inside = false;
-        int d = r + 1;
-        // real nodes around the leaf, at the virtual depths: coarse ones into the polynomial
-        for (; d <= dpoly; ++d) {
+        __syncwarp();
+        for (int e = lane; e < 36; e += 32) {
+            const int n0 = e / 9, j = (e / 3) % 3, l = e % 3;
+            float t = 0.f;
+#pragma unroll
+            for (int n1 = 0; n1 < 4; ++n1) t = fmaf(sm.T1[(4 * n0 + n1) * 3 + l], f4_at(pw[1][n1], j), t);
+            sm.T2[e] = t;
+        }
+        __syncwarp();
+        if (lane < 27) {
+            const int i = lane / 9, jl = lane % 9;
+            float t = 0.f;
+#pragma unroll
+            for (int n0 = 0; n0 < 4; ++n0) t = fmaf(sm.T2[9 * n0 + jl], f4_at(pw[0][n0], i), t);
+            coef += t;
+        }
+    }
+    // the ancestor polynomial's coefficients over the box (lane k < 27: coefficient k = 9i + 3j + l), one
+    // axis at a time through the blossom rows (the identity for a single-brick leaf), plus the shell part
+    const float* an = bix.anc + (i64)root * ANC_STRIDE;
+    float c = lane < 27 ? an[lane] : 0.f;
+    if (S > E) {
+        const int i = lane / 9, j = (lane / 3) % 3, l = lane % 3;
+        float t[3];
+        blossom_row(b[2] * E, (b[2] + 1) * E, S, l, t);
+        {
+            const int q = lane - l;
+            const float c0 = __shfl_sync(0xffffffffu, c, q), c1 = __shfl_sync(0xffffffffu, c, (q + 1) & 31),
+                        c2 = __shfl_sync(0xffffffffu, c, (q + 2) & 31);
+            c = fmaf(c2, t[2], fmaf(c1, t[1], c0 * t[0]));
+        }
+        blossom_row(b[1] * E, (b[1] + 1) * E, S, j, t);
+        {
+            const int q = lane - 3 * j;
+            const float c0 = __shfl_sync(0xffffffffu, c, q), c1 = __shfl_sync(0xffffffffu, c, (q + 3) & 31),
+                        c2 = __shfl_sync(0xffffffffu, c, (q + 6) & 31);
+            c = fmaf(c2, t[2], fmaf(c1, t[1], c0 * t[0]));
+        }
+        blossom_row(b[0] * E, (b[0] + 1) * E, S, i, t);
+        {
+            const int q = lane - 9 * i;
+            const float c0 = __shfl_sync(0xffffffffu, c, q), c1 = __shfl_sync(0xffffffffu, c, (q + 9) & 31),
+                        c2 = __shfl_sync(0xffffffffu, c, (q + 18) & 31);
+            c = fmaf(c2, t[2], fmaf(c1, t[1], c0 * t[0]));
+        }
+    }
+    c += coef;
+    float cmin = lane < 27 ? c : INFINITY, cmax = lane < 27 ? c : -INFINITY;
+    for (int o = 16; o; o >>= 1) {
+        s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+        fit += __shfl_xor_sync(0xffffffffu, fit, o);
+        // (a value that is not a number must not drop out of the range)
+        const float p = __shfl_xor_sync(0xffffffffu, cmin, o), q = __shfl_xor_sync(0xffffffffu, cmax, o);
+        cmin = (p < cmin || p != p) ? p : cmin;
+        cmax = (q > cmax || q != q) ? q : cmax;
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt) + (int)an[28];
+    s3 += an[27];
+    fit += an[29];
+    const signed char coarse = bound_sign_poly(cmin, cmax, 0.f, s3, fit, cnt, v.iso);
+    if (coarse == 0 || inside) return coarse;
+    // the finer terms together
+    {
+        float flo = 0.f, fhi = 0.f, famax = 0.f;
+        int fcnt = 0;
+        for (int d = dpoly + 1; d <= D; ++d) {
+            const int k = d - dpoly;
             int wlo[3], ext[3];
             bool cross = false;
             for (int ax = 0; ax < 3; ++ax) {
-                bool c;
-                window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], c);
-                cross |= c;
+                bool cr;
+                window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], cr);
+                cross |= cr;
             }
-            if (!cross) { inside = true; break; }   // nested windows: the finer ones lie inside the leaf too
-            if (ext[0] > PW || ext[1] > PW || ext[2] > PW) { ok = false; break; }   // (cannot happen)
-            const float4* pw[3];
-            for (int ax = 0; ax < 3; ++ax) pw[ax] = reinterpret_cast<const float4*>(row[ax] + d * PROW);
-            shell_poly(v, L, r, Lc, d, wlo, ext, pw, lane, s_stage[w], coef, s3, fit, cnt);
-        }
-        // the finer ones by intervals; only window cells outside the leaf can hold a real node
-        if (ok && !inside) {
-            for (; d <= D; ++d) {
-                int wlo[3], ext[3];
-                bool cross = false;
-                for (int ax = 0; ax < 3; ++ax) {
-                    bool c;
-                    window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], c);
-                    cross |= c;
+            if (!cross) break;
+            unsigned neg = 0, pos = 0;   // bits of the largest magnitudes on either side
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int g = lane + 32 * h;
+                const int N[3] = {plo[0] + (g >> 4), plo[1] + ((g >> 2) & 3), plo[2] + (g & 3)};
+                const int node = sm.id[cur][g];
+                bool touch = node >= 0;
+#pragma unroll
+                for (int ax = 0; ax < 3; ++ax) touch &= N[ax] >= (wlo[ax] >> k) && N[ax] <= ((wlo[ax] + ext[ax] - 1) >> k);
+                if (touch) {
+                    const float2 q = bix.below[BELOW * (node - bix.below0) + k - 1];
+                    neg = max(neg, __float_as_uint(-q.x) & 0x7fffffffu);
+                    pos = max(pos, __float_as_uint(q.y) & 0x7fffffffu);
                 }
-                if (!cross) break;
-                const float2* rw[3];
-                for (int ax = 0; ax < 3; ++ax) rw[ax] = reinterpret_cast<const float2*>(row[ax] + d * PROW);
-                shell_terms(v, L, r, Lc, d, D, wlo, ext, rw, lane, s_anchor[w], lo, hi, amax, cnt);
             }
+            const float xn = __uint_as_float(__reduce_max_sync(0xffffffffu, neg)),
+                        xp = __uint_as_float(__reduce_max_sync(0xffffffffu, pos)), xm = fmaxf(xn, xp);
+            if (xm == 0.f) continue;
+            const float2 bs = bix.bsum[d];
+            const float up = 1.0f + 9.5367431640625e-07f;
+            const float r3 = bs.x * bs.x * bs.x * up, n3 = 3.f * bs.y * bs.x * bs.x * up;
+            flo -= (xn * r3 + xm * n3) * up;
+            fhi += (xp * r3 + xm * n3) * up;
+            famax += xm * r3 * up;
+            fcnt += 27;
         }
-        // the coarse polynomial's Bernstein coefficients over the brick: the leaf's ancestor
-        // polynomial restricted to it (lane k < 27: coefficient k = 9i + 3j + l, through the
-        // blossom rows i, j, l of the three axes; the identity for a single-brick leaf) plus the
-        // shell part
-        const float* an = bix.anc + (i64)B.root * ANC_STRIDE;
-        __syncwarp();   // the previous brick's readers are done
-        if (lane < 27) s_coef[w][lane] = an[lane];
-        __syncwarp();
-        float cmin = INFINITY, cmax = -INFINITY;
-        if (lane < 27) {
-            float c = s_coef[w][lane];
-            if (nb > 1) {
-                float tx[3], ty[3], tz[3];
-                blossom_row(B.b[0] * E, (B.b[0] + 1) * E, S, lane / 9, tx);
-                blossom_row(B.b[1] * E, (B.b[1] + 1) * E, S, (lane / 3) % 3, ty);
-                blossom_row(B.b[2] * E, (B.b[2] + 1) * E, S, lane % 3, tz);
-                c = 0.f;
+        const signed char sg = bound_sign_poly(cmin + flo, cmax + fhi, famax, s3, fit, cnt + fcnt, v.iso);
+        if (sg != 0 || E > BR) return sg;
+    }
+    // the finer terms one by one; only window cells outside the leaf can hold a real node
+    float lo = 0.f, hi = 0.f, amax = 0.f;
+    int fcnt = 0;
+    for (int d = max(dpoly, r) + 1; d <= D; ++d) {
+        int wlo[3], ext[3];
+        bool cross = false;
+        for (int ax = 0; ax < 3; ++ax) {
+            bool cr;
+            window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], cr);
+            cross |= cr;
+        }
+        if (!cross) break;
+        const float2* rw[3];
+        for (int ax = 0; ax < 3; ++ax) rw[ax] = reinterpret_cast<const float2*>(row[ax] + d * PROW);
+        shell_terms(v, L, r, Lc, d, D, wlo, ext, rw, lane, sm.anchor, lo, hi, amax, fcnt);
+    }
+    for (int o = 16; o; o >>= 1) {
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+        amax += __shfl_xor_sync(0xffffffffu, amax, o);
+    }
+    fcnt = __reduce_add_sync(0xffffffffu, fcnt);
+    return bound_sign_poly(cmin + lo, cmax + hi, amax, s3, fit, cnt + fcnt, v.iso);
+}
+
+// One warp per super-brick (4^3 bricks of leaves with lattice edge >= 64): decided, its bricks get its sign;
+// undecided, it joins the list whose bricks k_brick_bound takes.
+constexpr int BB_BLOCK = 256;
+__global__ void __launch_bounds__(BB_BLOCK, 4) k_super_bound(VArgs v, BrickIndex bix, const i64* __restrict__ srow_prefix,
+                                                            const float* __restrict__ srows, i64 nsuper,
+                                                            signed char* __restrict__ sign, int* __restrict__ nopen,
+                                                            i64* __restrict__ open) {
+    __shared__ BoundShared sm[BB_BLOCK / 32];
+    const int D = v.e.D;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const DepthLayout& dl = bix.dl;
+    const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
+    for (i64 si = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; si < nsuper; si += nwarps) {
+        int dd = 0;
+        while (dd < D - 1 && dl.soff[dd + 1] <= si) ++dd;
+        const i64 loc = si - dl.soff[dd];
+        const int slg = dl.slg[dd], ns = 1 << slg;
+        const int root = dl.first[dd] + (int)(loc >> (3 * slg));
+        const VRoot R = v.roots[root];
+        const i64 l = loc & ((1ll << (3 * slg)) - 1);
+        const int b[3] = {(int)(l >> (2 * slg)), (int)(l >> slg) & (ns - 1), (int)l & (ns - 1)};
+        const float* row[3];
+        for (int ax = 0; ax < 3; ++ax) row[ax] = brick_row(srows, srow_prefix, D, root, ns, ax, b[ax]);
+        const signed char sg = bound_box(v, bix, root, R, b, SUPER, row, lane, sm[w]);
+        const int nb = 4 * ns;
+        const i64 first = bix.prefix[root] + ((i64)(4 * b[0]) * nb + 4 * b[1]) * nb + 4 * b[2];
+        if (sg != 0) {
 #pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        const float tij = tx[i] * ty[j];
-#pragma unroll
-                        for (int l = 0; l < 3; ++l) c = fmaf(s_coef[w][9 * i + 3 * j + l], tij * tz[l], c);
-                    }
+            for (int h = 0; h < 2; ++h) {
+                const int g = lane + 32 * h;
+                sign[first + ((i64)(g >> 4) * nb + ((g >> 2) & 3)) * nb + (g & 3)] = sg;
             }
-            c += coef;
-            cmin = cmax = c;
+        } else if (lane == 0) {
+            open[atomicAdd(nopen, 1)] = first;
         }
-        for (int o = 16; o; o >>= 1) {
-            lo += __shfl_xor_sync(0xffffffffu, lo, o);
-            hi += __shfl_xor_sync(0xffffffffu, hi, o);
-            amax += __shfl_xor_sync(0xffffffffu, amax, o);
-            s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-            fit += __shfl_xor_sync(0xffffffffu, fit, o);
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
-            cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    }
+}
+
+// One warp per brick: sign[bi] = 1 (all above iso), -1 (all below) or 0 (not proven), for the bricks of
+// the undecided super-bricks ('open': their first bricks) and those of [first, nbricks).
+// A single-brick leaf whose own real corners change sign ('has_tri') is left unproven at once:
+// its brick's corners include the leaf's corners, so its bound straddles iso (and a brick left
+// unproven is only evaluated exactly, which changes no value).
+// The launch has up to 256 blocks per SM: bricks differ in cost, and with 8 blocks per SM striding over
+// all of them the last blocks ran alone (22.0 -> 15.9 ms at 4 M points, 2.41 -> 1.90 on the 1M torus).
+__global__ void __launch_bounds__(BB_BLOCK, 4) k_brick_bound(VArgs v, BrickIndex bix, const int* __restrict__ nopen,
+                                                          const i64* __restrict__ open, i64 first, i64 nbricks,
+                                                          const int* __restrict__ has_tri,
+                                                          signed char* __restrict__ sign) {
+    __shared__ BoundShared sm[BB_BLOCK / 32];
+    const int D = v.e.D;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const i64 nsub = nopen ? 64ll * *nopen : 0;
+    const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
+    for (i64 it = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < nsub + (nbricks - first); it += nwarps) {
+        i64 bi = first + it - nsub;
+        if (it < nsub) {
+            const i64 f = open[it >> 6];
+            const VBrick F = brick_of(v, bix, f);
+            const i64 nb = 1ll << bix.dl.lg[v.roots[F.root].depth];
+            const int g = (int)it & 63;
+            bi = f + ((i64)(g >> 4) * nb + ((g >> 2) & 3)) * nb + (g & 3);
         }
-        if (lane == 0)
-            sign[bi] = ok ? bound_sign_poly(cmin + lo, cmax + hi, amax, s3 + an[27], fit + an[29], cnt + (int)an[28], v.iso)
-                          : (signed char)0;
+        const VBrick B = brick_of(v, bix, bi);
+        const VRoot R = v.roots[B.root];
+        const int r = R.depth, E = brick_edge(D, r), nb = (1 << (D - r)) / E;
+        signed char sg = 0;
+        if (!(nb == 1 && has_tri[R.node])) {
+            const float* row[3];
+            for (int ax = 0; ax < 3; ++ax) row[ax] = brick_row(bix.rows, bix.row_prefix, D, B.root, nb, ax, B.b[ax]);
+            sg = bound_box(v, bix, B.root, R, B.b, E, row, lane, sm[w]);
+        }
+        if (lane == 0) sign[bi] = sg;
     }
 }
 
@@ -2472,7 +2528,7 @@ void stage_mesh(Ctx& c) {
     int2* droot_list = nullptr;
     int nr = 0;
     RootLayout layout{};
-    i64 tot[4] = {0, 0, 0, 0}, nbig = 0;
+    i64 tot[4] = {0, 0, 0, 0}, nbig = 0, nlarge = 0;
     int nbatches = 1;
     {
         int* rpos = dalloc<int>(nCoarse + 1, s);
@@ -2507,7 +2563,8 @@ void stage_mesh(Ctx& c) {
                 layout.off[q][d] = tot[q];
                 tot[q] += (i64)cnt * layout.per[q][d];
             }
-            if (D - d >= 4) nbig = tot[0];   // bricks of leaves with lattice edge >= 16 come first
+            if (D - d >= 6) nlarge = tot[0];   // bricks of leaves with lattice edge >= 64 (super-bricks) come first
+            if (D - d >= 4) nbig = tot[0];     // then those of edge >= 16
             if (d < 3) nb += cnt;
             else if (cnt > 0) layout.batch[d] = ++nb;
         }
@@ -2569,15 +2626,23 @@ void stage_mesh(Ctx& c) {
         CK_LAUNCH();
         va.roots = droots;
         va.batch_root_flag = bflag;
-        const i64 nbricks = tot[0], nrows = tot[1], nsuper = tot[2], nsrows = tot[3];
+        const i64 nbricks = tot[0], nsuper = tot[2], nsrows = tot[3];
+        // Leaves of edge 2 (depth D - 1, the last roots) are not bounded but evaluated: the bound proves 1 to
+        // 9 % of them (4 M points at maxDepth 11, 1M torus) and, with its tables, costs 8 ns a brick where
+        // the evaluation takes 2.6.
+        const i64 nbound = layout.off[0][D - 1], nrows = layout.off[1][D - 1];
+        const int nrbound = layout.first[D - 1];
         i64* dbpre = dpre;
         i64* drpre = dpre + nr + 1;
         i64* dspre = dpre + 2 * (nr + 1);
         i64* dsrpre = dpre + 3 * (nr + 1);
         float* rows = dalloc<float>(nrows * PROW * (D + 1), s);
         int* up = dalloc<int>((i64)nr * BR_LEVELS, s);
-        float* anc = dalloc<float>((i64)nr * ANC_STRIDE, s);
-        BrickIndex bix{dbpre, drpre, nr, rows, up, anc, {}};
+        float* anc = dalloc<float>((i64)nrbound * ANC_STRIDE, s);
+        const i64 below0 = c.base[std::max(D - BELOW, 0)];
+        float2* below = dalloc<float2>(BELOW * (lo - below0), s);
+        float2* bsum = dalloc<float2>(D + 1, s);
+        BrickIndex bix{dbpre, drpre, nr, rows, up, anc, below, below0, bsum, {}};
         for (int d = 0; d <= D; ++d) {
             bix.dl.first[d] = layout.first[d];
             bix.dl.lg[d] = std::max(D - d - 3, 0);          // bricks per edge 2^(D-d) / min(2^(D-d), 8)
@@ -2589,17 +2654,28 @@ void stage_mesh(Ctx& c) {
         }
         c.kend(kg);
         const int kr = c.kbegin("brick_rows", (double)nrows * PROW * (D + 1) * 4);
-        k_brick_rows<<<grid_for(nrows * (D + 1), 128), 128, 0, s>>>(va, bix.dl, nrows, 0, c.d_has_tri, rows);
-        CK_LAUNCH();
+        if (nrows > 0) {
+            k_brick_rows<<<grid_for(nrows * (D + 1), 128), 128, 0, s>>>(va, bix.dl, nrows, 0, c.d_has_tri, rows);
+            CK_LAUNCH();
+        }
         float* srows = nullptr;
         if (nsrows > 0) {
-            srows = dalloc<float>(nsrows * ROW_PER_DEPTH * (D + 1), s);
+            srows = dalloc<float>(nsrows * PROW * (D + 1), s);
             k_brick_rows<<<grid_for(nsrows * (D + 1), 128), 128, 0, s>>>(va, bix.dl, nsrows, 1, c.d_has_tri, srows);
             CK_LAUNCH();
         }
         k_root_up<<<grid_for(nr, 256), 256, 0, s>>>(nd, droots, nr, up);
         CK_LAUNCH();
-        k_brick_xl<<<grid_for((i64)nr * 32, 32 * XL_WARPS), 32 * XL_WARPS, 0, s>>>(va, nr, c.d_has_tri, up, anc);
+        if (nrbound > 0) {
+            k_brick_xl<<<grid_for((i64)nrbound * 32, 32 * XL_WARPS), 32 * XL_WARPS, 0, s>>>(va, nrbound, c.d_has_tri, up, anc);
+            CK_LAUNCH();
+        }
+        for (int d = D - 1; d >= std::max(D - BELOW, 0); --d) {
+            k_x_below<<<grid_for(c.count[d], 256, 1ll << 30), 256, 0, s>>>(nd, c.x, c.base[d], c.base[d + 1], below0, D - d,
+                                                                           below);
+            CK_LAUNCH();
+        }
+        k_basis_sums<<<D + 1, 256, 0, s>>>(lb, D, bsum);
         CK_LAUNCH();
         c.kend(kr);
         unsigned char* culled = dalloc<unsigned char>(nbricks, s);
@@ -2609,43 +2685,47 @@ void stage_mesh(Ctx& c) {
         k_root_of<<<grid_for(nr, 256), 256, 0, s>>>(droots, nr, root_of);
         CK_LAUNCH();
         // compulsory: every brick row and the leaves' ancestor polynomial (super-bricks: their
-        // rows and the neighbour x) once, the sign written and read, the culled flag written
-        signed char* ssign = nullptr;
+        // rows) once, the sign written and read, the culled flag written
+        int* nopen = nullptr;
+        i64* open = nullptr;
         if (nsuper > 0) {
-            ssign = dalloc<signed char>(nsuper, s);
-            const int ksb = c.kbegin("super_bound", (double)nsrows * (6 + 2 * BR_WEXT) * (D + 1) * 4 +
-                                                        (double)nr * BR_LEVELS * 27 * 4 + (double)nsuper);
-            k_super_bound<<<grid_for(nsuper * 32, 256, (i64)c.sms * 8), 256, 0, s>>>(va, bix.dl, dsrpre, srows, up,
-                                                                                    nsuper, ssign);
+            nopen = dalloc<int>(1, s);
+            open = dalloc<i64>(nsuper, s);
+            CK(cudaMemsetAsync(nopen, 0, sizeof(int), s));
+            const int ksb = c.kbegin("super_bound", (double)nsrows * PROW * (D + 1) * 4 + (double)nr * ANC_STRIDE * 4 +
+                                                        (double)nlarge);
+            k_super_bound<<<grid_for(nsuper * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(va, bix, dsrpre, srows,
+                                                                                                nsuper, bsign, nopen, open);
             CK_LAUNCH();
             c.kend(ksb);
             if (c.profile) {   // statistics only
-                std::vector<signed char> hs(nsuper);
-                CK(cudaMemcpyAsync(hs.data(), ssign, nsuper, cudaMemcpyDeviceToHost, s));
-                CK(cudaStreamSynchronize(s));
                 c.super_bricks = nsuper;
-                c.super_decided = 0;
-                for (signed char v : hs) c.super_decided += (v != 0);
+                c.super_decided = nsuper - read_scalar(nopen, s);
             }
         }
-        // bricks of leaves with lattice edge >= 16 come first (roots are in depth order)
         const int kb = c.kbegin("brick_bound", (double)nrows * PROW * (D + 1) * 4 +
-                                                   (double)nr * ANC_STRIDE * 4 + (double)nbricks * 3);
-        k_brick_bound<<<grid_for(nbig * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(va, bix, 0, nbig, dspre,
-                                                                                         ssign, c.d_has_tri, bsign);
-        CK_LAUNCH();
+                                                   (double)nrbound * ANC_STRIDE * 4 + (double)nbound * 3);
+        if (nbig > 0) {
+            k_brick_bound<<<grid_for(nbig * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(
+                va, bix, nopen, open, nlarge, nbig, c.d_has_tri, bsign);
+            CK_LAUNCH();
+        }
         c.kend(kb);
-        const int kb2 = c.kbegin("brick_bound_small", (double)(nbricks - nbig) * 3);
-        if (nbricks > nbig) {
-            k_brick_bound<<<grid_for((nbricks - nbig) * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(
-                va, bix, nbig, nbricks, dspre, ssign, c.d_has_tri, bsign);
+        const int kb2 = c.kbegin("brick_bound_small", (double)(nbound - nbig) * 3);
+        CK(cudaMemsetAsync(bsign + nbound, 0, nbricks - nbound, s));
+        if (nbound > nbig) {
+            k_brick_bound<<<grid_for((nbound - nbig) * 32, BB_BLOCK, (i64)c.sms * 256), BB_BLOCK, 0, s>>>(
+                va, bix, nullptr, nullptr, nbig, nbound, c.d_has_tri, bsign);
             CK_LAUNCH();
         }
         k_brick_cull<<<grid_for(nbricks, 256), 256, 0, s>>>(va, bix, root_of, bsign, nbricks, culled);
         CK_LAUNCH();
         c.kend(kb2);
         dfree(bsign, s);
-        dfree(ssign, s);
+        dfree(nopen, s);
+        dfree(open, s);
+        dfree(below, s);
+        dfree(bsum, s);
         dfree(srows, s);
         dfree(anc, s);
         kg = c.kbegin("mesh_lists", 0.0);
