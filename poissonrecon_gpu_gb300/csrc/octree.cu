@@ -9,6 +9,13 @@
 // structure, so no hash table or atomic is needed and every field is exact
 // (the reference's racy parent assignment, main.cu:331,357, is not reproduced:
 // every slot receives its true parent).
+//
+// A point starts a run at every depth from the first at which its key differs
+// from its predecessor's, so one pass over the points counts the runs of all
+// depths, and a second one writes all depths' runs; one launch then fills the
+// nodes of all depths.  Depth by depth (flags, scan, the count read back, runs,
+// slots, fill) the stage was a chain of some ten launches and a host round trip
+// per depth: 0.50 of the 2.65 ms of 5,000 points at maxDepth 6.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -60,11 +67,32 @@ __global__ void k_bbox(const float* __restrict__ xyz, i64 n, unsigned* __restric
     }
 }
 
+// scale and corner of the cube from the box (ordered bits of min x y z, max x y z), as the reference's host
+// code computes them (main.cu:530-553)
+struct Cube {
+    float corner[3], scale;
+};
+__host__ __device__ inline Cube cube_of(const unsigned* mm) {
+    Cube c;
+    float scale = 1;
+    for (int a = 0; a < 3; ++a) {
+        const float mn = ord2f(mm[a]), mx = ord2f(mm[3 + a]);
+        if (!a || scale < mx - mn) scale = float(mx - mn);
+        c.corner[a] = float(mx + mn) / 2;
+    }
+    scale *= 1.25f;
+    for (int a = 0; a < 3; ++a) c.corner[a] -= scale / 2;
+    c.scale = scale;
+    return c;
+}
+
 // ----------------- normalisation + Morton key (main.cu:132-173,555-569) ------
 __global__ void k_normalise_encode(const float* __restrict__ in_xyz, const float* __restrict__ in_nrm, i64 n,
-                                   float cx, float cy, float cz, float scale, float nscale, int D,
+                                   const unsigned* __restrict__ mm, float nscale, int D,
                                    float* __restrict__ p_out, float* __restrict__ n_out, u64* __restrict__ keys,
                                    uint32_t* __restrict__ idx) {
+    const Cube cube = cube_of(mm);
+    const float cx = cube.corner[0], cy = cube.corner[1], cz = cube.corner[2], scale = cube.scale;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         float p[3] = {(in_xyz[3 * i] - cx) / scale, (in_xyz[3 * i + 1] - cy) / scale, (in_xyz[3 * i + 2] - cz) / scale};
         float nx = in_nrm[3 * i], ny = in_nrm[3 * i + 1], nz = in_nrm[3 * i + 2];
@@ -104,94 +132,143 @@ __global__ void k_gather_points(const uint32_t* __restrict__ idx, i64 n, const f
 }
 
 // ------------------------------- runs ---------------------------------------
-// head flag of a run of equal masked keys
-__global__ void k_head_flags(const u64* __restrict__ k, i64 n, u64 mask, int* __restrict__ f) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
-        f[i] = (i == 0 || ((k[i] & mask) != (k[i - 1] & mask))) ? 1 : 0;
-}
-// compacts run heads: unique key, first source index; every element learns its run rank
-__global__ void k_runs(const u64* __restrict__ k, i64 n, u64 mask, const int* __restrict__ f,
-                       const int* __restrict__ pos, u64* __restrict__ ukey, int* __restrict__ ufirst,
-                       int* __restrict__ rank_of) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        int r = pos[i] + f[i] - 1;
-        if (rank_of) rank_of[i] = r;
-        if (f[i]) {
-            ukey[r] = k[i] & mask;
-            ufirst[r] = (int)i;
-        }
-    }
-}
-__global__ void k_iota(int* __restrict__ out, i64 n) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) out[i] = (int)i;
-}
-// first point of a unique node = first point of its first child run
-__global__ void k_compose(const int* __restrict__ a, const int* __restrict__ b, i64 n, int* __restrict__ out) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) out[i] = a[b[i]];
-}
-// slot of each unique node inside its parent's group of 8, and the slot -> unique map
-__global__ void k_unique_slots(const u64* __restrict__ ukey, const int* __restrict__ uparent, i64 nu, int shift,
-                               int* __restrict__ uslot, int* __restrict__ slot2u) {
-    for (i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x; r < nu; r += (i64)gridDim.x * blockDim.x) {
-        int s = 8 * uparent[r] + (int)((ukey[r] >> shift) & 7);
-        uslot[r] = s;
-        slot2u[s] = (int)r;
-    }
+// first depth at which sorted point i differs from its predecessor: 0 for the first point, D + 1 when the
+// keys are equal (the point starts no run)
+__device__ __forceinline__ int first_depth(const u64* __restrict__ keys, i64 i, int D) {
+    if (i == 0) return 0;
+    const u64 x = keys[i] ^ keys[i - 1];
+    return x ? D - (63 - __clzll((i64)x)) / 3 : D + 1;
 }
 
-struct LevelArgs {
-    int d, D;
-    i64 base_prev, base_d, base_next;
-    i64 n_slots;          // count[d]
-    i64 N;                // points
-    i64 u_d, u_dm1;       // unique nodes at d and d-1
-    i64 u_last;           // unique nodes at depth D-1
+constexpr int LV_BLOCK = 256;
+constexpr int LV_ROUNDS = 4;
+constexpr int LV_TILE = LV_BLOCK * LV_ROUNDS;
+constexpr int LV_MAX = PRGPU_MAX_DEPTH + 1;   // depths 0..15
+
+// runs that start in each tile of LV_TILE points, per depth: cnt[d * ntiles + tile]
+__global__ void __launch_bounds__(LV_BLOCK) k_run_count(const u64* __restrict__ keys, i64 n, int D, i64 ntiles,
+                                                        int* __restrict__ cnt) {
+    __shared__ int h[LV_MAX];
+    if (threadIdx.x < LV_MAX) h[threadIdx.x] = 0;
+    __syncthreads();
+    int mine = 0;   // lane d: the warp's runs of depth d
+    for (int q = 0; q < LV_ROUNDS; ++q) {
+        const i64 i = (i64)blockIdx.x * LV_TILE + q * LV_BLOCK + threadIdx.x;
+        const int L = i < n ? first_depth(keys, i, D) : D + 1;
+        for (int d = 0; d <= D; ++d) {
+            const int c = __popc(__ballot_sync(0xffffffffu, L <= d));
+            if ((int)(threadIdx.x & 31) == d) mine += c;
+        }
+    }
+    if ((int)(threadIdx.x & 31) <= D) atomicAdd(&h[threadIdx.x & 31], mine);
+    __syncthreads();
+    if ((int)threadIdx.x <= D) cnt[(i64)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
+}
+
+// exclusive scan of each depth's counts over the tiles, in place (a block per depth); totals to U[d]
+__global__ void __launch_bounds__(1024) k_run_offsets(int* __restrict__ cnt, i64 ntiles, int* __restrict__ U) {
+    __shared__ int sw[32];
+    int* c = cnt + (i64)blockIdx.x * ntiles;
+    int run = 0;
+    for (i64 t0 = 0; t0 < ntiles; t0 += 1024) {
+        const i64 t = t0 + threadIdx.x;
+        const int v = t < ntiles ? c[t] : 0;
+        int total;
+        const int e = block_exclusive_sum<int>(v, sw, &total);
+        if (t < ntiles) c[t] = run + e;
+        run += total;
+    }
+    if (threadIdx.x == 0) U[blockIdx.x] = run;
+}
+
+// the runs of all depths
+struct Levels {
+    u64* key[LV_MAX];     // unique prefix (levels below masked)
+    int* pidx[LV_MAX];    // first point
+    int* slot[LV_MAX];    // slot among the depth's nodes: 8 * the parent's run + child code
+    int* first[LV_MAX];   // depths < D: first run one depth below
+    int* lo[LV_MAX];      // depths < D: first run of depth D - 1 below (its own number at D - 1)
+    int U[LV_MAX];        // runs
+    i64 base[LV_MAX + 1]; // first node of each depth
 };
 
-// fills one depth of the node arrays (one thread per slot); the empty-slot
-// conventions follow updateEmptyNodeInfo (main.cu:433-490)
-__global__ void k_fill_level(LevelArgs a, const u64* __restrict__ ukey_prev, const int* __restrict__ uslot_prev,
-                             const int* __restrict__ upidx_prev, const int* __restrict__ ulo_prev,
-                             const int* __restrict__ upidx_d, const int* __restrict__ ulo_d,
-                             const int* __restrict__ slot2u, NodeArrays nd) {
-    for (i64 s = (i64)blockIdx.x * blockDim.x + threadIdx.x; s < a.n_slots; s += (i64)gridDim.x * blockDim.x) {
-        const i64 g = s >> 3;
-        const int k = (int)(s & 7);
-        const i64 i = a.base_d + s;
-        const int shift = 3 * (a.D - a.d);
-        nd.key[i] = ukey_prev[g] | ((u64)k << shift);
-        nd.depth[i] = (int8_t)a.d;
-        nd.parent[i] = (int)(a.base_prev + uslot_prev[g]);
-        // per-sibling point and finest-slot counts
-        int ppre = 0, dpre = 0;
-        int my_pnum = 0, my_dnum = 0;
-        int r_self = -1;
-        for (int q = 0; q < 8; ++q) {
-            int r = slot2u[8 * g + q];
-            int pn = 0, dn = 0;
-            if (r >= 0) {
-                i64 next_p = (r + 1 < a.u_d) ? upidx_d[r + 1] : a.N;
-                pn = (int)(next_p - upidx_d[r]);
-                if (a.d < a.D) {
-                    i64 hi = (r + 1 < a.u_d) ? ulo_d[r + 1] : a.u_last;
-                    dn = (int)(8 * (hi - ulo_d[r]));
-                }
-            }
-            if (q < k) { ppre += pn; dpre += dn; }
-            if (q == k) { my_pnum = pn; my_dnum = dn; r_self = r; }
+__global__ void __launch_bounds__(LV_BLOCK) k_runs(const u64* __restrict__ keys, i64 n, int D, i64 ntiles,
+                                                   const int* __restrict__ off, Levels lv, int* __restrict__ point_node) {
+    __shared__ int wcnt[LV_BLOCK / 32][LV_MAX];
+    __shared__ int run[LV_MAX];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((int)threadIdx.x <= D) run[threadIdx.x] = off[(i64)threadIdx.x * ntiles + blockIdx.x];
+    const unsigned upto = 0xffffffffu >> (31 - lane);
+    for (int q = 0; q < LV_ROUNDS; ++q) {
+        const i64 i = (i64)blockIdx.x * LV_TILE + q * LV_BLOCK + threadIdx.x;
+        const int L = i < n ? first_depth(keys, i, D) : D + 1;
+        for (int d = 0; d <= D; ++d) {
+            const int c = __popc(__ballot_sync(0xffffffffu, L <= d));
+            if (lane == d) wcnt[w][d] = c;
         }
-        nd.pnum[i] = my_pnum;
-        nd.pidx[i] = upidx_prev[g] + ppre;
-        if (a.d == a.D) {
+        __syncthreads();
+        int before = 0, all = 0;   // lane d: runs of depth d before this warp, and in the round
+        if (lane <= D) {
+            for (int k = 0; k < LV_BLOCK / 32; ++k) {
+                if (k < w) before += wcnt[k][lane];
+                all += wcnt[k][lane];
+            }
+            before += run[lane];
+        }
+        const u64 key = i < n ? keys[i] : 0ull;
+        const unsigned b1 = __ballot_sync(0xffffffffu, L < D);
+        const int last = __shfl_sync(0xffffffffu, before, D - 1) + __popc(b1 & upto) - 1;   // its run of depth D - 1
+        int up = 0;                // this point's run one depth above
+        for (int d = 0; d <= D; ++d) {
+            const unsigned b = __ballot_sync(0xffffffffu, L <= d);
+            const int r = __shfl_sync(0xffffffffu, before, d) + __popc(b & upto) - 1;
+            const int slot = d ? 8 * up + (int)((key >> (3 * (D - d))) & 7) : 0;
+            if (L <= d) {
+                lv.key[d][r] = d ? key & ~((1ull << (3 * (D - d))) - 1) : 0ull;
+                lv.pidx[d][r] = (int)i;
+                lv.slot[d][r] = slot;
+                if (d < D) lv.lo[d][r] = last;
+                if (L < d) lv.first[d - 1][up] = r;   // the first run below the run that starts above
+            }
+            if (d == D && i < n) point_node[i] = (int)lv.base[D] + slot;
+            up = r;
+        }
+        __syncthreads();
+        if (w == 0 && lane <= D) run[lane] += all;
+        __syncthreads();
+    }
+}
+
+// Every depth's nodes (one thread per slot of the depths 1..D); the empty-slot
+// conventions follow updateEmptyNodeInfo (main.cu:433-490)
+__global__ void k_fill_nodes(Levels lv, int D, i64 N, i64 M, NodeArrays nd) {
+    for (i64 i = 1 + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (i64)gridDim.x * blockDim.x) {
+        int d = 1;
+        while (d < D && lv.base[d + 1] <= i) ++d;
+        const i64 s = i - lv.base[d], g = s >> 3;
+        const int k = (int)(s & 7), shift = 3 * (D - d);
+        nd.key[i] = lv.key[d - 1][g] | ((u64)k << shift);
+        nd.depth[i] = (int8_t)d;
+        nd.parent[i] = (int)(lv.base[d - 1] + lv.slot[d - 1][g]);
+        // the parent's children are the runs [f0, f1) of this depth, in slot order: the first at or after
+        // slot k, and the first after it
+        const int Ud = lv.U[d], f0 = lv.first[d - 1][g], f1 = g + 1 < lv.U[d - 1] ? lv.first[d - 1][g + 1] : Ud;
+        int r = f0;
+        while (r < f1 && (lv.slot[d][r] & 7) < k) ++r;
+        const bool self = r < f1 && (lv.slot[d][r] & 7) == k;
+        const int p0 = r < Ud ? lv.pidx[d][r] : (int)N, p1 = r + 1 < Ud ? lv.pidx[d][r + 1] : (int)N;
+        nd.pidx[i] = p0;
+        nd.pnum[i] = self ? p1 - p0 : 0;
+        if (d == D) {
             nd.didx[i] = (int)s;
             nd.dnum[i] = 1;
         } else {
-            nd.dnum[i] = my_dnum;
-            // parent's first finest slot: 8 * (rank of its first depth-(D-1) descendant)
-            int pdidx = (a.d - 1 == a.D - 1) ? (int)(8 * g) : 8 * ulo_prev[g];
-            nd.didx[i] = pdidx + dpre;
+            // finest slots: 8 per run of depth D - 1
+            const int l0 = r < Ud ? lv.lo[d][r] : lv.U[D - 1], l1 = r + 1 < Ud ? lv.lo[d][r + 1] : lv.U[D - 1];
+            nd.didx[i] = 8 * l0;
+            nd.dnum[i] = self ? 8 * (l1 - l0) : 0;
         }
-        nd.child0[i] = (r_self >= 0 && a.d < a.D) ? (int)(a.base_next + 8 * (i64)r_self) : -1;
+        nd.child0[i] = (self && d < D) ? (int)(lv.base[d + 1] + 8 * (i64)r) : -1;
     }
 }
 
@@ -248,44 +325,16 @@ __global__ void __launch_bounds__(256) k_neighbours(NodeArrays nd, i64 lo, i64 n
     }
 }
 
-__global__ void k_point_node(const int* __restrict__ leaf_rank, i64 n, const int* __restrict__ uslotD, i64 baseD,
-                             int* __restrict__ point_node) {
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
-        point_node[i] = (int)(baseD + uslotD[leaf_rank[i]]);
-}
-
 void stage_octree(Ctx& c) {
     cudaStream_t s = c.stream;
     const int D = c.D;
     const i64 N = c.N;
-    // ---- bounding box, scale and centre exactly as the reference host code
+    // ---- bounding box; scale and centre as the reference host code, on the device and below
     unsigned* mm = dalloc<unsigned>(6, s);
-    {
-        unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0, 0, 0};
-        CK(cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
-        k_bbox<<<grid_for(N, 256, 152 * 8), 256, 0, s>>>(c.in_xyz, N, mm);
-        CK_LAUNCH();
-        unsigned h[6];
-        CK(cudaMemcpyAsync(h, mm, sizeof h, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        float mn[3], mx[3];
-        for (int a = 0; a < 3; ++a) { mn[a] = ord2f(h[a]); mx[a] = ord2f(h[3 + a]); }
-        float scale = 1;
-        for (int a = 0; a < 3; ++a) {
-            if (!a || scale < mx[a] - mn[a]) scale = float(mx[a] - mn[a]);
-            c.center[a] = float(mx[a] + mn[a]) / 2;
-        }
-        scale *= 1.25f;
-        for (int a = 0; a < 3; ++a) c.center[a] -= scale / 2;
-        c.scale = scale;
-        if (!(scale > 0.f) || !std::isfinite(scale) || !std::isfinite(c.center[0]) || !std::isfinite(c.center[1]) ||
-            !std::isfinite(c.center[2])) {
-            dfree(mm, s);
-            set_last_error("degenerate bounding box (all points coincide or are not finite)");
-            throw Error{PRGPU_ERR_ARG, {0}};
-        }
-    }
-    dfree(mm, s);
+    const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0, 0, 0};
+    CK(cudaMemcpyAsync(mm, init, sizeof init, cudaMemcpyHostToDevice, s));
+    k_bbox<<<grid_for(N, 256, 152 * 8), 256, 0, s>>>(c.in_xyz, N, mm);
+    CK_LAUNCH();
     // ---- normalise + keys, sort, gather
     float* ptmp = dalloc<float>(3 * N, s);
     float* ntmp = dalloc<float>(3 * N, s);
@@ -293,8 +342,8 @@ void stage_octree(Ctx& c) {
     u64* ktmp = dalloc<u64>(N, s);
     uint32_t* idx = dalloc<uint32_t>(N, s);
     uint32_t* itmp = dalloc<uint32_t>(N, s);
-    k_normalise_encode<<<grid_for(N, 256), 256, 0, s>>>(c.in_xyz, c.in_nrm, N, c.center[0], c.center[1], c.center[2],
-                                                         c.scale, (float)(2 << D), D, ptmp, ntmp, keys, idx);
+    k_normalise_encode<<<grid_for(N, 256), 256, 0, s>>>(c.in_xyz, c.in_nrm, N, mm, (float)(2 << D), D, ptmp, ntmp, keys,
+                                                         idx);
     CK_LAUNCH();
     const int ks = c.kbegin("point_sort", (double)N * 12 * 2);
     radix_sort_pairs(keys, idx, ktmp, itmp, N, 3 * D, s);
@@ -310,59 +359,36 @@ void stage_octree(Ctx& c) {
     dfree(ptmp, s);
     dfree(ntmp, s);
 
-    // ---- unique nodes per depth
-    std::vector<u64*> ukey(D + 1, nullptr);
-    std::vector<int*> upidx(D + 1, nullptr), uparent(D + 1, nullptr), ufirstchild(D + 1, nullptr), ulo(D + 1, nullptr),
-        uslot(D + 1, nullptr), slot2u(D + 1, nullptr);
-    std::vector<i64> U(D + 1, 0);
-    int* flags = dalloc<int>(N, s);
-    int* pos = dalloc<int>(N + 1, s);
-    int* leaf_rank = dalloc<int>(N, s);
+    // ---- runs per depth; their counts and the bounding box come back in one read
+    const i64 ntiles = (N + LV_TILE - 1) / LV_TILE;
+    int* cnt = dalloc<int>((D + 1) * ntiles, s);
+    int* dU = dalloc<int>(LV_MAX, s);
+    k_run_count<<<(unsigned)ntiles, LV_BLOCK, 0, s>>>(keys, N, D, ntiles, cnt);
+    CK_LAUNCH();
+    k_run_offsets<<<D + 1, 1024, 0, s>>>(cnt, ntiles, dU);
+    CK_LAUNCH();
+    Levels lv{};
+    unsigned h[6];
+    CK(cudaMemcpyAsync(h, mm, sizeof h, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(lv.U, dU, (D + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    dfree(mm, s);
+    dfree(dU, s);
     {
-        k_head_flags<<<grid_for(N, 256), 256, 0, s>>>(keys, N, ~0ull, flags);
-        CK_LAUNCH();
-        exclusive_scan<int, int>(flags, pos, N, pos + N, s);
-        U[D] = read_scalar(pos + N, s);
-        ukey[D] = dalloc<u64>(U[D], s);
-        upidx[D] = dalloc<int>(U[D], s);
-        k_runs<<<grid_for(N, 256), 256, 0, s>>>(keys, N, ~0ull, flags, pos, ukey[D], upidx[D], leaf_rank);
-        CK_LAUNCH();
-    }
-    for (int d = D - 1; d >= 0; --d) {
-        const i64 n = U[d + 1];
-        u64 mask = ~((1ull << (3 * (D - d))) - 1);
-        k_head_flags<<<grid_for(n, 256), 256, 0, s>>>(ukey[d + 1], n, mask, flags);
-        CK_LAUNCH();
-        exclusive_scan<int, int>(flags, pos, n, pos + n, s);
-        U[d] = read_scalar(pos + n, s);
-        ukey[d] = dalloc<u64>(U[d], s);
-        ufirstchild[d] = dalloc<int>(U[d], s);
-        uparent[d + 1] = dalloc<int>(n, s);
-        k_runs<<<grid_for(n, 256), 256, 0, s>>>(ukey[d + 1], n, mask, flags, pos, ukey[d], ufirstchild[d],
-                                                 uparent[d + 1]);
-        CK_LAUNCH();
-        upidx[d] = dalloc<int>(U[d], s);
-        k_compose<<<grid_for(U[d], 256), 256, 0, s>>>(upidx[d + 1], ufirstchild[d], U[d], upidx[d]);
-        CK_LAUNCH();
-    }
-    dfree(flags, s);
-    dfree(pos, s);
-    // rank range of depth-(D-1) descendants: lo per unique node
-    if (D >= 1) {
-        ulo[D - 1] = dalloc<int>(U[D - 1], s);
-        k_iota<<<grid_for(U[D - 1], 256), 256, 0, s>>>(ulo[D - 1], U[D - 1]);
-        CK_LAUNCH();
-        for (int d = D - 2; d >= 0; --d) {
-            ulo[d] = dalloc<int>(U[d], s);
-            k_compose<<<grid_for(U[d], 256), 256, 0, s>>>(ulo[d + 1], ufirstchild[d], U[d], ulo[d]);
-            CK_LAUNCH();
+        const Cube cube = cube_of(h);
+        for (int a = 0; a < 3; ++a) c.center[a] = cube.corner[a];
+        c.scale = cube.scale;
+        if (!(c.scale > 0.f) || !std::isfinite(c.scale) || !std::isfinite(c.center[0]) ||
+            !std::isfinite(c.center[1]) || !std::isfinite(c.center[2])) {
+            set_last_error("degenerate bounding box (all points coincide or are not finite)");
+            throw Error{PRGPU_ERR_ARG, {0}};
         }
     }
     // ---- sizes
     c.count.assign(D + 1, 0);
     c.base.assign(D + 2, 0);
     c.count[0] = 1;
-    for (int d = 1; d <= D; ++d) c.count[d] = 8 * U[d - 1];
+    for (int d = 1; d <= D; ++d) c.count[d] = 8 * (i64)lv.U[d - 1];
     for (int d = 1; d <= D + 1; ++d) c.base[d] = c.base[d - 1] + c.count[d - 1];
     const i64 M = c.base[D + 1];
     if (M > 0x7fffffffLL) {
@@ -381,29 +407,29 @@ void stage_octree(Ctx& c) {
     nd.child0 = dalloc<int>(M, s);
     nd.depth = dalloc<int8_t>(M, s);
     nd.neigh = dalloc<int>(27 * M, s);
-    // ---- slots of unique nodes
-    uslot[0] = dalloc<int>(1, s);
-    CK(cudaMemsetAsync(uslot[0], 0, sizeof(int), s));
-    for (int d = 1; d <= D; ++d) {
-        uslot[d] = dalloc<int>(U[d], s);
-        slot2u[d] = dalloc<int>(c.count[d], s);
-        fill<int>(slot2u[d], c.count[d], -1, s);
-        k_unique_slots<<<grid_for(U[d], 256), 256, 0, s>>>(ukey[d], uparent[d], U[d], 3 * (D - d), uslot[d], slot2u[d]);
-        CK_LAUNCH();
+    // ---- the runs of all depths, each point's leaf, and the nodes
+    dfree(c.point_node, s);
+    c.point_node = dalloc<int>(N, s);
+    for (int d = 0; d <= D + 1; ++d) lv.base[d] = c.base[d];
+    for (int d = 0; d <= D; ++d) {
+        lv.key[d] = dalloc<u64>(lv.U[d], s);
+        lv.pidx[d] = dalloc<int>(lv.U[d], s);
+        lv.slot[d] = dalloc<int>(lv.U[d], s);
+        if (d < D) {
+            lv.first[d] = dalloc<int>(lv.U[d], s);
+            lv.lo[d] = dalloc<int>(lv.U[d], s);
+        }
     }
-    // ---- fill
+    k_runs<<<(unsigned)ntiles, LV_BLOCK, 0, s>>>(keys, N, D, ntiles, cnt, lv, c.point_node);
+    CK_LAUNCH();
     k_root<<<1, 1, 0, s>>>(nd, N, c.count[D], M);
     CK_LAUNCH();
-    for (int d = 1; d <= D; ++d) {
-        LevelArgs a;
-        a.d = d; a.D = D;
-        a.base_prev = c.base[d - 1]; a.base_d = c.base[d]; a.base_next = c.base[d + 1];
-        a.n_slots = c.count[d]; a.N = N; a.u_d = U[d]; a.u_dm1 = U[d - 1];
-        a.u_last = (D >= 1) ? U[D - 1] : 1;
-        k_fill_level<<<grid_for(c.count[d], 256), 256, 0, s>>>(a, ukey[d - 1], uslot[d - 1], upidx[d - 1],
-                                                                (d - 1 <= D - 2) ? ulo[d - 1] : nullptr, upidx[d],
-                                                                (d <= D - 1) ? ulo[d] : nullptr, slot2u[d], nd);
-        CK_LAUNCH();
+    k_fill_nodes<<<grid_for(M - 1, 256), 256, 0, s>>>(lv, D, N, M, nd);
+    CK_LAUNCH();
+    dfree(cnt, s);
+    dfree(keys, s);
+    for (int d = 0; d <= D; ++d) {
+        dfree(lv.key[d], s); dfree(lv.pidx[d], s); dfree(lv.slot[d], s); dfree(lv.first[d], s); dfree(lv.lo[d], s);
     }
     // ---- neighbours, top-down
     const int kn = c.kbegin("neighbours", (double)M * (108 + 8 + 4 + 4));
@@ -412,17 +438,6 @@ void stage_octree(Ctx& c) {
         CK_LAUNCH();
     }
     c.kend(kn);
-    // ---- point -> leaf
-    dfree(c.point_node, s);
-    c.point_node = dalloc<int>(N, s);
-    k_point_node<<<grid_for(N, 256), 256, 0, s>>>(leaf_rank, N, uslot[D], c.base[D], c.point_node);
-    CK_LAUNCH();
-    dfree(leaf_rank, s);
-    dfree(keys, s);
-    for (int d = 0; d <= D; ++d) {
-        dfree(ukey[d], s); dfree(upidx[d], s); dfree(uparent[d], s); dfree(ufirstchild[d], s);
-        dfree(ulo[d], s); dfree(uslot[d], s); dfree(slot2u[d], s);
-    }
 }
 
 }  // namespace prgpu

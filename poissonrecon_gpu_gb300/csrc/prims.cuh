@@ -99,11 +99,20 @@ __global__ void k_tile_reduce(const TI* __restrict__ in, i64 n, TO* __restrict__
     if (threadIdx.x == 0) partial[blockIdx.x] = tot;
 }
 
+// 'partial' (null: one tile): the tiles' sums, scanned when 'scanned', else summed here up to this tile
 template <class TI, class TO>
 __global__ void k_tile_scan(const TI* __restrict__ in, i64 n, TO* __restrict__ out,
-                            const TO* __restrict__ partial_scanned, TO* __restrict__ total_out) {
+                            const TO* __restrict__ partial, bool scanned, TO* __restrict__ total_out) {
     __shared__ TO sw[32];
     i64 base = (i64)blockIdx.x * SCAN_TILE + (i64)threadIdx.x * SCAN_ITEMS;
+    TO off = TO(0);
+    if (partial && scanned) {
+        off = partial[blockIdx.x];
+    } else if (partial) {
+        TO p = TO(0);
+        for (unsigned k = threadIdx.x; k < blockIdx.x; k += SCAN_BLOCK) p += partial[k];
+        block_exclusive_sum<TO>(p, sw, &off);
+    }
     TO v[SCAN_ITEMS];
     TO s = 0;
 #pragma unroll
@@ -113,7 +122,6 @@ __global__ void k_tile_scan(const TI* __restrict__ in, i64 n, TO* __restrict__ o
     }
     TO tot;
     TO pre = block_exclusive_sum<TO>(s, sw, &tot);
-    TO off = partial_scanned ? partial_scanned[blockIdx.x] : TO(0);
     TO run = off + pre;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
@@ -124,7 +132,10 @@ __global__ void k_tile_scan(const TI* __restrict__ in, i64 n, TO* __restrict__ o
 }
 
 // out[i] = sum_{k<i} in[k]; *total_dev (device pointer, optional) receives the sum.
-// 'in' and 'out' may alias.
+// 'in' and 'out' may alias.  Up to SCAN_SELF tiles each tile sums the sums of the tiles before it (at most
+// two loads a thread) instead of waiting for a scan of them: two launches in place of three, which is
+// what short scans cost (a few us each; a pass over 5,000 points makes 20 of them).
+constexpr i64 SCAN_SELF = 1024;
 template <class TI, class TO>
 void exclusive_scan(const TI* in, TO* out, i64 n, TO* total_dev, cudaStream_t s) {
     if (n <= 0) {
@@ -133,15 +144,16 @@ void exclusive_scan(const TI* in, TO* out, i64 n, TO* total_dev, cudaStream_t s)
     }
     i64 nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (nb == 1) {
-        k_tile_scan<TI, TO><<<1, SCAN_BLOCK, 0, s>>>(in, n, out, nullptr, total_dev);
+        k_tile_scan<TI, TO><<<1, SCAN_BLOCK, 0, s>>>(in, n, out, nullptr, false, total_dev);
         CK_LAUNCH();
         return;
     }
     TO* part = dalloc<TO>(nb, s);
     k_tile_reduce<TI, TO><<<(unsigned)nb, SCAN_BLOCK, 0, s>>>(in, n, part);
     CK_LAUNCH();
-    exclusive_scan<TO, TO>(part, part, nb, (TO*)nullptr, s);
-    k_tile_scan<TI, TO><<<(unsigned)nb, SCAN_BLOCK, 0, s>>>(in, n, out, part, total_dev);
+    const bool scanned = nb > SCAN_SELF;
+    if (scanned) exclusive_scan<TO, TO>(part, part, nb, (TO*)nullptr, s);
+    k_tile_scan<TI, TO><<<(unsigned)nb, SCAN_BLOCK, 0, s>>>(in, n, out, part, scanned, total_dev);
     CK_LAUNCH();
     dfree(part, s);
 }
