@@ -310,34 +310,6 @@ void stage_points(Ctx& c) {
 }
 
 // ------------------------------ corners -------------------------------------
-// owner of the corner 'kind' of real node i (min key among same-depth nodes
-// sharing the corner); returns the owner and the corner's kind in its frame
-__device__ __forceinline__ int corner_owner(const NodeArrays& nd, i64 i, int kind, int& okind) {
-    const int sx = kind & 1, sy = (kind >> 1) & 1, sz = (kind >> 2) & 1;
-    const i64 M = nd.M;
-    u64 best = ~0ull;
-    int own = -1;
-    okind = kind;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const int ex = e & 1, ey = (e >> 1) & 1, ez = (e >> 2) & 1;
-        const int dx = sx - ex, dy = sy - ey, dz = sz - ez;
-        const int j = 9 * (dx + 1) + 3 * (dy + 1) + (dz + 1);
-        const int nb = nd.neigh[(i64)j * M + i];
-        if (nb == -1) continue;
-        const u64 kk = nd.key[nb];
-        if (kk < best) { best = kk; own = nb; okind = ex | (ey << 1) | (ez << 2); }
-    }
-    return own;
-}
-
-__device__ __forceinline__ void corner_pos(const int xyz[3], int d, int kind, float q[3]) {
-    const float inv = 1.0f / (float)(1 << d);
-    q[0] = (float)(xyz[0] + (kind & 1)) * inv;
-    q[1] = (float)(xyz[1] + ((kind >> 1) & 1)) * inv;
-    q[2] = (float)(xyz[2] + ((kind >> 2) & 1)) * inv;
-}
-
 // value of corner 'kind' of owner o, minus the iso-value
 // (computeVertexImplicitFunctionValue main.cu:2259-2326, including its descent
 // through children[childrenVertexKind[kind]])
@@ -413,10 +385,24 @@ __global__ void k_finest_list(const unsigned char* __restrict__ owned_mask, cons
     }
 }
 
+// f(node, corner kind in its frame) for each of the existing same-depth nodes that share corner 'kind' of
+// node i, itself among them
+template <class F>
+__device__ __forceinline__ void corner_sharers(const NodeArrays& nd, i64 i, int kind, F f) {
+    const int sx = kind & 1, sy = (kind >> 1) & 1, sz = kind >> 2;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int j = 9 * (sx - (e & 1) + 1) + 3 * (sy - ((e >> 1) & 1) + 1) + (sz - (e >> 2) + 1);
+        const int nb = nd.neigh[(i64)j * nd.M + i];
+        if (nb != -1) f(nb, e);
+    }
+}
+
 // pass 2 (one thread per owned corner): walk_up_u from the owner at the corner,
-// the value of owner_corner_value (no descent at the finest depth)
+// the value of owner_corner_value (no descent at the finest depth), written to every cell that has the
+// corner.  (Each cell looking for the owner of each of its 8 corners reads 64 neighbours and keys.)
 __global__ void __launch_bounds__(128, 12) k_finest_corner_values(EvalArgs a, i64 lo, const int* __restrict__ list,
-                                                                 i64 ncorner, float iso, float* __restrict__ cval) {
+                                                                 i64 ncorner, float iso, float* __restrict__ cell_v) {
     const int D = a.D;
     for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < ncorner; q += (i64)gridDim.x * blockDim.x) {
         const int lk = list[q];
@@ -426,25 +412,71 @@ __global__ void __launch_bounds__(128, 12) k_finest_corner_values(EvalArgs a, i6
         int xyz[3];
         key_coords(a.nd.key[i], D, D, xyz);
         const int u[3] = {xyz[0] + (kind & 1), xyz[1] + ((kind >> 1) & 1), xyz[2] + (kind >> 2)};
-        cval[8 * l + kind] = walk_up_u(a, i, u, 0.f) - iso;
+        const float val = walk_up_u(a, i, u, 0.f) - iso;
+        corner_sharers(a.nd, i, kind, [&](int nb, int e) { cell_v[8 * ((i64)nb - lo) + e] = val; });
     }
 }
 
-// corner values of each finest cell (from the owners), cube category, triangle count
-__global__ void k_finest_cells(NodeArrays nd, i64 lo, i64 hi, const float* __restrict__ cval, float* __restrict__ cell_v,
-                               unsigned char* __restrict__ cat, int* __restrict__ ntri) {
-    for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
-        int cc = 0;
-        for (int kind = 0; kind < 8; ++kind) {
-            int ok;
-            const int own = corner_owner(nd, i, kind, ok);
-            const float v = cval[8 * ((i64)own - lo) + ok];
-            cell_v[8 * (i - lo) + kind] = v;
-            if (v < 0.f) cc |= 1 << c_vid[kind];
-        }
-        cat[i - lo] = (unsigned char)cc;
-        ntri[i - lo] = c_tri_count[cc];
+// Cells in tiles of CELL_TILE: the kernels that find the categories sum each tile's triangles, the sums are
+// scanned, and the emission kernels place a tile's active cells and triangles by a scan in the block.  (Lists
+// of active cells and triangle offsets, built by flags, scans and gathers over all cells, took a dozen
+// launches and as many bytes as the cells' corner values.)
+constexpr int CELL_BLOCK = 256;
+constexpr int CELL_ITEMS = 4;
+constexpr int CELL_TILE = CELL_ITEMS * CELL_BLOCK;
+constexpr int CELL_BITS = 10;
+static_assert(CELL_TILE == 1 << CELL_BITS, "");
+__device__ __forceinline__ void tile_triangles(int n, int* __restrict__ tile_tri) {
+    __shared__ int s_n[CELL_BLOCK / 32];
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) s_n[threadIdx.x >> 5] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = 0;
+        for (int k = 0; k < CELL_BLOCK / 32; ++k) t += s_n[k];
+        tile_tri[blockIdx.x] = t;
     }
+}
+// the tile's active cells in order, packed (cell in the tile) | (first triangle in the tile) << CELL_BITS, into
+// list; returns their number.  list: CELL_TILE ints of shared memory; all threads call
+__device__ __forceinline__ int tile_active(const unsigned char* __restrict__ cat, i64 total, int* list) {
+    __shared__ int sw[32];
+    const i64 c0 = (i64)blockIdx.x * CELL_TILE + CELL_ITEMS * threadIdx.x;
+    int nt[CELL_ITEMS], mine = 0;
+#pragma unroll
+    for (int k = 0; k < CELL_ITEMS; ++k) {
+        nt[k] = c0 + k < total ? c_tri_count[cat[c0 + k]] : 0;
+        mine += nt[k] ? (1 << 16) + nt[k] : 0;      // (active cells, triangles): at most 1024 and 5120
+    }
+    int all;
+    int at = block_exclusive_sum<int>(mine, sw, &all);
+#pragma unroll
+    for (int k = 0; k < CELL_ITEMS; ++k)
+        if (nt[k]) {
+            list[at >> 16] = (CELL_ITEMS * (int)threadIdx.x + k) | ((at & 0xffff) << CELL_BITS);
+            at += (1 << 16) + nt[k];
+        }
+    __syncthreads();
+    return all >> 16;
+}
+
+// cube category of each finest cell, the tile's triangles
+__global__ void __launch_bounds__(CELL_BLOCK) k_finest_cells(const float* __restrict__ cell_v, i64 n,
+                                                             unsigned char* __restrict__ cat, int* __restrict__ tile_tri) {
+    int tri = 0;
+    for (int q = 0; q < CELL_TILE / CELL_BLOCK; ++q) {
+        const i64 l = (i64)blockIdx.x * CELL_TILE + q * CELL_BLOCK + threadIdx.x;
+        if (l >= n) break;
+        const float4 v0 = reinterpret_cast<const float4*>(cell_v + 8 * l)[0], v1 = reinterpret_cast<const float4*>(cell_v + 8 * l)[1];
+        const float cv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        int cc = 0;
+#pragma unroll
+        for (int kind = 0; kind < 8; ++kind)
+            if (cv[kind] < 0.f) cc |= 1 << c_vid[kind];
+        cat[l] = (unsigned char)cc;
+        tri += c_tri_count[cc];
+    }
+    tile_triangles(tri, tile_tri);
 }
 
 // ------------------------------- faces ---------------------------------------
@@ -491,52 +523,59 @@ __global__ void k_mark_faces(NodeArrays nd, int D, i64 lo, i64 hi, const unsigne
     }
 }
 
-// corners of the leaves above the finest depth: mark each owner's corner once
-__global__ void k_coarse_need(NodeArrays nd, i64 lo, i64 hi, unsigned char* __restrict__ need) {
-    for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
-        if (nd.child0[i] != -1) continue;
-        for (int kind = 0; kind < 8; ++kind) {
-            int ok;
-            const int own = corner_owner(nd, i, kind, ok);
-            need[8 * (i64)own + ok] = 1;
-        }
-    }
-}
-// needed corners of each coarse node as a mask and a count
-__global__ void k_need_mask(const unsigned char* __restrict__ need, i64 n, unsigned char* __restrict__ mask,
-                            int* __restrict__ count) {
+// Corners of the leaves above the finest depth: each node's owned corners that a leaf shares, as a mask and a
+// count (a corner's owner is the least key among the existing same-depth nodes around it).
+__global__ void k_coarse_owned(NodeArrays nd, i64 n, unsigned char* __restrict__ mask, int* __restrict__ count) {
+    const i64 M = nd.M;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        unsigned m = 0;
+        const u64 ki = nd.key[i];
+        unsigned smaller = 0, leaf = 0;   // bit j: neighbour j exists and has a smaller key; is a leaf
 #pragma unroll
-        for (int k = 0; k < 8; ++k) m |= need[8 * i + k] ? (1u << k) : 0u;
-        mask[i] = (unsigned char)m;
-        count[i] = __popc(m);
+        for (int j = 0; j < 27; ++j) {
+            const int nb = nd.neigh[(i64)j * M + i];
+            if (nb == -1) continue;
+            if (j != 13 && nd.key[nb] < ki) smaller |= 1u << j;
+            if (nd.child0[nb] == -1) leaf |= 1u << j;
+        }
+        unsigned owned = 0;
+        if (i > 0)   // the root has no corner value of its own
+#pragma unroll
+            for (int kind = 0; kind < 8; ++kind) {
+                unsigned around = 0;
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    around |= 1u << (9 * ((kind & 1) - (e & 1) + 1) + 3 * (((kind >> 1) & 1) - ((e >> 1) & 1) + 1) +
+                                     ((kind >> 2) - (e >> 2) + 1));
+                if (!(smaller & around) && (leaf & around)) owned |= 1u << kind;
+            }
+        mask[i] = (unsigned char)owned;
+        count[i] = __popc(owned);
     }
 }
+// the listed corners (node << 3 | corner), each value to the leaves that have the corner
 __global__ void __launch_bounds__(128, 8) k_coarse_corner_list(EvalArgs a, const int* __restrict__ list, i64 n,
-                                                               float iso, float* __restrict__ cval) {
+                                                               float iso, float* __restrict__ leaf_v) {
     for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (i64)gridDim.x * blockDim.x) {
         const int lk = list[q];
-        cval[lk] = owner_corner_value(a, lk >> 3, lk & 7, iso);   // cval index = 8 node + corner
+        const float val = owner_corner_value(a, lk >> 3, lk & 7, iso);
+        corner_sharers(a.nd, lk >> 3, lk & 7, [&](int nb, int e) {
+            if (a.nd.child0[nb] == -1) leaf_v[8 * (i64)nb + e] = val;
+        });
     }
 }
 
 // leaves above the finest depth: sign change at their corners or a marked face
 // (ProcessLeafNodesAtOtherDepth main.cu:2957-2986, ifSubdivide :2988-2992)
-// (at most 64 registers: unbounded, the 8 corner-owner and 6 face-owner searches take 167
-// registers and leave one warp in eight resident; measured 0.84 -> 0.66 ms with the stage's lists)
-__global__ void __launch_bounds__(128, 8) k_coarse_leaves(EvalArgs a, i64 lo, i64 hi, const float* __restrict__ cval,
+__global__ void __launch_bounds__(128) k_coarse_leaves(NodeArrays nd, i64 lo, i64 hi, const float* __restrict__ leaf_v,
                                 const int* __restrict__ fflag, int* __restrict__ has_tri, int* __restrict__ has_int,
                                 int* __restrict__ is_root) {
-    const NodeArrays& nd = a.nd;
     for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
         if (nd.child0[i] != -1) { is_root[i] = 0; continue; }
+        const float4 v0 = reinterpret_cast<const float4*>(leaf_v + 8 * i)[0], v1 = reinterpret_cast<const float4*>(leaf_v + 8 * i)[1];
+        const float cv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         float v[8];
-        for (int kind = 0; kind < 8; ++kind) {
-            int ok;
-            const int own = corner_owner(nd, i, kind, ok);
-            v[c_vid[kind]] = cval[8 * (i64)own + ok];
-        }
+#pragma unroll
+        for (int kind = 0; kind < 8; ++kind) v[kind ^ ((kind >> 1) & 1)] = cv[kind];   // c_vid: the cube's vertex order
         const int sign = v[0] < 0 ? -1 : 1;
         int ht = 0;
         for (int j = 1; j < 8; ++j)
@@ -1674,12 +1713,33 @@ __global__ void k_root_of(const VRoot* __restrict__ roots, int nroots, int* __re
         root_of[roots[k].node] = k;
 }
 
-// live brick: root, brick coordinates; first corner value and first cell
+// live brick: root and brick coordinates
 struct LiveBrick {
     int root;
     int b[3];
-    i64 lat;
-    i64 cell;
+};
+// The live bricks in brick order.  Roots come in depth order, so the bricks of edge 8 come first, then those
+// of edge 4 and of edge 2: a brick's corner values and cells are numbered in closed form.
+struct LiveIndex {
+    const LiveBrick* live;
+    i64 n8, n4, n2;
+    __host__ __device__ i64 lattices() const { return 729 * n8 + 125 * n4 + 27 * n2; }
+    __host__ __device__ i64 cells() const { return 512 * n8 + 64 * n4 + 8 * n2; }
+    __device__ __forceinline__ i64 lat(i64 li) const {   // first corner value
+        if (li < n8) return 729 * li;
+        li -= n8;
+        return 729 * n8 + (li < n4 ? 125 * li : 125 * n4 + 27 * (li - n4));
+    }
+    // brick of cell e; its edge's logarithm and the cell in it
+    __device__ __forceinline__ i64 brick(i64 e, int& lg, int& loc) const {
+        if (e < 512 * n8) { lg = 3; loc = (int)(e & 511); return e >> 9; }
+        e -= 512 * n8;
+        if (e < 64 * n4) { lg = 2; loc = (int)(e & 63); return n8 + (e >> 6); }
+        e -= 64 * n4;
+        lg = 1;
+        loc = (int)(e & 7);
+        return n8 + n4 + (e >> 3);
+    }
 };
 // a corner of live brick li owned by another leaf of the batch, and the corner of that leaf's brick which
 // is the same point: brick << 10 | corner
@@ -1770,8 +1830,7 @@ __device__ __forceinline__ void column_level(const float xs[28], const float4& b
 // 8.7 ms, set-up and window loads waiting.
 template <int E, int NT>
 __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
-                                                   const LiveBrick* __restrict__ live, const int* __restrict__ list,
-                                                   i64 nlist, float* __restrict__ blat,
+                                                   LiveIndex lx, i64 first, i64 nlist, float* __restrict__ blat,
                                                    unsigned long long* __restrict__ nforeign,
                                                    ForeignCorner* __restrict__ foreign, i64 foreign_cap) {
     __shared__ BrickShared<E> sm;
@@ -1780,8 +1839,8 @@ __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, Br
     const EvalArgs& a = v.e;
     const int D = a.D;
     for (i64 it = blockIdx.x; it < nlist; it += gridDim.x) {
-        const int li = list[it];
-        const LiveBrick lb = live[li];
+        const int li = (int)(first + it);
+        const LiveBrick lb = lx.live[li];
         const VRoot R = v.roots[lb.root];
         const int r = R.depth, S = 1 << (D - r), L = R.node, nb = S / E;
         int Lc[3];
@@ -1932,7 +1991,7 @@ __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, Br
             }
             column_level<K1>(xs, sm.Bt[l * K1 + kx], sm.Bt[(BR_LEVELS + l) * K1 + ky], sm.Bt + (2 * BR_LEVELS + l) * K1, val);
         }
-        float* out = blat + lb.lat + (i64)ci * K1;
+        float* out = blat + lx.lat(li) + (i64)ci * K1;
         unsigned fmask = 0;                 // corners of the column that another leaf owns
         if (fposs) {
 #pragma unroll 1
@@ -1966,8 +2025,7 @@ __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, Br
 // 19.7 before); half of the issue slots idle on the gathers of x27 rows.
 constexpr int E2_WARPS = 4;
 __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
-                                                              const LiveBrick* __restrict__ live,
-                                                              const int* __restrict__ list, i64 nlist,
+                                                              LiveIndex lx, i64 first, i64 nlist,
                                                               float* __restrict__ blat,
                                                               unsigned long long* __restrict__ nforeign,
                                                               ForeignCorner* __restrict__ foreign, i64 foreign_cap) {
@@ -1985,7 +2043,7 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
         __syncwarp();                       // the previous bricks' readers are done
         for (int e = lane; e < nbr * 27; e += 32) {
             const int b = e / 27, j = e % 27;
-            const VRoot R = v.roots[live[list[it + b]].root];
+            const VRoot R = v.roots[lx.live[first + it + b].root];
             const int n = a.nd.neigh[(i64)j * a.nd.M + R.node];
             s_child[w][b][j] = n == -1 ? -1 : a.nd.child0[n];
             // batch_member's rule (R.depth >= 3: one batch per depth)
@@ -1993,7 +2051,7 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
         }
         for (int e = lane; e < nbr * BR_LEVELS; e += 32) {
             const int b = e / BR_LEVELS, l = e % BR_LEVELS;
-            if (l <= r) s_up[w][b][l] = bix.up[(i64)live[list[it + b]].root * BR_LEVELS + l];
+            if (l <= r) s_up[w][b][l] = bix.up[(i64)lx.live[first + it + b].root * BR_LEVELS + l];
         }
         __syncwarp();
         for (int e = lane; e < nbr * 64; e += 32) {
@@ -2004,8 +2062,8 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
         __syncwarp();
         const bool on = lane < 27 && gi < nbr;
         const int g = min(gi, nbr - 1);
-        const int li = list[it + g];
-        const i64 lat = live[li].lat;
+        const int li = (int)(first + it + g);
+        const i64 lat = lx.lat(li);
         int Lc[3];
         key_coords(a.nd.key[s_up[w][g][r]], r, D, Lc);
         const int g0[3] = {2 * Lc[0], 2 * Lc[1], 2 * Lc[2]};
@@ -2076,20 +2134,22 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
 // corners on a leaf's lower faces owned by a cell of another leaf L' of the
 // batch: the same value is a corner of L''s brick holding the owner cell, where
 // L' owns it -- copied when that brick is live, evaluated otherwise
-__global__ void k_foreign_fill(VArgs v, BrickIndex bix, const LiveBrick* __restrict__ live,
-                               const unsigned char* __restrict__ culled, const int* __restrict__ live_pos,
-                               const ForeignCorner* __restrict__ foreign, i64 n, float* __restrict__ blat,
-                               unsigned long long* __restrict__ nslow) {
+// (count[0]: the corners; count[2]: those evaluated.  The grid does not depend on the count, which the host
+// has not read.)
+__global__ void k_foreign_fill(VArgs v, BrickIndex bix, LiveIndex lx, const unsigned char* __restrict__ culled,
+                               const int* __restrict__ live_pos, const ForeignCorner* __restrict__ foreign, i64 cap,
+                               float* __restrict__ blat, unsigned long long* __restrict__ count) {
     const int D = v.e.D;
+    const i64 n = min((i64)count[0], cap);
     for (i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
         const ForeignCorner fe = foreign[f];
         const i64 brick = (i64)(fe.src >> 10);
         const int e = (int)(fe.src & 1023);
         float val;
         if (!culled[brick]) {
-            val = blat[live[live_pos[brick]].lat + e];
+            val = blat[lx.lat(live_pos[brick]) + e];
         } else {
-            atomicAdd(nslow, 1ull);
+            atomicAdd(&count[2], 1ull);
             // the owner brick's corner e, evaluated by its own leaf
             const VBrick B = brick_of(v, bix, brick);
             const VRoot R = v.roots[B.root];
@@ -2105,45 +2165,20 @@ __global__ void k_foreign_fill(VArgs v, BrickIndex bix, const LiveBrick* __restr
             }
             val = virtual_corner_value(v, R.node, r, oc, qc) - v.iso;
         }
-        blat[live[fe.li].lat + fe.e] = val;
+        blat[lx.lat(fe.li) + fe.e] = val;
     }
 }
 
 // live bricks in brick order
 __global__ void k_live_bricks(VArgs v, BrickIndex bix, const unsigned char* __restrict__ culled,
-                              const int* __restrict__ pos, i64 nbricks, LiveBrick* __restrict__ live,
-                              i64* __restrict__ lat_size, i64* __restrict__ cell_size) {
+                              const int* __restrict__ pos, i64 nbricks, LiveBrick* __restrict__ live) {
     for (i64 bi = (i64)blockIdx.x * blockDim.x + threadIdx.x; bi < nbricks; bi += (i64)gridDim.x * blockDim.x) {
         if (culled[bi]) continue;
         const VBrick B = brick_of(v, bix, bi);
-        const int E = brick_edge(v.e.D, v.roots[B.root].depth);
-        const int p = pos[bi];
         LiveBrick lb;
         lb.root = B.root;
         lb.b[0] = B.b[0]; lb.b[1] = B.b[1]; lb.b[2] = B.b[2];
-        lb.lat = 0;
-        lb.cell = 0;
-        live[p] = lb;
-        lat_size[p] = (i64)(E + 1) * (E + 1) * (E + 1);
-        cell_size[p] = (i64)E * E * E;
-    }
-}
-__global__ void k_live_offsets(LiveBrick* __restrict__ live, const i64* __restrict__ lat_pos,
-                               const i64* __restrict__ cell_pos, i64 n) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x) {
-        live[k].lat = lat_pos[k];
-        live[k].cell = cell_pos[k];
-    }
-}
-// live bricks split by edge: 8 (first list) and 2 or 4 (second list)
-// live bricks by edge: 8 (cnt[0]), 4 (cnt[1]) and 2 (cnt[5])
-__global__ void k_live_split(VArgs v, const LiveBrick* __restrict__ live, i64 n, int* __restrict__ big,
-                             int* __restrict__ mid, int* __restrict__ small, unsigned long long* __restrict__ cnt) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x) {
-        const int E = brick_edge(v.e.D, v.roots[live[k].root].depth);
-        if (E == BR) big[atomicAdd(&cnt[0], 1ull)] = (int)k;
-        else if (E == 4) mid[atomicAdd(&cnt[1], 1ull)] = (int)k;
-        else small[atomicAdd(&cnt[5], 1ull)] = (int)k;
+        live[pos[bi]] = lb;
     }
 }
 __global__ void k_live_flags(const unsigned char* __restrict__ culled, i64 n, int* __restrict__ f) {
@@ -2152,44 +2187,39 @@ __global__ void k_live_flags(const unsigned char* __restrict__ culled, i64 n, in
 }
 
 // ---- virtual cells: the cells of the live bricks
-struct VirtCells {
-    const LiveBrick* live;
-    i64 nlive;
-    const float* lat;              // corner values (minus iso) of the live bricks
-};
-
-// root, cell coordinates in the root's lattice and the 8 corner values of virtual cell e
-__device__ __forceinline__ int virt_cell(const VirtCells& vc, const VArgs& v, i64 e, int cu[3], float cv[8]) {
-    i64 lo = 0, hi = vc.nlive - 1;
-    while (lo < hi) {
-        const i64 mid = (lo + hi + 1) >> 1;
-        if (vc.live[mid].cell <= e) lo = mid; else hi = mid - 1;
-    }
-    const LiveBrick lb = vc.live[lo];
-    const int E = brick_edge(v.e.D, v.roots[lb.root].depth), E1 = E + 1;
-    const int loc = (int)(e - lb.cell);
-    const int l3[3] = {loc / (E * E), (loc / E) % E, loc % E};
-    cu[0] = lb.b[0] * E + l3[0];
-    cu[1] = lb.b[1] * E + l3[1];
-    cu[2] = lb.b[2] * E + l3[2];
-    const float* L = vc.lat + lb.lat;
-    for (int kind = 0; kind < 8; ++kind)
-        cv[kind] = L[((l3[0] + (kind & 1)) * E1 + (l3[1] + ((kind >> 1) & 1))) * E1 + (l3[2] + ((kind >> 2) & 1))];
+// brick and cell coordinates in its root's lattice of virtual cell e, and the cell's 8 corner values (minus iso)
+__device__ __forceinline__ int virt_cell(const LiveIndex& lx, const float* __restrict__ lat, i64 e, int cu[3], float cv[8]) {
+    int lg, loc;
+    const i64 li = lx.brick(e, lg, loc);
+    const int E = 1 << lg, E1 = E + 1;
+    const int l3[3] = {loc >> (2 * lg), (loc >> lg) & (E - 1), loc & (E - 1)};
+    const LiveBrick lb = lx.live[li];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) cu[ax] = lb.b[ax] * E + l3[ax];
+    const float* L = lat + lx.lat(li) + (l3[0] * E1 + l3[1]) * E1 + l3[2];
+#pragma unroll
+    for (int kind = 0; kind < 8; ++kind) cv[kind] = L[((kind & 1) * E1 + ((kind >> 1) & 1)) * E1 + (kind >> 2)];
     return lb.root;
 }
 
-__global__ void k_virtual_cells(VArgs v, VirtCells vc, i64 total, unsigned char* __restrict__ cat,
-                                int* __restrict__ ntri) {
-    for (i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
-        int cu[3];
-        float cv[8];
-        virt_cell(vc, v, e, cu, cv);
+__global__ void __launch_bounds__(CELL_BLOCK) k_virtual_cells(LiveIndex lx, const float* __restrict__ lat, i64 total,
+                                                              unsigned char* __restrict__ cat, int* __restrict__ tile_tri) {
+    int tri = 0;
+    for (int q = 0; q < CELL_TILE / CELL_BLOCK; ++q) {
+        const i64 e = (i64)blockIdx.x * CELL_TILE + q * CELL_BLOCK + threadIdx.x;
+        if (e >= total) break;
+        int lg, loc;
+        const i64 li = lx.brick(e, lg, loc);
+        const int E = 1 << lg, E1 = E + 1;
+        const float* L = lat + lx.lat(li) + ((loc >> (2 * lg)) * E1 + ((loc >> lg) & (E - 1))) * E1 + (loc & (E - 1));
         int cc = 0;
+#pragma unroll
         for (int kind = 0; kind < 8; ++kind)
-            if (cv[kind] < 0.f) cc |= 1 << c_vid[kind];
+            if (L[((kind & 1) * E1 + ((kind >> 1) & 1)) * E1 + (kind >> 2)] < 0.f) cc |= 1 << c_vid[kind];
         cat[e] = (unsigned char)cc;
-        ntri[e] = c_tri_count[cc];
+        tri += c_tri_count[cc];
     }
+    tile_triangles(tri, tile_tri);
 }
 
 // ---------------------------- triangle emission ------------------------------
@@ -2239,24 +2269,44 @@ __device__ __forceinline__ void edge_geom(int e, const int c[3], int lp[3], int&
     lp[a1] += b1;
 }
 
+// Emission of one cell's triangles: every triangle corner's edge key and crossing.  rev(a0, a1, b0, b1): the
+// edge at offsets b0, b1 along the axes a0, a1 runs reversed in its owner's frame; only edges along x do
+// (crossing's frame), so only they look for their owner.
+template <class R>
+__device__ __forceinline__ void emit_cell(const EmitArgs& em, const int c[3], const float cv[8], int cc, i64 tri, int batch,
+                                          R rev) {
+    const int nt = c_tri_count[cc];
+    for (int k = 0; k < 3 * nt; ++k) {
+        const int e = c_tri_edges[cc][k];
+        int lp[3], o, a0, a1, b0, b1;
+        edge_geom(e, c, lp, o, a0, a1, b0, b1);
+        const int ev0 = (b0 << a0) | (b1 << a1);   // corner kind of the lower end
+        const int ev1 = ev0 | (1 << o);
+        float p[3];
+        crossing(lp, o, o == 0 && rev(a0, a1, b0, b1), cv[ev0], cv[ev1], em.D, p);
+        const i64 slot = 3 * tri + k;
+        em.keys[slot] = edge_key(lp, o, em.D, batch, em.local_bits);
+        em.slot[slot] = (uint32_t)slot;
+        em.pos[3 * slot] = p[0];
+        em.pos[3 * slot + 1] = p[1];
+        em.pos[3 * slot + 2] = p[2];
+    }
+}
+
 // real finest cells
-__global__ void k_emit_real(NodeArrays nd, EmitArgs em, i64 lo, const int* __restrict__ active, i64 nactive,
-                            const unsigned char* __restrict__ cat, const int* __restrict__ tri_base,
-                            const float* __restrict__ cell_v) {
-    const int D = em.D;
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < nactive; t += (i64)gridDim.x * blockDim.x) {
-        const i64 s = active[t];
-        const i64 i = lo + s;
-        const int cc = cat[s];
-        const int nt = c_tri_count[cc];
+__global__ void __launch_bounds__(CELL_BLOCK, 5) k_emit_real(NodeArrays nd, EmitArgs em, i64 lo, i64 total,
+                                                          const unsigned char* __restrict__ cat,
+                                                          const i64* __restrict__ tile_first, const float* __restrict__ cell_v) {
+    __shared__ int list[CELL_TILE];
+    const int nact = tile_active(cat, total, list);
+    const i64 tri0 = em.tri_offset + tile_first[blockIdx.x];
+    for (int t = threadIdx.x; t < nact; t += CELL_BLOCK) {
+        const i64 s = (i64)blockIdx.x * CELL_TILE + (list[t] & (CELL_TILE - 1)), i = lo + s;
         int c[3];
-        key_coords(nd.key[i], D, D, c);
-        const float* cv = cell_v + 8 * s;
-        const i64 tb = tri_base[t];
-        for (int k = 0; k < 3 * nt; ++k) {
-            const int e = c_tri_edges[cc][k];
-            int lp[3], o, a0, a1, b0, b1;
-            edge_geom(e, c, lp, o, a0, a1, b0, b1);
+        key_coords(nd.key[i], em.D, em.D, c);
+        const float4 v0 = reinterpret_cast<const float4*>(cell_v + 8 * s)[0], v1 = reinterpret_cast<const float4*>(cell_v + 8 * s)[1];
+        const float cv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        emit_cell(em, c, cv, cat[s], tri0 + (list[t] >> CELL_BITS), 0, [&](int a0, int a1, int b0, int b1) {
             // edge owner among the real cells sharing it
             u64 best = ~0ull;
             int own_b0 = b0;
@@ -2265,46 +2315,33 @@ __global__ void k_emit_real(NodeArrays nd, EmitArgs em, i64 lo, const int* __res
                 int dxyz[3] = {0, 0, 0};
                 dxyz[a0] = d0;
                 dxyz[a1] = d1;
-                const int j = 9 * (dxyz[0] + 1) + 3 * (dxyz[1] + 1) + (dxyz[2] + 1);
-                const int nb = nd.neigh[(i64)j * nd.M + i];
+                const int nb = nd.neigh[(i64)(9 * (dxyz[0] + 1) + 3 * (dxyz[1] + 1) + (dxyz[2] + 1)) * nd.M + i];
                 if (nb == -1) continue;
                 const u64 kk = nd.key[nb];
                 if (kk < best) { best = kk; own_b0 = b0 - d0; }
             }
-            const bool rev = (o == 0 && own_b0 == 1);
-            const int ev0 = (b0 << a0) | (b1 << a1);   // corner kind of the lower end
-            const int ev1 = ev0 | (1 << o);
-            float p[3];
-            crossing(lp, o, rev, cv[ev0], cv[ev1], D, p);
-            const i64 slot = 3 * (tb + k / 3) + (k % 3);
-            em.keys[slot] = edge_key(lp, o, D, 0, em.local_bits);
-            em.slot[slot] = (uint32_t)slot;
-            em.pos[3 * slot] = p[0];
-            em.pos[3 * slot + 1] = p[1];
-            em.pos[3 * slot + 2] = p[2];
-        }
+            return own_b0 == 1;
+        });
     }
 }
 
-__global__ void k_emit_virtual(VArgs v, EmitArgs em, VirtCells vc, const i64* __restrict__ active, i64 nactive,
-                               const unsigned char* __restrict__ cat, const i64* __restrict__ tri_base) {
+__global__ void __launch_bounds__(CELL_BLOCK, 4) k_emit_virtual(VArgs v, EmitArgs em, LiveIndex lx, const float* __restrict__ lat,
+                                                             i64 total, const unsigned char* __restrict__ cat,
+                                                             const i64* __restrict__ tile_first) {
+    __shared__ int list[CELL_TILE];
+    const int nact = tile_active(cat, total, list);
     const int D = em.D;
-    for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < nactive; t += (i64)gridDim.x * blockDim.x) {
-        const i64 e = active[t];
+    const i64 tri0 = em.tri_offset + tile_first[blockIdx.x];
+    for (int t = threadIdx.x; t < nact; t += CELL_BLOCK) {
+        const i64 e = (i64)blockIdx.x * CELL_TILE + (list[t] & (CELL_TILE - 1));
         int cu[3];
         float cv[8];
-        const VRoot R = v.roots[virt_cell(vc, v, e, cu, cv)];
+        const VRoot R = v.roots[virt_cell(lx, lat, e, cu, cv)];
         const int S = 1 << (D - R.depth);
         int Lc[3];
         key_coords(v.e.nd.key[R.node], R.depth, D, Lc);
         const int c[3] = {Lc[0] * S + cu[0], Lc[1] * S + cu[1], Lc[2] * S + cu[2]};
-        const int cc = cat[e];
-        const int nt = c_tri_count[cc];
-        const i64 tb = em.tri_offset + tri_base[t];
-        for (int k = 0; k < 3 * nt; ++k) {
-            const int ed = c_tri_edges[cc][k];
-            int lp[3], o, a0, a1, b0, b1;
-            edge_geom(ed, c, lp, o, a0, a1, b0, b1);
+        emit_cell(em, c, cv, cat[e], tri0 + (list[t] >> CELL_BITS), em.weld ? 0 : R.batch, [&](int a0, int a1, int b0, int b1) {
             u64 best = ~0ull;
             int own_b0 = b0;
             for (int q = 0; q < 4; ++q) {
@@ -2316,18 +2353,8 @@ __global__ void k_emit_virtual(VArgs v, EmitArgs em, VirtCells vc, const i64* __
                 const u64 kk = cell_key_D(cell, D);
                 if (kk < best) { best = kk; own_b0 = b0 - d0; }
             }
-            const bool rev = (o == 0 && own_b0 == 1);
-            const int ev0 = (b0 << a0) | (b1 << a1);   // corner kind of the lower end
-            const int ev1 = ev0 | (1 << o);
-            float p[3];
-            crossing(lp, o, rev, cv[ev0], cv[ev1], D, p);
-            const i64 slot = 3 * (tb + k / 3) + (k % 3);
-            em.keys[slot] = edge_key(lp, o, D, em.weld ? 0 : R.batch, em.local_bits);
-            em.slot[slot] = (uint32_t)slot;
-            em.pos[3 * slot] = p[0];
-            em.pos[3 * slot + 1] = p[1];
-            em.pos[3 * slot + 2] = p[2];
-        }
+            return own_b0 == 1;
+        });
     }
 }
 
@@ -2394,26 +2421,6 @@ __global__ void k_key_heads(const u64* __restrict__ keys, i64 n, int* __restrict
     for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
         f[k] = (k == 0 || keys[k] != keys[k - 1]) ? 1 : 0;
 }
-__global__ void k_active_flags(const int* __restrict__ ntri, i64 n, int* __restrict__ f) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
-        f[k] = ntri[k] > 0 ? 1 : 0;
-}
-template <class TI>
-__global__ void k_compact_idx(const int* __restrict__ f, const int* __restrict__ pos, i64 n, TI* __restrict__ out) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
-        if (f[k]) out[pos[k]] = (TI)k;
-}
-__global__ void k_gather_ntri(const int* __restrict__ ntri, const i64* __restrict__ active, i64 n,
-                              i64* __restrict__ out) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
-        out[k] = ntri[active[k]];
-}
-__global__ void k_gather_ntri32(const int* __restrict__ ntri, const int* __restrict__ active, i64 n,
-                                int* __restrict__ out) {
-    for (i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (i64)gridDim.x * blockDim.x)
-        out[k] = ntri[active[k]];
-}
-
 void stage_mesh(Ctx& c) {
     ensure_mc_tables();
     cudaStream_t s = c.stream;
@@ -2434,10 +2441,11 @@ void stage_mesh(Ctx& c) {
     }
     c.kend(kx);
     // ---- finest corner values, categories
-    float* cval = dalloc<float>(8 * nD, s);
     float* cell_v = dalloc<float>(8 * nD, s);
     unsigned char* cat = dalloc<unsigned char>(nD, s);
-    int* ntri = dalloc<int>(nD, s);
+    const i64 rtiles = (nD + CELL_TILE - 1) / CELL_TILE;
+    int* rtri = dalloc<int>(rtiles, s);             // triangles of each tile of real cells
+    i64* rfirst = dalloc<i64>(rtiles + 1, s);       // first triangle of each tile, and their number
     int kt = c.kbegin("corner_values", (double)M * (108 + 8 + 4 + 4) + (double)nD * 8 * 4);
     {
         if (nD >= (1ll << 28)) {
@@ -2455,7 +2463,7 @@ void stage_mesh(Ctx& c) {
             int* olist = dalloc<int>(nown, s);
             k_finest_list<<<grid_for(nD, 256), 256, 0, s>>>(omask, ofirst, nD, olist);
             CK_LAUNCH();
-            k_finest_corner_values<<<grid_for(nown, 128, 1ll << 30), 128, 0, s>>>(ea, lo, olist, nown, c.iso, cval);
+            k_finest_corner_values<<<grid_for(nown, 128, 1ll << 30), 128, 0, s>>>(ea, lo, olist, nown, c.iso, cell_v);
             CK_LAUNCH();
             dfree(olist, s);
         }
@@ -2464,11 +2472,11 @@ void stage_mesh(Ctx& c) {
         dfree(ofirst, s);
     }
     c.kend(kt);
-    kt = c.kbegin("cells", (double)nD * (8 * 4 + 108 + 8 * 4 + 1 + 4));
-    k_finest_cells<<<grid_for(nD, 128, 1ll << 30), 128, 0, s>>>(nd, lo, M, cval, cell_v, cat, ntri);
+    kt = c.kbegin("cells", (double)nD * (8 * 4 + 1));
+    k_finest_cells<<<(unsigned)rtiles, CELL_BLOCK, 0, s>>>(cell_v, nD, cat, rtri);
     CK_LAUNCH();
+    exclusive_scan<int, i64>(rtri, rfirst, rtiles, rfirst + rtiles, s);
     c.kend(kt);
-    dfree(cval, s);
     // ---- face marks and subdivision roots
     int* fflag = dalloc<int>(6 * M, s);
     CK(cudaMemsetAsync(fflag, 0, (size_t)(6 * M) * sizeof(int), s));
@@ -2488,17 +2496,13 @@ void stage_mesh(Ctx& c) {
     CK(cudaMemsetAsync(is_root, 0, nCoarse * sizeof(int), s));
     if (nCoarse > 1) {
         const int kc = c.kbegin("coarse_leaves", (double)nCoarse * (4 + 108 + 8 + 3 * 4 + 8 * 4) + (double)M * 4);
-        unsigned char* need = dalloc<unsigned char>(8 * nCoarse, s);
-        float* ccv = dalloc<float>(8 * nCoarse, s);
-        CK(cudaMemsetAsync(need, 0, 8 * nCoarse, s));
-        k_coarse_need<<<grid_for(nCoarse - 1, 256), 256, 0, s>>>(nd, 1, nCoarse, need);
-        CK_LAUNCH();
+        float* leaf_v = dalloc<float>(8 * nCoarse, s);
         {
             // one thread per needed corner (list of (node << 3) | corner)
             unsigned char* nmask = dalloc<unsigned char>(nCoarse, s);
             int* ncnt = dalloc<int>(nCoarse, s);
             int* nfirst = dalloc<int>(nCoarse + 1, s);
-            k_need_mask<<<grid_for(nCoarse, 256), 256, 0, s>>>(need, nCoarse, nmask, ncnt);
+            k_coarse_owned<<<grid_for(nCoarse, 256), 256, 0, s>>>(nd, nCoarse, nmask, ncnt);
             CK_LAUNCH();
             exclusive_scan<int, int>(ncnt, nfirst, nCoarse, nfirst + nCoarse, s);
             const i64 nneed = read_scalar(nfirst + nCoarse, s);
@@ -2506,7 +2510,7 @@ void stage_mesh(Ctx& c) {
                 int* nlist = dalloc<int>(nneed, s);
                 k_finest_list<<<grid_for(nCoarse, 256), 256, 0, s>>>(nmask, nfirst, nCoarse, nlist);
                 CK_LAUNCH();
-                k_coarse_corner_list<<<grid_for(nneed, 128, 1ll << 30), 128, 0, s>>>(ea, nlist, nneed, c.iso, ccv);
+                k_coarse_corner_list<<<grid_for(nneed, 128, 1ll << 30), 128, 0, s>>>(ea, nlist, nneed, c.iso, leaf_v);
                 CK_LAUNCH();
                 dfree(nlist, s);
             }
@@ -2514,12 +2518,11 @@ void stage_mesh(Ctx& c) {
             dfree(ncnt, s);
             dfree(nfirst, s);
         }
-        k_coarse_leaves<<<grid_for(nCoarse - 1, 128, 1ll << 30), 128, 0, s>>>(ea, 1, nCoarse, ccv, fflag, has_tri,
+        k_coarse_leaves<<<grid_for(nCoarse - 1, 128, 1ll << 30), 128, 0, s>>>(nd, 1, nCoarse, leaf_v, fflag, has_tri,
                                                                              has_int, is_root);
         CK_LAUNCH();
         c.kend(kc);
-        dfree(need, s);
-        dfree(ccv, s);
+        dfree(leaf_v, s);
     }
     dfree(fflag, s);
     int kg = c.kbegin("mesh_lists", 0.0);
@@ -2572,47 +2575,27 @@ void stage_mesh(Ctx& c) {
     }
     dfree(is_root, s);
     c.subdivide_roots = nr;
-    // ---- real cells: active list, triangle bases
-    int* flags = dalloc<int>(std::max<i64>(nD, 1), s);
-    int* fpos = dalloc<int>(nD + 1, s);
-    k_active_flags<<<grid_for(nD, 256), 256, 0, s>>>(ntri, nD, flags);
-    CK_LAUNCH();
-    exclusive_scan<int, int>(flags, fpos, nD, fpos + nD, s);
-    const i64 nact_real = read_scalar(fpos + nD, s);
-    int* act_real = dalloc<int>(std::max<i64>(nact_real, 1), s);
-    k_compact_idx<int><<<grid_for(nD, 256), 256, 0, s>>>(flags, fpos, nD, act_real);
-    CK_LAUNCH();
-    int* tri_real = dalloc<int>(nact_real + 1, s);
-    {
-        int* tmp = dalloc<int>(std::max<i64>(nact_real, 1), s);
-        k_gather_ntri32<<<grid_for(nact_real, 256), 256, 0, s>>>(ntri, act_real, nact_real, tmp);
-        CK_LAUNCH();
-        exclusive_scan<int, int>(tmp, tri_real, nact_real, tri_real + nact_real, s);
-        dfree(tmp, s);
-    }
-    const i64 ntri_real = read_scalar(tri_real + nact_real, s);
-    dfree(flags, s);
-    dfree(fpos, s);
     c.kend(kg);
     // ---- virtual cells: every subdivided leaf cut into bricks, bounded and culled
     // before evaluation
-    i64 ntri_virt = 0, nact_virt = 0, total_cells = 0;
+    i64 total_cells = 0, vtiles = 0;
     c.total_bricks = 0;
     c.live_bricks = 0;
     c.foreign_corners = 0;
     c.foreign_slow = 0;
     VRoot* droots = nullptr;
-    i64 *act_virt = nullptr, *tri_virt = nullptr;
     unsigned char* vcat = nullptr;
-    int* vntri = nullptr;
+    i64* vfirst = nullptr;
     int* bflag = nullptr;
     float* lat_brick = nullptr;
     LiveBrick* live = nullptr;
+    unsigned long long* dcount = nullptr;   // foreign corners, window layout overflows, foreign corners evaluated
+    i64 fcap = 0;
+    LiveIndex lx{};
     VArgs va;
     va.e = ea;
     va.iso = c.iso;
     va.nroots = nr;
-    VirtCells vc{};
     if (nr > 0) {
         kg = c.kbegin("mesh_lists", 0.0);
         droots = dalloc<VRoot>(nr, s);
@@ -2734,130 +2717,95 @@ void stage_mesh(Ctx& c) {
         k_live_flags<<<grid_for(nbricks, 256), 256, 0, s>>>(culled, nbricks, bf);
         CK_LAUNCH();
         exclusive_scan<int, int>(bf, bp, nbricks, bp + nbricks, s);
-        const i64 nlive = read_scalar(bp + nbricks, s);
+        dfree(bf, s);
+        // live bricks of edge 8, and of edges 8 and 4, and in all: those before the first brick of depths
+        // D - 2 and D - 1, and before the end
+        int hl[3];
+        const i64 at[3] = {layout.off[0][std::max(D - 2, 0)], layout.off[0][D - 1], nbricks};
+        for (int q = 0; q < 3; ++q) CK(cudaMemcpyAsync(&hl[q], bp + at[q], sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        const i64 nlive = hl[2];
         c.total_bricks = nbricks;
         c.live_bricks = nlive;
         c.kend(kg);
         if (nlive > 0) {
             kg = c.kbegin("mesh_lists", 0.0);
             live = dalloc<LiveBrick>(nlive, s);
-            i64* lsz = dalloc<i64>(nlive, s);
-            i64* csz = dalloc<i64>(nlive, s);
-            i64* lpos = dalloc<i64>(nlive + 1, s);
-            i64* cpos = dalloc<i64>(nlive + 1, s);
-            k_live_bricks<<<grid_for(nbricks, 256), 256, 0, s>>>(va, bix, culled, bp, nbricks, live, lsz, csz);
+            lx = LiveIndex{live, hl[0], hl[1] - hl[0], hl[2] - hl[1]};
+            k_live_bricks<<<grid_for(nbricks, 256), 256, 0, s>>>(va, bix, culled, bp, nbricks, live);
             CK_LAUNCH();
-            exclusive_scan<i64, i64>(lsz, lpos, nlive, lpos + nlive, s);
-            exclusive_scan<i64, i64>(csz, cpos, nlive, cpos + nlive, s);
-            k_live_offsets<<<grid_for(nlive, 256), 256, 0, s>>>(live, lpos, cpos, nlive);
-            CK_LAUNCH();
-            const i64 lat_total = read_scalar(lpos + nlive, s);
-            total_cells = read_scalar(cpos + nlive, s);
-            lat_brick = dalloc<float>(lat_total, s);
-            // bricks of edge 8, 4 and 2 go to three instances of the evaluation
-            // counters: edge 8, edge 4, foreign corners, window layout overflows, foreign corners
-            // evaluated, edge 2
-            unsigned long long* cnt3 = dalloc<unsigned long long>(6, s);
-            int* lists = dalloc<int>(3 * nlive, s);
-            CK(cudaMemsetAsync(cnt3, 0, 6 * sizeof(unsigned long long), s));
-            k_live_split<<<grid_for(nlive, 256), 256, 0, s>>>(va, live, nlive, lists, lists + nlive,
-                                                              lists + 2 * nlive, cnt3);
-            CK_LAUNCH();
-            unsigned long long hc[6];
-            CK(cudaMemcpyAsync(hc, cnt3, sizeof hc, cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
+            total_cells = lx.cells();
+            lat_brick = dalloc<float>(lx.lattices(), s);
+            dcount = dalloc<unsigned long long>(3, s);
+            CK(cudaMemsetAsync(dcount, 0, 3 * sizeof(unsigned long long), s));
             // corners owned by another leaf: at most the lower-face corners of the live bricks
-            const i64 fcap = (i64)hc[0] * (9 * 9 * 9 - 8 * 8 * 8) + (i64)hc[1] * (5 * 5 * 5 - 4 * 4 * 4) +
-                             (i64)hc[5] * (3 * 3 * 3 - 2 * 2 * 2);
+            fcap = lx.lattices() - lx.cells();
             ForeignCorner* foreign = dalloc<ForeignCorner>(fcap, s);
             c.kend(kg);
             // compulsory: the corner values written (bricks of edge 8: 729 each)
-            const int ke = c.kbegin("brick_eval", (double)hc[0] * BR_CORNERS * 4);
-            if (hc[0] > 0) {
-                k_brick_eval<8, 96><<<grid_for((i64)hc[0], 1, (i64)c.sms * 16), 96, 0, s>>>(
-                    va, bix, root_of, live, lists, (i64)hc[0], lat_brick, cnt3 + 2, foreign, fcap);
+            const int ke = c.kbegin("brick_eval", (double)lx.n8 * BR_CORNERS * 4);
+            if (lx.n8 > 0) {
+                k_brick_eval<8, 96><<<grid_for(lx.n8, 1, (i64)c.sms * 16), 96, 0, s>>>(
+                    va, bix, root_of, lx, 0, lx.n8, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
             c.kend(ke);
-            const int ks = c.kbegin("brick_eval_small", (double)(lat_total - (i64)hc[0] * BR_CORNERS) * 4);
-            if (hc[1] > 0) {
-                k_brick_eval<4, 32><<<grid_for((i64)hc[1], 1, (i64)c.sms * 32), 32, 0, s>>>(
-                    va, bix, root_of, live, lists + nlive, (i64)hc[1], lat_brick, cnt3 + 2, foreign, fcap);
+            const int ks = c.kbegin("brick_eval_small", (double)(125 * lx.n4 + 27 * lx.n2) * 4);
+            if (lx.n4 > 0) {
+                k_brick_eval<4, 32><<<grid_for(lx.n4, 1, (i64)c.sms * 32), 32, 0, s>>>(
+                    va, bix, root_of, lx, lx.n8, lx.n4, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
-            if (hc[5] > 0) {
-                k_edge2_eval<<<grid_for((i64)hc[5], 3 * E2_WARPS, (i64)c.sms * 64), 32 * E2_WARPS, 0, s>>>(
-                    va, bix, root_of, live, lists + 2 * nlive, (i64)hc[5], lat_brick, cnt3 + 2, foreign, fcap);
+            if (lx.n2 > 0) {
+                k_edge2_eval<<<grid_for(lx.n2, 3 * E2_WARPS, (i64)c.sms * 64), 32 * E2_WARPS, 0, s>>>(
+                    va, bix, root_of, lx, lx.n8 + lx.n4, lx.n2, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
             c.kend(ks);
-            unsigned long long hf[2];
-            CK(cudaMemcpyAsync(hf, cnt3 + 2, sizeof hf, cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            c.foreign_corners = (i64)hf[0];
-            if (hf[1]) {
-                set_last_error("brick window layout overflow in %llu bricks", hf[1]);
-                throw Error{PRGPU_ERR_LIMIT, {0}};
-            }
-            if ((i64)hf[0] > fcap) {
-                set_last_error("foreign corner list overflow (%llu > %lld)", hf[0], (long long)fcap);
-                throw Error{PRGPU_ERR_LIMIT, {0}};
-            }
-            if (hf[0] > 0) {
-                const int kf = c.kbegin("foreign_fill", (double)hf[0] * 8);
-                k_foreign_fill<<<grid_for((i64)hf[0], 128, 1ll << 30), 128, 0, s>>>(
-                    va, bix, live, culled, bp, foreign, (i64)hf[0], lat_brick, cnt3 + 4);
-                CK_LAUNCH();
-                c.kend(kf);
-                c.foreign_slow = (i64)read_scalar(cnt3 + 4, s);
-            }
-            dfree(cnt3, s);
-            dfree(lists, s);
+            const int kf = c.kbegin("foreign_fill", 0.0);
+            k_foreign_fill<<<grid_for(fcap, 128, (i64)c.sms * 512), 128, 0, s>>>(va, bix, lx, culled, bp, foreign, fcap,
+                                                                                lat_brick, dcount);
+            CK_LAUNCH();
+            c.kend(kf);
             dfree(foreign, s);
-            dfree(lsz, s);
-            dfree(csz, s);
-            dfree(lpos, s);
-            dfree(cpos, s);
         }
-        dfree(bf, s);
         dfree(bp, s);
         dfree(culled, s);
         dfree(root_of, s);
         dfree(dpre, s);
         dfree(rows, s);
         dfree(up, s);
-        vc.live = live;
-        vc.nlive = nlive;
-        vc.lat = lat_brick;
         if (total_cells > 0) {
             vcat = dalloc<unsigned char>(total_cells, s);
-            vntri = dalloc<int>(total_cells, s);
+            vtiles = (total_cells + CELL_TILE - 1) / CELL_TILE;
+            int* vtri = dalloc<int>(vtiles, s);
+            vfirst = dalloc<i64>(vtiles + 1, s);
             const int kc2 = c.kbegin("virtual_cells", (double)total_cells * (8 * 4 + 5));
-            k_virtual_cells<<<grid_for(total_cells, 256, 1ll << 30), 256, 0, s>>>(va, vc, total_cells, vcat, vntri);
+            k_virtual_cells<<<(unsigned)vtiles, CELL_BLOCK, 0, s>>>(lx, lat_brick, total_cells, vcat, vtri);
             CK_LAUNCH();
+            exclusive_scan<int, i64>(vtri, vfirst, vtiles, vfirst + vtiles, s);
+            dfree(vtri, s);
             c.kend(kc2);
-            kg = c.kbegin("mesh_lists", 0.0);
-            int* vf = dalloc<int>(total_cells, s);
-            int* vp = dalloc<int>(total_cells + 1, s);
-            k_active_flags<<<grid_for(total_cells, 256), 256, 0, s>>>(vntri, total_cells, vf);
-            CK_LAUNCH();
-            exclusive_scan<int, int>(vf, vp, total_cells, vp + total_cells, s);
-            nact_virt = read_scalar(vp + total_cells, s);
-            act_virt = dalloc<i64>(std::max<i64>(nact_virt, 1), s);
-            k_compact_idx<i64><<<grid_for(total_cells, 256), 256, 0, s>>>(vf, vp, total_cells, act_virt);
-            CK_LAUNCH();
-            dfree(vf, s);
-            dfree(vp, s);
-            tri_virt = dalloc<i64>(nact_virt + 1, s);
-            i64* tmp = dalloc<i64>(std::max<i64>(nact_virt, 1), s);
-            k_gather_ntri<<<grid_for(nact_virt, 256), 256, 0, s>>>(vntri, act_virt, nact_virt, tmp);
-            CK_LAUNCH();
-            exclusive_scan<i64, i64>(tmp, tri_virt, nact_virt, tri_virt + nact_virt, s);
-            dfree(tmp, s);
-            ntri_virt = read_scalar(tri_virt + nact_virt, s);
-            c.kend(kg);
         }
     }
+    // the triangles of both kinds, and the checks and counts of the evaluation, in one read
+    i64 ntri_real = 0, ntri_virt = 0;
+    unsigned long long hc[3] = {0, 0, 0};
+    CK(cudaMemcpyAsync(&ntri_real, rfirst + rtiles, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    if (vfirst) CK(cudaMemcpyAsync(&ntri_virt, vfirst + vtiles, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    if (dcount) CK(cudaMemcpyAsync(hc, dcount, sizeof hc, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    dfree(dcount, s);
+    if (hc[1]) {
+        set_last_error("brick window layout overflow in %llu bricks", hc[1]);
+        throw Error{PRGPU_ERR_LIMIT, {0}};
+    }
+    if ((i64)hc[0] > fcap) {
+        set_last_error("foreign corner list overflow (%llu > %lld)", hc[0], (long long)fcap);
+        throw Error{PRGPU_ERR_LIMIT, {0}};
+    }
+    c.foreign_corners = (i64)hc[0];
+    c.foreign_slow = (i64)hc[2];
     c.virtual_cells = total_cells;
     // ---- emission, sort, vertex ids
     const i64 ntri_all = ntri_real + ntri_virt;
@@ -2887,16 +2835,14 @@ void stage_mesh(Ctx& c) {
         em.slot = dalloc<uint32_t>(nem, s);
         em.pos = dalloc<float>(3 * nem, s);
         const int kem = c.kbegin("emit", (double)nem * (8 + 4 + 12));
-        if (nact_real > 0) {
-            k_emit_real<<<grid_for(nact_real, 128, 1ll << 30), 128, 0, s>>>(nd, em, lo, act_real, nact_real, cat,
-                                                                            tri_real, cell_v);
+        if (ntri_real > 0) {
+            k_emit_real<<<(unsigned)rtiles, CELL_BLOCK, 0, s>>>(nd, em, lo, nD, cat, rfirst, cell_v);
             CK_LAUNCH();
         }
-        if (nact_virt > 0) {
+        if (ntri_virt > 0) {
             EmitArgs ev = em;
             ev.tri_offset = ntri_real;
-            k_emit_virtual<<<grid_for(nact_virt, 128, 1ll << 30), 128, 0, s>>>(va, ev, vc, act_virt, nact_virt, vcat,
-                                                                               tri_virt);
+            k_emit_virtual<<<(unsigned)vtiles, CELL_BLOCK, 0, s>>>(va, ev, lx, lat_brick, total_cells, vcat, vfirst);
             CK_LAUNCH();
         }
         c.kend(kem);
@@ -2931,16 +2877,15 @@ void stage_mesh(Ctx& c) {
         dfree(hf, s); dfree(hp, s); dfree(tri_vid, s); dfree(vpos, s);
         dfree(em.keys, s); dfree(em.slot, s); dfree(em.pos, s);
     }
-    dfree(act_real, s);
-    dfree(tri_real, s);
-    dfree(droots, s); dfree(droot_list, s); dfree(act_virt, s); dfree(tri_virt, s);
-    dfree(vcat, s); dfree(vntri, s); dfree(bflag, s);
+    dfree(rtri, s);
+    dfree(rfirst, s);
+    dfree(droots, s); dfree(droot_list, s);
+    dfree(vcat, s); dfree(vfirst, s); dfree(bflag, s);
     dfree(lat_brick, s); dfree(live, s);
     dfree(cell_v, s);
     dfree(x27, s);
     dfree(lb, s);
     dfree(cat, s);
-    dfree(ntri, s);
 }
 
 }  // namespace prgpu
