@@ -424,8 +424,6 @@ __global__ void __launch_bounds__(128, 12) k_finest_corner_values(EvalArgs a, i6
 constexpr int CELL_BLOCK = 256;
 constexpr int CELL_ITEMS = 4;
 constexpr int CELL_TILE = CELL_ITEMS * CELL_BLOCK;
-constexpr int CELL_BITS = 10;
-static_assert(CELL_TILE == 1 << CELL_BITS, "");
 __device__ __forceinline__ void tile_triangles(int n, int* __restrict__ tile_tri) {
     __shared__ int s_n[CELL_BLOCK / 32];
     n = __reduce_add_sync(0xffffffffu, n);
@@ -437,27 +435,31 @@ __device__ __forceinline__ void tile_triangles(int n, int* __restrict__ tile_tri
         tile_tri[blockIdx.x] = t;
     }
 }
-// the tile's active cells in order, packed (cell in the tile) | (first triangle in the tile) << CELL_BITS, into
-// list; returns their number.  list: CELL_TILE ints of shared memory; all threads call
-__device__ __forceinline__ int tile_active(const unsigned char* __restrict__ cat, i64 total, int* list) {
-    __shared__ int sw[32];
+// The tile's active cells: cell (in the tile) of each of its triangles, and each cell's first triangle, in
+// shared memory; returns the tile's triangles.  All threads call.
+struct TileShared {
+    unsigned short cell[5 * CELL_TILE];   // of triangle t (a cell has at most 5)
+    unsigned short first[CELL_TILE];      // first triangle of a cell
+    int sw[32];
+};
+__device__ __forceinline__ int tile_active(const unsigned char* __restrict__ cat, i64 total, TileShared& sm) {
     const i64 c0 = (i64)blockIdx.x * CELL_TILE + CELL_ITEMS * threadIdx.x;
     int nt[CELL_ITEMS], mine = 0;
 #pragma unroll
     for (int k = 0; k < CELL_ITEMS; ++k) {
         nt[k] = c0 + k < total ? c_tri_count[cat[c0 + k]] : 0;
-        mine += nt[k] ? (1 << 16) + nt[k] : 0;      // (active cells, triangles): at most 1024 and 5120
+        mine += nt[k];
     }
     int all;
-    int at = block_exclusive_sum<int>(mine, sw, &all);
+    int at = block_exclusive_sum<int>(mine, sm.sw, &all);
 #pragma unroll
-    for (int k = 0; k < CELL_ITEMS; ++k)
-        if (nt[k]) {
-            list[at >> 16] = (CELL_ITEMS * (int)threadIdx.x + k) | ((at & 0xffff) << CELL_BITS);
-            at += (1 << 16) + nt[k];
-        }
+    for (int k = 0; k < CELL_ITEMS; ++k) {
+        const int cell = CELL_ITEMS * (int)threadIdx.x + k;
+        sm.first[cell] = (unsigned short)at;
+        for (int t = 0; t < nt[k]; ++t) sm.cell[at++] = (unsigned short)cell;
+    }
     __syncthreads();
-    return all >> 16;
+    return all;
 }
 
 // cube category of each finest cell, the tile's triangles
@@ -2187,21 +2189,6 @@ __global__ void k_live_flags(const unsigned char* __restrict__ culled, i64 n, in
 }
 
 // ---- virtual cells: the cells of the live bricks
-// brick and cell coordinates in its root's lattice of virtual cell e, and the cell's 8 corner values (minus iso)
-__device__ __forceinline__ int virt_cell(const LiveIndex& lx, const float* __restrict__ lat, i64 e, int cu[3], float cv[8]) {
-    int lg, loc;
-    const i64 li = lx.brick(e, lg, loc);
-    const int E = 1 << lg, E1 = E + 1;
-    const int l3[3] = {loc >> (2 * lg), (loc >> lg) & (E - 1), loc & (E - 1)};
-    const LiveBrick lb = lx.live[li];
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) cu[ax] = lb.b[ax] * E + l3[ax];
-    const float* L = lat + lx.lat(li) + (l3[0] * E1 + l3[1]) * E1 + l3[2];
-#pragma unroll
-    for (int kind = 0; kind < 8; ++kind) cv[kind] = L[((kind & 1) * E1 + ((kind >> 1) & 1)) * E1 + (kind >> 2)];
-    return lb.root;
-}
-
 __global__ void __launch_bounds__(CELL_BLOCK) k_virtual_cells(LiveIndex lx, const float* __restrict__ lat, i64 total,
                                                               unsigned char* __restrict__ cat, int* __restrict__ tile_tri) {
     int tri = 0;
@@ -2269,92 +2256,98 @@ __device__ __forceinline__ void edge_geom(int e, const int c[3], int lp[3], int&
     lp[a1] += b1;
 }
 
-// Emission of one cell's triangles: every triangle corner's edge key and crossing.  rev(a0, a1, b0, b1): the
-// edge at offsets b0, b1 along the axes a0, a1 runs reversed in its owner's frame; only edges along x do
-// (crossing's frame), so only they look for their owner.
-template <class R>
-__device__ __forceinline__ void emit_cell(const EmitArgs& em, const int c[3], const float cv[8], int cc, i64 tri, int batch,
-                                          R rev) {
-    const int nt = c_tri_count[cc];
-    for (int k = 0; k < 3 * nt; ++k) {
-        const int e = c_tri_edges[cc][k];
-        int lp[3], o, a0, a1, b0, b1;
-        edge_geom(e, c, lp, o, a0, a1, b0, b1);
-        const int ev0 = (b0 << a0) | (b1 << a1);   // corner kind of the lower end
-        const int ev1 = ev0 | (1 << o);
-        float p[3];
-        crossing(lp, o, o == 0 && rev(a0, a1, b0, b1), cv[ev0], cv[ev1], em.D, p);
-        const i64 slot = 3 * tri + k;
-        em.keys[slot] = edge_key(lp, o, em.D, batch, em.local_bits);
-        em.slot[slot] = (uint32_t)slot;
-        em.pos[3 * slot] = p[0];
-        em.pos[3 * slot + 1] = p[1];
-        em.pos[3 * slot + 2] = p[2];
-    }
+// Emission: a thread per triangle corner, in the order of the output, so that a warp writes 32 consecutive
+// keys, slots and positions.  (A thread per cell writes its corners one by one, every store of a warp
+// spread over 32 sectors: 0.52 ms for the 9.2 M corners of the 1M torus, 220 MB.)
+// Corner k of the cell's triangles: its edge's key and crossing.  rev(a0, a1, b0, b1): the edge at offsets
+// b0, b1 along the axes a0, a1 runs reversed in its owner's frame; only edges along x do (crossing's
+// frame), so only they look for their owner.
+template <class V, class R>
+__device__ __forceinline__ void emit_corner(const EmitArgs& em, const int c[3], V value, int cc, int k, i64 slot, int batch,
+                                            R rev) {
+    const int e = c_tri_edges[cc][k];
+    int lp[3], o, a0, a1, b0, b1;
+    edge_geom(e, c, lp, o, a0, a1, b0, b1);
+    const int ev0 = (b0 << a0) | (b1 << a1);   // corner kind of the lower end
+    const int ev1 = ev0 | (1 << o);
+    float p[3];
+    crossing(lp, o, o == 0 && rev(a0, a1, b0, b1), value(ev0), value(ev1), em.D, p);
+    em.keys[slot] = edge_key(lp, o, em.D, batch, em.local_bits);
+    em.slot[slot] = (uint32_t)slot;
+    em.pos[3 * slot] = p[0];
+    em.pos[3 * slot + 1] = p[1];
+    em.pos[3 * slot + 2] = p[2];
 }
 
 // real finest cells
-__global__ void __launch_bounds__(CELL_BLOCK, 5) k_emit_real(NodeArrays nd, EmitArgs em, i64 lo, i64 total,
+__global__ void __launch_bounds__(CELL_BLOCK) k_emit_real(NodeArrays nd, EmitArgs em, i64 lo, i64 total,
                                                           const unsigned char* __restrict__ cat,
                                                           const i64* __restrict__ tile_first, const float* __restrict__ cell_v) {
-    __shared__ int list[CELL_TILE];
-    const int nact = tile_active(cat, total, list);
-    const i64 tri0 = em.tri_offset + tile_first[blockIdx.x];
-    for (int t = threadIdx.x; t < nact; t += CELL_BLOCK) {
-        const i64 s = (i64)blockIdx.x * CELL_TILE + (list[t] & (CELL_TILE - 1)), i = lo + s;
+    __shared__ TileShared sm;
+    const int n = 3 * tile_active(cat, total, sm);
+    const i64 slot0 = 3 * (em.tri_offset + tile_first[blockIdx.x]);
+    for (int q = threadIdx.x; q < n; q += CELL_BLOCK) {
+        const int cell = sm.cell[q / 3];
+        const i64 s = (i64)blockIdx.x * CELL_TILE + cell, i = lo + s;
         int c[3];
         key_coords(nd.key[i], em.D, em.D, c);
-        const float4 v0 = reinterpret_cast<const float4*>(cell_v + 8 * s)[0], v1 = reinterpret_cast<const float4*>(cell_v + 8 * s)[1];
-        const float cv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        emit_cell(em, c, cv, cat[s], tri0 + (list[t] >> CELL_BITS), 0, [&](int a0, int a1, int b0, int b1) {
-            // edge owner among the real cells sharing it
-            u64 best = ~0ull;
-            int own_b0 = b0;
-            for (int q = 0; q < 4; ++q) {
-                const int d0 = b0 - (q & 1), d1 = b1 - ((q >> 1) & 1);
-                int dxyz[3] = {0, 0, 0};
-                dxyz[a0] = d0;
-                dxyz[a1] = d1;
-                const int nb = nd.neigh[(i64)(9 * (dxyz[0] + 1) + 3 * (dxyz[1] + 1) + (dxyz[2] + 1)) * nd.M + i];
-                if (nb == -1) continue;
-                const u64 kk = nd.key[nb];
-                if (kk < best) { best = kk; own_b0 = b0 - d0; }
-            }
-            return own_b0 == 1;
-        });
+        const float* cv = cell_v + 8 * s;
+        emit_corner(em, c, [&](int kind) { return cv[kind]; }, cat[s], q - 3 * sm.first[cell], slot0 + q, 0,
+                    [&](int a0, int a1, int b0, int b1) {
+                        // edge owner among the real cells sharing it
+                        u64 best = ~0ull;
+                        int own_b0 = b0;
+                        for (int t = 0; t < 4; ++t) {
+                            const int d0 = b0 - (t & 1), d1 = b1 - ((t >> 1) & 1);
+                            int dxyz[3] = {0, 0, 0};
+                            dxyz[a0] = d0;
+                            dxyz[a1] = d1;
+                            const int nb = nd.neigh[(i64)(9 * (dxyz[0] + 1) + 3 * (dxyz[1] + 1) + (dxyz[2] + 1)) * nd.M + i];
+                            if (nb == -1) continue;
+                            const u64 kk = nd.key[nb];
+                            if (kk < best) { best = kk; own_b0 = b0 - d0; }
+                        }
+                        return own_b0 == 1;
+                    });
     }
 }
 
-__global__ void __launch_bounds__(CELL_BLOCK, 4) k_emit_virtual(VArgs v, EmitArgs em, LiveIndex lx, const float* __restrict__ lat,
+__global__ void __launch_bounds__(CELL_BLOCK) k_emit_virtual(VArgs v, EmitArgs em, LiveIndex lx, const float* __restrict__ lat,
                                                              i64 total, const unsigned char* __restrict__ cat,
                                                              const i64* __restrict__ tile_first) {
-    __shared__ int list[CELL_TILE];
-    const int nact = tile_active(cat, total, list);
+    __shared__ TileShared sm;
+    const int n = 3 * tile_active(cat, total, sm);
     const int D = em.D;
-    const i64 tri0 = em.tri_offset + tile_first[blockIdx.x];
-    for (int t = threadIdx.x; t < nact; t += CELL_BLOCK) {
-        const i64 e = (i64)blockIdx.x * CELL_TILE + (list[t] & (CELL_TILE - 1));
-        int cu[3];
-        float cv[8];
-        const VRoot R = v.roots[virt_cell(lx, lat, e, cu, cv)];
+    const i64 slot0 = 3 * (em.tri_offset + tile_first[blockIdx.x]);
+    for (int q = threadIdx.x; q < n; q += CELL_BLOCK) {
+        const int cell = sm.cell[q / 3];
+        const i64 e = (i64)blockIdx.x * CELL_TILE + cell;
+        int lg, loc;
+        const i64 li = lx.brick(e, lg, loc);
+        const int E = 1 << lg, E1 = E + 1;
+        const int l3[3] = {loc >> (2 * lg), (loc >> lg) & (E - 1), loc & (E - 1)};
+        const LiveBrick lb = lx.live[li];
+        const VRoot R = v.roots[lb.root];
         const int S = 1 << (D - R.depth);
         int Lc[3];
         key_coords(v.e.nd.key[R.node], R.depth, D, Lc);
-        const int c[3] = {Lc[0] * S + cu[0], Lc[1] * S + cu[1], Lc[2] * S + cu[2]};
-        emit_cell(em, c, cv, cat[e], tri0 + (list[t] >> CELL_BITS), em.weld ? 0 : R.batch, [&](int a0, int a1, int b0, int b1) {
-            u64 best = ~0ull;
-            int own_b0 = b0;
-            for (int q = 0; q < 4; ++q) {
-                const int d0 = b0 - (q & 1), d1 = b1 - ((q >> 1) & 1);
-                int cell[3] = {c[0], c[1], c[2]};
-                cell[a0] += d0;
-                cell[a1] += d1;
-                if (batch_member(v, R, Lc, cell) < 0) continue;
-                const u64 kk = cell_key_D(cell, D);
-                if (kk < best) { best = kk; own_b0 = b0 - d0; }
-            }
-            return own_b0 == 1;
-        });
+        const int c[3] = {Lc[0] * S + lb.b[0] * E + l3[0], Lc[1] * S + lb.b[1] * E + l3[1], Lc[2] * S + lb.b[2] * E + l3[2]};
+        const float* L = lat + lx.lat(li) + (l3[0] * E1 + l3[1]) * E1 + l3[2];
+        emit_corner(em, c, [&](int kind) { return L[((kind & 1) * E1 + ((kind >> 1) & 1)) * E1 + (kind >> 2)]; }, cat[e],
+                    q - 3 * sm.first[cell], slot0 + q, em.weld ? 0 : R.batch, [&](int a0, int a1, int b0, int b1) {
+                        u64 best = ~0ull;
+                        int own_b0 = b0;
+                        for (int t = 0; t < 4; ++t) {
+                            const int d0 = b0 - (t & 1), d1 = b1 - ((t >> 1) & 1);
+                            int oc[3] = {c[0], c[1], c[2]};
+                            oc[a0] += d0;
+                            oc[a1] += d1;
+                            if (batch_member(v, R, Lc, oc) < 0) continue;
+                            const u64 kk = cell_key_D(oc, D);
+                            if (kk < best) { best = kk; own_b0 = b0 - d0; }
+                        }
+                        return own_b0 == 1;
+                    });
     }
 }
 
