@@ -150,6 +150,18 @@ int prgpu_reconstruct(void* ctx, const float* xyz, const float* nrm, int64_t n, 
 int prgpu_reconstruct_batch(void* ctx, const float* xyz, const float* nrm, const int64_t* offsets,
                             const int32_t* depths, int32_t ncloud, prgpu_mesh* outs);
 
+/* The same with the meshes written straight into the caller's memory: once cloud k's size is known, alloc (from
+ * the host thread that ran it, up to four at a time) sets *vertices and *triangles to room for 3 n_vertices floats
+ * and 3 n_triangles int32 and returns 0; outs[k] points there and is not for prgpu_mesh_free.  A null alloc is prgpu_reconstruct_batch. */
+typedef int (*prgpu_mesh_alloc)(void* user, int32_t cloud, int64_t n_vertices, int64_t n_triangles, float** vertices,
+                                int32_t** triangles);
+int prgpu_reconstruct_batch_into(void* ctx, const float* xyz, const float* nrm, const int64_t* offsets,
+                                 const int32_t* depths, int32_t ncloud, prgpu_mesh_alloc alloc, void* user,
+                                 prgpu_mesh* outs);
+
+/* Copies a mesh to the caller's arrays (3 floats per vertex, 3 int32 per triangle), large ones by several threads. */
+int prgpu_copy_mesh(const prgpu_mesh* mesh, float* vertices, int32_t* triangles);
+
 /* Releases a mesh returned by prgpu_reconstruct_batch and zeroes it. */
 int prgpu_mesh_free(prgpu_mesh* mesh);
 

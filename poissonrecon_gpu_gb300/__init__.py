@@ -62,6 +62,11 @@ class Mesh(ctypes.Structure):
                 ("vertices", ctypes.POINTER(ctypes.c_float)), ("triangles", ctypes.POINTER(ctypes.c_int32))]
 
 
+# prgpu_mesh_alloc
+MeshAlloc = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_int64,
+                             ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p))
+
+
 class NodeArrays(ctypes.Structure):
     _fields_ = [("n_nodes", ctypes.c_int64), ("max_depth", ctypes.c_int32),
                 ("base", ctypes.c_void_p), ("key", ctypes.c_void_p), ("pidx", ctypes.c_void_p),
@@ -87,6 +92,9 @@ SIGNATURES = {
     "prgpu_get_mesh": (ctypes.c_int, [_VP, ctypes.POINTER(Mesh)]),
     "prgpu_reconstruct": (ctypes.c_int, [_VP, _VP, _VP, _I64, ctypes.POINTER(Mesh)]),
     "prgpu_reconstruct_batch": (ctypes.c_int, [_VP, _VP, _VP, _VP, _VP, ctypes.c_int32, ctypes.POINTER(Mesh)]),
+    "prgpu_reconstruct_batch_into": (ctypes.c_int, [_VP, _VP, _VP, _VP, _VP, ctypes.c_int32, MeshAlloc, _VP,
+                                                    ctypes.POINTER(Mesh)]),
+    "prgpu_copy_mesh": (ctypes.c_int, [ctypes.POINTER(Mesh), _VP, _VP]),
     "prgpu_mesh_free": (ctypes.c_int, [ctypes.POINTER(Mesh)]),
     "prgpu_get_array": (ctypes.c_int, [_VP, ctypes.c_char_p, _VP, _I64, ctypes.POINTER(_I64)]),
     "prgpu_set_array": (ctypes.c_int, [_VP, ctypes.c_char_p, _VP, _I64]),
@@ -241,10 +249,8 @@ class Reconstructor:
     def mesh(self):
         m = Mesh()
         _check(_lib().prgpu_get_mesh(self._h, ctypes.byref(m)), "prgpu_get_mesh")
-        v = np.ctypeslib.as_array(m.vertices, shape=(m.n_vertices * 3,)).reshape(-1, 3).copy() \
-            if m.n_vertices else np.zeros((0, 3), np.float32)
-        f = np.ctypeslib.as_array(m.triangles, shape=(m.n_triangles * 3,)).reshape(-1, 3).copy() \
-            if m.n_triangles else np.zeros((0, 3), np.int32)
+        v, f = np.empty((m.n_vertices, 3), np.float32), np.empty((m.n_triangles, 3), np.int32)
+        _check(_lib().prgpu_copy_mesh(ctypes.byref(m), v.ctypes.data, f.ctypes.data), "prgpu_copy_mesh")
         return v, f
 
     def reconstruct(self, xyz, nrm):
@@ -265,18 +271,20 @@ class Reconstructor:
         offsets[1:] = np.cumsum([len(c[0]) for c in clouds])
         dep = None if depths is None else np.ascontiguousarray(depths, dtype=np.int32)
         outs = (Mesh * max(len(clouds), 1))()
-        _check(_lib().prgpu_reconstruct_batch(self._h, xyz.ctypes.data, nrm.ctypes.data, offsets.ctypes.data,
-                                              None if dep is None else dep.ctypes.data, len(clouds), outs),
-               "prgpu_reconstruct_batch")
-        result = []
-        for k in range(len(clouds)):
-            m = outs[k]
-            v = np.ctypeslib.as_array(m.vertices, shape=(m.n_vertices * 3,)).reshape(-1, 3).copy() \
-                if m.n_vertices else np.zeros((0, 3), np.float32)
-            f = np.ctypeslib.as_array(m.triangles, shape=(m.n_triangles * 3,)).reshape(-1, 3).copy() \
-                if m.n_triangles else np.zeros((0, 3), np.int32)
-            _lib().prgpu_mesh_free(ctypes.byref(m))
-            result.append((v, f))
+        result = [None] * len(clouds)
+
+        def alloc(_, k, nv, nt, pv, pf):          # called on the library's host threads
+            try:
+                v, f = np.empty((nv, 3), np.float32), np.empty((nt, 3), np.int32)
+            except MemoryError:
+                return 1
+            result[k] = v, f
+            pv[0], pf[0] = v.ctypes.data, f.ctypes.data
+            return 0
+
+        _check(_lib().prgpu_reconstruct_batch_into(self._h, xyz.ctypes.data, nrm.ctypes.data, offsets.ctypes.data,
+                                                   None if dep is None else dep.ctypes.data, len(clouds),
+                                                   MeshAlloc(alloc), None, outs), "prgpu_reconstruct_batch")
         return result
 
     # ---- arrays

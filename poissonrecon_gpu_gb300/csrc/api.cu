@@ -417,18 +417,69 @@ int prgpu_mesh_free(prgpu_mesh* m) {
     return PRGPU_OK;
 }
 
-// a reconstructed mesh copied into memory the caller releases with prgpu_mesh_free
-static int copy_mesh_out(const prgpu_mesh& m, prgpu_mesh* out) {
-    float* vv = (float*)malloc(sizeof(float) * 3 * (size_t)std::max<int64_t>(m.n_vertices, 1));
-    int32_t* ff = (int32_t*)malloc(sizeof(int32_t) * 3 * (size_t)std::max<int64_t>(m.n_triangles, 1));
-    if (!vv || !ff) {
-        free(vv);
-        free(ff);
+// A copy into memory written for the first time: its pages are mapped and zeroed as they are touched, which holds one
+// thread to about 12 GB/s, so large copies are cut at 2 MB boundaries of the destination and shared by several threads:
+// 40 MB 2.6 -> 0.6 ms, 120 MB 10 -> 1.9 ms, 360 MB 31 -> 5 ms.  Below 16 MB the allocator often hands out memory that
+// is mapped already, and one thread is the faster (12 MB: 0.40 ms against 0.44; fresh memory 0.81 against 0.47).
+// A thread that cannot be started leaves its part to the caller.
+constexpr size_t COPY_WIDE = (size_t)16 << 20, COPY_PART = (size_t)4 << 20, COPY_PAGE = (size_t)2 << 20;
+constexpr size_t COPY_THREADS = 8;
+
+static void copy_wide(void* dst, const void* src, size_t bytes) {
+    if (bytes < COPY_WIDE) {
+        if (bytes) memcpy(dst, src, bytes);
+        return;
+    }
+    const size_t parts = std::min(COPY_THREADS, bytes / COPY_PART);
+    auto cut = [&](size_t k) -> size_t {   // where part k begins
+        if (k == 0) return 0;
+        if (k >= parts) return bytes;
+        const size_t at = (size_t)dst + bytes / parts * k;
+        return std::min(bytes, (at + COPY_PAGE - 1) / COPY_PAGE * COPY_PAGE - (size_t)dst);
+    };
+    auto part = [&](size_t k) { memcpy((char*)dst + cut(k), (const char*)src + cut(k), cut(k + 1) - cut(k)); };
+    std::thread th[COPY_THREADS];
+    size_t started = 1;
+    try {
+        for (; started < parts; ++started) th[started] = std::thread(part, started);
+    } catch (...) {
+    }
+    part(0);
+    for (size_t k = started; k < parts; ++k) part(k);
+    for (size_t k = 1; k < started; ++k) th[k].join();
+}
+
+int prgpu_copy_mesh(const prgpu_mesh* m, float* vertices, int32_t* triangles) {
+    if (!m || (m->n_vertices && (!m->vertices || !vertices)) || (m->n_triangles && (!m->triangles || !triangles))) {
+        set_last_error("prgpu_copy_mesh: invalid argument");
+        return PRGPU_ERR_ARG;
+    }
+    copy_wide(vertices, m->vertices, sizeof(float) * 3 * (size_t)m->n_vertices);
+    copy_wide(triangles, m->triangles, sizeof(int32_t) * 3 * (size_t)m->n_triangles);
+    return PRGPU_OK;
+}
+
+// a reconstructed mesh copied into memory from alloc (malloc when it is null)
+static int copy_mesh_out(const prgpu_mesh& m, prgpu_mesh_alloc alloc, void* user, int32_t cloud, prgpu_mesh* out) {
+    float* vv = nullptr;
+    int32_t* ff = nullptr;
+    bool room;
+    if (alloc) {
+        room = alloc(user, cloud, m.n_vertices, m.n_triangles, &vv, &ff) == 0 && (vv || !m.n_vertices) && (ff || !m.n_triangles);
+    } else {
+        vv = (float*)malloc(sizeof(float) * 3 * (size_t)std::max<int64_t>(m.n_vertices, 1));
+        ff = (int32_t*)malloc(sizeof(int32_t) * 3 * (size_t)std::max<int64_t>(m.n_triangles, 1));
+        room = vv && ff;
+        if (!room) {
+            free(vv);
+            free(ff);
+        }
+    }
+    if (!room) {
         set_last_error("host allocation failed");
         return PRGPU_ERR_NOMEM;
     }
-    memcpy(vv, m.vertices, sizeof(float) * 3 * (size_t)m.n_vertices);
-    memcpy(ff, m.triangles, sizeof(int32_t) * 3 * (size_t)m.n_triangles);
+    prgpu_copy_mesh(&m, vv, ff);
     out->vertices = vv;
     out->triangles = ff;
     out->n_vertices = m.n_vertices;
@@ -446,6 +497,12 @@ constexpr int64_t BATCH_SHARED_POINTS = 4000000;
 
 int prgpu_reconstruct_batch(void* h, const float* xyz, const float* nrm, const int64_t* offsets,
                             const int32_t* depths, int32_t ncloud, prgpu_mesh* outs) {
+    return prgpu_reconstruct_batch_into(h, xyz, nrm, offsets, depths, ncloud, nullptr, nullptr, outs);
+}
+
+int prgpu_reconstruct_batch_into(void* h, const float* xyz, const float* nrm, const int64_t* offsets,
+                                 const int32_t* depths, int32_t ncloud, prgpu_mesh_alloc alloc, void* user,
+                                 prgpu_mesh* outs) {
     Ctx* c = as_ctx(h);
     if (!c || !xyz || !nrm || !offsets || !outs || ncloud < 0) {
         set_last_error("prgpu_reconstruct_batch: invalid argument");
@@ -483,7 +540,7 @@ int prgpu_reconstruct_batch(void* h, const float* xyz, const float* nrm, const i
         w->D = depths ? depths[k] : D0;
         prgpu_mesh m;
         int rc = prgpu_reconstruct(w, xyz + 3 * offsets[k], nrm + 3 * offsets[k], offsets[k + 1] - offsets[k], &m);
-        if (rc == PRGPU_OK) rc = copy_mesh_out(m, &outs[k]);
+        if (rc == PRGPU_OK) rc = copy_mesh_out(m, alloc, user, k, &outs[k]);
         if (rc != PRGPU_OK) fail(k, rc);
         return rc == PRGPU_OK;
     };
@@ -519,7 +576,10 @@ int prgpu_reconstruct_batch(void* h, const float* xyz, const float* nrm, const i
             if (!run(c, k)) break;
     c->D = D0;
     if (err_cloud >= 0) {
-        for (int k = 0; k < ncloud; ++k) prgpu_mesh_free(&outs[k]);
+        for (int k = 0; k < ncloud; ++k) {
+            if (!alloc) prgpu_mesh_free(&outs[k]);
+            outs[k] = prgpu_mesh{};
+        }
         set_last_error("prgpu_reconstruct_batch: cloud %d: %s", err_cloud, err_msg.c_str());
         return err_rc;
     }
