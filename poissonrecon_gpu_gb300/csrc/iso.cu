@@ -744,6 +744,13 @@ constexpr int BELOW = 5;           // depths below a node whose range of x k_x_b
 
 __device__ __forceinline__ int brick_edge(int D, int r) { return min(1 << (D - r), BR); }
 
+// 16 bytes from global to shared memory without a register in between; async_wait returns when this thread's are there
+__device__ __forceinline__ void async_copy16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Roots are in depth order and every root of depth d has the same number of bricks
 // (8^lg[d]) and super-bricks (8^slg[d]), so the root of a brick follows from the
 // per-depth counts without a search.
@@ -1827,8 +1834,8 @@ __device__ __forceinline__ void column_level(const float xs[28], const float4& b
 }
 
 // Bricks of edge 8 (96 threads, 81 columns) and 4 (a warp, 25 columns).  4 M points, maxDepth 11: 109 K
-// bricks of edge 8 in 3.8 ms (7.9 with a thread per corner and a descent per window cell), 0.4 M of edge 4
-// in 3.2.  At most 85 registers, so that 7 blocks share an SM: with 128 (5 blocks) the edge-8 bricks take
+// bricks of edge 8 in 3.5 ms (7.9 with a thread per corner and a descent per window cell; 3.8 with 16 blocks
+// per SM striding over the bricks, some of them left with one more at the end), 0.4 M of edge 4 in 3.  At most 85 registers, so that 7 blocks share an SM: with 128 (5 blocks) the edge-8 bricks take
 // 8.7 ms, set-up and window loads waiting.
 template <int E, int NT>
 __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
@@ -2023,69 +2030,116 @@ __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, Br
 // The only virtual depth is the finest, and its window, the 4x4x4 cells around the leaf, are the children
 // of the leaf's 27 neighbours, so a cell's x is two loads away without a descent.  A level costs a warp 45
 // instructions of arithmetic per brick where a lane per corner takes 81 on 27 of 32 lanes, and its set-up
-// is shared by three.  4 M points, maxDepth 11, 1.6 M such bricks: 4.1 ms (with the edge-4 bricks 7.4 ms,
-// 19.7 before); half of the issue slots idle on the gathers of x27 rows.
-constexpr int E2_WARPS = 4;
+// is shared by three.  The x27 rows and basis entries of all levels are fetched by asynchronous copies at
+// once, beside the gathers of the window, so that a warp waits for one latency instead of one per level.
+// 4 M points, maxDepth 11, 1.6 M such bricks, with the edge-4 bricks: 7.1 -> 5.9 ms (19.7 with a lane per
+// corner); without a bound on the registers (119): 0.5 ms less than at 96.
+constexpr int E2_WARPS = 2;
+struct E2Warp {                        // a warp's share of shared memory, before the levels
+    float x[3][64];                    // finest-depth window
+    int child[3][27], member[3][27];   // the leaf's neighbours: first child, leaf of the batch (-1: none)
+    int up[3][BR_LEVELS];
+    int pad[2];
+};
+constexpr int E2_ROWS = 3 * 7, E2_BASIS = 3 * 9;   // float4 per level: x27 rows (below the finest), basis entries
+static_assert(sizeof(E2Warp) % 16 == 0, "the levels follow at 16-byte alignment");
+inline size_t edge2_shared(int D) { return E2_WARPS * (sizeof(E2Warp) + 16 * (size_t)(E2_ROWS * D + E2_BASIS * (D + 1))); }
+static_assert(E2_WARPS * (sizeof(E2Warp) + 16 * (E2_ROWS * PRGPU_MAX_DEPTH + E2_BASIS * (PRGPU_MAX_DEPTH + 1))) <= 48 * 1024,
+              "dynamic shared memory without an opt-in");
 __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickIndex bix, const int* __restrict__ root_of,
                                                               LiveIndex lx, i64 first, i64 nlist,
                                                               float* __restrict__ blat,
                                                               unsigned long long* __restrict__ nforeign,
                                                               ForeignCorner* __restrict__ foreign, i64 foreign_cap) {
-    __shared__ float s_x[E2_WARPS][3][64];
-    __shared__ int s_child[E2_WARPS][3][27];
-    __shared__ int s_member[E2_WARPS][3][27];
-    __shared__ int s_up[E2_WARPS][3][BR_LEVELS];
+    extern __shared__ float4 e2_shared[];
     const EvalArgs& a = v.e;
     const int D = a.D, r = D - 1;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    char* mine = reinterpret_cast<char*>(e2_shared) +
+                 w * (sizeof(E2Warp) + 16 * (size_t)(E2_ROWS * D + E2_BASIS * (D + 1)));
+    E2Warp& sm = *reinterpret_cast<E2Warp*>(mine);
+    float4* s_row = reinterpret_cast<float4*>(mine + sizeof(E2Warp));   // [level][brick][7]
+    float4* s_bt = s_row + E2_ROWS * D;                                 // [level][brick][axis][corner]
     const int gi = min(lane / 9, 2), ci = lane - 9 * gi < 9 ? lane - 9 * gi : 8, kx = ci / 3, ky = ci % 3;
+    const int rb = min(lane / 7, 2), rq = lane % 7;    // the row entry this lane fetches (lanes below 21)
     const i64 nwarps = (i64)gridDim.x * E2_WARPS;
     for (i64 it = ((i64)blockIdx.x * E2_WARPS + w) * 3; it < nlist; it += nwarps * 3) {
         const int nbr = (int)min(nlist - it, (i64)3);
         __syncwarp();                       // the previous bricks' readers are done
-        for (int e = lane; e < nbr * 27; e += 32) {
-            const int b = e / 27, j = e % 27;
-            const VRoot R = v.roots[lx.live[first + it + b].root];
-            const int n = a.nd.neigh[(i64)j * a.nd.M + R.node];
-            s_child[w][b][j] = n == -1 ? -1 : a.nd.child0[n];
-            // batch_member's rule (R.depth >= 3: one batch per depth)
-            s_member[w][b][j] = j == 13 ? R.node : (r >= 3 && n != -1 && v.batch_root_flag[n] == R.batch) ? n : -1;
-        }
         for (int e = lane; e < nbr * BR_LEVELS; e += 32) {
             const int b = e / BR_LEVELS, l = e % BR_LEVELS;
-            if (l <= r) s_up[w][b][l] = bix.up[(i64)lx.live[first + it + b].root * BR_LEVELS + l];
-        }
-        __syncwarp();
-        for (int e = lane; e < nbr * 64; e += 32) {
-            const int b = e >> 6, cell = e & 63, bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
-            const int c0 = s_child[w][b][9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
-            s_x[w][b][cell] = c0 == -1 ? 0.f : a.x[c0 + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
+            if (l <= r) sm.up[b][l] = bix.up[(i64)lx.live[first + it + b].root * BR_LEVELS + l];
         }
         __syncwarp();
         const bool on = lane < 27 && gi < nbr;
         const int g = min(gi, nbr - 1);
-        const int li = (int)(first + it + g);
-        const i64 lat = lx.lat(li);
         int Lc[3];
-        key_coords(a.nd.key[s_up[w][g][r]], r, D, Lc);
+        key_coords(a.nd.key[sm.up[g][r]], r, D, Lc);
         const int g0[3] = {2 * Lc[0], 2 * Lc[1], 2 * Lc[2]};
         const int u[3] = {g0[0] + kx, g0[1] + ky, g0[2]};
+        int nb[3], ch[3];                   // neighbours and their first children, loads side by side
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int e = lane + 32 * m;
+            nb[m] = e < nbr * 27 ? a.nd.neigh[(i64)(e % 27) * a.nd.M + sm.up[e / 27][r]] : -1;
+        }
+        {
+            // lanes below 27: entry k = ky of axis kx of brick g
+            const int ax = kx, k = ky, gax = ax == 0 ? g0[0] : ax == 1 ? g0[1] : g0[2];
+            for (int l = 0; l <= r; ++l) {
+                const int sh = D - l, c = gax >> sh;
+                if (lane < 27)
+                    async_copy16(s_bt + l * E2_BASIS + lane, &a.lb[lattice_offset(D, l) + (i64)c * ((1 << sh) + 1) + (gax + k - (c << sh))]);
+                if (lane < 21 && rb < nbr)
+                    async_copy16(s_row + l * E2_ROWS + lane,
+                                 reinterpret_cast<const float4*>(a.x27 + (i64)sm.up[rb][l] * X27_STRIDE) + rq);
+            }
+            // the finest depth: owner cell = the one below the corner, its own on the leaf's lower face
+            if (lane < 27)
+                async_copy16(s_bt + D * E2_BASIS + lane, &a.lb[lattice_offset(D, D) + 2 * (i64)(gax + (k == 2)) + (k - (k == 2))]);
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) ch[m] = nb[m] == -1 ? -1 : a.nd.child0[nb[m]];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int e = lane + 32 * m, b = e / 27, j = e % 27;
+            if (e >= nbr * 27) break;
+            sm.child[b][j] = ch[m];
+            // batch_member's rule (r >= 3: the roots of a depth are one batch)
+            sm.member[b][j] = j == 13 ? sm.up[b][r] : (r >= 3 && nb[m] != -1 && v.batch_root_flag[nb[m]] == v.roots[lx.live[first + it + b].root].batch) ? nb[m] : -1;
+        }
+        __syncwarp();
+        {
+            float xv[6];
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                const int b = m >> 1, cell = lane + 32 * (m & 1), bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
+                const int c0 = b < nbr ? sm.child[b][9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)] : -1;
+                xv[m] = c0 == -1 ? 0.f : a.x[c0 + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
+            }
+#pragma unroll
+            for (int m = 0; m < 6; ++m) sm.x[m >> 1][lane + 32 * (m & 1)] = xv[m];
+        }
+        async_wait();
+        __syncwarp();
+        const int li = (int)(first + it + g);
+        const i64 lat = lx.lat(li);
         float val[3] = {0.f, 0.f, 0.f};
         {
-            // the finest depth: owner cell = the one below the corner, its own on the leaf's lower face
             const int sx = kx == 2, sy = ky == 2;
-            const float4 fx = lattice_at(a, D, g0[0] + sx, kx - sx), fy = lattice_at(a, D, g0[1] + sy, ky - sy);
+            const float4* bt = s_bt + D * E2_BASIS + 9 * g;
+            const float4 fx = bt[kx], fy = bt[3 + ky];
             const float x3[3] = {fx.x, fx.y, fx.z}, y3[3] = {fy.x, fy.y, fy.z};
             float p[4][9];
 #pragma unroll
             for (int z = 0; z < 4; ++z)
 #pragma unroll
                 for (int j = 0; j < 9; ++j)
-                    p[z][j] = s_x[w][g][(sx + j / 3) * 16 + (sy + j % 3) * 4 + z] * x3[j / 3] * y3[j % 3];
+                    p[z][j] = sm.x[g][(sx + j / 3) * 16 + (sy + j % 3) * 4 + z] * x3[j / 3] * y3[j % 3];
 #pragma unroll
             for (int kz = 0; kz < 3; ++kz) {
                 const int sz = kz == 2;
-                const float4 fz = lattice_at(a, D, g0[2] + sz, kz - sz);
+                const float4 fz = bt[6 + kz];
                 const float z3[3] = {fz.x, fz.y, fz.z};
 #pragma unroll
                 for (int j = 0; j < 27; ++j) val[kz] = fmaf(p[sz + j % 3][j / 3], z3[j % 3], val[kz]);
@@ -2093,23 +2147,15 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
         }
 #pragma unroll 1
         for (int l = r; l >= 0; --l) {
-            const float4* row = reinterpret_cast<const float4*>(a.x27 + (i64)s_up[w][g][l] * X27_STRIDE);
+            const float4* row = s_row + l * E2_ROWS + 7 * g;
             float xs[28];
 #pragma unroll
             for (int q = 0; q < 7; ++q) {
                 const float4 f = row[q];
                 xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
             }
-            const int sh = D - l;
-            int c[3], k[3];
-#pragma unroll
-            for (int ax = 0; ax < 3; ++ax) {
-                c[ax] = Lc[ax] >> (r - l);
-                k[ax] = u[ax] - (c[ax] << sh);
-            }
-            const float4* bz = a.lb + lattice_offset(D, l) + (i64)c[2] * ((1 << sh) + 1) + k[2];
-            const float4 b3[3] = {bz[0], bz[1], bz[2]};
-            column_level<3>(xs, lattice_at(a, l, c[0], k[0]), lattice_at(a, l, c[1], k[1]), b3, val);
+            const float4* bt = s_bt + l * E2_BASIS + 9 * g;
+            column_level<3>(xs, bt[kx], bt[3 + ky], bt + 6, val);
         }
         unsigned fmask = 0;
 #pragma unroll
@@ -2118,8 +2164,8 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
             int oc[3] = {0, 0, 0};
             int own = -1;
             const bool low = on && (kx == 0 || ky == 0 || kz == 0);
-            if (low) own = corner_owner_cell(D, r, Lc, qc, s_member[w][g], oc);
-            const bool isf = low && own != s_up[w][g][r];
+            if (low) own = corner_owner_cell(D, r, Lc, qc, sm.member[g], oc);
+            const bool isf = low && own != sm.up[g][r];
             const u64 src = isf ? foreign_src(D, r, 2, bix.dl, root_of[own], oc, qc) : 0ull;
             push_foreign(isf, li, ci * 3 + kz, src, nforeign, foreign, foreign_cap);
             if (isf) fmask |= 1u << kz;
@@ -2738,19 +2784,19 @@ void stage_mesh(Ctx& c) {
             // compulsory: the corner values written (bricks of edge 8: 729 each)
             const int ke = c.kbegin("brick_eval", (double)lx.n8 * BR_CORNERS * 4);
             if (lx.n8 > 0) {
-                k_brick_eval<8, 96><<<grid_for(lx.n8, 1, (i64)c.sms * 16), 96, 0, s>>>(
+                k_brick_eval<8, 96><<<grid_for(lx.n8, 1, 1ll << 30), 96, 0, s>>>(
                     va, bix, root_of, lx, 0, lx.n8, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
             c.kend(ke);
             const int ks = c.kbegin("brick_eval_small", (double)(125 * lx.n4 + 27 * lx.n2) * 4);
             if (lx.n4 > 0) {
-                k_brick_eval<4, 32><<<grid_for(lx.n4, 1, (i64)c.sms * 32), 32, 0, s>>>(
+                k_brick_eval<4, 32><<<grid_for(lx.n4, 1, 1ll << 30), 32, 0, s>>>(
                     va, bix, root_of, lx, lx.n8, lx.n4, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
             if (lx.n2 > 0) {
-                k_edge2_eval<<<grid_for(lx.n2, 3 * E2_WARPS, (i64)c.sms * 64), 32 * E2_WARPS, 0, s>>>(
+                k_edge2_eval<<<grid_for(lx.n2, 3 * E2_WARPS, 1ll << 30), 32 * E2_WARPS, edge2_shared(D), s>>>(
                     va, bix, root_of, lx, lx.n8 + lx.n4, lx.n2, lat_brick, dcount, foreign, fcap);
                 CK_LAUNCH();
             }
