@@ -2262,7 +2262,6 @@ struct EmitArgs {
     int weld;           // 1: keys without the batch (vertices shared across batches)
     i64 tri_offset;     // first global triangle of this emission
     u64* keys;          // 3 per triangle
-    uint32_t* slot;     // payload: 3*t+q
     float* pos;         // 3 floats per emission
 };
 
@@ -2319,7 +2318,6 @@ __device__ __forceinline__ void emit_corner(const EmitArgs& em, const int c[3], 
     float p[3];
     crossing(lp, o, o == 0 && rev(a0, a1, b0, b1), value(ev0), value(ev1), em.D, p);
     em.keys[slot] = edge_key(lp, o, em.D, batch, em.local_bits);
-    em.slot[slot] = (uint32_t)slot;
     em.pos[3 * slot] = p[0];
     em.pos[3 * slot + 1] = p[1];
     em.pos[3 * slot + 2] = p[2];
@@ -2871,9 +2869,8 @@ void stage_mesh(Ctx& c) {
         em.weld = c.params.weld ? 1 : 0;
         em.tri_offset = 0;
         em.keys = dalloc<u64>(nem, s);
-        em.slot = dalloc<uint32_t>(nem, s);
         em.pos = dalloc<float>(3 * nem, s);
-        const int kem = c.kbegin("emit", (double)nem * (8 + 4 + 12));
+        const int kem = c.kbegin("emit", (double)nem * (8 + 12));
         if (ntri_real > 0) {
             k_emit_real<<<(unsigned)rtiles, CELL_BLOCK, 0, s>>>(nd, em, lo, nD, cat, rfirst, cell_v);
             CK_LAUNCH();
@@ -2886,9 +2883,9 @@ void stage_mesh(Ctx& c) {
         }
         c.kend(kem);
         u64* ktmp = dalloc<u64>(nem, s);
-        uint32_t* stmp = dalloc<uint32_t>(nem, s);
+        uint32_t *slot = dalloc<uint32_t>(nem, s), *stmp = dalloc<uint32_t>(nem, s);
         const int ks = c.kbegin("edge_sort", (double)nem * 12 * 2);
-        radix_sort_pairs(em.keys, em.slot, ktmp, stmp, nem, local_bits + batch_bits, s);
+        radix_sort_pairs(em.keys, slot, ktmp, stmp, nem, local_bits + batch_bits, s);
         c.kend(ks);
         dfree(ktmp, s);
         dfree(stmp, s);
@@ -2901,7 +2898,7 @@ void stage_mesh(Ctx& c) {
         const i64 nvert = read_scalar(hp + nem, s);
         int32_t* tri_vid = dalloc<int32_t>(nem, s);
         float* vpos = dalloc<float>(3 * std::max<i64>(nvert, 1), s);
-        k_vertex_ids<<<grid_for(nem, 256), 256, 0, s>>>(em.keys, em.slot, nem, hp, em.pos, c.scale,
+        k_vertex_ids<<<grid_for(nem, 256), 256, 0, s>>>(em.keys, slot, nem, hp, em.pos, c.scale,
                                                         make_float3(c.center[0], c.center[1], c.center[2]),
                                                         tri_vid, vpos);
         CK_LAUNCH();
@@ -2914,7 +2911,7 @@ void stage_mesh(Ctx& c) {
         c.kend(kd);
         CK(cudaStreamSynchronize(s));
         dfree(hf, s); dfree(hp, s); dfree(tri_vid, s); dfree(vpos, s);
-        dfree(em.keys, s); dfree(em.slot, s); dfree(em.pos, s);
+        dfree(em.keys, s); dfree(slot, s); dfree(em.pos, s);
     }
     dfree(rtri, s);
     dfree(rfirst, s);

@@ -89,8 +89,7 @@ __host__ __device__ inline Cube cube_of(const unsigned* mm) {
 // ----------------- normalisation + Morton key (main.cu:132-173,555-569) ------
 __global__ void k_normalise_encode(const float* __restrict__ in_xyz, const float* __restrict__ in_nrm, i64 n,
                                    const unsigned* __restrict__ mm, float nscale, int D,
-                                   float* __restrict__ p_out, float* __restrict__ n_out, u64* __restrict__ keys,
-                                   uint32_t* __restrict__ idx) {
+                                   float* __restrict__ p_out, float* __restrict__ n_out, u64* __restrict__ keys) {
     const Cube cube = cube_of(mm);
     const float cx = cube.corner[0], cy = cube.corner[1], cz = cube.corner[2], scale = cube.scale;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -115,7 +114,6 @@ __global__ void k_normalise_encode(const float* __restrict__ in_xyz, const float
             w *= 0.5f;
         }
         keys[i] = key;
-        idx[i] = (uint32_t)i;
     }
 }
 
@@ -342,8 +340,7 @@ void stage_octree(Ctx& c) {
     u64* ktmp = dalloc<u64>(N, s);
     uint32_t* idx = dalloc<uint32_t>(N, s);
     uint32_t* itmp = dalloc<uint32_t>(N, s);
-    k_normalise_encode<<<grid_for(N, 256), 256, 0, s>>>(c.in_xyz, c.in_nrm, N, mm, (float)(2 << D), D, ptmp, ntmp, keys,
-                                                         idx);
+    k_normalise_encode<<<grid_for(N, 256), 256, 0, s>>>(c.in_xyz, c.in_nrm, N, mm, (float)(2 << D), D, ptmp, ntmp, keys);
     CK_LAUNCH();
     const int ks = c.kbegin("point_sort", (double)N * 12 * 2);
     radix_sort_pairs(keys, idx, ktmp, itmp, N, 3 * D, s);

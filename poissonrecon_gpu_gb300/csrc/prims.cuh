@@ -1,5 +1,5 @@
 // Device primitives: exclusive scan, stable LSD radix sort of (u64 key, u32
-// value) pairs with a shared-memory digit-binned scatter, and compaction.
+// index) pairs, and compaction.
 // All work on the caller's stream; temporary memory comes from the stream's
 // memory pool (cudaMallocAsync).
 #pragma once
@@ -159,98 +159,203 @@ void exclusive_scan(const TI* in, TO* out, i64 n, TO* total_dev, cudaStream_t s)
 }
 
 // ----------------------------- radix sort -----------------------------------
+// Stable LSD sort of (key, index) pairs, 8 bits a pass, one launch per pass behind one that counts the digits
+// of all passes.  A tile ranks its 4,096 keys warp by warp (a warp's 512 consecutive keys against counters of
+// its own, without a barrier), publishes its count per digit, adds the counts of the tiles before it
+// (look-back) and writes its elements from shared memory in digit order, so that each digit's run is written
+// at once.  24 bytes move per element and pass, where a count, a scan and a scatter moved 32 and wrote
+// every element by itself.  Tiles are numbered as their blocks start, so a tile waits for running ones
+// only; a wait that runs out (RS_POLLS) ends in counting the missing tiles' keys instead.
+// Bound by the latency of a tile's phases (load, rank, look back, write) at two blocks per SM: three (80
+// registers, spilling) and tiles of 2,048 are slower, 0.47 and 0.48 ms on the second line.  Against three
+// launches a pass: 15 K keys of 20 bits 0.099 -> 0.040 ms, 9.2 M of 36 bits (corners of the 1M torus)
+// 0.585 -> 0.42, 80 M of 39 bits 4.5 -> 3.3.
 constexpr int RS_BLOCK = 256;
+constexpr int RS_WARPS = RS_BLOCK / 32;
 constexpr int RS_ITEMS = 16;
 constexpr int RS_TILE = RS_BLOCK * RS_ITEMS;
 constexpr int RS_BINS = 256;
+static_assert(RS_BLOCK == RS_BINS, "a thread per digit value");
+constexpr int RS_PASSES = 8;
+constexpr int RS_POLLS = 1 << 20;
+constexpr int RS_LOOK = 16;              // tiles a look-back step reads at once
+constexpr size_t RS_SHARED = RS_TILE * (sizeof(u64) + sizeof(uint32_t));
 
-static __global__ void k_rs_hist(const u64* __restrict__ keys, i64 n, int shift, u64 mask, unsigned* __restrict__ hist,
-                          int nblocks) {
-    __shared__ unsigned h[RS_BINS];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    i64 base = (i64)blockIdx.x * RS_TILE;
-#pragma unroll 4
-    for (int i = 0; i < RS_ITEMS; ++i) {
-        i64 e = base + (i64)i * RS_BLOCK + threadIdx.x;
-        if (e < n) atomicAdd(&h[(unsigned)((keys[e] >> shift) & mask)], 1u);
-    }
-    __syncthreads();
-    hist[(i64)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
-}
+struct RsCounts {
+    unsigned hist[RS_PASSES][RS_BINS];   // of the digits, all keys
+    unsigned ticket[RS_PASSES];          // tiles started
+};
 
-// Stable scatter: elements of a tile are ranked in index order, round by round.
-static __global__ void k_rs_scatter(const u64* __restrict__ kin, const uint32_t* __restrict__ vin, i64 n, int shift, u64 mask,
-                             const unsigned* __restrict__ offs, int nblocks, u64* __restrict__ kout,
-                             uint32_t* __restrict__ vout) {
-    __shared__ unsigned wcnt[RS_BLOCK / 32][RS_BINS];
-    __shared__ unsigned run[RS_BINS];
-    __shared__ unsigned goff[RS_BINS];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    run[t] = 0;
-    goff[t] = offs[(i64)t * nblocks + blockIdx.x];
-    const unsigned lt = (1u << lane) - 1u;
-    i64 base = (i64)blockIdx.x * RS_TILE;
-    for (int i = 0; i < RS_ITEMS; ++i) {
+static __global__ void __launch_bounds__(RS_BLOCK) k_rs_hist(const u64* __restrict__ keys, i64 n, int nbits,
+                                                             RsCounts* __restrict__ counts) {
+    __shared__ unsigned h[RS_PASSES][RS_BINS];
 #pragma unroll
-        for (int w = 0; w < RS_BLOCK / 32; ++w) wcnt[w][t] = 0;
-        __syncthreads();
-        i64 e = base + (i64)i * RS_BLOCK + t;
-        bool valid = e < n;
-        u64 k = valid ? kin[e] : 0;
-        uint32_t v = valid ? vin[e] : 0;
-        unsigned dig = valid ? (unsigned)((k >> shift) & mask) : 0xffffffffu;
-        unsigned peers = __match_any_sync(0xffffffffu, dig);
-        unsigned lrank = __popc(peers & lt);
-        if (valid && lrank == 0) wcnt[warp][dig] = __popc(peers);
-        __syncthreads();
-        {
-            unsigned r = run[t];
+    for (int p = 0; p < RS_PASSES; ++p) h[p][threadIdx.x] = 0;
+    __syncthreads();
+    const i64 stride = (i64)gridDim.x * RS_BLOCK * 4;
+    for (i64 e0 = (i64)blockIdx.x * RS_BLOCK * 4; e0 < n; e0 += stride) {
+        u64 k[4];
 #pragma unroll
-            for (int w = 0; w < RS_BLOCK / 32; ++w) {
-                unsigned c = wcnt[w][t];
-                wcnt[w][t] = r;
-                r += c;
+        for (int i = 0; i < 4; ++i) {
+            const i64 e = e0 + i * RS_BLOCK + threadIdx.x;
+            k[i] = e < n ? keys[e] : ~0ull;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool valid = e0 + i * RS_BLOCK + threadIdx.x < n;
+            for (int p = 0; 8 * p < nbits; ++p) {
+                const unsigned mask = nbits - 8 * p < 8 ? (1u << (nbits - 8 * p)) - 1u : 255u;
+                const unsigned dig = valid ? (unsigned)(k[i] >> (8 * p)) & mask : RS_BINS;
+                // the upper digits of neighbouring keys agree: one addition for the warp
+                if (__all_sync(0xffffffffu, dig == __shfl_sync(0xffffffffu, dig, 0))) {
+                    if (valid && (threadIdx.x & 31) == 0) atomicAdd(&h[p][dig], 32u);
+                } else if (valid) {
+                    atomicAdd(&h[p][dig], 1u);
+                }
             }
-            run[t] = r;
         }
-        __syncthreads();
-        if (valid) {
-            unsigned pos = goff[dig] + wcnt[warp][dig] + lrank;
-            kout[pos] = k;
-            vout[pos] = v;
+    }
+    __syncthreads();
+    for (int p = 0; 8 * p < nbits; ++p)
+        if (h[p][threadIdx.x]) atomicAdd(&counts->hist[p][threadIdx.x], h[p][threadIdx.x]);
+}
+
+// Elements of digit t in the tiles before 'tile'.  A tile's word is its tag << 32 | count: tag 2 pass + 1 with the
+// tile's own count, 2 pass + 2 with the count of all tiles up to it; words of earlier passes have lower tags.
+__device__ __forceinline__ unsigned rs_look_back(const u64* status, unsigned tag, int tile, const u64* __restrict__ kin,
+                                                 int shift, unsigned mask) {
+    const unsigned t = threadIdx.x;
+    unsigned before = 0;
+    int at = tile - 1, polls = 0;
+    while (at >= 0) {
+        u64 w[RS_LOOK];
+#pragma unroll
+        for (int j = 0; j < RS_LOOK; ++j)
+            w[j] = at - j >= 0 ? *(volatile const u64*)&status[(i64)(at - j) * RS_BINS + t] : (u64)(tag + 1) << 32;
+        int got = 0;
+        bool open = true, done = false;
+#pragma unroll
+        for (int j = 0; j < RS_LOOK; ++j) {
+            const unsigned wt = (unsigned)(w[j] >> 32);
+            open = open && wt >= tag;
+            if (open) {
+                before += (unsigned)w[j];
+                ++got;
+                if (wt > tag) {
+                    done = true;
+                    open = false;
+                }
+            }
         }
-        __syncthreads();
+        if (done) return before;
+        at -= got;
+        if (got == 0 && ++polls >= RS_POLLS) {
+            for (i64 e = 0; e < (i64)(at + 1) * RS_TILE; ++e) before += ((unsigned)(kin[e] >> shift) & mask) == t;
+            return before;
+        }
+    }
+    return before;
+}
+
+// vin null: the index of each element (the first pass)
+static __global__ void __launch_bounds__(RS_BLOCK, 2) k_rs_pass(const u64* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                                                i64 n, int pass, unsigned mask,
+                                                                RsCounts* __restrict__ counts, u64* status,
+                                                                u64* __restrict__ kout, uint32_t* __restrict__ vout) {
+    extern __shared__ u64 rs_shared[];
+    u64* skey = rs_shared;
+    uint32_t* sval = reinterpret_cast<uint32_t*>(rs_shared + RS_TILE);
+    __shared__ unsigned wcnt[RS_WARPS][RS_BINS];
+    __shared__ unsigned lbase[RS_BINS], gbase[RS_BINS], sw[32];
+    __shared__ int s_tile;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, shift = 8 * pass;
+    const unsigned lt = (1u << lane) - 1u, tag = 2u * pass + 1u;
+    if (t == 0) s_tile = (int)atomicAdd(&counts->ticket[pass], 1u);
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = 0;
+    __syncthreads();
+    const int tile = s_tile;
+    const i64 first = (i64)tile * RS_TILE, mine = first + warp * (32 * RS_ITEMS) + lane;
+    u64 key[RS_ITEMS];
+    uint32_t val[RS_ITEMS];
+    unsigned short rank[RS_ITEMS];
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; ++i) {
+        const i64 e = mine + 32 * i;
+        key[i] = e < n ? kin[e] : 0;
+        val[i] = e < n ? (vin ? vin[e] : (uint32_t)e) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; ++i) {
+        const bool valid = mine + 32 * i < n;
+        const unsigned dig = (unsigned)(key[i] >> shift) & mask;
+        const unsigned peers = __match_any_sync(0xffffffffu, valid ? dig : RS_BINS);
+        const unsigned r = wcnt[warp][dig];
+        __syncwarp();
+        if (valid && (peers & lt) == 0) wcnt[warp][dig] = r + __popc(peers);
+        __syncwarp();
+        rank[i] = (unsigned short)(r + __popc(peers & lt));
+    }
+    __syncthreads();
+    unsigned total = 0;                  // of digit t in this tile
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; ++w) {
+        const unsigned c = wcnt[w][t];
+        wcnt[w][t] = total;
+        total += c;
+    }
+    u64* mineword = status + (i64)tile * RS_BINS + t;
+    if (tile > 0) *(volatile u64*)mineword = ((u64)tag << 32) | total;
+    unsigned all;
+    const unsigned local = block_exclusive_sum<unsigned>(total, sw, &all);
+    lbase[t] = local;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; ++i) {
+        if (mine + 32 * i < n) {
+            const unsigned dig = (unsigned)(key[i] >> shift) & mask;
+            const unsigned p = lbase[dig] + wcnt[warp][dig] + rank[i];
+            skey[p] = key[i];
+            sval[p] = val[i];
+        }
+    }
+    const unsigned start = block_exclusive_sum<unsigned>(counts->hist[pass][t], sw, &all);
+    const unsigned before = rs_look_back(status, tag, tile, kin, shift, mask);
+    *(volatile u64*)mineword = ((u64)(tag + 1) << 32) | (before + total);
+    gbase[t] = start + before - local;   // modulo 2^32
+    __syncthreads();
+    const int m = (int)min(n - first, (i64)RS_TILE);
+    for (int q = t; q < m; q += RS_BLOCK) {
+        const u64 k = skey[q];
+        const unsigned pos = gbase[(unsigned)(k >> shift) & mask] + q;
+        kout[pos] = k;
+        vout[pos] = sval[q];
     }
 }
 
-// Sorts n (key,value) pairs by key bits [0, nbits); stable.  Result ends in
-// (keys, vals); tmp buffers are supplied by the caller.
-inline void radix_sort_pairs(u64* keys, uint32_t* vals, u64* ktmp, uint32_t* vtmp, i64 n, int nbits,
-                             cudaStream_t s) {
-    if (n <= 1 || nbits <= 0) return;
-    const int nb = (int)((n + RS_TILE - 1) / RS_TILE);
-    unsigned* hist = dalloc<unsigned>((i64)RS_BINS * nb, s);
-    u64 *ka = keys, *kb = ktmp;
-    uint32_t *va = vals, *vb = vtmp;
-    int passes = 0;
-    for (int shift = 0; shift < nbits; shift += 8) {
-        int bits = nbits - shift < 8 ? nbits - shift : 8;
-        u64 mask = (1ull << bits) - 1;
-        k_rs_hist<<<nb, RS_BLOCK, 0, s>>>(ka, n, shift, mask, hist, nb);
+// Sorts n keys (below 2^31) by bits [0, nbits) and gives the index each came from, stable.  The result ends in
+// (keys, vals); the four buffers may change roles.
+inline void radix_sort_pairs(u64*& keys, uint32_t*& vals, u64*& ktmp, uint32_t*& vtmp, i64 n, int nbits, cudaStream_t s) {
+    if (n <= 0) return;
+    nbits = std::max(nbits, 1);
+    const i64 nb = (n + RS_TILE - 1) / RS_TILE;
+    static_assert(sizeof(RsCounts) % sizeof(u64) == 0, "the tiles' words follow the counts");
+    const i64 head = sizeof(RsCounts) / sizeof(u64);
+    u64* work = dalloc<u64>(head + nb * RS_BINS, s);
+    RsCounts* counts = reinterpret_cast<RsCounts*>(work);
+    CK(cudaMemsetAsync(work, 0, (size_t)(head + nb * RS_BINS) * sizeof(u64), s));
+    k_rs_hist<<<grid_for(n, RS_BLOCK * 8, 152 * 8), RS_BLOCK, 0, s>>>(keys, n, nbits, counts);
+    CK_LAUNCH();
+    CK(cudaFuncSetAttribute(k_rs_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SHARED));
+    for (int pass = 0; 8 * pass < nbits; ++pass) {
+        const unsigned mask = nbits - 8 * pass < 8 ? (1u << (nbits - 8 * pass)) - 1u : 255u;
+        k_rs_pass<<<(unsigned)nb, RS_BLOCK, RS_SHARED, s>>>(keys, pass ? vals : nullptr, n, pass, mask, counts, work + head,
+                                                            ktmp, vtmp);
         CK_LAUNCH();
-        exclusive_scan<unsigned, unsigned>(hist, hist, (i64)RS_BINS * nb, (unsigned*)nullptr, s);
-        k_rs_scatter<<<nb, RS_BLOCK, 0, s>>>(ka, va, n, shift, mask, hist, nb, kb, vb);
-        CK_LAUNCH();
-        u64* kt = ka; ka = kb; kb = kt;
-        uint32_t* vt = va; va = vb; vb = vt;
-        ++passes;
+        std::swap(keys, ktmp);
+        std::swap(vals, vtmp);
     }
-    if (passes & 1) {
-        CK(cudaMemcpyAsync(keys, ka, (size_t)n * sizeof(u64), cudaMemcpyDeviceToDevice, s));
-        CK(cudaMemcpyAsync(vals, va, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    }
-    dfree(hist, s);
+    dfree(work, s);
 }
 
 // ---------------------------- small helpers ---------------------------------
