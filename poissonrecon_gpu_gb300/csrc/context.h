@@ -69,6 +69,10 @@ struct PinnedBuf {
     T& operator[](i64 k) { return ptr[k]; }
 };
 
+// The sibling-group table row by row: a group's 27 first-child indices (and a pad), so that a
+// warp's consecutive groups are one contiguous run of the table.
+constexpr int GN_ROW = 28;
+
 struct Ctx {
     prgpu_params params;
     std::vector<Ctx*> workers;          // contexts of prgpu_reconstruct_batch's host threads

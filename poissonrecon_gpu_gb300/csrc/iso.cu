@@ -339,39 +339,7 @@ __device__ float owner_corner_value(const EvalArgs& a, i64 o, int kind, float is
     return val - iso;
 }
 
-// finest-depth corners: each corner evaluated by its owner.  A node owns a
-// corner when no other existing node of the 8 around it has a smaller key.
-// Pass 1 (one thread per node): the mask of owned corners and their count.
-__global__ void k_finest_owned(NodeArrays nd, i64 lo, i64 hi, unsigned char* __restrict__ owned_mask,
-                               int* __restrict__ owned_count) {
-    const i64 M = nd.M;
-    for (i64 i = lo + (i64)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (i64)gridDim.x * blockDim.x) {
-        const u64 ki = nd.key[i];
-        unsigned smaller = 0;   // bit j: neighbour j exists and has a smaller key
-#pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            if (j == 13) continue;
-            const int nb = nd.neigh[(i64)j * M + i];
-            if (nb != -1 && nd.key[nb] < ki) smaller |= 1u << j;
-        }
-        unsigned owned = 0;
-#pragma unroll
-        for (int kind = 0; kind < 8; ++kind) {
-            const int sx = kind & 1, sy = (kind >> 1) & 1, sz = kind >> 2;
-            bool own = true;
-#pragma unroll
-            for (int e = 1; e < 8; ++e) {
-                const int j = 9 * (sx - (e & 1) + 1) + 3 * (sy - ((e >> 1) & 1) + 1) + (sz - (e >> 2) + 1);
-                if ((smaller >> j) & 1) own = false;
-            }
-            if (own) owned |= 1u << kind;
-        }
-        owned_mask[i - lo] = (unsigned char)owned;
-        owned_count[i - lo] = __popc(owned);
-    }
-}
-
-// the owned corners as a list: (finest slot << 3) | corner
+// the owned corners as a list: (node << 3) | corner
 __global__ void k_finest_list(const unsigned char* __restrict__ owned_mask, const int* __restrict__ first, i64 nD,
                               int* __restrict__ list) {
     for (i64 l = (i64)blockIdx.x * blockDim.x + threadIdx.x; l < nD; l += (i64)gridDim.x * blockDim.x) {
@@ -395,25 +363,6 @@ __device__ __forceinline__ void corner_sharers(const NodeArrays& nd, i64 i, int 
         const int j = 9 * (sx - (e & 1) + 1) + 3 * (sy - ((e >> 1) & 1) + 1) + (sz - (e >> 2) + 1);
         const int nb = nd.neigh[(i64)j * nd.M + i];
         if (nb != -1) f(nb, e);
-    }
-}
-
-// pass 2 (one thread per owned corner): walk_up_u from the owner at the corner,
-// the value of owner_corner_value (no descent at the finest depth), written to every cell that has the
-// corner.  (Each cell looking for the owner of each of its 8 corners reads 64 neighbours and keys.)
-__global__ void __launch_bounds__(128, 12) k_finest_corner_values(EvalArgs a, i64 lo, const int* __restrict__ list,
-                                                                 i64 ncorner, float iso, float* __restrict__ cell_v) {
-    const int D = a.D;
-    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < ncorner; q += (i64)gridDim.x * blockDim.x) {
-        const int lk = list[q];
-        const i64 l = lk >> 3;
-        const int kind = lk & 7;
-        const i64 i = lo + l;
-        int xyz[3];
-        key_coords(a.nd.key[i], D, D, xyz);
-        const int u[3] = {xyz[0] + (kind & 1), xyz[1] + ((kind >> 1) & 1), xyz[2] + (kind >> 2)};
-        const float val = walk_up_u(a, i, u, 0.f) - iso;
-        corner_sharers(a.nd, i, kind, [&](int nb, int e) { cell_v[8 * ((i64)nb - lo) + e] = val; });
     }
 }
 
@@ -2179,6 +2128,162 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
     }
 }
 
+// Corners of the finest cells, by sibling groups, four to a warp.  A group's 2x2x2 cells have 3x3x3 corners.
+// The cells around them are the 4x4x4 block of the children of the parent's 27 neighbours (the group table:
+// sibling groups are whole), so which exist and which of them precede the group in key order are 27 bits, and
+// a corner is the group's own when none of its 8 cells that exists precedes the group; its owner is then the
+// lowest of the group's cells at it.  The window, the ancestors' x27 rows and the walk are those of the
+// edge-2 bricks above: a column of up to three corners along z per lane, here only the columns that own any (a surface fills about
+// half of the 36), and each value goes to the cells of the block that share the corner, without a look at
+// their neighbour tables.  The values and their order of summation are owner_corner_value's.
+// 1M torus 0.90 -> 0.54 ms, 4M displaced sphere 3.9 -> 2.3, where a pass over the nodes' neighbours and keys
+// found the owners and a thread per owned corner walked up alone.  Two thirds of it is arithmetic; fetching
+// every group's rows, shared or not, cost 0.16 ms on the torus, and the basis entries a level ahead gain nothing.
+constexpr int FC_GROUPS = 4, FC_WARPS = 2;
+struct FcWarp {
+    unsigned long long before[FC_GROUPS];       // cells of the block that exist and precede the group, a bit each
+    float x[FC_GROUPS][65];                     // windows; a warp reads 0, 4, 16 and 20 on of each, in banks of their own
+    int gn[FC_GROUPS * GN_ROW];
+    int up[FC_GROUPS][BR_LEVELS];               // the parent and its ancestors, by depth
+    int cell[FC_GROUPS][3];                     // coordinates of the group's first cell
+    unsigned char row[FC_GROUPS][BR_LEVELS];    // the group whose copy of the ancestor's row serves this one
+    unsigned short col[40];                     // group, column and owned corners of the columns that own any
+};
+constexpr int FC_ROWS = FC_GROUPS * 7;          // float4 per level
+static_assert(sizeof(FcWarp) % 16 == 0, "the rows follow at 16-byte alignment");
+static_assert(FC_WARPS * (sizeof(FcWarp) + 16 * FC_ROWS * PRGPU_MAX_DEPTH) <= 48 * 1024,
+              "dynamic shared memory without an opt-in");
+inline size_t finest_shared(int D) { return FC_WARPS * (sizeof(FcWarp) + 16 * (size_t)FC_ROWS * D); }
+__global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, const int* __restrict__ gn_rows,
+                                                                  i64 gfirst, i64 ng, i64 lo, float iso, float* __restrict__ cell_v) {
+    extern __shared__ float4 fc_shared[];
+    const int D = a.D, r = D - 1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    char* mine = reinterpret_cast<char*>(fc_shared) + w * (sizeof(FcWarp) + 16 * (size_t)FC_ROWS * D);
+    FcWarp& sm = *reinterpret_cast<FcWarp*>(mine);
+    float4* s_row = reinterpret_cast<float4*>(mine + sizeof(FcWarp));   // [level][group][7]
+    const i64 g1 = ((i64)blockIdx.x * FC_WARPS + w) * FC_GROUPS;
+    if (g1 >= ng) return;
+    const int nbr = (int)min(ng - g1, (i64)FC_GROUPS);
+#pragma unroll
+    for (int m = 0; m < (FC_GROUPS * GN_ROW + 31) / 32; ++m) {
+        const int e = lane + 32 * m;
+        if (e < FC_GROUPS * GN_ROW) sm.gn[e] = e < nbr * GN_ROW ? gn_rows[(gfirst + g1) * GN_ROW + e] : -1;
+    }
+    if (lane < nbr) {
+        int n = (int)(lo + 8 * (g1 + lane));
+        for (int l = r; l >= 0; --l) {
+            n = a.nd.parent[n];
+            sm.up[lane][l] = n;
+        }
+        int c[3];
+        key_coords(a.nd.key[lo + 8 * (g1 + lane)], D, D, c);
+        for (int ax = 0; ax < 3; ++ax) sm.cell[lane][ax] = c[ax];
+    }
+    __syncwarp();
+    {
+        // neighbouring groups share their upper ancestors: a row is fetched by the first group that has it
+        const int b = lane / 7, q = lane % 7;
+        if (b < nbr)
+            for (int l = 0; l <= r; ++l) {
+                const int n = sm.up[b][l];
+                int first = b;
+                while (first > 0 && sm.up[first - 1][l] == n) --first;
+                if (first == b)
+                    async_copy16(s_row + l * FC_ROWS + lane, reinterpret_cast<const float4*>(a.x27 + (i64)n * X27_STRIDE) + q);
+                if (q == 0) sm.row[b][l] = (unsigned char)first;
+            }
+    }
+    {
+        float xv[2 * FC_GROUPS];
+#pragma unroll
+        for (int m = 0; m < 2 * FC_GROUPS; ++m) {
+            const int g = m >> 1, cell = lane + 32 * (m & 1), bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
+            const int cn = sm.gn[g * GN_ROW + 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
+            xv[m] = cn == -1 ? 0.f : a.x[cn + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
+            const unsigned b = __ballot_sync(0xffffffffu, cn != -1 && cn < sm.gn[g * GN_ROW + 13]);
+            if (lane == 0) reinterpret_cast<unsigned*>(sm.before)[m] = b;
+        }
+#pragma unroll
+        for (int m = 0; m < 2 * FC_GROUPS; ++m) sm.x[m >> 1][lane + 32 * (m & 1)] = xv[m];
+    }
+    __syncwarp();
+    int ncol = 0;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const int e = lane + 32 * m, g = e / 9, kx = e % 9 / 3, ky = e % 3;
+        int bits = 0;
+        if (e < 9 * nbr)
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz)   // the 2x2x2 cells at the corner
+                if (!(sm.before[g] & (0x330033ull << (16 * kx + 4 * ky + kz)))) bits |= 1 << kz;
+        const unsigned some = __ballot_sync(0xffffffffu, bits != 0);
+        if (bits) sm.col[ncol + __popc(some & ((1u << lane) - 1u))] = (unsigned short)(e << 3 | bits);
+        ncol += __popc(some);
+    }
+    async_wait();
+    __syncwarp();
+    for (int c0 = 0; c0 < ncol; c0 += 32) {
+        const int entry = sm.col[min(c0 + lane, ncol - 1)];
+        const int bits = c0 + lane < ncol ? entry & 7 : 0, e = entry >> 3, g = e / 9, kx = e % 9 / 3, ky = e % 3;
+        const int g0[3] = {sm.cell[g][0], sm.cell[g][1], sm.cell[g][2]};
+        float val[3] = {0.f, 0.f, 0.f};
+        {
+            // the finest depth: owner cell = the one below the corner, its own on the group's lower face
+            const int sx = kx == 2, sy = ky == 2;
+            const float4 fx = lattice_at(a, D, g0[0] + sx, kx - sx), fy = lattice_at(a, D, g0[1] + sy, ky - sy);
+            const float x3[3] = {fx.x, fx.y, fx.z}, y3[3] = {fy.x, fy.y, fy.z};
+            float p[4][9];
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+#pragma unroll
+                for (int j = 0; j < 9; ++j)
+                    p[z][j] = sm.x[g][(sx + j / 3) * 16 + (sy + j % 3) * 4 + z] * x3[j / 3] * y3[j % 3];
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz) {
+                const int sz = kz == 2;
+                const float4 fz = lattice_at(a, D, g0[2] + sz, kz - sz);
+                const float z3[3] = {fz.x, fz.y, fz.z};
+#pragma unroll
+                for (int j = 0; j < 27; ++j) val[kz] = fmaf(p[sz + j % 3][j / 3], z3[j % 3], val[kz]);
+            }
+        }
+#pragma unroll 1
+        for (int l = r; l >= 0; --l) {
+            const int sh = D - l;
+            int c[3], k[3];
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                c[ax] = g0[ax] >> sh;
+                k[ax] = g0[ax] - (c[ax] << sh);
+            }
+            const float4* bz = &a.lb[lattice_offset(D, l) + (i64)c[2] * ((1 << sh) + 1) + k[2]];
+            const float4 b3[3] = {bz[0], bz[1], bz[2]};
+            const float4* row = s_row + l * FC_ROWS + 7 * sm.row[g][l];
+            float xs[28];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const float4 f = row[q];
+                xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
+            }
+            column_level<3>(xs, lattice_at(a, l, c[0], k[0] + kx), lattice_at(a, l, c[1], k[1] + ky), b3, val);
+        }
+#pragma unroll
+        for (int kz = 0; kz < 3; ++kz) {
+            if (!((bits >> kz) & 1)) continue;
+            const float v = val[kz] - iso;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {       // the cells at the corner, in block coordinates
+                const int bx = kx + (q & 1), by = ky + ((q >> 1) & 1), bz = kz + (q >> 2);
+                const int cn = sm.gn[g * GN_ROW + 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
+                if (cn == -1) continue;
+                const int cell = cn + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1));
+                cell_v[8 * ((i64)cell - lo) + (q ^ 7)] = v;
+            }
+        }
+    }
+}
+
 // corners on a leaf's lower faces owned by a cell of another leaf L' of the
 // batch: the same value is a corner of L''s brick holding the owner cell, where
 // L' owns it -- copied when that brick is live, evaluated otherwise
@@ -2489,24 +2594,12 @@ void stage_mesh(Ctx& c) {
             set_last_error("%lld finest nodes exceed the corner list's 2^28", (long long)nD);
             throw Error{PRGPU_ERR_LIMIT, {0}};
         }
-        unsigned char* omask = dalloc<unsigned char>(nD, s);
-        int* ocnt = dalloc<int>(nD, s);
-        int* ofirst = dalloc<int>(nD + 1, s);
-        k_finest_owned<<<grid_for(nD, 256), 256, 0, s>>>(nd, lo, M, omask, ocnt);
+        const i64 gfirst = (lo - 1) / 8, ng = nD / 8;
+        ensure_group_rows(c);
         CK_LAUNCH();
-        exclusive_scan<int, int>(ocnt, ofirst, nD, ofirst + nD, s);
-        const i64 nown = read_scalar(ofirst + nD, s);
-        if (nown > 0) {
-            int* olist = dalloc<int>(nown, s);
-            k_finest_list<<<grid_for(nD, 256), 256, 0, s>>>(omask, ofirst, nD, olist);
-            CK_LAUNCH();
-            k_finest_corner_values<<<grid_for(nown, 128, 1ll << 30), 128, 0, s>>>(ea, lo, olist, nown, c.iso, cell_v);
-            CK_LAUNCH();
-            dfree(olist, s);
-        }
-        dfree(omask, s);
-        dfree(ocnt, s);
-        dfree(ofirst, s);
+        k_finest_corners<<<(unsigned)((ng + FC_GROUPS * FC_WARPS - 1) / (FC_GROUPS * FC_WARPS)), 32 * FC_WARPS, finest_shared(D), s>>>(
+            ea, c.gn_rows, gfirst, ng, lo, c.iso, cell_v);
+        CK_LAUNCH();
     }
     c.kend(kt);
     kt = c.kbegin("cells", (double)nD * (8 * 4 + 1));
