@@ -310,60 +310,22 @@ void stage_points(Ctx& c) {
 }
 
 // ------------------------------ corners -------------------------------------
-// value of corner 'kind' of owner o, minus the iso-value
-// (computeVertexImplicitFunctionValue main.cu:2259-2326, including its descent
-// through children[childrenVertexKind[kind]])
-__device__ float owner_corner_value(const EvalArgs& a, i64 o, int kind, float iso) {
-    const int d = a.nd.depth[o];
-    int xyz[3];
-    key_coords(a.nd.key[o], d, a.D, xyz);
-    // the corner as a finest-lattice point: (xyz + bit) / 2^d = u / 2^D exactly
-    const int sh = a.D - d;
-    const int u[3] = {(xyz[0] + (kind & 1)) << sh, (xyz[1] + ((kind >> 1) & 1)) << sh, (xyz[2] + ((kind >> 2) & 1)) << sh};
-    float val = 0.f;
-    if (o > 0) {
-        val = walk_up_u(a, o, u, val);
-        const int exceed = c_vid[kind];
-        i64 node = o;
-        int cx[3] = {xyz[0], xyz[1], xyz[2]};
-        for (int dd = d + 1; dd <= a.D; ++dd) {
-            const int c0 = a.nd.child0[node];
-            if (c0 == -1) break;
-            node = c0 + exceed;   // child 'exceed': its coordinates are the parent's doubled plus its bits
-            cx[0] = (cx[0] << 1) | ((exceed >> 2) & 1);
-            cx[1] = (cx[1] << 1) | ((exceed >> 1) & 1);
-            cx[2] = (cx[2] << 1) | (exceed & 1);
-            val = level_sum_u(a, node, dd, cx, u, val);
-        }
+// A corner's value is its owner's (computeVertexImplicitFunctionValue main.cu:2259-2326): the walk from the owner to
+// the root, then, where the owner has children, the descent through children[childrenVertexKind[kind]] added here
+__device__ __forceinline__ float corner_descent(const EvalArgs& a, i64 node, int d, int kind, int cx, int cy, int cz,
+                                                const int u[3], float val) {
+    const int exceed = c_vid[kind];
+    int c[3] = {cx, cy, cz};
+    for (int dd = d + 1; dd <= a.D; ++dd) {
+        const int c0 = a.nd.child0[node];
+        if (c0 == -1) break;
+        node = c0 + exceed;   // child 'exceed': its coordinates are the parent's doubled plus its bits
+        c[0] = (c[0] << 1) | ((exceed >> 2) & 1);
+        c[1] = (c[1] << 1) | ((exceed >> 1) & 1);
+        c[2] = (c[2] << 1) | (exceed & 1);
+        val = level_sum_u(a, node, dd, c, u, val);
     }
-    return val - iso;
-}
-
-// the owned corners as a list: (node << 3) | corner
-__global__ void k_finest_list(const unsigned char* __restrict__ owned_mask, const int* __restrict__ first, i64 nD,
-                              int* __restrict__ list) {
-    for (i64 l = (i64)blockIdx.x * blockDim.x + threadIdx.x; l < nD; l += (i64)gridDim.x * blockDim.x) {
-        unsigned m = owned_mask[l];
-        int q = first[l];
-        while (m) {
-            const int kind = __ffs(m) - 1;
-            list[q++] = (int)(l << 3) | kind;
-            m &= m - 1;
-        }
-    }
-}
-
-// f(node, corner kind in its frame) for each of the existing same-depth nodes that share corner 'kind' of
-// node i, itself among them
-template <class F>
-__device__ __forceinline__ void corner_sharers(const NodeArrays& nd, i64 i, int kind, F f) {
-    const int sx = kind & 1, sy = (kind >> 1) & 1, sz = kind >> 2;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const int j = 9 * (sx - (e & 1) + 1) + 3 * (sy - ((e >> 1) & 1) + 1) + (sz - (e >> 2) + 1);
-        const int nb = nd.neigh[(i64)j * nd.M + i];
-        if (nb != -1) f(nb, e);
-    }
+    return val;
 }
 
 // Cells in tiles of CELL_TILE: the kernels that find the categories sum each tile's triangles, the sums are
@@ -471,47 +433,6 @@ __global__ void k_mark_faces(NodeArrays nd, int D, i64 lo, i64 hi, const unsigne
                 fflag[6 * (i64)o + k] = 1;
             }
         }
-    }
-}
-
-// Corners of the leaves above the finest depth: each node's owned corners that a leaf shares, as a mask and a
-// count (a corner's owner is the least key among the existing same-depth nodes around it).
-__global__ void k_coarse_owned(NodeArrays nd, i64 n, unsigned char* __restrict__ mask, int* __restrict__ count) {
-    const i64 M = nd.M;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const u64 ki = nd.key[i];
-        unsigned smaller = 0, leaf = 0;   // bit j: neighbour j exists and has a smaller key; is a leaf
-#pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            const int nb = nd.neigh[(i64)j * M + i];
-            if (nb == -1) continue;
-            if (j != 13 && nd.key[nb] < ki) smaller |= 1u << j;
-            if (nd.child0[nb] == -1) leaf |= 1u << j;
-        }
-        unsigned owned = 0;
-        if (i > 0)   // the root has no corner value of its own
-#pragma unroll
-            for (int kind = 0; kind < 8; ++kind) {
-                unsigned around = 0;
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    around |= 1u << (9 * ((kind & 1) - (e & 1) + 1) + 3 * (((kind >> 1) & 1) - ((e >> 1) & 1) + 1) +
-                                     ((kind >> 2) - (e >> 2) + 1));
-                if (!(smaller & around) && (leaf & around)) owned |= 1u << kind;
-            }
-        mask[i] = (unsigned char)owned;
-        count[i] = __popc(owned);
-    }
-}
-// the listed corners (node << 3 | corner), each value to the leaves that have the corner
-__global__ void __launch_bounds__(128, 8) k_coarse_corner_list(EvalArgs a, const int* __restrict__ list, i64 n,
-                                                               float iso, float* __restrict__ leaf_v) {
-    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (i64)gridDim.x * blockDim.x) {
-        const int lk = list[q];
-        const float val = owner_corner_value(a, lk >> 3, lk & 7, iso);
-        corner_sharers(a.nd, lk >> 3, lk & 7, [&](int nb, int e) {
-            if (a.nd.child0[nb] == -1) leaf_v[8 * (i64)nb + e] = val;
-        });
     }
 }
 
@@ -2128,36 +2049,47 @@ __global__ void __launch_bounds__(32 * E2_WARPS) k_edge2_eval(VArgs v, BrickInde
     }
 }
 
-// Corners of the finest cells, by sibling groups, four to a warp.  A group's 2x2x2 cells have 3x3x3 corners.
+// Corners by sibling groups, four to a warp.  A group's 2x2x2 cells have 3x3x3 corners.
 // The cells around them are the 4x4x4 block of the children of the parent's 27 neighbours (the group table:
 // sibling groups are whole), so which exist and which of them precede the group in key order are 27 bits, and
 // a corner is the group's own when none of its 8 cells that exists precedes the group; its owner is then the
 // lowest of the group's cells at it.  The window, the ancestors' x27 rows and the walk are those of the
 // edge-2 bricks above: a column of up to three corners along z per lane, here only the columns that own any (a surface fills about
 // half of the 36), and each value goes to the cells of the block that share the corner, without a look at
-// their neighbour tables.  The values and their order of summation are owner_corner_value's.
-// 1M torus 0.90 -> 0.54 ms, 4M displaced sphere 3.9 -> 2.3, where a pass over the nodes' neighbours and keys
+// their neighbour tables.
+// COARSE: the groups above the finest depth (a warp's may lie at two depths), of whose corners only those that a
+// leaf shares are wanted; an owner with children adds its descent, the corners one to a lane.  Corners and flags of
+// the coarse leaves, 50k sphere 0.088 -> 0.051 ms, 100k superquadric 0.215 -> 0.177, 1M torus 0.48 -> 0.46 (4M
+// displaced sphere 2.3 either way, bound by the descents).
+// Finest cells: 1M torus 0.90 -> 0.56 ms, 4M displaced sphere 3.9 -> 2.4, where a pass over the nodes' neighbours and keys
 // found the owners and a thread per owned corner walked up alone.  Two thirds of it is arithmetic; fetching
 // every group's rows, shared or not, cost 0.16 ms on the torus, and the basis entries a level ahead gain nothing.
 constexpr int FC_GROUPS = 4, FC_WARPS = 2;
 struct FcWarp {
+    unsigned long long leaf[FC_GROUPS];         // COARSE: the leaves among the cells of the block
     unsigned long long before[FC_GROUPS];       // cells of the block that exist and precede the group, a bit each
     float x[FC_GROUPS][65];                     // windows; a warp reads 0, 4, 16 and 20 on of each, in banks of their own
     int gn[FC_GROUPS * GN_ROW];
     int up[FC_GROUPS][BR_LEVELS];               // the parent and its ancestors, by depth
+    int depth[FC_GROUPS];
     int cell[FC_GROUPS][3];                     // coordinates of the group's first cell
     unsigned char row[FC_GROUPS][BR_LEVELS];    // the group whose copy of the ancestor's row serves this one
+    float val[96];                              // COARSE: corners of a round of columns
+    unsigned char corner[96];
     unsigned short col[40];                     // group, column and owned corners of the columns that own any
 };
 constexpr int FC_ROWS = FC_GROUPS * 7;          // float4 per level
 static_assert(sizeof(FcWarp) % 16 == 0, "the rows follow at 16-byte alignment");
 static_assert(FC_WARPS * (sizeof(FcWarp) + 16 * FC_ROWS * PRGPU_MAX_DEPTH) <= 48 * 1024,
               "dynamic shared memory without an opt-in");
-inline size_t finest_shared(int D) { return FC_WARPS * (sizeof(FcWarp) + 16 * (size_t)FC_ROWS * D); }
-__global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, const int* __restrict__ gn_rows,
-                                                                  i64 gfirst, i64 ng, i64 lo, float iso, float* __restrict__ cell_v) {
+inline unsigned group_blocks(i64 ng) { return (unsigned)((ng + FC_GROUPS * FC_WARPS - 1) / (FC_GROUPS * FC_WARPS)); }
+inline size_t group_shared(int D) { return FC_WARPS * (sizeof(FcWarp) + 16 * (size_t)FC_ROWS * D); }
+// out: eight values per cell from node out0 on
+template <bool COARSE>
+__global__ void __launch_bounds__(32 * FC_WARPS) k_group_corners(EvalArgs a, const int* __restrict__ gn_rows, i64 gfirst,
+                                                                 i64 ng, float iso, float* __restrict__ out, i64 out0) {
     extern __shared__ float4 fc_shared[];
-    const int D = a.D, r = D - 1;
+    const int D = a.D;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     char* mine = reinterpret_cast<char*>(fc_shared) + w * (sizeof(FcWarp) + 16 * (size_t)FC_ROWS * D);
     FcWarp& sm = *reinterpret_cast<FcWarp*>(mine);
@@ -2171,41 +2103,60 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, co
         if (e < FC_GROUPS * GN_ROW) sm.gn[e] = e < nbr * GN_ROW ? gn_rows[(gfirst + g1) * GN_ROW + e] : -1;
     }
     if (lane < nbr) {
-        int n = (int)(lo + 8 * (g1 + lane));
-        for (int l = r; l >= 0; --l) {
-            n = a.nd.parent[n];
-            sm.up[lane][l] = n;
+        const i64 first = 1 + 8 * (gfirst + g1 + lane);
+        const int d = COARSE ? a.nd.depth[first] : D;
+        sm.depth[lane] = d;
+        int n = (int)first;
+        for (int l = D - 1; l >= 0; --l) {
+            if (!COARSE || l < d) n = a.nd.parent[n];
+            sm.up[lane][l] = !COARSE || l < d ? n : -1;
         }
         int c[3];
-        key_coords(a.nd.key[lo + 8 * (g1 + lane)], D, D, c);
+        key_coords(a.nd.key[first], d, D, c);
         for (int ax = 0; ax < 3; ++ax) sm.cell[lane][ax] = c[ax];
     }
     __syncwarp();
-    {
-        // neighbouring groups share their upper ancestors: a row is fetched by the first group that has it
-        const int b = lane / 7, q = lane % 7;
-        if (b < nbr)
-            for (int l = 0; l <= r; ++l) {
-                const int n = sm.up[b][l];
-                int first = b;
-                while (first > 0 && sm.up[first - 1][l] == n) --first;
-                if (first == b)
-                    async_copy16(s_row + l * FC_ROWS + lane, reinterpret_cast<const float4*>(a.x27 + (i64)n * X27_STRIDE) + q);
-                if (q == 0) sm.row[b][l] = (unsigned char)first;
-            }
+    int node[2 * FC_GROUPS];                    // this lane's cells of the blocks, -1: absent
+#pragma unroll
+    for (int m = 0; m < 2 * FC_GROUPS; ++m) {
+        const int g = m >> 1, cell = lane + 32 * (m & 1), bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
+        const int cn = sm.gn[g * GN_ROW + 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
+        node[m] = cn == -1 ? -1 : cn + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1));
+        const unsigned b = __ballot_sync(0xffffffffu, cn != -1 && cn < sm.gn[g * GN_ROW + 13]);
+        if (lane == 0) reinterpret_cast<unsigned*>(sm.before)[m] = b;
     }
-    {
-        float xv[2 * FC_GROUPS];
+    auto stage = [&]() {
+        {
+            // neighbouring groups share their upper ancestors: a row is fetched by the first group that has it
+            const int b = lane / 7, q = lane % 7;
+            if (b < nbr)
+                for (int l = 0; l < sm.depth[b]; ++l) {
+                    const int n = sm.up[b][l];
+                    int first = b;
+                    while (first > 0 && sm.up[first - 1][l] == n) --first;
+                    if (first == b)
+                        async_copy16(s_row + l * FC_ROWS + lane, reinterpret_cast<const float4*>(a.x27 + (i64)n * X27_STRIDE) + q);
+                    if (q == 0) sm.row[b][l] = (unsigned char)first;
+                }
+        }
+        {
+            float xv[2 * FC_GROUPS];
+#pragma unroll
+            for (int m = 0; m < 2 * FC_GROUPS; ++m) xv[m] = node[m] == -1 ? 0.f : a.x[node[m]];
+#pragma unroll
+            for (int m = 0; m < 2 * FC_GROUPS; ++m) sm.x[m >> 1][lane + 32 * (m & 1)] = xv[m];
+        }
+    };
+    if (!COARSE) stage();
+    if (COARSE) {
+        bool leaf[2 * FC_GROUPS];
+#pragma unroll
+        for (int m = 0; m < 2 * FC_GROUPS; ++m) leaf[m] = node[m] != -1 && a.nd.child0[node[m]] == -1;
 #pragma unroll
         for (int m = 0; m < 2 * FC_GROUPS; ++m) {
-            const int g = m >> 1, cell = lane + 32 * (m & 1), bx = cell >> 4, by = (cell >> 2) & 3, bz = cell & 3;
-            const int cn = sm.gn[g * GN_ROW + 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
-            xv[m] = cn == -1 ? 0.f : a.x[cn + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1))];
-            const unsigned b = __ballot_sync(0xffffffffu, cn != -1 && cn < sm.gn[g * GN_ROW + 13]);
-            if (lane == 0) reinterpret_cast<unsigned*>(sm.before)[m] = b;
+            const unsigned b = __ballot_sync(0xffffffffu, leaf[m]);
+            if (lane == 0) reinterpret_cast<unsigned*>(sm.leaf)[m] = b;
         }
-#pragma unroll
-        for (int m = 0; m < 2 * FC_GROUPS; ++m) sm.x[m >> 1][lane + 32 * (m & 1)] = xv[m];
     }
     __syncwarp();
     int ncol = 0;
@@ -2215,11 +2166,17 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, co
         int bits = 0;
         if (e < 9 * nbr)
 #pragma unroll
-            for (int kz = 0; kz < 3; ++kz)   // the 2x2x2 cells at the corner
-                if (!(sm.before[g] & (0x330033ull << (16 * kx + 4 * ky + kz)))) bits |= 1 << kz;
+            for (int kz = 0; kz < 3; ++kz) {
+                const unsigned long long at = 0x330033ull << (16 * kx + 4 * ky + kz);   // the 2x2x2 cells at the corner
+                if (!(sm.before[g] & at) && (!COARSE || (sm.leaf[g] & at))) bits |= 1 << kz;
+            }
         const unsigned some = __ballot_sync(0xffffffffu, bits != 0);
         if (bits) sm.col[ncol + __popc(some & ((1u << lane) - 1u))] = (unsigned short)(e << 3 | bits);
         ncol += __popc(some);
+    }
+    if (COARSE) {                               // nothing to fetch where no corner is wanted
+        if (ncol == 0) return;
+        stage();
     }
     async_wait();
     __syncwarp();
@@ -2227,11 +2184,13 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, co
         const int entry = sm.col[min(c0 + lane, ncol - 1)];
         const int bits = c0 + lane < ncol ? entry & 7 : 0, e = entry >> 3, g = e / 9, kx = e % 9 / 3, ky = e % 3;
         const int g0[3] = {sm.cell[g][0], sm.cell[g][1], sm.cell[g][2]};
+        const int d = COARSE ? sm.depth[g] : D, sh0 = D - d;   // corner k of the group: (g0 + k) << sh0 on the lattice
         float val[3] = {0.f, 0.f, 0.f};
         {
-            // the finest depth: owner cell = the one below the corner, its own on the group's lower face
+            // the group's depth: owner cell = the one below the corner, its own on the group's lower face
             const int sx = kx == 2, sy = ky == 2;
-            const float4 fx = lattice_at(a, D, g0[0] + sx, kx - sx), fy = lattice_at(a, D, g0[1] + sy, ky - sy);
+            const float4 fx = lattice_at(a, d, g0[0] + sx, (kx - sx) << sh0),
+                         fy = lattice_at(a, d, g0[1] + sy, (ky - sy) << sh0);
             const float x3[3] = {fx.x, fx.y, fx.z}, y3[3] = {fy.x, fy.y, fy.z};
             float p[4][9];
 #pragma unroll
@@ -2242,23 +2201,23 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, co
 #pragma unroll
             for (int kz = 0; kz < 3; ++kz) {
                 const int sz = kz == 2;
-                const float4 fz = lattice_at(a, D, g0[2] + sz, kz - sz);
+                const float4 fz = lattice_at(a, d, g0[2] + sz, (kz - sz) << sh0);
                 const float z3[3] = {fz.x, fz.y, fz.z};
 #pragma unroll
                 for (int j = 0; j < 27; ++j) val[kz] = fmaf(p[sz + j % 3][j / 3], z3[j % 3], val[kz]);
             }
         }
 #pragma unroll 1
-        for (int l = r; l >= 0; --l) {
+        for (int l = d - 1; l >= 0; --l) {
             const int sh = D - l;
             int c[3], k[3];
 #pragma unroll
             for (int ax = 0; ax < 3; ++ax) {
-                c[ax] = g0[ax] >> sh;
-                k[ax] = g0[ax] - (c[ax] << sh);
+                c[ax] = g0[ax] >> (d - l);
+                k[ax] = (g0[ax] << sh0) - (c[ax] << sh);
             }
             const float4* bz = &a.lb[lattice_offset(D, l) + (i64)c[2] * ((1 << sh) + 1) + k[2]];
-            const float4 b3[3] = {bz[0], bz[1], bz[2]};
+            const float4 b3[3] = {bz[0], bz[1 << sh0], bz[2 << sh0]};
             const float4* row = s_row + l * FC_ROWS + 7 * sm.row[g][l];
             float xs[28];
 #pragma unroll
@@ -2266,20 +2225,47 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_finest_corners(EvalArgs a, co
                 const float4 f = row[q];
                 xs[4 * q] = f.x; xs[4 * q + 1] = f.y; xs[4 * q + 2] = f.z; xs[4 * q + 3] = f.w;
             }
-            column_level<3>(xs, lattice_at(a, l, c[0], k[0] + kx), lattice_at(a, l, c[1], k[1] + ky), b3, val);
+            column_level<3>(xs, lattice_at(a, l, c[0], k[0] + (kx << sh0)), lattice_at(a, l, c[1], k[1] + (ky << sh0)), b3, val);
         }
-#pragma unroll
-        for (int kz = 0; kz < 3; ++kz) {
-            if (!((bits >> kz) & 1)) continue;
-            const float v = val[kz] - iso;
+        auto scatter = [&](int g, int kx, int ky, int kz, float v) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {       // the cells at the corner, in block coordinates
                 const int bx = kx + (q & 1), by = ky + ((q >> 1) & 1), bz = kz + (q >> 2);
                 const int cn = sm.gn[g * GN_ROW + 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1)];
-                if (cn == -1) continue;
+                if (cn == -1 || (COARSE && !((sm.leaf[g] >> (16 * bx + 4 * by + bz)) & 1))) continue;
                 const int cell = cn + ((((bx + 1) & 1) << 2) | (((by + 1) & 1) << 1) | ((bz + 1) & 1));
-                cell_v[8 * ((i64)cell - lo) + (q ^ 7)] = v;
+                out[8 * ((i64)cell - out0) + (q ^ 7)] = v;
             }
+        };
+        if (!COARSE) {
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz)
+                if ((bits >> kz) & 1) scatter(g, kx, ky, kz, val[kz] - iso);
+            continue;
+        }
+        // a descent is a walk of its own: the corners one to a lane
+        __syncwarp();
+        int n = 0;
+#pragma unroll
+        for (int kz = 0; kz < 3; ++kz) {
+            const bool own = (bits >> kz) & 1;
+            const unsigned some = __ballot_sync(0xffffffffu, own);
+            if (own) {
+                const int at = n + __popc(some & ((1u << lane) - 1u));
+                sm.val[at] = val[kz];
+                sm.corner[at] = (unsigned char)(3 * e + kz);
+            }
+            n += __popc(some);
+        }
+        __syncwarp();
+        for (int q = lane; q < n; q += 32) {
+            const int e = sm.corner[q] / 3, kz = sm.corner[q] % 3, g = e / 9, kx = e % 9 / 3, ky = e % 3;
+            const int sx = kx == 2, sy = ky == 2, sz = kz == 2, d = sm.depth[g], sh0 = D - d;
+            const int X = sm.cell[g][0], Y = sm.cell[g][1], Z = sm.cell[g][2];
+            const int u[3] = {(X + kx) << sh0, (Y + ky) << sh0, (Z + kz) << sh0};
+            const float v = corner_descent(a, sm.gn[g * GN_ROW + 13] + (sx << 2 | sy << 1 | sz), d,
+                                           (kx - sx) | (ky - sy) << 1 | (kz - sz) << 2, X + sx, Y + sy, Z + sz, u, sm.val[q]);
+            scatter(g, kx, ky, kz, v - iso);
         }
     }
 }
@@ -2597,8 +2583,8 @@ void stage_mesh(Ctx& c) {
         const i64 gfirst = (lo - 1) / 8, ng = nD / 8;
         ensure_group_rows(c);
         CK_LAUNCH();
-        k_finest_corners<<<(unsigned)((ng + FC_GROUPS * FC_WARPS - 1) / (FC_GROUPS * FC_WARPS)), 32 * FC_WARPS, finest_shared(D), s>>>(
-            ea, c.gn_rows, gfirst, ng, lo, c.iso, cell_v);
+        k_group_corners<false><<<group_blocks(ng), 32 * FC_WARPS, group_shared(D), s>>>(ea, c.gn_rows, gfirst, ng, c.iso,
+                                                                                       cell_v, lo);
         CK_LAUNCH();
     }
     c.kend(kt);
@@ -2627,27 +2613,9 @@ void stage_mesh(Ctx& c) {
     if (nCoarse > 1) {
         const int kc = c.kbegin("coarse_leaves", (double)nCoarse * (4 + 108 + 8 + 3 * 4 + 8 * 4) + (double)M * 4);
         float* leaf_v = dalloc<float>(8 * nCoarse, s);
-        {
-            // one thread per needed corner (list of (node << 3) | corner)
-            unsigned char* nmask = dalloc<unsigned char>(nCoarse, s);
-            int* ncnt = dalloc<int>(nCoarse, s);
-            int* nfirst = dalloc<int>(nCoarse + 1, s);
-            k_coarse_owned<<<grid_for(nCoarse, 256), 256, 0, s>>>(nd, nCoarse, nmask, ncnt);
-            CK_LAUNCH();
-            exclusive_scan<int, int>(ncnt, nfirst, nCoarse, nfirst + nCoarse, s);
-            const i64 nneed = read_scalar(nfirst + nCoarse, s);
-            if (nneed > 0) {
-                int* nlist = dalloc<int>(nneed, s);
-                k_finest_list<<<grid_for(nCoarse, 256), 256, 0, s>>>(nmask, nfirst, nCoarse, nlist);
-                CK_LAUNCH();
-                k_coarse_corner_list<<<grid_for(nneed, 128, 1ll << 30), 128, 0, s>>>(ea, nlist, nneed, c.iso, leaf_v);
-                CK_LAUNCH();
-                dfree(nlist, s);
-            }
-            dfree(nmask, s);
-            dfree(ncnt, s);
-            dfree(nfirst, s);
-        }
+        const i64 ng = (lo - 1) / 8;
+        k_group_corners<true><<<group_blocks(ng), 32 * FC_WARPS, group_shared(D), s>>>(ea, c.gn_rows, 0, ng, c.iso, leaf_v, 0);
+        CK_LAUNCH();
         k_coarse_leaves<<<grid_for(nCoarse - 1, 128, 1ll << 30), 128, 0, s>>>(nd, 1, nCoarse, leaf_v, fflag, has_tri,
                                                                              has_int, is_root);
         CK_LAUNCH();
