@@ -1,6 +1,6 @@
-"""Corner values by sibling groups, four groups to a warp, of the finest cells and of the leaves above them: group counts around that, blocks with
-every neighbour present (a filled volume), cells at the ends of the domain, lone groups far apart, and the shallowest
-tree: the mesh bit for bit the oracle's for the same coefficients."""
+"""Corner values by sibling groups, four groups to a warp, of the finest cells and of the leaves above them: group
+counts around that, blocks with every neighbour present (a filled volume), cells at the ends of the domain, lone
+groups far apart, and the shallowest tree: the mesh bit for bit the oracle's for the same coefficients."""
 import numpy as np
 import pytest
 
