@@ -6,7 +6,8 @@
 //   * corners, edges and faces are not materialised as records; each cell finds
 //     the owner of a corner/edge/face (the minimum key among the cells that
 //     share it, as initVertexOwner/initEdgeArray/initFaceArray do) from its
-//     neighbour table, and a corner value is evaluated once, by its owner;
+//     neighbour table or its sibling group's, and a corner value is evaluated
+//     once, by its owner;
 //   * edge vertices are de-duplicated by sorting edge keys (batch, lattice
 //     edge) instead of by owner back-links, one sort for the whole mesh;
 //   * subdivided leaves are never expanded into node arrays: their finest cells
@@ -586,7 +587,7 @@ __device__ __forceinline__ u64 cell_key_D(const int c[3], int D) { return coords
 //   BT[d][t][k]   basis value at corner k of the function of cell V_k + t - 1
 //                 (depth d > r, V_k = (corner - 1) >> (D - d), t = 0..3; t = 3
 //                 serves owner cells V_k + 1) or of ancestor cell + t - 1
-//                 (depth d <= r); built per live brick by k_brick_eval
+//                 (depth d <= r); read per live brick from the lattice table
 //   RA[l][t]      range over k of BT[l][t][k], l <= r
 //   RW[d][n]      range (with 0) of the depth-d function of window cell n over
 //                 the corners whose owner cell is within one cell of it
@@ -2715,7 +2716,6 @@ void stage_mesh(Ctx& c) {
         const int nrbound = layout.first[D - 1];
         i64* dbpre = dpre;
         i64* drpre = dpre + nr + 1;
-        i64* dspre = dpre + 2 * (nr + 1);
         i64* dsrpre = dpre + 3 * (nr + 1);
         float* rows = dalloc<float>(nrows * PROW * (D + 1), s);
         int* up = dalloc<int>((i64)nr * BR_LEVELS, s);

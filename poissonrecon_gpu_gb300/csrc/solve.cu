@@ -10,7 +10,7 @@
 // the others), so ONE persistent cooperative launch solves all of them at
 // once: the co-resident blocks are partitioned between the depths in
 // proportion to their row counts, and each partition runs its own CG with its
-// own grid barrier.  Barriers spin with an iteration limit; on expiry the
+// own grid sums.  Their waits have an iteration limit; on expiry the
 // kernel records PRGPU_ERR_TIMEOUT and returns.
 //
 // Matrix-vector product by sibling groups: the 8 children of a node are
