@@ -2274,38 +2274,70 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_group_corners(EvalArgs a, con
 // corners on a leaf's lower faces owned by a cell of another leaf L' of the
 // batch: the same value is a corner of L''s brick holding the owner cell, where
 // L' owns it -- copied when that brick is live, evaluated otherwise
-// (count[0]: the corners; count[2]: those evaluated.  The grid does not depend on the count, which the host
-// has not read.)
+// (count[0]: the corners; count[2]: those evaluated.  The grids do not depend on the counts, which the host
+// has not read.)  A few in a hundred are evaluated, at a hundred times the cost of a copy.  LIST: they are listed by
+// the launch that copies and evaluated by one of their own, one to a thread, instead of each holding up a warp of
+// copies: 27 M corners (4M displaced sphere) 2.36 -> 1.50 ms, 101 M 8.5 -> 5.3, 1.3 M (1M torus) 0.174 -> 0.150.
+// Below FF_LISTED lower-face corners of live bricks one launch that does both is the faster, the evaluation's chain of loads
+// being most of either: 0.44 M corners 0.065 against 0.085 ms.  The list takes the corners [at, at + FF_SPAN), count[3]
+// of them.
+constexpr i64 FF_SPAN = 1ll << 31, FF_LISTED = 1ll << 21;
+// the owner brick's corner, evaluated by its own leaf
+__device__ __forceinline__ float foreign_value(const VArgs& v, const BrickIndex& bix, u64 src) {
+    const int D = v.e.D, e = (int)(src & 1023);
+    const VBrick B = brick_of(v, bix, (i64)(src >> 10));
+    const VRoot R = v.roots[B.root];
+    const int r = R.depth, S = 1 << (D - r), E = brick_edge(D, r), E1 = E + 1;
+    int Lc[3];
+    key_coords(v.e.nd.key[R.node], r, D, Lc);
+    const int kk[3] = {e / (E1 * E1), (e / E1) % E1, e % E1};
+    int oc[3], qc[3];
+    for (int ax = 0; ax < 3; ++ax) {
+        const int l0 = Lc[ax] * S;
+        qc[ax] = l0 + B.b[ax] * E + kk[ax];
+        oc[ax] = max(qc[ax] - 1, l0);
+    }
+    return virtual_corner_value(v, R.node, r, oc, qc) - v.iso;
+}
+template <bool LIST>
 __global__ void k_foreign_fill(VArgs v, BrickIndex bix, LiveIndex lx, const unsigned char* __restrict__ culled,
-                               const int* __restrict__ live_pos, const ForeignCorner* __restrict__ foreign, i64 cap,
-                               float* __restrict__ blat, unsigned long long* __restrict__ count) {
-    const int D = v.e.D;
-    const i64 n = min((i64)count[0], cap);
-    for (i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
-        const ForeignCorner fe = foreign[f];
-        const i64 brick = (i64)(fe.src >> 10);
-        const int e = (int)(fe.src & 1023);
-        float val;
-        if (!culled[brick]) {
-            val = blat[lx.lat(live_pos[brick]) + e];
-        } else {
-            atomicAdd(&count[2], 1ull);
-            // the owner brick's corner e, evaluated by its own leaf
-            const VBrick B = brick_of(v, bix, brick);
-            const VRoot R = v.roots[B.root];
-            const int r = R.depth, S = 1 << (D - r), E = brick_edge(D, r), E1 = E + 1;
-            int Lc[3];
-            key_coords(v.e.nd.key[R.node], r, D, Lc);
-            const int kk[3] = {e / (E1 * E1), (e / E1) % E1, e % E1};
-            int oc[3], qc[3];
-            for (int ax = 0; ax < 3; ++ax) {
-                const int l0 = Lc[ax] * S;
-                qc[ax] = l0 + B.b[ax] * E + kk[ax];
-                oc[ax] = max(qc[ax] - 1, l0);
+                               const int* __restrict__ live_pos, const ForeignCorner* __restrict__ foreign, i64 at, i64 cap,
+                               float* __restrict__ blat, unsigned* __restrict__ list, unsigned long long* __restrict__ count) {
+    const i64 n = min(min((i64)count[0], cap), at + FF_SPAN);
+    for (i64 f0 = at + (i64)blockIdx.x * blockDim.x; f0 < n; f0 += (i64)gridDim.x * blockDim.x) {
+        const i64 f = f0 + threadIdx.x;
+        bool slow = false;
+        if (f < n) {
+            const ForeignCorner fe = foreign[f];
+            const i64 brick = (i64)(fe.src >> 10);
+            slow = culled[brick];
+            if (!slow) {
+                blat[lx.lat(fe.li) + fe.e] = blat[lx.lat(live_pos[brick]) + (int)(fe.src & 1023)];
+            } else if (!LIST) {
+                atomicAdd(&count[2], 1ull);
+                blat[lx.lat(fe.li) + fe.e] = foreign_value(v, bix, fe.src);
             }
-            val = virtual_corner_value(v, R.node, r, oc, qc) - v.iso;
         }
-        blat[lx.lat(fe.li) + fe.e] = val;
+        if (!LIST) continue;
+        const unsigned m = __ballot_sync(0xffffffffu, slow);
+        if (!m) continue;
+        const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+        unsigned base = 0;
+        if (lane == leader) {
+            base = (unsigned)atomicAdd(&count[3], (unsigned long long)__popc(m));
+            atomicAdd(&count[2], (unsigned long long)__popc(m));
+        }
+        base = __shfl_sync(0xffffffffu, base, leader);
+        if (slow) list[base + __popc(m & ((1u << lane) - 1u))] = (unsigned)(f - at);
+    }
+}
+__global__ void k_foreign_eval(VArgs v, BrickIndex bix, LiveIndex lx, const ForeignCorner* __restrict__ foreign, i64 at,
+                               const unsigned* __restrict__ list, float* __restrict__ blat,
+                               const unsigned long long* __restrict__ count) {
+    const i64 n = (i64)count[3];
+    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (i64)gridDim.x * blockDim.x) {
+        const ForeignCorner fe = foreign[at + list[q]];
+        blat[lx.lat(fe.li) + fe.e] = foreign_value(v, bix, fe.src);
     }
 }
 
@@ -2834,8 +2866,8 @@ void stage_mesh(Ctx& c) {
             CK_LAUNCH();
             total_cells = lx.cells();
             lat_brick = dalloc<float>(lx.lattices(), s);
-            dcount = dalloc<unsigned long long>(3, s);
-            CK(cudaMemsetAsync(dcount, 0, 3 * sizeof(unsigned long long), s));
+            dcount = dalloc<unsigned long long>(4, s);
+            CK(cudaMemsetAsync(dcount, 0, 4 * sizeof(unsigned long long), s));
             // corners owned by another leaf: at most the lower-face corners of the live bricks
             fcap = lx.lattices() - lx.cells();
             ForeignCorner* foreign = dalloc<ForeignCorner>(fcap, s);
@@ -2861,9 +2893,24 @@ void stage_mesh(Ctx& c) {
             }
             c.kend(ks);
             const int kf = c.kbegin("foreign_fill", 0.0);
-            k_foreign_fill<<<grid_for(fcap, 128, (i64)c.sms * 512), 128, 0, s>>>(va, bix, lx, culled, bp, foreign, fcap,
-                                                                                lat_brick, dcount);
-            CK_LAUNCH();
+            if (fcap < FF_LISTED) {
+                k_foreign_fill<false><<<grid_for(fcap, 128, (i64)c.sms * 512), 128, 0, s>>>(va, bix, lx, culled, bp, foreign, 0,
+                                                                                           fcap, lat_brick, nullptr, dcount);
+                CK_LAUNCH();
+            } else {
+                unsigned* list = dalloc<unsigned>(std::min(fcap, FF_SPAN), s);
+                for (i64 at = 0; at < fcap; at += FF_SPAN) {
+                    if (at) CK(cudaMemsetAsync(dcount + 3, 0, sizeof(unsigned long long), s));
+                    const i64 span = std::min(fcap - at, FF_SPAN);
+                    k_foreign_fill<true><<<grid_for(span, 256, (i64)c.sms * 128), 256, 0, s>>>(
+                        va, bix, lx, culled, bp, foreign, at, fcap, lat_brick, list, dcount);
+                    CK_LAUNCH();
+                    k_foreign_eval<<<grid_for(span, 64, (i64)c.sms * 256), 64, 0, s>>>(va, bix, lx, foreign, at, list, lat_brick,
+                                                                                       dcount);
+                    CK_LAUNCH();
+                }
+                dfree(list, s);
+            }
             c.kend(kf);
             dfree(foreign, s);
         }
