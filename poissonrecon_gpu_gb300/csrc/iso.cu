@@ -1287,6 +1287,7 @@ __device__ __forceinline__ signed char bound_box(const VArgs& v, const BrickInde
         sm.id[0][lane] = sm.id[0][lane + 32] = -1;
         __syncwarp();
         if (lane < 27) sm.id[0][(lane / 9) * 16 + ((lane / 3) % 3) * 4 + lane % 3] = n;
+        __syncwarp();   // (a single-brick leaf has no coarse depth: the finer terms below are the next to read)
     }
     bool inside = false;
     for (int d = r + 1; d <= dpoly; ++d) {

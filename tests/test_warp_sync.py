@@ -1,0 +1,36 @@
+"""Shared memory passed between lanes is ordered by a barrier on every path.
+
+CUDA orders the lanes' accesses to shared memory at barriers only; shuffles, votes and warp reductions exchange
+registers.  A missing barrier shows in no result as long as the lanes run in step, so it is looked for in the text."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "poissonrecon_gpu_gb300", "csrc")
+
+
+def _body(text, head):
+    """The braces' contents after the first 'head'."""
+    at = text.index("{", text.index(head))
+    depth = 0
+    for k in range(at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[k], 0)
+        if depth == 0:
+            return text[at + 1:k], k + 1
+    raise ValueError(head)
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_bound_box_orders_the_neighbours_before_the_finer_terms():
+    # a leaf that is one brick of edge 8 or 4 has no depth of the coarse loop: the path without the loop's body
+    text, _ = _body(_source("iso.cu"), "signed char bound_box(")
+    loop = "for (int d = r + 1; d <= dpoly; ++d)"
+    _, end = _body(text, loop)
+    path = text[:text.index(loop)] + text[end:]
+    scatter = path.index("sm.id[0][(lane / 9)")
+    reads = path.index("sm.id[cur][g]")
+    assert scatter < reads
+    assert re.search(r"__sync(warp|threads)\(\)", path[scatter:reads])
