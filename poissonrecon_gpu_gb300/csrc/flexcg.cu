@@ -320,7 +320,10 @@ __global__ void __launch_bounds__(FCG_THREADS, 1) k_fcg_all(FcgArgs a, const CgD
 #pragma unroll
         for (int j = 0; j < FCG_NV; ++j) v[j] = acc[j];
         const bool r = reduce(v);
-        return r && !*(volatile int*)a.err;
+        // A wait that gave up (an MMA's, or one of another depth's) ends the solve.  err may be set between two
+        // threads' reads of it, so one read decides for the block: its warps leave together or not at all.
+        const int gave_up = __syncthreads_or(threadIdx.x == 0 && *(volatile int*)a.err != 0);
+        return r && !gave_up;
     };
 
     double rz_prev = bb, rr_prev = bb;

@@ -1,7 +1,8 @@
-"""Shared memory passed between lanes is ordered by a barrier on every path.
+"""Barriers that no result shows, looked for in the text.
 
 CUDA orders the lanes' accesses to shared memory at barriers only; shuffles, votes and warp reductions exchange
-registers.  A missing barrier shows in no result as long as the lanes run in step, so it is looked for in the text."""
+registers.  A missing barrier shows in no result as long as the lanes run in step.  A block whose warps decide
+differently to leave a loop waits at a barrier for ever, which no test may bring about on a GPU."""
 import os
 import re
 
@@ -34,3 +35,12 @@ def test_bound_box_orders_the_neighbours_before_the_finer_terms():
     reads = path.index("sm.id[cur][g]")
     assert scatter < reads
     assert re.search(r"__sync(warp|threads)\(\)", path[scatter:reads])
+
+
+def test_flexible_cg_leaves_by_one_read_of_the_error_flag():
+    # another depth's wait may set the flag between two threads' reads of it
+    text, _ = _body(_source("flexcg.cu"), "k_fcg_all(FcgArgs a")
+    reads = re.findall(r"[^\n;]*\*\s*\(volatile int\*\)\s*a\.err[^\n;]*", text)
+    assert reads
+    for r in reads:
+        assert re.search(r"__syncthreads_(or|and)\(threadIdx\.x == 0 &&", r), r
