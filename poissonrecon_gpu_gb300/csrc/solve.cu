@@ -25,6 +25,7 @@
 // q = A p = s + beta q_prev (p = r + beta p_prev), so each cell is gathered once
 // per iteration (one vector) rather than forming p at every group that reads it.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -846,6 +847,49 @@ __device__ __forceinline__ double csr_stream(const CsrArgs& a, int first, int st
     return loc;
 }
 
+// Whether the streamed product is the faster one for this system, from 32 consecutive rows per warp spread over the
+// matrix: at least 3 in 4 of them have to fit (votes of 1 and -3), which they do when
+//  * the entries at one place of the 32 rows (eight places are looked at) mostly lie within CSR_NEAR columns: matrix
+//    pieces fill an SM's shared memory, so p is gathered through the 40 KB of L1 that are left, and where these do not
+//    hold it a thread per row, with most of 256 KB and twice the warps, is the faster;
+//  * within CSR_NEAR_TIGHT for rows of more than CSR_LONG_NNZ entries on average, and when 16 of the rows or more start
+//    in one bank (rows of 64 entries: 32 lanes in one);
+//  * their lanes' shares are alike, unless the longest row is an eighth of a piece at most: a piece holds parts of few
+//    long rows, so most lanes idle when those are longer than the others.
+// us an iteration, a thread per row against streamed, 1 M rows: 27 entries within 1,024 columns 91 and 65, within
+// 8,192 106 and 106, within 32,768 140 and 188, anywhere 173 and 216; 64 entries within 8,192 columns 508 and 546, 125
+// entries 425 and 553; rows of 1 to 319 entries 586 and 842; 81 entries a row on average, all in every fourth row,
+// 388 and 484.  With 500 K rows, 27 entries: 57 and 40, 67 and 52, 80 and 97, 104 and 116.
+constexpr int CSR_STREAM_NNZ = 16, CSR_LONG_NNZ = 88, CSR_STREAM_NNZ_MAX = 128, CSR_STREAM_ROWS = 1 << 17;
+constexpr int CSR_NEAR = 5120, CSR_NEAR_TIGHT = 1280;
+constexpr int CSR_LOOK_BLOCKS = 304;
+__host__ __device__ constexpr bool csr_stream_length(i64 nz, i64 n) {
+    return nz / n >= CSR_STREAM_NNZ && nz / n <= CSR_STREAM_NNZ_MAX;
+}
+__global__ void __launch_bounds__(CG_BLOCK) k_csr_look(CsrArgs a, int* __restrict__ vote) {
+    const i64 nwarps = (i64)gridDim.x * (CG_BLOCK / 32), warp = (i64)blockIdx.x * (CG_BLOCK / 32) + (threadIdx.x >> 5);
+    const i64 nz = (i64)a.rowptr[a.n] - a.rowptr[0];
+    const CsrRows r = csr_rows_load(a, warp * (((i64)a.n + 31) / 32) / nwarps);
+    const int len = min(max(r.e1 - r.e0, 0), 1 << 24), step = len >> 3;
+    const int crowd = __reduce_max_sync(0xffffffffu, __popc(__match_any_sync(0xffffffffu, r.e0 & 31)));
+    const bool longer = nz / a.n > CSR_LONG_NNZ;
+    const int within = crowd < 16 && !longer ? CSR_NEAR : CSR_NEAR_TIGHT;
+    int c[8], near = 0, seen = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c[k] = step > 0 || k < len ? a.col[r.e0 + (step > 0 ? k * step : k)] : -1;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int hi = __reduce_max_sync(0xffffffffu, c[k]), lo = __reduce_min_sync(0xffffffffu, c[k] < 0 ? INT_MAX : c[k]);
+        if (hi < 0) continue;                          // no row has this place
+        ++seen;
+        near += hi - lo < within;
+    }
+    const unsigned total = __reduce_add_sync(0xffffffffu, (unsigned)len), most = __reduce_max_sync(0xffffffffu, (unsigned)len);
+    const bool even = most <= CSR_CHUNK / 8 || 32 * (u64)most <= (longer ? total + total / 4 : 3 * (u64)total);
+    const bool fits = 4 * near >= 3 * seen && even && csr_stream_length(nz, a.n);
+    if ((threadIdx.x & 31) == 0) atomicAdd(vote, fits ? 1 : -3);
+}
+
 // f over this thread's rows, four at a time: load (row, slot) for all four first
 template <class L, class F>
 __device__ __forceinline__ void csr_each(i64 start, i64 stride, i64 n, L load, F use) {
@@ -934,26 +978,12 @@ __global__ void __launch_bounds__(STREAM ? CSR_BLOCK : CG_BLOCK, STREAM ? 1 : 4)
     }
 }
 
-// Where the streamed product is the faster one (us an iteration, a thread per row against streamed): 27
-// entries a row, 1 M rows 98 against 67, 100 K rows 20 against 23; 7 entries, 1 M rows 33 against 54; 64
-// entries, 1 M rows (rows 16 quads apart, so lanes meet in a bank) 486 against 478.  A wrong nz only picks
-// the slower of two products.
-constexpr int CSR_STREAM_NNZ = 16, CSR_STREAM_ROWS = 1 << 17;
-
 int cg_csr_impl(int n, int nz, const int* rowptr, const int* col, const float* val, const float* rhs, float* x, float tol,
                 int max_iter, int* iters, float* ms) {
     cudaStream_t s = 0;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const bool stream = nz / std::max(n, 1) >= CSR_STREAM_NNZ && n >= CSR_STREAM_ROWS;
-    const int block = stream ? CSR_BLOCK : CG_BLOCK, dsmem = stream ? CSR_DSMEM : 0;
-    void (*kernel)(CsrArgs) = stream ? k_cg_csr<true> : k_cg_csr<false>;
-    if (stream) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CSR_DSMEM));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, dsmem));
-    const i64 want = ((i64)n + block - 1) / block;
-    const int G = (int)std::max<i64>(1, std::min<i64>((i64)sms * std::max(per_sm, 1), want));
-    const i64 words = grid_sum_words(G + 2, 1);
     float *r = nullptr, *p = nullptr, *q = nullptr;
     PartState* st = nullptr;
     u64* slots = nullptr;
@@ -962,17 +992,14 @@ int cg_csr_impl(int n, int nz, const int* rowptr, const int* col, const float* v
     CK(cudaMalloc(&p, sizeof(float) * std::max(n, 1)));
     CK(cudaMalloc(&q, sizeof(float) * std::max(n, 1)));
     CK(cudaMalloc(&st, sizeof(PartState)));
-    CK(cudaMalloc(&slots, sizeof(u64) * words));
     CK(cudaMalloc(&err, sizeof(int)));
     CK(cudaMemset(st, 0, sizeof(PartState)));
-    CK(cudaMemset(slots, 0, sizeof(u64) * words));
     CK(cudaMemset(err, 0, sizeof(int)));
     CsrArgs a;
     a.n = n; a.rowptr = rowptr; a.col = col; a.val = val; a.b = rhs; a.x = x; a.r = r; a.p = p; a.q = q;
     a.tol2 = tol * tol;
     a.max_iter = max_iter;
     a.state = st;
-    a.slots = slots;
     a.err = err;
     const WaitLimits wl = wait_limits();
     a.spin_limit = wl.spin_limit;
@@ -980,6 +1007,28 @@ int cg_csr_impl(int n, int nz, const int* rowptr, const int* col, const float* v
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
+    // A system whose size and number of entries allow the streamed product is looked at on the device (k_csr_look, which
+    // also sees a wrong nz: a few us and a read); a thread per row takes what is declined there and the rest.  Below
+    // CSR_STREAM_ROWS rows neither is the faster for all: 98,304 rows of 27 entries 23 us an iteration and 20, of 48 entries
+    // 36 and 41.
+    bool stream = n >= CSR_STREAM_ROWS && csr_stream_length(nz, n);
+    if (stream) {
+        k_csr_look<<<CSR_LOOK_BLOCKS, CG_BLOCK, 0, s>>>(a, &st->status);
+        CK_LAUNCH();
+        int vote = 0;
+        CK(cudaMemcpy(&vote, &st->status, sizeof vote, cudaMemcpyDeviceToHost));
+        stream = vote >= 0;
+    }
+    const int block = stream ? CSR_BLOCK : CG_BLOCK, dsmem = stream ? CSR_DSMEM : 0;
+    void (*kernel)(CsrArgs) = stream ? k_cg_csr<true> : k_cg_csr<false>;
+    if (stream) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CSR_DSMEM));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, dsmem));
+    const i64 want = ((i64)n + block - 1) / block;
+    const int G = (int)std::max<i64>(1, std::min<i64>((i64)sms * std::max(per_sm, 1), want));
+    const i64 words = grid_sum_words(G + 2, 1);
+    CK(cudaMalloc(&slots, sizeof(u64) * words));
+    CK(cudaMemset(slots, 0, sizeof(u64) * words));
+    a.slots = slots;
     void* kargs[] = {(void*)&a};
     CK(cudaEventRecord(e0, s));
     CK(cudaLaunchCooperativeKernel((void*)kernel, dim3(G), dim3(block), kargs, dsmem, s));
