@@ -450,7 +450,8 @@ static void copy_wide(void* dst, const void* src, size_t bytes) {
 }
 
 int prgpu_copy_mesh(const prgpu_mesh* m, float* vertices, int32_t* triangles) {
-    if (!m || (m->n_vertices && (!m->vertices || !vertices)) || (m->n_triangles && (!m->triangles || !triangles))) {
+    if (!m || m->n_vertices < 0 || m->n_triangles < 0 || (m->n_vertices && (!m->vertices || !vertices)) ||
+        (m->n_triangles && (!m->triangles || !triangles))) {
         set_last_error("prgpu_copy_mesh: invalid argument");
         return PRGPU_ERR_ARG;
     }
