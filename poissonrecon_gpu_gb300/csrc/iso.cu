@@ -2616,7 +2616,6 @@ void stage_mesh(Ctx& c) {
         }
         const i64 gfirst = (lo - 1) / 8, ng = nD / 8;
         ensure_group_rows(c);
-        CK_LAUNCH();
         k_group_corners<false><<<group_blocks(ng), 32 * FC_WARPS, group_shared(D), s>>>(ea, c.gn_rows, gfirst, ng, c.iso,
                                                                                        cell_v, lo);
         CK_LAUNCH();
