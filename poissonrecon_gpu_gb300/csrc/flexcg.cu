@@ -60,9 +60,7 @@ struct FcgArgs {
     int max_iter;
     i64 M;
     const int* neigh;       // 27 x M
-    const int* gn;          // group table
     const int* gnr;         // the group table row by row (GN_ROW per group)
-    i64 ngroups;
     const float* b;
     float* x;
     float* ra;              // residual, two buffers used alternately
@@ -571,9 +569,7 @@ void stage_solve_learned(Ctx& c) {
     a.max_iter = c.params.cg_max_iter;
     a.M = M;
     a.neigh = c.nodes.neigh;
-    a.gn = c.gn;
     a.gnr = c.gn_rows;
-    a.ngroups = (M - 1) / 8;
     a.b = c.divergence;
     a.x = c.x;
     a.ra = ra;

@@ -737,18 +737,15 @@ __device__ __forceinline__ bool foreign_neighbour(int j, const int b[3], int nb)
 }
 
 // window of depth d around a brick (edge B) along one axis: origin and extent
-// of the cells the brick's owner cells can reach (one more upper cell when
-// 'extra': owner cells of foreign corners on the leaf's upper faces); 'cross'
-// when that reaches outside the leaf
-__device__ __forceinline__ void window_axis(int g0, int B, int Lc_ax, int r, int d, int D, int extra, int& wlo,
-                                            int& ext, bool& cross) {
+// of the cells the brick's owner cells can reach; 'cross' when that reaches outside the leaf
+__device__ __forceinline__ void window_axis(int g0, int B, int Lc_ax, int r, int d, int D, int& wlo, int& ext, bool& cross) {
     const int sh = D - d, span = 1 << (d - r);
     const int llo = Lc_ax * span;
     // the first corner's owner cell: the one below it, or its own on the leaf's lower face
     const int Vlo = (g0 == (llo << sh)) ? (g0 >> sh) : ((g0 - 1) >> sh), Vhi = (g0 + B - 1) >> sh;
     cross = (Vlo - 1 < llo || Vhi + 1 >= llo + span);
     wlo = Vlo - 1;
-    ext = Vhi - Vlo + 3 + extra;
+    ext = Vhi - Vlo + 3;
 }
 
 // BT[d][0..3][k] of the brick row starting at corner g0 (see above): the corner is in the closure of its
@@ -806,7 +803,6 @@ __device__ __forceinline__ int outside_boxes(const int wlo[3], const int ext[3],
     return nb;   // what is left lies inside the leaf
 }
 
-// one thread per (brick row, depth)
 // root k's batch id on its node (depth >= 3; shallower roots are single-root batches)
 __global__ void k_batch_flags(const VRoot* __restrict__ roots, int nroots, int* __restrict__ bflag) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nroots; k += gridDim.x * blockDim.x)
@@ -850,7 +846,7 @@ __global__ void k_brick_rows(VArgs v, DepthLayout dl, i64 nrows, int super, cons
         {
             int wlo, ext;
             bool cross;
-            window_axis(g0, B, Lc[ax], r, d, D, 0, wlo, ext, cross);
+            window_axis(g0, B, Lc[ax], r, d, D, wlo, ext, cross);
             const int sh = D - d, lim = 1 << d;
             // the term of window cell N at corner k: its basis value where the corner's owner cell
             // (the lower-face corner owns its own cell) is within one cell of N, else 0
@@ -1295,7 +1291,7 @@ __device__ __forceinline__ signed char bound_box(const VArgs& v, const BrickInde
         bool cross = false;
         for (int ax = 0; ax < 3; ++ax) {
             bool c;
-            window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], c);
+            window_axis(g0[ax], E, Lc[ax], r, d, D, wlo[ax], ext[ax], c);
             cross |= c;
         }
         if (!cross) { inside = true; break; }   // nested windows: the finer ones lie inside the leaf too
@@ -1411,7 +1407,7 @@ __device__ __forceinline__ signed char bound_box(const VArgs& v, const BrickInde
             bool cross = false;
             for (int ax = 0; ax < 3; ++ax) {
                 bool cr;
-                window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], cr);
+                window_axis(g0[ax], E, Lc[ax], r, d, D, wlo[ax], ext[ax], cr);
                 cross |= cr;
             }
             if (!cross) break;
@@ -1452,7 +1448,7 @@ __device__ __forceinline__ signed char bound_box(const VArgs& v, const BrickInde
         bool cross = false;
         for (int ax = 0; ax < 3; ++ax) {
             bool cr;
-            window_axis(g0[ax], E, Lc[ax], r, d, D, 0, wlo[ax], ext[ax], cr);
+            window_axis(g0[ax], E, Lc[ax], r, d, D, wlo[ax], ext[ax], cr);
             cross |= cr;
         }
         if (!cross) break;
@@ -1749,7 +1745,7 @@ __global__ void __launch_bounds__(NT, E == BR ? 7 : 24) k_brick_eval(VArgs v, Br
             if (lane > r && lane <= D) {
                 for (int ax = 0; ax < 3; ++ax) {
                     bool c;
-                    window_axis(g0[ax], E, Lc[ax], r, lane, D, 0, wl[ax], we[ax], c);
+                    window_axis(g0[ax], E, Lc[ax], r, lane, D, wl[ax], we[ax], c);
                     cross |= c;
                 }
                 if (cross) size = we[0] * we[1] * we[2];
@@ -2610,8 +2606,9 @@ void stage_mesh(Ctx& c) {
     i64* rfirst = dalloc<i64>(rtiles + 1, s);       // first triangle of each tile, and their number
     int kt = c.kbegin("corner_values", (double)M * (108 + 8 + 4 + 4) + (double)nD * 8 * 4);
     {
+        // (no index here needs this bound; no tree of that size, 41 GB of nodes, has been meshed)
         if (nD >= (1ll << 28)) {
-            set_last_error("%lld finest nodes exceed the corner list's 2^28", (long long)nD);
+            set_last_error("a mesh from %lld finest nodes: 2^28 or more are not taken", (long long)nD);
             throw Error{PRGPU_ERR_LIMIT, {0}};
         }
         const i64 gfirst = (lo - 1) / 8, ng = nD / 8;

@@ -37,16 +37,13 @@ namespace prgpu {
 
 
 struct CgArgs {
-    int ndepth;
     int mode;               // prgpu_solve_mode
     float tol2;             // reference mode: float(tol)*float(tol)
     double rel2;            // relative mode: tol^2
     int max_iter;
     i64 M;
     const int* neigh;       // 27 x M
-    const int* gn;          // 27 x ngroups: first child of each neighbour of a sibling group's parent, or -1
-    const int* gnr;         // the same, GN_ROW per group
-    i64 ngroups;            // sibling groups (nodes 1..M-1, 8 per group)
+    const int* gnr;         // GN_ROW per sibling group: first child of each neighbour of its parent, or -1
     const float* b;
     float* x;
     float* r;
@@ -599,9 +596,7 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
     float* p = dalloc<float>(M, s);
     float* q = dalloc<float>(M, s);
     // sibling-group table for the matrix-vector products
-    const i64 ngroups = (M - 1) / 8;
     ensure_group_rows(c);
-    const int* gn = c.gn;
     // co-resident capacity
     int dev = c.device, sms = 0, per_sm = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -624,7 +619,6 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
     CK(cudaMemsetAsync(st, 0, (D + 1) * sizeof(PartState), s));
     CK(cudaMemsetAsync(err, 0, sizeof(int), s));
     CgArgs a;
-    a.ndepth = D + 1;
     a.mode = mode;
     const float tolf = (float)c.params.cg_tol;
     a.tol2 = tolf * tolf;
@@ -632,9 +626,7 @@ void stage_solve_depths(Ctx& c, int d0, int d1, int mode, const float* rhs) {
     a.max_iter = c.params.cg_max_iter;
     a.M = M;
     a.neigh = c.nodes.neigh;
-    a.gn = gn;
     a.gnr = c.gn_rows;
-    a.ngroups = ngroups;
     a.b = rhs ? rhs : c.divergence;
     a.x = c.x;
     a.r = r;
