@@ -226,6 +226,9 @@ const char* prgpu_last_error(void);
  *                             launch has -- an arrival that never comes -- and give up
  *                             after arg polls of about 32 ns, so a solve returns
  *                             PRGPU_ERR_TIMEOUT without hanging (arg >= 1);
+ *   PRGPU_HOOK_SORT_POLLS     the radix sort's tiles look at the tiles before them at most arg
+ *                             times in a row without news, then count their keys themselves
+ *                             (arg >= 0; the result is the same);
  *   PRGPU_HOOK_POOL_USED      *out = bytes the current device's memory pool has handed out
  *                             and not taken back (after a device synchronisation).
  * out may be NULL except for PRGPU_HOOK_POOL_USED. */
@@ -233,7 +236,8 @@ enum {
     PRGPU_HOOK_CLEAR = 0,
     PRGPU_HOOK_FAIL_ALLOC = 1,
     PRGPU_HOOK_BARRIER_WAIT = 2,
-    PRGPU_HOOK_POOL_USED = 3
+    PRGPU_HOOK_POOL_USED = 3,
+    PRGPU_HOOK_SORT_POLLS = 4
 };
 int prgpu_test_hook(int32_t what, int64_t arg, int64_t* out);
 

@@ -51,6 +51,10 @@ struct WaitLimits {
     int extra = 0;
 };
 WaitLimits wait_limits();   // current settings (host)
+// The radix sort's tiles look at the tiles before them at most so often in a row without news, then count their keys
+// themselves: the same result without the wait.  PRGPU_HOOK_SORT_POLLS sets the limit.
+constexpr int DEFAULT_SORT_POLLS = 1 << 20;
+int sort_poll_limit();
 #define CK_LAUNCH()                            \
     do {                                       \
         ++::prgpu::g_kernel_launches;          \

@@ -165,7 +165,7 @@ void exclusive_scan(const TI* in, TO* out, i64 n, TO* total_dev, cudaStream_t s)
 // (look-back) and writes its elements from shared memory in digit order, so that each digit's run is written
 // at once.  24 bytes move per element and pass, where a count, a scan and a scatter moved 32 and wrote
 // every element by itself.  Tiles are numbered as their blocks start, so a tile waits for running ones
-// only; a wait that runs out (RS_POLLS) ends in counting the missing tiles' keys instead.
+// only; a wait that runs out (sort_poll_limit) ends in counting the earlier tiles' keys instead.
 // Bound by the latency of a tile's phases (load, rank, look back, write) at two blocks per SM: three (80
 // registers, spilling) and tiles of 2,048 are slower, 0.47 and 0.48 ms on the second line.  Against three
 // launches a pass: 15 K keys of 20 bits 0.099 -> 0.040 ms, 9.2 M of 36 bits (corners of the 1M torus)
@@ -177,7 +177,6 @@ constexpr int RS_TILE = RS_BLOCK * RS_ITEMS;
 constexpr int RS_BINS = 256;
 static_assert(RS_BLOCK == RS_BINS, "a thread per digit value");
 constexpr int RS_PASSES = 8;
-constexpr int RS_POLLS = 1 << 20;
 constexpr int RS_LOOK = 16;              // tiles a look-back step reads at once
 constexpr size_t RS_SHARED = RS_TILE * (sizeof(u64) + sizeof(uint32_t));
 
@@ -220,14 +219,15 @@ static __global__ void __launch_bounds__(RS_BLOCK) k_rs_hist(const u64* __restri
         if (h[p][threadIdx.x]) atomicAdd(&counts->hist[p][threadIdx.x], h[p][threadIdx.x]);
 }
 
-// Elements of digit t in the tiles before 'tile'.  A tile's word is its tag << 32 | count: tag 2 pass + 1 with the
-// tile's own count, 2 pass + 2 with the count of all tiles up to it; words of earlier passes have lower tags.
-__device__ __forceinline__ unsigned rs_look_back(const u64* status, unsigned tag, int tile, const u64* __restrict__ kin,
-                                                 int shift, unsigned mask) {
+// Elements of digit t in the tiles before 'tile'; false after 'limit' polls in a row that found no further tile.  A
+// tile's word is its tag << 32 | count: tag 2 pass + 1 with the tile's own count, 2 pass + 2 with the count of all tiles
+// up to it; words of earlier passes have lower tags.
+__device__ __forceinline__ bool rs_look_back(const u64* status, unsigned tag, int tile, int limit, unsigned& before) {
     const unsigned t = threadIdx.x;
-    unsigned before = 0;
+    before = 0;
     int at = tile - 1, polls = 0;
     while (at >= 0) {
+        if (polls >= limit) return false;
         u64 w[RS_LOOK];
 #pragma unroll
         for (int j = 0; j < RS_LOOK; ++j)
@@ -247,19 +247,16 @@ __device__ __forceinline__ unsigned rs_look_back(const u64* status, unsigned tag
                 }
             }
         }
-        if (done) return before;
+        if (done) return true;
         at -= got;
-        if (got == 0 && ++polls >= RS_POLLS) {
-            for (i64 e = 0; e < (i64)(at + 1) * RS_TILE; ++e) before += ((unsigned)(kin[e] >> shift) & mask) == t;
-            return before;
-        }
+        polls = got ? 0 : polls + 1;
     }
-    return before;
+    return true;
 }
 
 // vin null: the index of each element (the first pass)
 static __global__ void __launch_bounds__(RS_BLOCK, 2) k_rs_pass(const u64* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                                i64 n, int pass, unsigned mask,
+                                                                i64 n, int pass, unsigned mask, int poll_limit,
                                                                 RsCounts* __restrict__ counts, u64* status,
                                                                 u64* __restrict__ kout, uint32_t* __restrict__ vout) {
     extern __shared__ u64 rs_shared[];
@@ -320,10 +317,20 @@ static __global__ void __launch_bounds__(RS_BLOCK, 2) k_rs_pass(const u64* __res
         }
     }
     const unsigned start = block_exclusive_sum<unsigned>(counts->hist[pass][t], sw, &all);
-    const unsigned before = rs_look_back(status, tag, tile, kin, shift, mask);
-    *(volatile u64*)mineword = ((u64)(tag + 1) << 32) | (before + total);
+    unsigned before;
+    const bool known = rs_look_back(status, tag, tile, poll_limit, before);
+    if (known) *(volatile u64*)mineword = ((u64)(tag + 1) << 32) | (before + total);
     gbase[t] = start + before - local;   // modulo 2^32
-    __syncthreads();
+    if (__syncthreads_or(!known)) {      // a wait ran out: the block counts the keys of the tiles before its own
+        gbase[t] = 0;
+        __syncthreads();
+        for (i64 e = t; e < first; e += RS_BLOCK) atomicAdd(&gbase[(unsigned)(kin[e] >> shift) & mask], 1u);
+        __syncthreads();
+        before = gbase[t];
+        if (!known) *(volatile u64*)mineword = ((u64)(tag + 1) << 32) | (before + total);
+        gbase[t] = start + before - local;
+        __syncthreads();
+    }
     const int m = (int)min(n - first, (i64)RS_TILE);
     for (int q = t; q < m; q += RS_BLOCK) {
         const u64 k = skey[q];
@@ -347,10 +354,11 @@ inline void radix_sort_pairs(u64*& keys, uint32_t*& vals, u64*& ktmp, uint32_t*&
     k_rs_hist<<<grid_for(n, RS_BLOCK * 8, 152 * 8), RS_BLOCK, 0, s>>>(keys, n, nbits, counts);
     CK_LAUNCH();
     CK(cudaFuncSetAttribute(k_rs_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SHARED));
+    const int limit = sort_poll_limit();
     for (int pass = 0; 8 * pass < nbits; ++pass) {
         const unsigned mask = nbits - 8 * pass < 8 ? (1u << (nbits - 8 * pass)) - 1u : 255u;
-        k_rs_pass<<<(unsigned)nb, RS_BLOCK, RS_SHARED, s>>>(keys, pass ? vals : nullptr, n, pass, mask, counts, work + head,
-                                                            ktmp, vtmp);
+        k_rs_pass<<<(unsigned)nb, RS_BLOCK, RS_SHARED, s>>>(keys, pass ? vals : nullptr, n, pass, mask, limit, counts,
+                                                            work + head, ktmp, vtmp);
         CK_LAUNCH();
         std::swap(keys, ktmp);
         std::swap(vals, vtmp);
