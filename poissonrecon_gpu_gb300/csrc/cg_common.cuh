@@ -47,10 +47,10 @@ __host__ __device__ constexpr int stencil_class(int j) {
 // cycles, so a butterfly of doubles in each warp of a block, five blocks an SM, costs microseconds per
 // reduction; a solve does two reductions an iteration.  Here the lanes' values are aligned to the
 // largest exponent as 58-bit integers (one REDUX), split in limbs of 24 bits that 32 lanes cannot
-// overflow, and added by three more REDUX.  What alignment drops is below 2^-58 of the largest value
-// per lane, at most 2^-53 of it in all: no more than one rounding of a double addition.  The sum is
-// then rounded once to a double.  Non-finite or tiny (exponent field below 64) values take the
-// butterfly.  Every lane gets the result.
+// overflow, and added by three more REDUX.  What alignment drops is below 2^-57 of the largest value's
+// power of two per lane, 2^-52 of it in all: two roundings of a double addition at most.  The sum is then
+// rounded once to a double.  Values that are not finite or whose sum may not be (exponent field from
+// 0x7fa), and tiny ones (below 64), take the butterfly.  Every lane gets the result.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum_butterfly(double v) {
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -74,7 +74,7 @@ __device__ __forceinline__ double warp_sum(double v) {
     const u64 b = (u64)__double_as_longlong(v);
     const int e = (int)(b >> 52) & 0x7ff;
     const int emax = __reduce_max_sync(0xffffffffu, e);
-    if (emax < 64 || emax == 0x7ff) {
+    if (emax < 64 || emax >= 0x7fa) {
         if (!__any_sync(0xffffffffu, v != 0.0)) return 0.0;
         return warp_sum_butterfly(v);
     }
@@ -95,7 +95,8 @@ struct FSum {
     }
     __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
-// the pairs' 24-bit mantissas aligned to the largest exponent with 33 bits below
+// the pairs' 24-bit mantissas aligned to the largest exponent with 33 bits below: below 2^-56 of the largest
+// float's power of two is dropped per float, 2^-50 of it in all 64
 __device__ __forceinline__ double warp_sum(const FSum& v) {
     const unsigned bh = __float_as_uint(v.h), bl = __float_as_uint(v.l);
     const int eh = (int)(bh >> 23) & 255, el = (int)(bl >> 23) & 255;
