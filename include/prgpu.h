@@ -229,6 +229,8 @@ const char* prgpu_last_error(void);
  *   PRGPU_HOOK_SORT_POLLS     the radix sort's tiles look at the tiles before them at most arg
  *                             times in a row without news, then count their keys themselves
  *                             (arg >= 0; the result is the same);
+ *   PRGPU_HOOK_FOREIGN_SPAN   the mesh stage fills the brick corners that another leaf owns in
+ *                             spans of arg corners (arg >= 1; the result is the same);
  *   PRGPU_HOOK_POOL_USED      *out = bytes the current device's memory pool has handed out
  *                             and not taken back (after a device synchronisation).
  * out may be NULL except for PRGPU_HOOK_POOL_USED. */
@@ -237,7 +239,8 @@ enum {
     PRGPU_HOOK_FAIL_ALLOC = 1,
     PRGPU_HOOK_BARRIER_WAIT = 2,
     PRGPU_HOOK_POOL_USED = 3,
-    PRGPU_HOOK_SORT_POLLS = 4
+    PRGPU_HOOK_SORT_POLLS = 4,
+    PRGPU_HOOK_FOREIGN_SPAN = 5
 };
 int prgpu_test_hook(int32_t what, int64_t arg, int64_t* out);
 

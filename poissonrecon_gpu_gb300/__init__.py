@@ -445,7 +445,7 @@ def kernel_launches() -> int:
     return int(_lib().prgpu_kernel_launches())
 
 
-HOOK_CLEAR, HOOK_FAIL_ALLOC, HOOK_BARRIER_WAIT, HOOK_POOL_USED, HOOK_SORT_POLLS = 0, 1, 2, 3, 4
+HOOK_CLEAR, HOOK_FAIL_ALLOC, HOOK_BARRIER_WAIT, HOOK_POOL_USED, HOOK_SORT_POLLS, HOOK_FOREIGN_SPAN = 0, 1, 2, 3, 4, 5
 
 
 def test_hook(what: int, arg: int = 0) -> int:

@@ -23,6 +23,8 @@ static std::atomic<long long> g_spin_limit(DEFAULT_SPIN_LIMIT);
 static std::atomic<int> g_wait_extra(0);
 static std::atomic<int> g_sort_polls(DEFAULT_SORT_POLLS);
 int sort_poll_limit() { return g_sort_polls.load(); }
+static std::atomic<long long> g_foreign_span(0);
+i64 foreign_span_hook() { return g_foreign_span.load(); }
 WaitLimits wait_limits() {
     WaitLimits w;
     w.spin_limit = g_spin_limit.load();
@@ -896,6 +898,7 @@ int prgpu_test_hook(int32_t what, int64_t arg, int64_t* out) {
         g_spin_limit = DEFAULT_SPIN_LIMIT;
         g_wait_extra = 0;
         g_sort_polls = DEFAULT_SORT_POLLS;
+        g_foreign_span = 0;
         return PRGPU_OK;
     case PRGPU_HOOK_FAIL_ALLOC:
         if (arg < 1) return PRGPU_ERR_ARG;
@@ -909,6 +912,10 @@ int prgpu_test_hook(int32_t what, int64_t arg, int64_t* out) {
     case PRGPU_HOOK_SORT_POLLS:
         if (arg < 0 || arg > DEFAULT_SORT_POLLS) return PRGPU_ERR_ARG;
         g_sort_polls = (int)arg;
+        return PRGPU_OK;
+    case PRGPU_HOOK_FOREIGN_SPAN:
+        if (arg < 1) return PRGPU_ERR_ARG;
+        g_foreign_span = arg;
         return PRGPU_OK;
     case PRGPU_HOOK_POOL_USED: {
         if (!out) return PRGPU_ERR_ARG;

@@ -55,6 +55,7 @@ WaitLimits wait_limits();   // current settings (host)
 // themselves: the same result without the wait.  PRGPU_HOOK_SORT_POLLS sets the limit.
 constexpr int DEFAULT_SORT_POLLS = 1 << 20;
 int sort_poll_limit();
+i64 foreign_span_hook();   // PRGPU_HOOK_FOREIGN_SPAN (0: off)
 #define CK_LAUNCH()                            \
     do {                                       \
         ++::prgpu::g_kernel_launches;          \

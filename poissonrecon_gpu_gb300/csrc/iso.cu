@@ -2276,8 +2276,9 @@ __global__ void __launch_bounds__(32 * FC_WARPS) k_group_corners(EvalArgs a, con
 // the launch that copies and evaluated by one of their own, one to a thread, instead of each holding up a warp of
 // copies: 27 M corners (4M displaced sphere) 2.36 -> 1.50 ms, 101 M 8.5 -> 5.3, 1.3 M (1M torus) 0.174 -> 0.150.
 // Below FF_LISTED lower-face corners of live bricks one launch that does both is the faster, the evaluation's chain of loads
-// being most of either: 0.44 M corners 0.065 against 0.085 ms.  The list takes the corners [at, at + FF_SPAN), count[3]
-// of them.
+// being most of either: 0.44 M corners 0.065 against 0.085 ms.  A launch with a list takes the corners [at, end), at most
+// FF_SPAN, whose numbers from 'at' on the list holds; count[3] of them.  (PRGPU_HOOK_FOREIGN_SPAN: lists for every size, of
+// shorter spans.)
 constexpr i64 FF_SPAN = 1ll << 31, FF_LISTED = 1ll << 21;
 // the owner brick's corner, evaluated by its own leaf
 __device__ __forceinline__ float foreign_value(const VArgs& v, const BrickIndex& bix, u64 src) {
@@ -2298,9 +2299,9 @@ __device__ __forceinline__ float foreign_value(const VArgs& v, const BrickIndex&
 }
 template <bool LIST>
 __global__ void k_foreign_fill(VArgs v, BrickIndex bix, LiveIndex lx, const unsigned char* __restrict__ culled,
-                               const int* __restrict__ live_pos, const ForeignCorner* __restrict__ foreign, i64 at, i64 cap,
+                               const int* __restrict__ live_pos, const ForeignCorner* __restrict__ foreign, i64 at, i64 end,
                                float* __restrict__ blat, unsigned* __restrict__ list, unsigned long long* __restrict__ count) {
-    const i64 n = min(min((i64)count[0], cap), at + FF_SPAN);
+    const i64 n = min((i64)count[0], end);
     for (i64 f0 = at + (i64)blockIdx.x * blockDim.x; f0 < n; f0 += (i64)gridDim.x * blockDim.x) {
         const i64 f = f0 + threadIdx.x;
         bool slow = false;
@@ -2890,20 +2891,22 @@ void stage_mesh(Ctx& c) {
             }
             c.kend(ks);
             const int kf = c.kbegin("foreign_fill", 0.0);
-            if (fcap < FF_LISTED) {
+            const i64 hook = foreign_span_hook();
+            if (fcap < FF_LISTED && !hook) {
                 k_foreign_fill<false><<<grid_for(fcap, 128, (i64)c.sms * 512), 128, 0, s>>>(va, bix, lx, culled, bp, foreign, 0,
                                                                                            fcap, lat_brick, nullptr, dcount);
                 CK_LAUNCH();
             } else {
-                unsigned* list = dalloc<unsigned>(std::min(fcap, FF_SPAN), s);
-                for (i64 at = 0; at < fcap; at += FF_SPAN) {
+                const i64 span = std::min(fcap, hook ? hook : FF_SPAN);
+                unsigned* list = dalloc<unsigned>(span, s);
+                for (i64 at = 0; at < fcap; at += span) {
                     if (at) CK(cudaMemsetAsync(dcount + 3, 0, sizeof(unsigned long long), s));
-                    const i64 span = std::min(fcap - at, FF_SPAN);
-                    k_foreign_fill<true><<<grid_for(span, 256, (i64)c.sms * 128), 256, 0, s>>>(
-                        va, bix, lx, culled, bp, foreign, at, fcap, lat_brick, list, dcount);
+                    const i64 end = std::min(fcap, at + span);
+                    k_foreign_fill<true><<<grid_for(end - at, 256, (i64)c.sms * 128), 256, 0, s>>>(
+                        va, bix, lx, culled, bp, foreign, at, end, lat_brick, list, dcount);
                     CK_LAUNCH();
-                    k_foreign_eval<<<grid_for(span, 64, (i64)c.sms * 256), 64, 0, s>>>(va, bix, lx, foreign, at, list, lat_brick,
-                                                                                       dcount);
+                    k_foreign_eval<<<grid_for(end - at, 64, (i64)c.sms * 256), 64, 0, s>>>(va, bix, lx, foreign, at, list,
+                                                                                           lat_brick, dcount);
                     CK_LAUNCH();
                 }
                 dfree(list, s);
