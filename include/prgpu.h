@@ -224,7 +224,7 @@ const char* prgpu_last_error(void);
  *                             the device were out of memory (arg >= 1);
  *   PRGPU_HOOK_BARRIER_WAIT   the solvers' grid barriers expect one block more than the
  *                             launch has -- an arrival that never comes -- and give up
- *                             after arg polls of about 32 ns, so a solve returns
+ *                             after arg polls of about 0.3 us, so a solve returns
  *                             PRGPU_ERR_TIMEOUT without hanging (arg >= 1);
  *   PRGPU_HOOK_SORT_POLLS     the radix sort's tiles look at the tiles before them at most arg
  *                             times in a row without news, then count their keys themselves

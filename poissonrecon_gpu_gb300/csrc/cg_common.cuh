@@ -1,6 +1,6 @@
 // Definitions shared by the plain (solve.cu) and the flexible (flexcg.cu)
-// persistent CG kernels: per-depth partition state and reduction barriers, the
-// per-depth stencil description, block sums and compensated partial sums.
+// persistent CG kernels: per-depth partition state, the per-depth stencil
+// description, compensated partial sums, and sums over warps and grids.
 #pragma once
 #include "common.cuh"
 
@@ -189,8 +189,7 @@ struct GridSumShared {
 
 // The sum in two calls, so that work that needs neither its result nor other blocks' data runs while
 // the partials travel.  grid_publish: v (per thread) summed over the block and published.  grid_collect:
-// every thread gets the partition's sums in out.  The block has a multiple of 32 threads and, with
-// partitions of more than GS_ALL blocks, NV = 1.
+// every thread gets the partition's sums in out.  The block has a multiple of 32 threads.
 template <int NV, class V>
 __device__ __forceinline__ void grid_publish(const GridSum& g, unsigned epoch, bool data, const V (&v)[NV],
                                              GridSumShared<NV>& sm) {

@@ -41,11 +41,13 @@ const char* last_error();
 // every kernel launch is followed by CK_LAUNCH(), which also counts it
 extern std::atomic<unsigned long long> g_kernel_launches;
 
-// Bounded waits of the persistent solver kernels: a barrier polls at most
-// spin_limit times (about 32-64 ns apart) and then records PRGPU_ERR_TIMEOUT.
+// Bounded waits of the persistent solver kernels: a grid sum polls a block's
+// value at most spin_limit times (a poll, an L2 read and a short sleep, takes 0.31 us
+// by solves whose wait ran out after 2^14 to 2^18 polls) and then records
+// PRGPU_ERR_TIMEOUT; blocks that wait for the block that gave up see the record.
 // PRGPU_HOOK_BARRIER_WAIT sets extra = 1 (an arrival that never comes) and a
 // small limit, so tests reach the timeout path without a real hang.
-constexpr long long DEFAULT_SPIN_LIMIT = 1ll << 24;   // about half a second
+constexpr long long DEFAULT_SPIN_LIMIT = 1ll << 24;   // about 5 seconds
 struct WaitLimits {
     long long spin_limit = DEFAULT_SPIN_LIMIT;
     int extra = 0;

@@ -2739,9 +2739,10 @@ void stage_mesh(Ctx& c) {
         va.roots = droots;
         va.batch_root_flag = bflag;
         const i64 nbricks = tot[0], nsuper = tot[2], nsrows = tot[3];
-        // Leaves of edge 2 (depth D - 1, the last roots) are not bounded but evaluated: the bound proves 1 to
-        // 9 % of them (4 M points at maxDepth 11, 1M torus) and, with its tables, costs 8 ns a brick where
-        // the evaluation takes 2.6.
+        // Leaves of edge 2 (depth D - 1, the last roots) are not bounded but evaluated: the bound proves at most
+        // 9 % of them (4 M points at maxDepth 11, 1M torus, an open plane; below 1 % of those of noisy spheres, a
+        // filled volume, outliers and random normals) and, with its tables, costs 8 ns a brick where the
+        // evaluation takes 2.6.
         const i64 nbound = layout.off[0][D - 1], nrows = layout.off[1][D - 1];
         const int nrbound = layout.first[D - 1];
         i64* dbpre = dpre;

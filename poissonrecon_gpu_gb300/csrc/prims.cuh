@@ -160,7 +160,8 @@ void exclusive_scan(const TI* in, TO* out, i64 n, TO* total_dev, cudaStream_t s)
 
 // ----------------------------- radix sort -----------------------------------
 // Stable LSD sort of (key, index) pairs, 8 bits a pass, one launch per pass behind one that counts the digits
-// of all passes.  A tile ranks its 4,096 keys warp by warp (a warp's 512 consecutive keys against counters of
+// of all passes (the scheme of Adinets and Merrill's Onesweep, 2022, with the look-back of Merrill and
+// Garland's single-pass scan, 2016).  A tile ranks its 4,096 keys warp by warp (a warp's 512 consecutive keys against counters of
 // its own, without a barrier), publishes its count per digit, adds the counts of the tiles before it
 // (look-back) and writes its elements from shared memory in digit order, so that each digit's run is written
 // at once.  24 bytes move per element and pass, where a count, a scan and a scatter moved 32 and wrote

@@ -17,7 +17,8 @@ __device__ __forceinline__ float finest_center(int off, int D) {
 // centre (main.cu:913-964), a product of one value per axis.  A sample meets the 27 nodes around its leaf,
 // so along an axis only three centres: nine values per sample, where evaluating them per (node, sample)
 // pair takes 81, each with the shifted polynomial's arithmetic.  Per sample: its normal (and a pad), then the
-// values of the centres one cell below, at and above its leaf along x, y and z (and three pads).
+// values of the centres one cell below, at and above its leaf along x, y and z (and three pads): 64 bytes a
+// sample for the stage, 1.9 GB for 30 M.
 constexpr int SW_STRIDE = 16;
 __global__ void k_sample_weights(NodeArrays nd, int D, CPoly f, const float* __restrict__ pts, const float* __restrict__ nrm,
                                  const int* __restrict__ point_node, i64 n, float4* __restrict__ out, int stable) {
