@@ -271,20 +271,24 @@ class Reconstructor:
         offsets[1:] = np.cumsum([len(c[0]) for c in clouds])
         dep = None if depths is None else np.ascontiguousarray(depths, dtype=np.int32)
         outs = (Mesh * max(len(clouds), 1))()
-        result = [None] * len(clouds)
+        result, raised = [None] * len(clouds), []
 
         def alloc(_, k, nv, nt, pv, pf):          # called on the library's host threads
             try:
                 v, f = np.empty((nv, 3), np.float32), np.empty((nt, 3), np.int32)
-            except MemoryError:
+                result[k] = v, f
+                pv[0], pf[0] = v.ctypes.data, f.ctypes.data
+                return 0
+            except BaseException as e:            # (an interrupt too, which ctypes would drop)
+                raised.append(e)
                 return 1
-            result[k] = v, f
-            pv[0], pf[0] = v.ctypes.data, f.ctypes.data
-            return 0
 
-        _check(_lib().prgpu_reconstruct_batch_into(self._h, xyz.ctypes.data, nrm.ctypes.data, offsets.ctypes.data,
-                                                   None if dep is None else dep.ctypes.data, len(clouds),
-                                                   MeshAlloc(alloc), None, outs), "prgpu_reconstruct_batch")
+        rc = _lib().prgpu_reconstruct_batch_into(self._h, xyz.ctypes.data, nrm.ctypes.data, offsets.ctypes.data,
+                                                 None if dep is None else dep.ctypes.data, len(clouds),
+                                                 MeshAlloc(alloc), None, outs)
+        if raised:
+            raise raised[0]
+        _check(rc, "prgpu_reconstruct_batch")
         return result
 
     # ---- arrays
